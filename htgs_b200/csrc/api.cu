@@ -68,6 +68,7 @@ struct FrameLayout {
     PrimBuffers prim;
     InstBuffers inst;
     uint2* tile_ranges;
+    uint32_t* tile_order;
     size_t bytes;
 };
 
@@ -86,6 +87,7 @@ FrameLayout carve_frame(void* blob, int n_primitives, int n_tiles, const SortPla
     L.prim.block_offsets = c.take<uint32_t>(prim_blocks + 1);
     L.prim.visible_list = c.take<uint32_t>(n);
     L.tile_ranges = c.take<uint2>(size_t(n_tiles));
+    L.tile_order = c.take<uint32_t>(size_t(n_tiles));
     const uint64_t cap = instance_capacity > 0xfffffff0ull ? 0xfffffff0ull : instance_capacity;
     L.inst.capacity = uint32_t(cap);
     L.inst.sort_blocks_cap = uint32_t((cap + kSortTile - 1) / kSortTile);
@@ -290,7 +292,7 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
     if (f.fast && !ctx->fast_deterministic) {
         if ((err = launch_bin_unordered(scene, geo, L.prim, L.inst.prims[plan.final_buffer], L.inst.capacity, L.tile_ranges, L.status, ctx->sm_count,
                                         stream, prof ? ev + 3 : nullptr, launches)) != cudaSuccess) return fail_cuda(err, "unordered binning");
-    } else if ((err = launch_emit_sort_ranges(view.mode, scene, geo, plan, L.prim, L.inst, L.tile_ranges, L.status, ctx->sm_count, stream,
+    } else if ((err = launch_emit_sort_ranges(view.mode, scene, geo, plan, L.prim, L.inst, L.tile_ranges, L.tile_order, L.status, ctx->sm_count, stream,
                                               prof ? ev + 3 : nullptr, launches)) != cudaSuccess) return fail_cuda(err, "binning");
     if (front_priority) {
         if ((err = cudaEventRecord(ctx->front_end, stream)) != cudaSuccess) return fail_cuda(err, "front event record");
@@ -302,7 +304,7 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
                                       stream)) != cudaSuccess) return fail_cuda(err, "max weights");
     } else if (f.fast) {
         if ((err = launch_blend_fast(view.mode, view.K, geo, L.prim, prims_sorted, L.tile_ranges, out.image, out.to_chw, L.status, stream)) != cudaSuccess) return fail_cuda(err, "fast blend");
-    } else if ((err = launch_blend(view.mode, view.K, false, geo, L.prim, prims_sorted, L.tile_ranges, out, TrainPixelBuffers{}, L.status, stream)) != cudaSuccess) return fail_cuda(err, "blend");
+    } else if ((err = launch_blend(view, false, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out, TrainPixelBuffers{}, L.status, stream)) != cudaSuccess) return fail_cuda(err, "blend");
     *launches += 1;
     if (prof) cudaEventRecord(ev[6], stream);
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
@@ -624,6 +626,16 @@ InstLayout carve_instance_blob(void* blob, const SortPlan& plan, uint64_t capaci
     return L;
 }
 
+struct TileLayout { uint2* ranges; uint32_t* order; size_t bytes; };
+TileLayout carve_tile_blob(void* blob, const FrameGeometry& geo) {
+    TileLayout L{};
+    Carver c(blob);
+    L.ranges = c.take<uint2>(size_t(geo.n_tiles));
+    L.order = c.take<uint32_t>(size_t(geo.n_tiles));
+    L.bytes = align_up(c.offset + 1);
+    return L;
+}
+
 struct PixelLayout { TrainPixelBuffers px; size_t bytes; };
 PixelLayout carve_pixel_blob(void* blob, int mode, int K, const FrameGeometry& geo) {
     PixelLayout L{};
@@ -650,7 +662,7 @@ int htgs_forward_blob_sizes(const HtgsScene* scene, const HtgsView* view, size_t
     if (rc != HTGS_OK) return rc;
     const FrameGeometry geo = make_geometry(view->mode, view->width, view->height);
     if (per_primitive_bytes) *per_primitive_bytes = carve_primitive_blob(nullptr, scene->n_primitives).bytes;
-    if (per_tile_bytes) *per_tile_bytes = align_up(sizeof(uint2) * size_t(geo.n_tiles) + 1);
+    if (per_tile_bytes) *per_tile_bytes = carve_tile_blob(nullptr, geo).bytes;
     if (per_pixel_bytes) *per_pixel_bytes = carve_pixel_blob(nullptr, view->mode, view->K, geo).bytes;
     return HTGS_OK;
 }
@@ -708,15 +720,15 @@ int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView
     const InstLayout I = carve_instance_blob(blobs->per_instance, plan, n_instances);
     const PixelLayout X = carve_pixel_blob(blobs->per_pixel, view->mode, view->K, geo);
     if (!blobs->per_primitive || blobs->per_primitive_bytes < P.bytes || !blobs->per_instance || blobs->per_instance_bytes < I.bytes ||
-        !blobs->per_pixel || blobs->per_pixel_bytes < X.bytes || !blobs->per_tile || blobs->per_tile_bytes < sizeof(uint2) * size_t(geo.n_tiles))
+        !blobs->per_pixel || blobs->per_pixel_bytes < X.bytes || !blobs->per_tile || blobs->per_tile_bytes < carve_tile_blob(nullptr, geo).bytes)
         return fail(HTGS_ERR_WORKSPACE_TOO_SMALL, "a forward blob is missing or too small");
-    uint2* tile_ranges = static_cast<uint2*>(blobs->per_tile);
+    const TileLayout T = carve_tile_blob(blobs->per_tile, geo);
     uint32_t launches = 0;
     cudaError_t err;
-    if ((err = launch_emit_sort_ranges(view->mode, *scene, geo, plan, P.prim, I.inst, tile_ranges, P.status, ctx->sm_count, stream, nullptr, &launches)) != cudaSuccess)
+    if ((err = launch_emit_sort_ranges(view->mode, *scene, geo, plan, P.prim, I.inst, T.ranges, T.order, P.status, ctx->sm_count, stream, nullptr, &launches)) != cudaSuccess)
         return fail_cuda(err, "binning");
     const BlendOutputs out{image, nullptr, nullptr, true, false, false};
-    if ((err = launch_blend(view->mode, view->K, true, geo, P.prim, I.inst.prims[plan.final_buffer], tile_ranges, out, X.px, P.status, stream)) != cudaSuccess)
+    if ((err = launch_blend(*view, true, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order, out, X.px, P.status, stream)) != cudaSuccess)
         return fail_cuda(err, "blend");
     if ((err = cudaMemcpyAsync(ctx->host_status, P.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
     if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(err, "synchronise");

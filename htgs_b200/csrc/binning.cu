@@ -441,11 +441,64 @@ template <typename KeyT> constexpr size_t scatter_smem_bytes(int bits = kMaxRadi
     return (size_t(kSortWarps + 3) * (size_t(1) << bits) + kSortTile) * sizeof(uint32_t) + size_t(kSortTile) * sizeof(KeyT);
 }
 
+// Tiles by the length of their lists, longest first, in half-octave classes: blocks start in this order, so that the long lists do
+// not end up as the tail of a launch.  Inside a class the order is that of the image up to a few thousand tiles, which keeps
+// tiles that share Gaussians together in time.  Run by one block of 1024 threads.
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderClasses = 64;
+__device__ __forceinline__ uint32_t order_class(uint2 range) {
+    const uint32_t n = range.y - range.x;
+    if (n < 2) return kOrderClasses - 1;
+    const uint32_t log2n = 31u - __clz(int(n));
+    return uint32_t(kOrderClasses - 1) - min(2u * log2n + ((n >> (log2n - 1)) & 1u) - 1u, uint32_t(kOrderClasses - 1));
+}
+__device__ __forceinline__ void order_tiles(const uint2* ranges, uint32_t* order, uint32_t n_tiles) {
+    __shared__ uint32_t start[kOrderClasses];
+    constexpr int kUnroll = 4;
+    if (threadIdx.x < kOrderClasses) start[threadIdx.x] = 0;
+    __syncthreads();
+    #pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        for (uint32_t base = 0; base < n_tiles; base += kOrderThreads * kUnroll) {
+            uint2 r[kUnroll];
+            #pragma unroll
+            for (int i = 0; i < kUnroll; ++i) {
+                const uint32_t t = base + i * kOrderThreads + threadIdx.x;
+                r[i] = t < n_tiles ? __ldcg(ranges + t) : make_uint2(0u, 0u);
+            }
+            #pragma unroll
+            for (int i = 0; i < kUnroll; ++i) {
+                const uint32_t t = base + i * kOrderThreads + threadIdx.x;
+                const bool valid = t < n_tiles;
+                const uint32_t c = order_class(r[i]);
+                // one shared-memory atomic per class and warp
+                const uint32_t same = __match_any_sync(0xffffffffu, valid ? c : 0xffffffffu);
+                const int leader = __ffs(same) - 1;
+                uint32_t at = 0;
+                if (valid && int(threadIdx.x & 31u) == leader) at = atomicAdd(&start[c], uint32_t(__popc(same)));
+                at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & lanemask_lt());
+                if (pass == 1 && valid) order[at] = t;
+            }
+        }
+        __syncthreads();
+        if (pass == 0) {
+            if (threadIdx.x < 32) {
+                const uint32_t a = start[2 * threadIdx.x], b = start[2 * threadIdx.x + 1];
+                const uint32_t inc = warp_inclusive_scan(a + b);
+                start[2 * threadIdx.x] = inc - a - b;
+                start[2 * threadIdx.x + 1] = inc - b;
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // Tile ranges from the sorted keys (rasterization/src/shared_kernels.cu:56-95); ranges were zeroed before.
 // A thread takes kRangeRun consecutive keys with one 16-byte load (plus the key in front of them), so the sorted keys
 // are read once, in full sectors, and a thread has all its loads in flight before its first comparison.
 template <typename KeyT>
-__global__ void __launch_bounds__(256) tile_ranges_kernel(const KeyT* __restrict__ keys, uint2* __restrict__ ranges, const FrameStatus* status, uint32_t capacity) {
+__global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* __restrict__ keys, uint2* __restrict__ ranges, uint32_t* __restrict__ order,
+                                                                    FrameStatus* status, uint32_t capacity, uint32_t n_tiles) {
     constexpr uint32_t kRangeRun = 16 / sizeof(KeyT);            // 8 / 4 / 2 keys per 16-byte load
     const uint32_t n = frame_instances(status, capacity);
     const uint32_t n_runs = (n + kRangeRun - 1) / kRangeRun;
@@ -472,25 +525,36 @@ __global__ void __launch_bounds__(256) tile_ranges_kernel(const KeyT* __restrict
             }
         }
     }
+    __shared__ bool is_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(&status->range_blocks_done, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (is_last) {
+        __threadfence();
+        order_tiles(ranges, order, n_tiles);
+    }
 }
 
 template <typename KeyT>
 cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst,
-                               uint2* tile_ranges, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
+                               uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
     cudaError_t err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream);
     if (err != cudaSuccess) return err;
     if (prim_blocks == 0 || inst.capacity == 0) {
-        if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); cudaEventRecord(ev[2], stream); }
-        return cudaSuccess;
+        if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); }
+        tile_ranges_kernel<KeyT><<<1, kOrderThreads, 0, stream>>>(static_cast<const KeyT*>(inst.keys[0]), tile_ranges, tile_order, status, 0u, uint32_t(geo.n_tiles));
+        if (ev) cudaEventRecord(ev[2], stream);
+        if (launches) *launches += 1;
+        return cudaGetLastError();
     }
     emit_instances_kernel<KeyT><<<prim_blocks, kPreprocessBlock, 0, stream>>>(
         prim.n_touched, prim.bounds, prim.eval, prim.block_sums, prim.block_offsets, static_cast<KeyT*>(inst.keys[0]), inst.prims[0], n,
         uint32_t(geo.grid_w), inst.capacity, status);
     if (ev) cudaEventRecord(ev[0], stream);
     if (launches) *launches += 1;
-    const uint32_t persistent = uint32_t(sm_count) * 4;
     static PerDeviceOnce configured;
     err = configured.run([] { return cudaFuncSetAttribute(radix_scatter_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(scatter_smem_bytes<KeyT>())); });
     if (err != cudaSuccess) return err;
@@ -518,7 +582,8 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
         }
     }
     if (ev) cudaEventRecord(ev[1], stream);
-    tile_ranges_kernel<KeyT><<<persistent, 256, 0, stream>>>(static_cast<const KeyT*>(inst.keys[cur]), tile_ranges, status, inst.capacity);
+    tile_ranges_kernel<KeyT><<<uint32_t(sm_count), kOrderThreads, 0, stream>>>(static_cast<const KeyT*>(inst.keys[cur]), tile_ranges, tile_order, status, inst.capacity,
+                                                                                uint32_t(geo.n_tiles));
     if (ev) cudaEventRecord(ev[2], stream);
     if (launches) *launches += 1;
     return cudaGetLastError();
@@ -536,13 +601,13 @@ cudaError_t launch_scan_only(const HtgsScene& scene, const PrimBuffers& prim, ui
 }
 
 cudaError_t launch_emit_sort_ranges(int mode, const HtgsScene& scene, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim,
-                                    const InstBuffers& inst, uint2* tile_ranges, FrameStatus* status, int sm_count, cudaStream_t stream,
+                                    const InstBuffers& inst, uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream,
                                     cudaEvent_t* stage_events, uint32_t* launches) {
     (void)mode;
     switch (plan.key_bytes) {
-        case 2: return emit_sort_ranges_t<uint16_t>(scene, geo, plan, prim, inst, tile_ranges, status, sm_count, stream, stage_events, launches);
-        case 4: return emit_sort_ranges_t<uint32_t>(scene, geo, plan, prim, inst, tile_ranges, status, sm_count, stream, stage_events, launches);
-        case 8: return emit_sort_ranges_t<uint64_t>(scene, geo, plan, prim, inst, tile_ranges, status, sm_count, stream, stage_events, launches);
+        case 2: return emit_sort_ranges_t<uint16_t>(scene, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
+        case 4: return emit_sort_ranges_t<uint32_t>(scene, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
+        case 8: return emit_sort_ranges_t<uint64_t>(scene, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
         default: return cudaErrorInvalidValue;
     }
 }

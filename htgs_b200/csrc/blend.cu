@@ -8,72 +8,106 @@
 // The per-fragment arithmetic (planes through the pixel ray, rho^2, G, alpha, depth of the point
 // of maximum contribution) and every threshold decision are kept operation for operation, and each
 // pixel still sees its tile's instances in list order, so results match the reference bit for bit.
-// How the work is organised is different:
+// How the work is organised is different.  A CTA is ONE warp and blends 8 x 4 pixels, half of a tile (an eighth of
+// GLOBAL_ORDERING's 16 x 16 tile, whose lists have to be the reference's; its pixels share no state).  Nothing is shared
+// between warps, so there is no block barrier, a short list frees its resources at once, and the warp runs this pipeline
+// over its tile's list:
 //
-//  1. Staging.  One thread per instance of a batch starts ONE 80-byte bulk asynchronous copy (TMA,
-//     cp.async.bulk) of the Gaussian's evaluation record into shared memory, completion tracked by an
-//     mbarrier, and publishes the Gaussian's conservative screen-space outline (5 floats).  Index and
-//     outline of the NEXT batch are prefetched into registers while the current batch is processed.
-//  2. Candidate masks (overlap the copies in flight).  Inside a warp, lane l takes Gaussian l of the
-//     batch and evaluates the 3-flop outline test at each of the warp's 32 pixels; one warp ballot per
-//     pixel transposes the result, so that afterwards lane p holds the bit mask of the Gaussians that
-//     can touch pixel p.  No divergence, no shared-memory queue.
-//  3. Exact pass.  After the mbarrier completes, every lane walks the set bits of its own mask, so
-//     (almost) every iteration of every lane is an accepted fragment: the expensive part (IEEE divide,
-//     expf, depth, K-buffer insertion) runs converged instead of once per Gaussian per warp.  Every mode
-//     evaluates two candidates per trip for instruction-level parallelism and commits them in list order.
-//  4. K-buffer.  Registers hold only (depth, slot) pairs; the payloads live in a shared-memory pool of
-//     K+1 slots per pixel, so an insertion moves 2 registers per level instead of 5-6.  The buffer
-//     references K slots, one is free: a new fragment is written to the free slot, the insertion
-//     chain carries (depth, slot) pairs exactly like the reference's swap chain carries whole
-//     fragments, and the slot that falls out of the chain becomes the free one.
+//  1. Filter.  Lane = instance: 32 instances at a time, the conservative outline of the Gaussian (an ellipse) is cut with the
+//     four pixel rows, which gives a 32-bit mask of the pixels it can touch.  Instances that touch none (half of a list:
+//     lists come from tile boxes) are dropped, the others wait in a queue, in list order.
+//  2. Window.  Records are staged in two halves of 16; each lane's 80-byte bulk asynchronous copy (TMA, cp.async.bulk)
+//     brings one, an mbarrier per half tracks them, and the next instances are filtered while they fly.  The masks of a
+//     half are transposed (16 x 32 bits, shuffles), so that lane = pixel holds the bits of its own candidates: the
+//     older half in the upper 16 bits of a word, the newer one below.
+//  3. Exact pass.  Every lane walks the bits of its own word from the top; almost every step of every lane is an accepted
+//     fragment.  A half is replaced when no lane has a bit of it left; lanes that are ahead work on the newer half
+//     meanwhile, so lanes wait for the pixel with the most fragments only over a tile, not over every batch of 64 (lanes busy
+//     per step: 0.92 instead of 0.83 at 1297 x 840, 3 M Gaussians).
+//  4. K-buffer (core_buffer.cuh).  The K nearest core fragments lie unsorted in shared memory, 12 bytes each; an insertion
+//     overwrites the one that falls out and costs the same for every K.  The colour of the entry that will fall out next is
+//     fetched from its record right after the insertion before, so that it has arrived when it is needed.
+//
+// Blocks start in the order of `tile_order`, long lists first: the last blocks of a launch are short ones.
+//
+// What bounds it: instruction issue (1.0e9 warp instructions at 3 M Gaussians, 1297 x 840, K = 16, 7.3 M instances; 65 % of the
+// issue slots), at the 22 warps per SM that the K-buffers leave (K = 32: 14).  Measured against the form with one CTA of 64 pixels,
+// candidate masks by ballots and the chain in registers: K = 16 at that size 1660 -> 1185 us, K = 32 at 4K with 8 M Gaussians
+// 46.6 -> 34.9 ms, training forward 1813 -> 1370 us, GLOBAL_ORDERING (1.5 M, 980 x 545) 351 -> 262 us.
+#include <algorithm>
+#include <type_traits>
+
+#include "core_buffer.cuh"
 #include "kernels.h"
 
 namespace htgs {
 
 namespace {
 
-// Pixels one CTA blends.  The binning tile of GLOBAL_ORDERING is 16x16 (its lists have to be the reference's), but its
-// blend walks a list with per-pixel early termination and no state shared between pixels, so each binning tile is blended
-// by split_x * split_y independent CTAs that read the same list: more and shorter-lived CTAs, a tighter outline test per
-// CTA, and a CTA stops as soon as ITS pixels are opaque.
-#ifndef HTGS_GO_BLEND_W
-#define HTGS_GO_BLEND_W 8
-#define HTGS_GO_BLEND_H 8
-#endif
-template <int MODE> struct TileShape {
-    static constexpr bool split = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
-    static constexpr int tw = split ? HTGS_GO_BLEND_W : ModeTraits<MODE>::tile_w, th = split ? HTGS_GO_BLEND_H : ModeTraits<MODE>::tile_h;
-    static constexpr int split_x = ModeTraits<MODE>::tile_w / tw, split_y = ModeTraits<MODE>::tile_h / th;
-    static constexpr int threads = tw * th;
-    static constexpr int warps = threads / 32;
-    static constexpr int rows_per_warp = 32 / tw;
-    static constexpr int batch = threads;            // instances staged per iteration (one per thread)
-    static constexpr int chunk = 64;                 // candidate masks are built and consumed 64 instances at a time
-    static constexpr int chunks = batch / chunk;
+constexpr int kBlockW = 8, kBlockH = 4;          // pixels of a warp
+constexpr int kHalf = 16;                        // records per half of the window
+constexpr int kQueue = 64;                       // survivors of the filter that wait for a place: fewer than kHalf before a step of 32
+
+// The unsorted buffer from four entries on, where the depth range allows it (core_key_window); the chain otherwise.
+enum class Buffer { chain, keys, keys_and_colours };
+template <int K, Buffer BUFFER> struct CoreOf { using type = SortedCore<K, 32>; };
+template <int K> struct CoreOf<K, Buffer::keys> { using type = UnsortedCore<K, 32, false>; };
+template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = UnsortedCore<K, 32, true>; };
+struct NoCore { static constexpr bool keeps_colour = false; static constexpr size_t smem_bytes = 0; };
+
+template <int MODE, int K, Buffer BUFFER, bool TRAIN> struct SmemLayout {
+    static constexpr bool has_kbuffer = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
+    using Core = typename std::conditional<has_kbuffer, typename CoreOf<K, BUFFER>::type, NoCore>::type;
+    static constexpr size_t record_off = 0;
+    static constexpr size_t core_off = record_off + 2 * kHalf * sizeof(EvalRecord);
+    static constexpr size_t queue_prim_off = core_off + Core::smem_bytes;
+    static constexpr size_t queue_mask_off = queue_prim_off + kQueue * 4;
+    static constexpr size_t queue_pos_off = queue_mask_off + kQueue * 4;
+    static constexpr bool has_pos = has_kbuffer && TRAIN;
+    static constexpr size_t word_off = queue_pos_off + (has_pos ? kQueue * 4 : 0);       // what a K-buffer entry is filed under, per staged record
+    static constexpr size_t bar_off = word_off + (has_kbuffer ? 2 * kHalf * 4 : 0);
+    static constexpr size_t total = bar_off + 2 * 8;
 };
 
-template <int MODE, int K, bool TRAIN> struct SmemLayout {
-    using TS = TileShape<MODE>;
-    static constexpr bool has_kbuffer = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
-    static constexpr bool has_prim = (MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K) || (MODE == HTGS_MODE_HYBRID_BLEND && TRAIN);
-    static constexpr bool has_pool_idx = (MODE == HTGS_MODE_HYBRID_BLEND && TRAIN);
-    static constexpr int pool_elem = (MODE == HTGS_MODE_HYBRID_BLEND) ? 16 : (MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K ? 8 : 0);
-    static constexpr size_t eval_off = 0;
-    static constexpr size_t eval_bytes = size_t(TS::batch) * sizeof(EvalRecord);
-    static constexpr size_t cull4_off = eval_off + eval_bytes;
-    static constexpr size_t cull4_bytes = size_t(TS::batch) * 16;
-    static constexpr size_t cullc_off = cull4_off + cull4_bytes;
-    static constexpr size_t cullc_bytes = size_t(TS::batch) * 4;
-    static constexpr size_t prim_off = cullc_off + cullc_bytes;
-    static constexpr size_t prim_bytes = has_prim ? size_t(TS::batch) * 4 : 0;
-    static constexpr size_t bar_off = (prim_off + prim_bytes + 15) & ~size_t(15);
-    static constexpr size_t pool_off = bar_off + 16;
-    static constexpr size_t pool_bytes = has_kbuffer ? size_t(K + 1) * TS::threads * pool_elem : 0;
-    static constexpr size_t pool_idx_off = pool_off + pool_bytes;
-    static constexpr size_t pool_idx_bytes = has_pool_idx ? size_t(K + 1) * TS::threads * 4 : 0;
-    static constexpr size_t total = pool_idx_off + pool_idx_bytes;
-};
+__device__ __forceinline__ float sqrt_approx(float x) { float y; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+
+// Pixels of the 8 x 4 block at (x0, y0) that the outline a dx^2 + b2 dx dy + c dy^2 <= 1 about (cx, cy) can touch: bit
+// (row * 8 + column).  A row is cut in an interval; 0.01 pixel is added at both ends, far more than the roundings here and
+// far less than the 0.3 pixel by which the outline was inflated.
+__device__ __forceinline__ uint32_t outline_mask(const float4& c0, float cc, float x0, float y0) {
+    if (c0.z == 0.0f) return c0.x > 1e30f ? 0u : 0xffffffffu;   // nothing can be accepted / no proper ellipse: every pixel is a candidate
+    const float a_rcp = __fdividef(1.0f, c0.z);
+    const float slope = -0.5f * c0.w * a_rcp;                   // centre of the interval per unit of dy
+    const float shrink = slope * slope - cc * a_rcp;            // half width^2 = 1/a + shrink * dy^2
+    const float left = c0.x - x0, dy0 = y0 - c0.y;
+    uint32_t mask = 0;
+    #pragma unroll
+    for (int r = 0; r < kBlockH; ++r) {
+        const float dy = dy0 + float(r);
+        const float half_sq = fmaf(shrink * dy, dy, a_rcp);
+        const float mid = fmaf(slope, dy, left);
+        const float half = half_sq >= 0.0f ? sqrt_approx(half_sq) + 0.01f : -16.0f;
+        const int lo = max(__float2int_ru(mid - half), 0), hi = min(__float2int_rd(mid + half), kBlockW - 1);
+        const uint32_t row = ((2u << (hi & 31)) - 1u) & ~((1u << (lo & 31)) - 1u);       // bits lo..hi
+        if (lo <= hi) mask |= row << (r * kBlockW);
+    }
+    return mask;
+}
+
+// Lane i < 16 holds the pixel mask of survivor i; the result has, in lane = pixel, bit 15 - i set if survivor i can touch it.
+__device__ __forceinline__ uint32_t transpose_masks(uint32_t mask, uint32_t lane) {
+    uint32_t x = __shfl_sync(0xffffffffu, mask, 15u - (lane & 15u)) >> (lane & 16u);     // row 15 - i of a 16 x 16 block per half warp
+    #pragma unroll
+    for (int d = 8; d > 0; d >>= 1) {
+        const uint32_t low = d == 8 ? 0x00ffu : d == 4 ? 0x0f0fu : d == 2 ? 0x3333u : 0x5555u;
+        const bool up = lane & uint32_t(d);
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, d);
+        const uint32_t t = __funnelshift_l(y, y, up ? 32u - d : d);
+        const uint32_t keep = up ? ~low : low;
+        x = (x & keep) | (t & ~keep);
+    }
+    return x & 0xffffu;
+}
 
 // The shared per-fragment front end (hybrid_blend/kernels/inference.cuh:137-148).
 struct FragmentFront {
@@ -93,251 +127,193 @@ __device__ __forceinline__ FragmentFront fragment_front(const float4& VPMT1, con
     return f;
 }
 
-// The reference's insertion chain (hybrid_blend/kernels/inference.cuh:159-167) on (depth, slot) pairs:
-//     for k: if (carried.depth < kd[k]) swap(carried, entry[k]);
-// Because kd is sorted, the DEPTH carried into level k is always max(depth, kd[k-1]) - with or without ties -
-// so every level's comparison and new depth are computed from the old buffer in parallel; only the carried
-// slot is still passed from level to level (one select per level on the critical path instead of a compare
-// and a select).  Results, including the reference's behaviour for equal depths, are bit-identical to the chain.
-// On return `depth` is the depth of the entry that fell out of the buffer and the result its slot.
-// Slot numbers travel as floats (0..K are exact): the two selects per level that pass the slots along the chain become
-// one add and two multiply-adds on the FMA pipes, which are mostly idle in this kernel, instead of two instructions on
-// the ALU pipe that bounds it.  The comparison is materialised as 1.0f / 0.0f by a single `set` instruction.
-using slot_t = float;
-__device__ __forceinline__ uint32_t slot_index(slot_t s) { return uint32_t(__float2int_rz(s)); }
-__device__ __forceinline__ float less_than_as_float(float a, float b) {
-    float r;
-    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
-template <int K>
-__device__ __forceinline__ slot_t kbuffer_insert(float (&kd)[K], slot_t (&ks)[K], float& depth, slot_t slot) {
-    float p[K];
-    float nd[K];
-    #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const float carried = k == 0 ? depth : fmaxf(depth, kd[k - 1]);
-        p[k] = less_than_as_float(carried, kd[k]);
-        nd[k] = fminf(carried, kd[k]);   // = carried where carried < kd[k], else kd[k]
-    }
-    const float out_depth = fmaxf(depth, kd[K - 1]);
-    #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const slot_t mine = ks[k];
-        const float t = slot - mine;
-        ks[k] = fmaf(t, p[k], mine);      // p ? slot : mine
-        slot = fmaf(-t, p[k], slot);      // p ? mine : slot
-        kd[k] = nd[k];
-    }
-    depth = out_depth;
-    return slot;
-}
-
-template <int MODE, int K, bool TRAIN, bool STATS>
-__global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
-    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
+template <int MODE, int K, Buffer BUFFER, bool TRAIN, bool STATS>
+__global__ void __launch_bounds__(32) blend_kernel(
+    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, float* __restrict__ image, float* __restrict__ depth_out, float* __restrict__ alpha_out,
-    TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw, bool use_median_depth, FrameStatus* status)
+    TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw, bool use_median_depth, int32_t key_base, FrameStatus* status)
 {
     using MT = ModeTraits<MODE>;
-    using TS = TileShape<MODE>;
-    using SL = SmemLayout<MODE, K, TRAIN>;
+    using SL = SmemLayout<MODE, K, BUFFER, TRAIN>;
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
+    constexpr uint32_t kTileX = MT::tile_w / kBlockW, kTileY = MT::tile_h / kBlockH;     // blocks per binning tile
     extern __shared__ __align__(128) unsigned char smem[];
-    EvalRecord* s_eval = reinterpret_cast<EvalRecord*>(smem + SL::eval_off);
-    float4* s_cull4 = reinterpret_cast<float4*>(smem + SL::cull4_off);
-    float* s_cullc = reinterpret_cast<float*>(smem + SL::cullc_off);
-    [[maybe_unused]] uint32_t* s_prim = reinterpret_cast<uint32_t*>(smem + SL::prim_off);
+    EvalRecord* s_record = reinterpret_cast<EvalRecord*>(smem + SL::record_off);
+    uint32_t* s_queue_prim = reinterpret_cast<uint32_t*>(smem + SL::queue_prim_off);
+    uint32_t* s_queue_mask = reinterpret_cast<uint32_t*>(smem + SL::queue_mask_off);
+    [[maybe_unused]] uint32_t* s_queue_pos = reinterpret_cast<uint32_t*>(smem + SL::queue_pos_off);
+    [[maybe_unused]] uint32_t* s_word = reinterpret_cast<uint32_t*>(smem + SL::word_off);
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + SL::bar_off);
 
-    const uint32_t tid = threadIdx.x;
-    const uint32_t warp = tid >> 5, lane = tid & 31;
-    const uint32_t tile_x = blockIdx.x, tile_y = blockIdx.y;
-    const uint32_t px_i = tile_x * TS::tw + (tid % TS::tw);
-    const uint32_t py_i = tile_y * TS::th + (tid / TS::tw);
+    const uint32_t lane = threadIdx.x;
+    const uint32_t tile = __ldg(tile_order + blockIdx.x / (kTileX * kTileY)), part = blockIdx.x % (kTileX * kTileY);
+    const uint32_t block_x = (tile % grid_w) * kTileX + part % kTileX, block_y = (tile / grid_w) * kTileY + part / kTileX;
+    if (block_x * kBlockW >= width || block_y * kBlockH >= height) return;       // a ragged edge leaves blocks without pixels
+    const uint32_t px_i = block_x * kBlockW + (lane & 7u);
+    const uint32_t py_i = block_y * kBlockH + (lane >> 3);
     const bool inside = px_i < width && py_i < height;
     const float pixel_x = __uint2float_rn(px_i);
     const float pixel_y = __uint2float_rn(py_i);
+    const float block_x0 = float(block_x * kBlockW), block_y0 = float(block_y * kBlockH);
 
-    if (tid == 0) { mbar_init(s_bar, TS::threads); mbar_fence_init(); }
+    if (lane < 2) mbar_init(s_bar + lane, 1);
+    mbar_fence_init();
 
     // ---- per-pixel state -------------------------------------------------------------------
-    [[maybe_unused]] float kd[SL::has_kbuffer ? K : 1];
-    [[maybe_unused]] slot_t ks[SL::has_kbuffer ? K : 1];
-    [[maybe_unused]] float4* pool4 = reinterpret_cast<float4*>(smem + SL::pool_off);
-    [[maybe_unused]] float2* pool2 = reinterpret_cast<float2*>(smem + SL::pool_off);
-    [[maybe_unused]] uint32_t* pool_idx = reinterpret_cast<uint32_t*>(smem + SL::pool_idx_off);
-    [[maybe_unused]] uint32_t free_slot = K;   // index of the pool slot no buffer entry refers to
-    if constexpr (SL::has_kbuffer) {
-        #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            kd[k] = FLT_MAX; ks[k] = slot_t(k);
-            if constexpr (kHybrid) pool4[k * TS::threads + tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            else pool2[k * TS::threads + tid] = make_float2(0.0f, __uint_as_float(0xffffffffu));
-            if constexpr (SL::has_pool_idx) pool_idx[k * TS::threads + tid] = 0xffffffffu;
-        }
-    }
+    [[maybe_unused]] typename SL::Core core;
+    // what is known of the entry that falls out of the buffer next: payload and colour, zero for an empty entry
+    [[maybe_unused]] uint2 last = make_uint2(0u, kNoEntry);
+    [[maybe_unused]] float3 last_rgb = make_float3(0.0f, 0.0f, 0.0f);
+    if constexpr (SL::has_kbuffer) core.init(smem + SL::core_off, lane, key_base);
     // HYBRID tail / OIT accumulators / GLOBAL_ORDERING running blend
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // HB: premultiplied tail rgba; OIT: alpha-weighted rgb,depth; GO: rgb, depth
     float acc_depth = 0.0f;                              // HB: depth * alpha of the tail; OIT: alpha sum
     float transmittance = 1.0f;                          // HB: tail; OIT / GO: pixel
     bool done = !inside;
 
-    const uint2 range = tile_ranges[(tile_y / TS::split_y) * grid_w + tile_x / TS::split_x];   // grid_w counts binning tiles
-    uint32_t phase = 0;
+    const uint2 range = tile_ranges[tile];
+    // colour of the Gaussian that a payload's word names: its index, or (training) its position in the tile's list
+    [[maybe_unused]] auto colour_of = [&](uint32_t word) -> float3 {
+        const uint32_t g = TRAIN ? __ldg(prims_sorted + range.x + word) : word;
+        const float4 second = ldg4(reinterpret_cast<const float*>(cull + g) + 4);
+        return make_float3(second.y, second.z, second.w);
+    };
     bool wait_failed = false;
     [[maybe_unused]] uint32_t stat_candidates = 0, stat_accepted = 0, stat_trips = 0, stat_trips_inserting = 0, stat_insertions = 0;
-    // pixel rectangle of this warp (tw x rows_per_warp pixels; lane = row * tw + column)
-    const float rect_x0 = float(tile_x * TS::tw);
-    const float rect_y0 = float(tile_y * TS::th + warp * TS::rows_per_warp);
 
-    // prefetch registers: Gaussian index and outline of the instance this thread stages next
-    uint32_t g_next = 0;
-    float4 c0_next = make_float4(__int_as_float(0x7f800000), 0.0f, 0.0f, 0.0f);   // "reject everything"
-    float cc_next = 0.0f;
-    if (range.x + tid < range.y) {
-        g_next = __ldg(prims_sorted + range.x + tid);
-        c0_next = ldg4(reinterpret_cast<const float*>(cull + g_next));
-        cc_next = __ldg(reinterpret_cast<const float*>(cull + g_next) + 4);
-    }
-    __syncthreads();
+    // ---- 1. filter: the 32 instances from `next` on; their outlines and the indices of the 32 behind them are on their way ----
+    uint32_t next = range.x + lane;                      // the instance this lane tests next
+    uint32_t g_here = 0, g_ahead = 0;
+    float4 outline = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float outline_c = 0.0f;
+    auto request_outline = [&](uint32_t g) {
+        outline = ldg4(reinterpret_cast<const float*>(cull + g));
+        outline_c = __ldg(reinterpret_cast<const float*>(cull + g) + 4);
+    };
+    if (next < range.y) { g_here = __ldg(prims_sorted + next); request_outline(g_here); }
+    if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
+    uint32_t queue_head = 0, queued = 0;
+    auto filter = [&]() {
+        uint32_t mask = 0;
+        if (next < range.y) mask = outline_mask(outline, outline_c, block_x0, block_y0);
+        const uint32_t survivors = __ballot_sync(0xffffffffu, mask != 0);
+        if (mask != 0) {
+            const uint32_t at = (queue_head + queued + __popc(survivors & lanemask_lt())) & uint32_t(kQueue - 1);
+            s_queue_prim[at] = g_here;
+            s_queue_mask[at] = mask;
+            if constexpr (SL::has_pos) s_queue_pos[at] = next - range.x;
+        }
+        queued += __popc(survivors);
+        next += 32;
+        g_here = g_ahead;
+        if (next < range.y) request_outline(g_here);
+        if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
+    };
+    while (queued < kHalf && next - lane < range.y) filter();
+    __syncwarp();
 
-    for (uint32_t batch_begin = range.x; batch_begin < range.y; batch_begin += TS::batch) {
-        if constexpr (kGlobal) {
-            if (__syncthreads_count(done) == TS::threads) break;
-        } else {
-            __syncthreads();
+    uint32_t window = 0;                                 // this pixel's candidates: bits 31..16 the older half, 15..0 the newer half
+    uint32_t phases = 0;                                 // parity of each half's barrier
+    for (uint32_t half = 0;; half ^= 1u) {
+        // ---- 2. replace the half that no lane needs any more ----------------------------------------------------------
+        const uint32_t count = min(queued, uint32_t(kHalf));
+        if (count != 0) {
+            uint32_t g = 0, mask = 0;
+            const uint32_t slot = half * kHalf + (uint32_t(kHalf) - 1u - (lane & uint32_t(kHalf - 1)));
+            if (lane < count) {
+                const uint32_t at = (queue_head + lane) & uint32_t(kQueue - 1);
+                g = s_queue_prim[at];
+                mask = s_queue_mask[at];
+                if constexpr (SL::has_kbuffer) s_word[slot] = TRAIN ? s_queue_pos[at] : g;
+            }
+            if (lane == 0) mbar_arrive_expect_tx(s_bar + half, count * uint32_t(sizeof(EvalRecord)));
+            __syncwarp();
+            if (lane < count) bulk_copy_g2s(s_record + slot, eval + g, uint32_t(sizeof(EvalRecord)), s_bar + half);
+            queue_head += count;
+            queued -= count;
+            const uint32_t mine = transpose_masks(mask, lane);
+            if (!done) window |= mine;
+            if constexpr (STATS) stat_candidates += __popc(done ? 0u : mine);
+            while (queued < kHalf && next - lane < range.y) filter();
+            if (!mbar_wait_bounded(s_bar + half, (phases >> half) & 1u)) wait_failed = true;
+            phases ^= 1u << half;
+            __syncwarp();
+        } else if (!__any_sync(0xffffffffu, window != 0)) {
+            break;
         }
-        // ---- 1. staging: one instance per thread, from the prefetch registers ------------------------
-        const bool valid_inst = batch_begin + tid < range.y;
-        s_cull4[tid] = c0_next;
-        s_cullc[tid] = cc_next;
-        if (valid_inst) {
-            mbar_arrive_expect_tx(s_bar, uint32_t(sizeof(EvalRecord)));
-            bulk_copy_g2s(s_eval + tid, eval + g_next, uint32_t(sizeof(EvalRecord)), s_bar);
-            if constexpr (SL::has_prim) s_prim[tid] = g_next;
-        } else {
-            mbar_arrive(s_bar);
-        }
-        const uint32_t inst_next = batch_begin + TS::batch + tid;
-        const bool valid_next = inst_next < range.y;
-        if (valid_next) g_next = __ldg(prims_sorted + inst_next);
-        __syncthreads();
-        bool copies_landed = false;
-        #pragma unroll 1
-        for (int chunk = 0; chunk < TS::chunks; ++chunk) {
-            // ---- 2. candidate masks: lane = Gaussian, one ballot per pixel of the warp --------------
-            uint64_t cand = 0;
-            {
-                #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const uint32_t j = chunk * TS::chunk + half * 32 + lane;
-                    const float4 c0 = s_cull4[j];
-                    const float cc = s_cullc[j];
-                    const float dx0 = rect_x0 - c0.x, dy0 = rect_y0 - c0.y;
-                    uint32_t mine = 0;
-                    #pragma unroll
-                    for (int r = 0; r < TS::rows_per_warp; ++r) {
-                        const float dy = dy0 + float(r);
-                        const float b2dy = c0.w * dy, cdy2 = cc * dy * dy;
-                        #pragma unroll
-                        for (int i = 0; i < TS::tw; ++i) {
-                            const float dx = dx0 + float(i);
-                            const float q = dx * (c0.z * dx + b2dy) + cdy2;
-                            const uint32_t touched = __ballot_sync(0xffffffffu, q <= 1.0f);
-                            if (int(lane) == r * TS::tw + i) mine = touched;
-                        }
-                    }
-                    cand |= uint64_t(mine) << (32 * half);
-                }
-                if (done) cand = 0;
-            }
-            if (chunk == 0) {   // the index prefetched before the barrier has arrived by now
-                if (valid_next) {
-                    c0_next = ldg4(reinterpret_cast<const float*>(cull + g_next));
-                    cc_next = __ldg(reinterpret_cast<const float*>(cull + g_next) + 4);
-                } else {
-                    c0_next = make_float4(__int_as_float(0x7f800000), 0.0f, 0.0f, 0.0f);
-                    cc_next = 0.0f;
-                }
-            }
-            // ---- 3. exact pass ------------------------------------------------------------------------
-            if (!copies_landed) {
-                if (!mbar_wait_bounded(s_bar, phase)) wait_failed = true;
-                phase ^= 1;
-                copies_landed = true;
-            }
-            const uint32_t n_cand = __popcll(cand);
-            if constexpr (STATS) stat_candidates += n_cand;
-            const uint32_t n_iter = __reduce_max_sync(0xffffffffu, n_cand);
-            const uint32_t chunk_base = chunk * TS::chunk;
-            auto pop_candidate = [&](bool& valid) -> uint32_t {
-                valid = cand != 0;
-                const uint32_t j = valid ? uint32_t(__ffsll((long long)cand) - 1) : 0u;
-                cand &= cand - 1;
-                return chunk_base + j;
-            };
+        // ---- 3. exact pass: until no lane has a candidate of the older half left ---------------------------------------
+        const uint32_t flip = half * kHalf;              // bit j of the window is record j ^ flip
+        auto pop_candidate = [&](bool& valid) -> uint32_t {
+            valid = window != 0;
+            const uint32_t j = uint32_t(31 - __clz(int(window | 1u)));
+            window &= ~(1u << j);
+            return j ^ flip;
+        };
+        while (__any_sync(0xffffffffu, window >= 0x10000u)) {
             if constexpr (kHybrid) {
                 // Two candidates per trip: their evaluations are independent instruction streams (the compiler
                 // interleaves them), which hides the latency of the divide / expf / dot chains; the buffer
                 // and tail updates then happen strictly in list order.
-                // Inference keeps premultiplied colours in the buffer (inference.cuh:158), the training forward
-                // keeps (rgb, alpha) and the Gaussian index (forward.cuh:159-171).
                 auto evaluate = [&](bool valid, uint32_t j, float& depth, float4& frag) -> bool {
-                    const float4* rec = reinterpret_cast<const float4*>(s_eval + j);
+                    const float4* rec = reinterpret_cast<const float4*>(s_record + j);
                     const FragmentFront fr = fragment_front(rec[0], rec[1], rec[2], pixel_x, pixel_y);
                     const float numerator_rho2 = fr.numerator_rho2;
                     const float denominator = fr.denominator;
                     const bool inside_cutoff = !(numerator_rho2 > MT::max_cutoff_sq * denominator);
-                    const float denominator_rcp = 1.0f / denominator;
+                    const float denominator_rcp = reciprocal_rn(denominator);
                     const float4 rgba_in = rec[4];
                     const float G = expf(-0.5f * numerator_rho2 * denominator_rcp);
                     const float alpha = fminf(rgba_in.w * G, kMaxFragmentAlpha);
                     const float3 eval_point_diag = cross(fr.d, fr.m) * denominator_rcp;
                     const float4 MT3 = rec[3];
                     depth = dot(f3(MT3), eval_point_diag) + MT3.w;
-                    if constexpr (TRAIN) frag = make_float4(rgba_in.x, rgba_in.y, rgba_in.z, alpha);
-                    else frag = make_float4(rgba_in.x * alpha, rgba_in.y * alpha, rgba_in.z * alpha, alpha);
+                    frag = make_float4(rgba_in.x, rgba_in.y, rgba_in.z, alpha);
                     return valid && inside_cutoff && !(alpha < MT::min_alpha);
                 };
                 auto commit = [&](float depth, float4 frag, uint32_t j) {
                     if constexpr (STATS) ++stat_accepted;
-                    if (depth < kd[K - 1] && frag.w >= MT::min_alpha_core) {
-                        pool4[free_slot * TS::threads + tid] = frag;
-                        if constexpr (TRAIN) pool_idx[free_slot * TS::threads + tid] = batch_begin - range.x + j;   // position in the tile's list: what the backward pass looks up
-                        free_slot = slot_index(kbuffer_insert<K>(kd, ks, depth, slot_t(free_slot)));   // the entry that fell out: a real fragment or an empty one
-                        frag = pool4[free_slot * TS::threads + tid];
+                    if (depth < core.limit() && frag.w >= MT::min_alpha_core) {
+                        const float limit = core.limit();
+                        const uint2 payload = make_uint2(__float_as_uint(frag.w), s_word[j]);   // training: what the backward pass looks up
+                        // what falls out is a fragment, or nothing (alpha 0; its colour does not matter)
+                        if constexpr (SL::Core::keeps_colour) {
+                            float3 rgb = f3(frag);
+                            core.replace(depth, payload, last, rgb);
+                            frag = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(last.x));
+                        } else {
+                            if (!core.replace(depth, payload, last, last_rgb)) last_rgb = colour_of(last.y);
+                            frag = make_float4(last_rgb.x, last_rgb.y, last_rgb.z, __uint_as_float(last.x));
+                            if (core.last(last)) last_rgb = colour_of(last.y);
+                        }
+                        depth = limit;
                     }
                     if constexpr (TRAIN) {
                         acc += make_float4(frag.x * frag.w, frag.y * frag.w, frag.z * frag.w, frag.w);
-                    } else {
-                        acc += frag;
+                    } else {       // premultiplied colours are rounded before they are summed (inference.cuh:158)
+                        acc += make_float4(__fmul_rn(frag.x, frag.w), __fmul_rn(frag.y, frag.w), __fmul_rn(frag.z, frag.w), frag.w);
                         if (!use_median_depth) acc_depth += depth * frag.w;
                     }
                     transmittance *= 1.0f - frag.w;
                 };
-                for (uint32_t it = 0; it < n_iter; it += 2) {
-                    bool v0, v1;
-                    const uint32_t j0 = pop_candidate(v0);
-                    const uint32_t j1 = pop_candidate(v1);
-                    float depth0, depth1;
-                    float4 frag0, frag1;
-                    const bool ok0 = evaluate(v0, j0, depth0, frag0);
-                    const bool ok1 = evaluate(v1, j1, depth1, frag1);
-                    if constexpr (STATS) {   // how often the insertion chain runs for the warp (the branch in commit is the warp vote)
-                        const bool in0 = ok0 && depth0 < kd[K - 1] && frag0.w >= MT::min_alpha_core;
-                        stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in0) ? 1 : 0; stat_insertions += in0 ? 1 : 0;
-                    }
-                    if (ok0) commit(depth0, frag0, j0);
-                    if constexpr (STATS) {
-                        const bool in1 = ok1 && depth1 < kd[K - 1] && frag1.w >= MT::min_alpha_core;
-                        stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in1) ? 1 : 0; stat_insertions += in1 ? 1 : 0;
-                    }
-                    if (ok1) commit(depth1, frag1, j1);
+                bool v0, v1;
+                const uint32_t j0 = pop_candidate(v0);
+                const uint32_t j1 = pop_candidate(v1);
+                float depth0, depth1;
+                float4 frag0, frag1;
+                const bool ok0 = evaluate(v0, j0, depth0, frag0);
+                const bool ok1 = evaluate(v1, j1, depth1, frag1);
+                if constexpr (STATS) {   // how often a lane of the warp inserts
+                    const bool in0 = ok0 && depth0 < core.limit() && frag0.w >= MT::min_alpha_core;
+                    stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in0) ? 1 : 0; stat_insertions += in0 ? 1 : 0;
                 }
+                if (ok0) commit(depth0, frag0, j0);
+                if constexpr (STATS) {
+                    const bool in1 = ok1 && depth1 < core.limit() && frag1.w >= MT::min_alpha_core;
+                    stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in1) ? 1 : 0; stat_insertions += in1 ? 1 : 0;
+                }
+                if (ok1) commit(depth1, frag1, j1);
             } else {
                 // The other three modes use the same two-candidates-per-trip shape: both evaluations (divide, expf, depth) are
                 // independent instruction streams; the state updates happen in list order.  A fragment counts iff it passes
@@ -346,12 +322,12 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
                 // alpha_blend_global_ordering/kernels/inference.cuh:139-160, oit_blend/kernels/inference.cuh:139-160).
                 constexpr bool kNeedsPointDepth = kFirstK || (!kGlobal && !TRAIN);
                 auto evaluate = [&](bool valid, uint32_t j, float& alpha, float& depth, float4& rgba_in) -> bool {
-                    const float4* rec = reinterpret_cast<const float4*>(s_eval + j);
+                    const float4* rec = reinterpret_cast<const float4*>(s_record + j);
                     const FragmentFront fr = fragment_front(rec[0], rec[1], rec[2], pixel_x, pixel_y);
                     const float numerator_rho2 = fr.numerator_rho2;
                     const float denominator = fr.denominator;
                     const bool inside_cutoff = !(numerator_rho2 > MT::max_cutoff_sq * denominator);
-                    const float denominator_rcp = 1.0f / denominator;
+                    const float denominator_rcp = reciprocal_rn(denominator);
                     rgba_in = rec[4];
                     const float G = expf(-0.5f * numerator_rho2 * denominator_rcp);
                     alpha = fminf(rgba_in.w * G, kMaxFragmentAlpha);
@@ -366,10 +342,10 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
                 };
                 auto commit = [&](uint32_t j, float alpha, float depth, const float4& rgba_in) {
                     if constexpr (kFirstK) {
-                        if (depth >= kd[K - 1]) return;
+                        if (depth >= core.limit()) return;
                         if constexpr (STATS) ++stat_accepted;
-                        pool2[free_slot * TS::threads + tid] = make_float2(alpha, __uint_as_float(TRAIN ? batch_begin - range.x + j : s_prim[j]));
-                        free_slot = slot_index(kbuffer_insert<K>(kd, ks, depth, slot_t(free_slot)));
+                        core.last(last);
+                        core.replace(depth, make_uint2(__float_as_uint(alpha), s_word[j]), last, last_rgb);   // what falls out is dropped
                     } else if constexpr (kGlobal) {
                         if (done) return;
                         if constexpr (STATS) ++stat_accepted;
@@ -380,7 +356,7 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
                             else acc.w += blending_weight * depth;
                         }
                         transmittance *= 1.0f - alpha;
-                        if (transmittance < kTransmittanceThreshold) done = true;
+                        if (transmittance < kTransmittanceThreshold) { done = true; window = 0; }
                     } else {   // OIT_BLEND
                         if constexpr (STATS) ++stat_accepted;
                         if constexpr (TRAIN) {
@@ -392,19 +368,19 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
                         transmittance *= 1.0f - alpha;
                     }
                 };
-                for (uint32_t it = 0; it < n_iter; it += 2) {
-                    bool v0, v1;
-                    const uint32_t j0 = pop_candidate(v0);
-                    const uint32_t j1 = pop_candidate(v1);
-                    float alpha0, alpha1, depth0, depth1;
-                    float4 rgba0, rgba1;
-                    const bool ok0 = evaluate(v0, j0, alpha0, depth0, rgba0);
-                    const bool ok1 = evaluate(v1, j1, alpha1, depth1, rgba1);
-                    if (ok0) commit(j0, alpha0, depth0, rgba0);
-                    if (ok1) commit(j1, alpha1, depth1, rgba1);
-                }
+                bool v0, v1;
+                const uint32_t j0 = pop_candidate(v0);
+                const uint32_t j1 = pop_candidate(v1);
+                float alpha0, alpha1, depth0, depth1;
+                float4 rgba0, rgba1;
+                const bool ok0 = evaluate(v0, j0, alpha0, depth0, rgba0);
+                const bool ok1 = evaluate(v1, j1, alpha1, depth1, rgba1);
+                if (ok0) commit(j0, alpha0, depth0, rgba0);
+                if (ok1) commit(j1, alpha1, depth1, rgba1);
             }
-        }   // chunk loop
+        }
+        if constexpr (kGlobal) { if (__all_sync(0xffffffffu, done)) break; }
+        window <<= 16;
     }
 
     if (wait_failed) atomicOr(&status->error, 1u);
@@ -418,13 +394,14 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
         }
     }
     if (!inside) return;
+    if constexpr (SL::has_kbuffer) core.finish();
 
     const uint32_t pixel_idx = width * py_i + px_i;
     const uint32_t n_pixels = width * height;
 
     if constexpr (TRAIN) {
         // ---- training forward: unclamped CHW image + what the backward pass needs per pixel ------------
-        const uint32_t slot_base = (tile_y * grid_w + tile_x) * TS::threads + tid;   // tile-major pixel slot
+        const uint32_t slot_base = tile * 64u + part * 32u + lane;   // tile-major pixel slot (modes with 8 x 8 tiles)
         const uint32_t PP = tout.padded_pixels;
         float3 rgb_pixel = make_float3(0.0f, 0.0f, 0.0f);
         if constexpr (kHybrid) {
@@ -432,11 +409,14 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
             float transmittance_core = 1.0f;
             #pragma unroll
             for (int k = 0; k < K; ++k) {
-                if (transmittance_core >= kTransmittanceThreshold) {
-                    const float4 rgba = pool4[slot_index(ks[k]) * TS::threads + tid];
-                    const float blending_weight = transmittance_core * rgba.w;
-                    rgb_pixel += blending_weight * f3(rgba);
-                    transmittance_core *= 1.0f - rgba.w;
+                float depth;
+                uint2 payload;
+                const bool stored = core.entry(k, depth, payload);
+                if (transmittance_core >= kTransmittanceThreshold && stored) {
+                    const float alpha = __uint_as_float(payload.x);
+                    const float blending_weight = transmittance_core * alpha;
+                    rgb_pixel += blending_weight * colour_of(payload.y);
+                    transmittance_core *= 1.0f - alpha;
                     if (transmittance_core < kTransmittanceThreshold) transmittance_core = 0.0f;
                 }
             }
@@ -455,11 +435,13 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
             transmittance_core = 1.0f;
             #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const uint32_t primitive_idx = pool_idx[slot_index(ks[k]) * TS::threads + tid];
-                const bool skip = primitive_idx == 0xffffffffu || transmittance_core < kTransmittanceThreshold;
-                tout.idx_core[k * PP + slot_base] = skip ? 0xffffffffu : primitive_idx;
+                float depth;
+                uint2 payload;
+                const bool skip = !core.entry(k, depth, payload) || transmittance_core < kTransmittanceThreshold;
+                tout.idx_core[k * PP + slot_base] = skip ? kNoEntry : payload.y;
                 if (!skip) {
-                    const float4 rgba = pool4[slot_index(ks[k]) * TS::threads + tid];
+                    const float3 rgb = colour_of(payload.y);
+                    const float4 rgba = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(payload.x));
                     const float blending_weight = transmittance_core * rgba.w;
                     rgb_pixel_new += blending_weight * f3(rgba);
                     const float one_minus_alpha = 1.0f - rgba.w;
@@ -477,21 +459,16 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
             // alpha_blend_first_k/kernels/forward.cuh:167-213
             float t = 1.0f;
             bool stop = false;
-            float3 rgbs_core[K];
             #pragma unroll
             for (int k = 0; k < K; ++k) {
-                rgbs_core[k] = make_float3(0.0f, 0.0f, 0.0f);
                 if (!stop && t >= kTransmittanceThreshold) {
-                    const float2 cell = pool2[slot_index(ks[k]) * TS::threads + tid];
-                    const uint32_t position = __float_as_uint(cell.y);       // in the tile's list (training stores positions)
-                    if (position == 0xffffffffu) stop = true;
+                    float depth;
+                    uint2 payload;
+                    if (!core.entry(k, depth, payload)) stop = true;
                     else {
-                        const float alpha = cell.x;
-                        const uint32_t primitive_idx = __ldg(prims_sorted + range.x + position);
-                        const float3 rgb = f3(ldg4(reinterpret_cast<const float*>(eval + primitive_idx) + 16));
-                        rgbs_core[k] = rgb;
+                        const float alpha = __uint_as_float(payload.x);
                         const float blending_weight = t * alpha;
-                        rgb_pixel += blending_weight * rgb;
+                        rgb_pixel += blending_weight * colour_of(payload.y);
                         t *= 1.0f - alpha;
                     }
                 }
@@ -500,13 +477,13 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
             t = 1.0f;
             #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const float2 cell = pool2[slot_index(ks[k]) * TS::threads + tid];
-                const uint32_t primitive_idx = __float_as_uint(cell.y);
-                const bool skip = primitive_idx == 0xffffffffu || t < kTransmittanceThreshold;
-                tout.idx_core[k * PP + slot_base] = skip ? 0xffffffffu : primitive_idx;
+                float depth;
+                uint2 payload;
+                const bool skip = !core.entry(k, depth, payload) || t < kTransmittanceThreshold;
+                tout.idx_core[k * PP + slot_base] = skip ? kNoEntry : payload.y;
                 if (!skip) {
-                    const float alpha = cell.x;
-                    const float3 rgb = rgbs_core[k];
+                    const float alpha = __uint_as_float(payload.x);
+                    const float3 rgb = colour_of(payload.y);
                     const float blending_weight = t * alpha;
                     rgb_pixel_new += blending_weight * rgb;
                     const float one_minus_alpha = 1.0f - alpha;
@@ -546,13 +523,16 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
         float transmittance_core = 1.0f;
         #pragma unroll
         for (int k = 0; k < K; ++k) {
-            if (transmittance_core >= kTransmittanceThreshold) {
-                const float4 rgba_premultiplied = pool4[slot_index(ks[k]) * TS::threads + tid];
-                rgb_pixel += transmittance_core * f3(rgba_premultiplied);
-                const float depth = kd[k];
-                if (use_median_depth) depth_pixel = (transmittance_core > 0.5f && depth < FLT_MAX) ? depth : depth_pixel;
-                else depth_pixel += transmittance_core * rgba_premultiplied.w * depth;
-                transmittance_core *= 1.0f - rgba_premultiplied.w;
+            float depth;
+            uint2 payload;
+            const bool stored = core.entry(k, depth, payload);
+            if (transmittance_core >= kTransmittanceThreshold && stored) {
+                const float alpha = __uint_as_float(payload.x);
+                const float3 rgb = colour_of(payload.y);
+                rgb_pixel += transmittance_core * make_float3(__fmul_rn(rgb.x, alpha), __fmul_rn(rgb.y, alpha), __fmul_rn(rgb.z, alpha));
+                if (use_median_depth) depth_pixel = transmittance_core > 0.5f ? depth : depth_pixel;
+                else depth_pixel += transmittance_core * alpha * depth;
+                transmittance_core *= 1.0f - alpha;
             }
         }
         float total_alpha = 1.0f - transmittance_core;
@@ -571,15 +551,13 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
         #pragma unroll
         for (int k = 0; k < K; ++k) {
             if (!stop && t >= kTransmittanceThreshold) {
-                const float2 cell = pool2[slot_index(ks[k]) * TS::threads + tid];
-                const uint32_t primitive_idx = __float_as_uint(cell.y);
-                if (primitive_idx == 0xffffffffu) { stop = true; }
+                float depth;
+                uint2 payload;
+                if (!core.entry(k, depth, payload)) { stop = true; }
                 else {
-                    const float alpha = cell.x;
+                    const float alpha = __uint_as_float(payload.x);
                     const float blending_weight = t * alpha;
-                    const float4 rgba = ldg4(reinterpret_cast<const float*>(eval + primitive_idx) + 16);
-                    rgb_pixel += blending_weight * f3(rgba);
-                    const float depth = kd[k];
+                    rgb_pixel += blending_weight * colour_of(payload.y);
                     if (use_median_depth) depth_pixel = (t > 0.5f) ? depth : depth_pixel;
                     else depth_pixel += blending_weight * depth;
                     t *= 1.0f - alpha;
@@ -620,40 +598,60 @@ __global__ void __launch_bounds__(TileShape<MODE>::threads) blend_kernel(
     }
 }
 
-template <int MODE, int K, bool TRAIN, bool STATS>
-cudaError_t launch_blend_t(const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
-                           const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
-    using SL = SmemLayout<MODE, K, TRAIN>;
-    auto kernel = blend_kernel<MODE, K, TRAIN, STATS>;
+template <int MODE, int K, Buffer BUFFER, bool TRAIN, bool STATS>
+cudaError_t launch_blend_t(const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
+                           const BlendOutputs& out, const TrainPixelBuffers& tout, int32_t key_base, FrameStatus* status, cudaStream_t stream) {
+    using SL = SmemLayout<MODE, K, BUFFER, TRAIN>;
+    auto kernel = blend_kernel<MODE, K, BUFFER, TRAIN, STATS>;
     static PerDeviceOnce configured;
-    const cudaError_t err = configured.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SL::total)); });
+    const cudaError_t err = configured.run([&] {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SL::total));
+        return e;
+    });
     if (err != cudaSuccess) return err;
-    using TS = TileShape<MODE>;
-    const dim3 grid((geo.width + TS::tw - 1) / TS::tw, (geo.height + TS::th - 1) / TS::th, 1);
-    kernel<<<grid, TS::threads, SL::total, stream>>>(tile_ranges, prims_sorted, prim.eval, prim.cull, out.image, out.depth, out.alpha, tout,
+    using MT = ModeTraits<MODE>;
+    const uint32_t grid = uint32_t(geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
+    kernel<<<grid, 32, SL::total, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, out.image, out.depth, out.alpha, tout,
                                                                   uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w), out.to_chw,
-                                                                  out.use_median_depth, status);
+                                                                  out.use_median_depth, key_base, status);
     return cudaGetLastError();
 }
 
-template <int MODE, int K>
-cudaError_t launch_mode_k(bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
-                          const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
-    if (train) return launch_blend_t<MODE, K, true, false>(geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-    return out.collect_stats ? launch_blend_t<MODE, K, false, true>(geo, prim, prims_sorted, tile_ranges, out, tout, status, stream)
-                             : launch_blend_t<MODE, K, false, false>(geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
+template <int MODE, int K, Buffer BUFFER>
+cudaError_t launch_mode_k(bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
+                          const BlendOutputs& out, const TrainPixelBuffers& tout, int32_t key_base, FrameStatus* status, cudaStream_t stream) {
+    if (train) return launch_blend_t<MODE, K, BUFFER, true, false>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, key_base, status, stream);
+    return out.collect_stats ? launch_blend_t<MODE, K, BUFFER, false, true>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, key_base, status, stream)
+                             : launch_blend_t<MODE, K, BUFFER, false, false>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, key_base, status, stream);
 }
 
 // K is rounded down to a power of two <= 32 (hybrid_blend/inference.cu:15-28)
 template <int MODE>
-cudaError_t launch_mode(bool train, int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
-                        const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
-    if (K >= 32) return launch_mode_k<MODE, 32>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-    if (K >= 16) return launch_mode_k<MODE, 16>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-    if (K >= 8) return launch_mode_k<MODE, 8>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-    if (K >= 4) return launch_mode_k<MODE, 4>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-    if (K >= 2) return launch_mode_k<MODE, 2>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-    return launch_mode_k<MODE, 1>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
+cudaError_t launch_mode(bool train, int K, float near_plane, float far_plane, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
+                        const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
+    const int k = effective_k(MODE, K);
+    const CoreKeyWindow window = core_key_window(k, near_plane, far_plane);
+    // A grid that is resident at once leaves shared memory unused, and its time is that of its longest list: there the buffer keeps
+    // the colours too (24 bytes an entry), so that an insertion does not wait for one (256 x 256, 16384 Gaussians: 232 -> 197 us;
+    // at 1297 x 840 it costs occupancy: 1181 -> 1333 us).
+    auto one_wave = [&](size_t smem) {
+        const int per_sm = int(std::min<size_t>(32, (227 * 1024) / (smem + 1024)));
+        return !train && !out.collect_stats && geo.n_tiles * 2 <= per_sm * sm_count_of_current_device();
+    };
+    switch (k) {
+#define HTGS_K(N) case N: \
+        if (window.covers && one_wave(SmemLayout<MODE, N, Buffer::keys_and_colours, false>::total)) \
+            return launch_blend_t<MODE, N, MODE == HTGS_MODE_HYBRID_BLEND ? Buffer::keys_and_colours : Buffer::keys, false, false>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, window.base, status, stream); \
+        return window.covers ? launch_mode_k<MODE, N, Buffer::keys>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, window.base, status, stream) \
+                                               : launch_mode_k<MODE, N, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
+        HTGS_K(32)
+        HTGS_K(16)
+        HTGS_K(8)
+        HTGS_K(4)
+#undef HTGS_K
+        case 2: return launch_mode_k<MODE, 2, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
+        default: return launch_mode_k<MODE, 1, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
+    }
 }
 
 }  // namespace
@@ -663,13 +661,13 @@ int effective_k(int mode, int K) {
     return K >= 32 ? 32 : K >= 16 ? 16 : K >= 8 ? 8 : K >= 4 ? 4 : K >= 2 ? 2 : 1;
 }
 
-cudaError_t launch_blend(int mode, int K, bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
-                         const uint2* tile_ranges, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
-    switch (mode) {
-        case HTGS_MODE_HYBRID_BLEND: return launch_mode<HTGS_MODE_HYBRID_BLEND>(train, K, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-        case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_mode<HTGS_MODE_ALPHA_BLEND_FIRST_K>(train, K, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-        case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: return launch_mode_k<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING, 1>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
-        case HTGS_MODE_OIT_BLEND: return launch_mode_k<HTGS_MODE_OIT_BLEND, 1>(train, geo, prim, prims_sorted, tile_ranges, out, tout, status, stream);
+cudaError_t launch_blend(const HtgsView& view, bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
+                         const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
+    switch (view.mode) {
+        case HTGS_MODE_HYBRID_BLEND: return launch_mode<HTGS_MODE_HYBRID_BLEND>(train, view.K, view.near_plane, view.far_plane, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, status, stream);
+        case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_mode<HTGS_MODE_ALPHA_BLEND_FIRST_K>(train, view.K, view.near_plane, view.far_plane, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, status, stream);
+        case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: return launch_mode_k<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING, 1, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
+        case HTGS_MODE_OIT_BLEND: return launch_mode_k<HTGS_MODE_OIT_BLEND, 1, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -68,6 +68,7 @@ struct FrameGeometry {
 FrameGeometry make_geometry(int mode, int width, int height);
 
 // preprocess.cu
+int sm_count_of_current_device();
 // `fast_records`: write FastRecord instead of EvalRecord (inference of the modes launch_blend_fast supports).
 cudaError_t launch_preprocess(int mode, bool train, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo,
                               const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream, bool fast_records = false);
@@ -75,9 +76,10 @@ cudaError_t launch_preprocess(int mode, bool train, const HtgsScene& scene, cons
 // binning.cu: scan of block sums, instance emission, stable radix sort, tile ranges.
 // Everything after the scan reads the instance count from `status` on the device.
 cudaError_t launch_scan_only(const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream);
+// `tile_order`: receives the tiles, long lists first (the blend kernels start them in this order).
 // `stage_events` (optional): events recorded after emission, after the sort and after the range kernel.
 cudaError_t launch_emit_sort_ranges(int mode, const HtgsScene& scene, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim,
-                                    const InstBuffers& inst, uint2* tile_ranges, FrameStatus* status, int sm_count, cudaStream_t stream,
+                                    const InstBuffers& inst, uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream,
                                     cudaEvent_t* stage_events = nullptr, uint32_t* launches = nullptr);
 
 // binning_unordered.cu: per-tile lists without sort keys (counting sort with atomics; the order inside a list is not
@@ -106,8 +108,8 @@ struct TrainPixelBuffers {
 };
 
 int effective_k(int mode, int K);
-cudaError_t launch_blend(int mode, int K, bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
-                         const uint2* tile_ranges, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream);
+cudaError_t launch_blend(const HtgsView& view, bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
+                         const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream);
 
 // blend_fast.cu: relaxed-precision inference (RGB only) for HYBRID_BLEND, ALPHA_BLEND_FIRST_K and OIT_BLEND.  `supports` tells
 // whether (mode, K) has a fast kernel; these kernels do not depend on the order of a tile's list.

@@ -302,26 +302,15 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
             // The fragment evaluation measures from the projected centre, the outline test from the centre of
             // the outline: the record carries the (small) difference, so that outline centre + difference
             // gives the projected centre to better than float32 resolution at the pixel's magnitude.
-            cr.cx_lo = float(centre[0] - double(cr.cx));
-            cr.cy_lo = float(centre[1] - double(cr.cy));
+            cr.r = float(centre[0] - double(cr.cx));
+            cr.g = float(centre[1] - double(cr.cy));
+        } else {
+            cr.r = rgb.x; cr.g = rgb.y; cr.b = rgb.z;
         }
         float4* cdst = reinterpret_cast<float4*>(out.cull + gi);
         cdst[0] = make_float4(cr.cx, cr.cy, cr.a, cr.b2);
-        cdst[1] = make_float4(cr.c, cr.cx_lo, cr.cy_lo, 0.0f);
+        cdst[1] = make_float4(cr.c, cr.r, cr.g, cr.b);
     }
-}
-
-int sm_count_of_current_device() {
-    static std::atomic<int> cached[64] = {};
-    int device = 0;
-    cudaGetDevice(&device);
-    if (device < 0 || device >= 64) return 148;
-    int n = cached[device].load(std::memory_order_relaxed);
-    if (!n) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
-        cached[device].store(n, std::memory_order_relaxed);
-    }
-    return n;
 }
 
 template <int MODE, bool TRAIN, bool FAST>
@@ -341,6 +330,19 @@ cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGe
 }
 
 }  // namespace
+
+int sm_count_of_current_device() {
+    static std::atomic<int> cached[64] = {};
+    int device = 0;
+    cudaGetDevice(&device);
+    if (device < 0 || device >= 64) return 148;
+    int n = cached[device].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
+        cached[device].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
 
 cudaError_t launch_preprocess(int mode, bool train, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo,
                               const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream, bool fast_records) {

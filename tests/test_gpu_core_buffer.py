@@ -1,0 +1,60 @@
+"""GPU: the K-buffer's two forms (unsorted keys, insertion chain) and the pixel blocks at ragged edges.
+
+The unsorted form serves depth ranges its keys cover, the chain everything else; a far plane of 3e38 selects the chain for a
+scene that both see in full, so the two renders have to agree bit for bit, ties in depth included.
+"""
+import numpy as np
+import pytest
+
+import harness
+from htgs_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def scene_with_ties(n, width, height, K, mode, seed=5):
+    scene = scenes.tiny_scene(n=n, size=max(width, height), seed=seed, mode=mode, K=K, sh_degree=1)
+    # every third Gaussian sits where its predecessor sits, with the same shape: equal depth at every pixel, other colour and opacity
+    for a in (scene.positions, scene.scales, scene.rotations):
+        a[2::3] = a[1::3][: len(a[2::3])]
+    view = scene.views[0]
+    view.width, view.height = width, height
+    return scene, view
+
+
+def render(scene, view, mode, K, near, far, median):
+    import torch
+    tb = harness.ours()
+    wide = scenes.make_view(view.M, view.width, view.height, 256.0, 256.0, view.width / 2.0, view.height / 2.0, near, far)
+    st = harness.settings_for(tb, scene, wide, mode, K)
+    image, depth = tb.rasterize(*harness.scene_tensors(scene), st, True, median)
+    torch.cuda.synchronize()
+    return image.cpu().numpy(), depth.cpu().numpy()
+
+
+@pytest.mark.parametrize("mode,K", [(0, 4), (0, 8), (0, 16), (0, 32), (1, 4), (1, 8), (1, 16), (1, 32)])
+@pytest.mark.parametrize("n,width,height", [(6000, 256, 256), (40, 7, 3), (900, 129, 61), (3000, 33, 250)])
+def test_unsorted_buffer_equals_the_chain(mode, K, n, width, height):
+    scene, view = scene_with_ties(n, width, height, K, mode)
+    for median in (False, True):
+        got = render(scene, view, mode, K, 0.2, 100.0, median)
+        want = render(scene, view, mode, K, 0.2, 3e38, median)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        assert got[0].max() > 0.0
+
+
+@pytest.mark.parametrize("mode,K", [(0, 8), (1, 16)])
+def test_training_forward_and_gradients_agree_between_the_two_forms(mode, K):
+    import torch
+    tb = harness.ours()
+    scene, view = scene_with_ties(3000, 131, 77, K, mode)
+    outs = []
+    for near, far in ((0.2, 100.0), (0.2, 3e38)):
+        wide = scenes.make_view(view.M, view.width, view.height, 256.0, 256.0, view.width / 2.0, view.height / 2.0, near, far)
+        tensors = [t.requires_grad_() for t in harness.scene_tensors(scene)]
+        image = tb.diff_rasterize(*tensors, torch.empty(0, device="cuda"), harness.settings_for(tb, scene, wide, mode, K), False)
+        image.square().sum().backward()
+        outs.append((image.detach(), [t.grad for t in tensors]))
+    assert torch.equal(outs[0][0], outs[1][0])
+    for a, b in zip(outs[0][1], outs[1][1]):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-5 * float(b.abs().max()))
