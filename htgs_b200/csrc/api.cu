@@ -272,7 +272,6 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
         ctx->events_created = true;
     }
     cudaEvent_t* ev = ctx->events;   // 0 start, 1 preprocess, 2 scan, 3 emit, 4 sort, 5 ranges, 6 blend
-    out.collect_stats = ctx->collect_stats;
     cudaStream_t const caller_stream = stream;
     const bool front_priority = ctx->front_priority;
     if (front_priority) {
@@ -281,9 +280,10 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
         if ((err = cudaStreamWaitEvent(ctx->front_stream, ctx->front_begin, 0)) != cudaSuccess) return fail_cuda(err, "front stream wait");
         stream = ctx->front_stream;
     }
+    const int outline_mode = f.max_weights ? max_weights_mode(view.mode, ctx->max_weights_tail_credit) : view.mode;
     if ((err = cudaMemsetAsync(L.status, 0, sizeof(FrameStatus), stream)) != cudaSuccess) return fail_cuda(err, "status reset");
     if (prof) cudaEventRecord(ev[0], stream);
-    if ((err = launch_preprocess(view.mode, false, scene, view, geo, L.prim, L.status, stream, f.fast)) != cudaSuccess) return fail_cuda(err, "preprocess");
+    if ((err = launch_preprocess(view.mode, false, scene, view, geo, L.prim, L.status, stream, outline_mode, f.fast)) != cudaSuccess) return fail_cuda(err, "preprocess");
     if (prof) cudaEventRecord(ev[1], stream);
     if ((err = launch_scan_only(scene, L.prim, L.inst.capacity, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
     if (prof) cudaEventRecord(ev[2], stream);
@@ -300,11 +300,11 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
         stream = caller_stream;
     }
     if (f.max_weights) {
-        if ((err = launch_max_weights(view.mode, view.K, geo, L.prim, prims_sorted, L.tile_ranges, f.max_weights, f.weight_threshold, ctx->max_weights_tail_credit,
+        if ((err = launch_max_weights(view, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, L.status, f.max_weights, f.weight_threshold, ctx->max_weights_tail_credit,
                                       stream)) != cudaSuccess) return fail_cuda(err, "max weights");
     } else if (f.fast) {
         if ((err = launch_blend_fast(view.mode, view.K, geo, L.prim, prims_sorted, L.tile_ranges, out.image, out.to_chw, L.status, stream)) != cudaSuccess) return fail_cuda(err, "fast blend");
-    } else if ((err = launch_blend(view, false, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out, TrainPixelBuffers{}, L.status, stream)) != cudaSuccess) return fail_cuda(err, "blend");
+    } else if ((err = launch_blend(view.mode, ctx->collect_stats ? BlendTask::image_with_statistics : BlendTask::image, view, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out, TrainPixelBuffers{}, L.status, stream)) != cudaSuccess) return fail_cuda(err, "blend");
     *launches += 1;
     if (prof) cudaEventRecord(ev[6], stream);
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
@@ -350,7 +350,7 @@ static int begin_frame(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
     f.geo = make_geometry(view->mode, view->width, view->height);
     f.fast = fast && !max_weights && blend_fast_supports(view->mode, view->K);   // other modes / K: the exact kernels serve the fast entry point
     f.plan = make_sort_plan(view->mode, f.geo.n_tiles);
-    f.out = BlendOutputs{image, depth, alpha, to_chw != 0, use_median_depth != 0, false};
+    f.out = BlendOutputs{image, depth, alpha, to_chw != 0, use_median_depth != 0, nullptr, 0.0f};
     f.workspace = workspace; f.workspace_bytes = workspace_bytes;
     f.max_weights = max_weights; f.weight_threshold = weight_threshold;
     if (workspace == nullptr) {
@@ -696,7 +696,7 @@ int htgs_forward_begin(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
     const FrameGeometry geo = make_geometry(view->mode, view->width, view->height);
     cudaError_t err;
     if ((err = cudaMemsetAsync(L.status, 0, sizeof(FrameStatus), stream)) != cudaSuccess) return fail_cuda(err, "status reset");
-    if ((err = launch_preprocess(view->mode, true, *scene, *view, geo, L.prim, L.status, stream)) != cudaSuccess) return fail_cuda(err, "preprocess");
+    if ((err = launch_preprocess(view->mode, true, *scene, *view, geo, L.prim, L.status, stream, view->mode)) != cudaSuccess) return fail_cuda(err, "preprocess");
     if ((err = launch_scan_only(*scene, L.prim, 0xfffffff0u, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
     if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(err, "synchronise");
@@ -727,8 +727,8 @@ int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView
     cudaError_t err;
     if ((err = launch_emit_sort_ranges(view->mode, *scene, geo, plan, P.prim, I.inst, T.ranges, T.order, P.status, ctx->sm_count, stream, nullptr, &launches)) != cudaSuccess)
         return fail_cuda(err, "binning");
-    const BlendOutputs out{image, nullptr, nullptr, true, false, false};
-    if ((err = launch_blend(*view, true, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order, out, X.px, P.status, stream)) != cudaSuccess)
+    const BlendOutputs out{image, nullptr, nullptr, true, false, nullptr, 0.0f};
+    if ((err = launch_blend(view->mode, BlendTask::training, *view, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order, out, X.px, P.status, stream)) != cudaSuccess)
         return fail_cuda(err, "blend");
     if ((err = cudaMemcpyAsync(ctx->host_status, P.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
     if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(err, "synchronise");

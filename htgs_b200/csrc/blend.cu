@@ -55,7 +55,7 @@ template <int K> struct CoreOf<K, Buffer::keys> { using type = UnsortedCore<K, 3
 template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = UnsortedCore<K, 32, true>; };
 struct NoCore { static constexpr bool keeps_colour = false; static constexpr size_t smem_bytes = 0; };
 
-template <int MODE, int K, Buffer BUFFER, bool TRAIN> struct SmemLayout {
+template <int MODE, int K, Buffer BUFFER, BlendTask TASK> struct SmemLayout {
     static constexpr bool has_kbuffer = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
     using Core = typename std::conditional<has_kbuffer, typename CoreOf<K, BUFFER>::type, NoCore>::type;
     static constexpr size_t record_off = 0;
@@ -63,9 +63,10 @@ template <int MODE, int K, Buffer BUFFER, bool TRAIN> struct SmemLayout {
     static constexpr size_t queue_prim_off = core_off + Core::smem_bytes;
     static constexpr size_t queue_mask_off = queue_prim_off + kQueue * 4;
     static constexpr size_t queue_pos_off = queue_mask_off + kQueue * 4;
-    static constexpr bool has_pos = has_kbuffer && TRAIN;
+    static constexpr bool has_pos = has_kbuffer && TASK == BlendTask::training;
+    static constexpr bool has_word = has_kbuffer || TASK == BlendTask::max_weights;
     static constexpr size_t word_off = queue_pos_off + (has_pos ? kQueue * 4 : 0);       // what a K-buffer entry is filed under, per staged record
-    static constexpr size_t bar_off = word_off + (has_kbuffer ? 2 * kHalf * 4 : 0);
+    static constexpr size_t bar_off = word_off + (has_word ? 2 * kHalf * 4 : 0);
     static constexpr size_t total = bar_off + 2 * 8;
 };
 
@@ -127,14 +128,16 @@ __device__ __forceinline__ FragmentFront fragment_front(const float4& VPMT1, con
     return f;
 }
 
-template <int MODE, int K, Buffer BUFFER, bool TRAIN, bool STATS>
+template <int MODE, int K, Buffer BUFFER, BlendTask TASK>
 __global__ void __launch_bounds__(32) blend_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, float* __restrict__ image, float* __restrict__ depth_out, float* __restrict__ alpha_out,
-    TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw, bool use_median_depth, int32_t key_base, FrameStatus* status)
+    unsigned int* __restrict__ max_weights, float weight_threshold, TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
+    bool use_median_depth, int32_t key_base, FrameStatus* status)
 {
     using MT = ModeTraits<MODE>;
-    using SL = SmemLayout<MODE, K, BUFFER, TRAIN>;
+    using SL = SmemLayout<MODE, K, BUFFER, TASK>;
+    constexpr bool TRAIN = TASK == BlendTask::training, STATS = TASK == BlendTask::image_with_statistics, WEIGHTS = TASK == BlendTask::max_weights;
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
@@ -226,7 +229,7 @@ __global__ void __launch_bounds__(32) blend_kernel(
                 const uint32_t at = (queue_head + lane) & uint32_t(kQueue - 1);
                 g = s_queue_prim[at];
                 mask = s_queue_mask[at];
-                if constexpr (SL::has_kbuffer) s_word[slot] = TRAIN ? s_queue_pos[at] : g;
+                if constexpr (SL::has_word) s_word[slot] = TRAIN ? s_queue_pos[at] : g;
             }
             if (lane == 0) mbar_arrive_expect_tx(s_bar + half, count * uint32_t(sizeof(EvalRecord)));
             __syncwarp();
@@ -350,6 +353,7 @@ __global__ void __launch_bounds__(32) blend_kernel(
                         if (done) return;
                         if constexpr (STATS) ++stat_accepted;
                         const float blending_weight = transmittance * alpha;
+                        if constexpr (WEIGHTS) { if (!(blending_weight < weight_threshold)) raise_weight(max_weights, s_word[j], blending_weight); }
                         acc.x += blending_weight * rgba_in.x; acc.y += blending_weight * rgba_in.y; acc.z += blending_weight * rgba_in.z;
                         if constexpr (!TRAIN) {
                             if (use_median_depth) acc.w = (transmittance > 0.5f) ? depth : acc.w;
@@ -399,7 +403,24 @@ __global__ void __launch_bounds__(32) blend_kernel(
     const uint32_t pixel_idx = width * py_i + px_i;
     const uint32_t n_pixels = width * height;
 
-    if constexpr (TRAIN) {
+    if constexpr (WEIGHTS) {
+        // ---- largest weights (alpha_blend_first_k/kernels/update_max_weights.cuh; GLOBAL_ORDERING raises them on the way) ----
+        if constexpr (kFirstK) {
+            float t = 1.0f;
+            #pragma unroll
+            for (int k = 0; k < K; ++k) {
+                float depth;
+                uint2 payload;
+                const bool stored = core.entry(k, depth, payload);
+                const float alpha = __uint_as_float(payload.x);
+                const float blending_weight = t * alpha;
+                t *= 1.0f - alpha;
+                if (t < kTransmittanceThreshold) t = 0.0f;
+                if (stored && !(blending_weight < weight_threshold)) raise_weight(max_weights, payload.y, blending_weight);
+            }
+        }
+        return;
+    } else if constexpr (TRAIN) {
         // ---- training forward: unclamped CHW image + what the backward pass needs per pixel ------------
         const uint32_t slot_base = tile * 64u + part * 32u + lane;   // tile-major pixel slot (modes with 8 x 8 tiles)
         const uint32_t PP = tout.padded_pixels;
@@ -598,59 +619,79 @@ __global__ void __launch_bounds__(32) blend_kernel(
     }
 }
 
-template <int MODE, int K, Buffer BUFFER, bool TRAIN, bool STATS>
-cudaError_t launch_blend_t(const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
-                           const BlendOutputs& out, const TrainPixelBuffers& tout, int32_t key_base, FrameStatus* status, cudaStream_t stream) {
-    using SL = SmemLayout<MODE, K, BUFFER, TRAIN>;
-    auto kernel = blend_kernel<MODE, K, BUFFER, TRAIN, STATS>;
-    static PerDeviceOnce configured;
-    const cudaError_t err = configured.run([&] {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SL::total));
-        return e;
-    });
-    if (err != cudaSuccess) return err;
+struct BlendLaunch {
+    FrameGeometry geo;
+    PrimBuffers prim;
+    const uint32_t* prims_sorted;
+    const uint2* tile_ranges;
+    const uint32_t* tile_order;
+    BlendOutputs out;
+    TrainPixelBuffers tout;
+    FrameStatus* status;
+    cudaStream_t stream;
+};
+
+template <int MODE, int K, Buffer BUFFER, BlendTask TASK>
+cudaError_t launch_task(const BlendLaunch& l, int32_t key_base) {
+    using SL = SmemLayout<MODE, K, BUFFER, TASK>;
     using MT = ModeTraits<MODE>;
-    const uint32_t grid = uint32_t(geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
-    kernel<<<grid, 32, SL::total, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, out.image, out.depth, out.alpha, tout,
-                                                                  uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w), out.to_chw,
-                                                                  out.use_median_depth, key_base, status);
+    auto kernel = blend_kernel<MODE, K, BUFFER, TASK>;
+    if constexpr (SL::total > 48 * 1024) {
+        static PerDeviceOnce configured;
+        const cudaError_t err = configured.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SL::total)); });
+        if (err != cudaSuccess) return err;
+    }
+    const uint32_t grid = uint32_t(l.geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
+    kernel<<<grid, 32, SL::total, l.stream>>>(l.tile_ranges, l.tile_order, l.prims_sorted, l.prim.eval, l.prim.cull, l.out.image, l.out.depth, l.out.alpha,
+                                              reinterpret_cast<unsigned int*>(l.out.max_weights), l.out.weight_threshold, l.tout, uint32_t(l.geo.width),
+                                              uint32_t(l.geo.height), uint32_t(l.geo.grid_w), l.out.to_chw, l.out.use_median_depth, key_base, l.status);
     return cudaGetLastError();
 }
 
 template <int MODE, int K, Buffer BUFFER>
-cudaError_t launch_mode_k(bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
-                          const BlendOutputs& out, const TrainPixelBuffers& tout, int32_t key_base, FrameStatus* status, cudaStream_t stream) {
-    if (train) return launch_blend_t<MODE, K, BUFFER, true, false>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, key_base, status, stream);
-    return out.collect_stats ? launch_blend_t<MODE, K, BUFFER, false, true>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, key_base, status, stream)
-                             : launch_blend_t<MODE, K, BUFFER, false, false>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, key_base, status, stream);
+cudaError_t launch_buffer(const BlendLaunch& l, BlendTask task, int32_t key_base) {
+    switch (task) {
+        case BlendTask::image: return launch_task<MODE, K, BUFFER, BlendTask::image>(l, key_base);
+        case BlendTask::image_with_statistics: return launch_task<MODE, K, BUFFER, BlendTask::image_with_statistics>(l, key_base);
+        case BlendTask::training: return launch_task<MODE, K, BUFFER, BlendTask::training>(l, key_base);
+        case BlendTask::max_weights:
+            if constexpr (MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K || MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING)
+                return launch_task<MODE, K, BUFFER, BlendTask::max_weights>(l, key_base);
+    }
+    return cudaErrorInvalidValue;
 }
 
-// K is rounded down to a power of two <= 32 (hybrid_blend/inference.cu:15-28)
+// K is rounded down to a power of two <= 32 (hybrid_blend/inference.cu:15-28).  Below four entries the chain is shorter than a row
+// update; it also serves depth ranges that the keys do not cover.
+template <int MODE, int K>
+cudaError_t launch_k(const BlendLaunch& l, BlendTask task, const HtgsView& view) {
+    if constexpr (K < 4) {
+        return launch_buffer<MODE, K, Buffer::chain>(l, task, 0);
+    } else {
+        const CoreKeyWindow window = core_key_window(K, view.near_plane, view.far_plane);
+        if (!window.covers) return launch_buffer<MODE, K, Buffer::chain>(l, task, 0);
+        // A grid that is resident at once leaves shared memory unused, and its time is that of its longest list: there the buffer
+        // keeps the colours too (24 bytes an entry), so that an insertion does not wait for one (256 x 256, 16384 Gaussians:
+        // 232 -> 197 us; at 1297 x 840 it costs occupancy: 1181 -> 1333 us).
+        if constexpr (MODE == HTGS_MODE_HYBRID_BLEND) {
+            constexpr size_t smem = SmemLayout<MODE, K, Buffer::keys_and_colours, BlendTask::image>::total;
+            constexpr int per_sm = int((227 * 1024) / (smem + 1024)) < 32 ? int((227 * 1024) / (smem + 1024)) : 32;
+            if (task == BlendTask::image && l.geo.n_tiles * 2 <= per_sm * sm_count_of_current_device())
+                return launch_task<MODE, K, Buffer::keys_and_colours, BlendTask::image>(l, window.base);
+        }
+        return launch_buffer<MODE, K, Buffer::keys>(l, task, window.base);
+    }
+}
+
 template <int MODE>
-cudaError_t launch_mode(bool train, int K, float near_plane, float far_plane, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
-                        const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
-    const int k = effective_k(MODE, K);
-    const CoreKeyWindow window = core_key_window(k, near_plane, far_plane);
-    // A grid that is resident at once leaves shared memory unused, and its time is that of its longest list: there the buffer keeps
-    // the colours too (24 bytes an entry), so that an insertion does not wait for one (256 x 256, 16384 Gaussians: 232 -> 197 us;
-    // at 1297 x 840 it costs occupancy: 1181 -> 1333 us).
-    auto one_wave = [&](size_t smem) {
-        const int per_sm = int(std::min<size_t>(32, (227 * 1024) / (smem + 1024)));
-        return !train && !out.collect_stats && geo.n_tiles * 2 <= per_sm * sm_count_of_current_device();
-    };
-    switch (k) {
-#define HTGS_K(N) case N: \
-        if (window.covers && one_wave(SmemLayout<MODE, N, Buffer::keys_and_colours, false>::total)) \
-            return launch_blend_t<MODE, N, MODE == HTGS_MODE_HYBRID_BLEND ? Buffer::keys_and_colours : Buffer::keys, false, false>(geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, window.base, status, stream); \
-        return window.covers ? launch_mode_k<MODE, N, Buffer::keys>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, window.base, status, stream) \
-                                               : launch_mode_k<MODE, N, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
-        HTGS_K(32)
-        HTGS_K(16)
-        HTGS_K(8)
-        HTGS_K(4)
-#undef HTGS_K
-        case 2: return launch_mode_k<MODE, 2, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
-        default: return launch_mode_k<MODE, 1, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
+cudaError_t launch_mode(const BlendLaunch& l, BlendTask task, const HtgsView& view) {
+    switch (effective_k(MODE, view.K)) {
+        case 32: return launch_k<MODE, 32>(l, task, view);
+        case 16: return launch_k<MODE, 16>(l, task, view);
+        case 8: return launch_k<MODE, 8>(l, task, view);
+        case 4: return launch_k<MODE, 4>(l, task, view);
+        case 2: return launch_k<MODE, 2>(l, task, view);
+        default: return launch_k<MODE, 1>(l, task, view);
     }
 }
 
@@ -661,13 +702,15 @@ int effective_k(int mode, int K) {
     return K >= 32 ? 32 : K >= 16 ? 16 : K >= 8 ? 8 : K >= 4 ? 4 : K >= 2 ? 2 : 1;
 }
 
-cudaError_t launch_blend(const HtgsView& view, bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
-                         const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream) {
-    switch (view.mode) {
-        case HTGS_MODE_HYBRID_BLEND: return launch_mode<HTGS_MODE_HYBRID_BLEND>(train, view.K, view.near_plane, view.far_plane, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, status, stream);
-        case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_mode<HTGS_MODE_ALPHA_BLEND_FIRST_K>(train, view.K, view.near_plane, view.far_plane, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, status, stream);
-        case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: return launch_mode_k<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING, 1, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
-        case HTGS_MODE_OIT_BLEND: return launch_mode_k<HTGS_MODE_OIT_BLEND, 1, Buffer::chain>(train, geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, 0, status, stream);
+cudaError_t launch_blend(int mode, BlendTask task, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
+                         const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status,
+                         cudaStream_t stream) {
+    const BlendLaunch l{geo, prim, prims_sorted, tile_ranges, tile_order, out, tout, status, stream};
+    switch (mode) {
+        case HTGS_MODE_HYBRID_BLEND: return launch_mode<HTGS_MODE_HYBRID_BLEND>(l, task, view);
+        case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_mode<HTGS_MODE_ALPHA_BLEND_FIRST_K>(l, task, view);
+        case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: return launch_buffer<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING, 1, Buffer::chain>(l, task, 0);
+        case HTGS_MODE_OIT_BLEND: return launch_buffer<HTGS_MODE_OIT_BLEND, 1, Buffer::chain>(l, task, 0);
         default: return cudaErrorInvalidValue;
     }
 }

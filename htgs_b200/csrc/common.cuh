@@ -162,6 +162,12 @@ __device__ __forceinline__ float reciprocal_rn(float x) {
 
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 
+// update_max_weights: the largest weight of a Gaussian, as the bits of a non-negative float
+__device__ __forceinline__ void raise_weight(unsigned int* max_weights, uint32_t primitive_idx, float weight) {
+    const unsigned int bits = __float_as_uint(weight);
+    if (max_weights[primitive_idx] < bits) atomicMax(&max_weights[primitive_idx], bits);
+}
+
 // ---------------------------------------------------------------------------
 // PTX wrappers: mbarrier + bulk asynchronous copy (TMA, non-tensor, single-CTA destination)
 // ---------------------------------------------------------------------------

@@ -69,9 +69,10 @@ FrameGeometry make_geometry(int mode, int width, int height);
 
 // preprocess.cu
 int sm_count_of_current_device();
+// `outline_mode`: whose thresholds the conservative outlines are for; the view's mode, or a stricter one if only its fragments count.
 // `fast_records`: write FastRecord instead of EvalRecord (inference of the modes launch_blend_fast supports).
 cudaError_t launch_preprocess(int mode, bool train, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo,
-                              const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream, bool fast_records = false);
+                              const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream, int outline_mode, bool fast_records = false);
 
 // binning.cu: scan of block sums, instance emission, stable radix sort, tile ranges.
 // Everything after the scan reads the instance count from `status` on the device.
@@ -96,8 +97,10 @@ struct BlendOutputs {
     float* alpha;     // may be null
     bool to_chw;
     bool use_median_depth;
-    bool collect_stats;
+    float* max_weights;       // BlendTask::max_weights
+    float weight_threshold;
 };
+enum class BlendTask { image, image_with_statistics, training, max_weights };
 // per-pixel buffers the training forward leaves for the backward pass; pixel slots are tile-major
 // (slot = tile * pixels_per_tile + pixel_in_tile) and every array is plane-major over `padded_pixels` slots
 struct TrainPixelBuffers {
@@ -108,7 +111,8 @@ struct TrainPixelBuffers {
 };
 
 int effective_k(int mode, int K);
-cudaError_t launch_blend(const HtgsView& view, bool train, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
+// `mode` is the view's, but for BlendTask::max_weights (weights.cu); max_weights exists for FIRST_K and GLOBAL_ORDERING.
+cudaError_t launch_blend(int mode, BlendTask task, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
                          const uint2* tile_ranges, const uint32_t* tile_order, const BlendOutputs& out, const TrainPixelBuffers& tout, FrameStatus* status, cudaStream_t stream);
 
 // blend_fast.cu: relaxed-precision inference (RGB only) for HYBRID_BLEND, ALPHA_BLEND_FIRST_K and OIT_BLEND.  `supports` tells
@@ -118,9 +122,10 @@ cudaError_t launch_blend_fast(int mode, int K, const FrameGeometry& geo, const P
                               float* image, bool to_chw, FrameStatus* status, cudaStream_t stream);
 
 // weights.cu
+int max_weights_mode(int mode, bool credit_tail);     // the mode whose rule decides which fragments count
 // `credit_tail` (HYBRID_BLEND only): also run the second walk that credits `alpha * tail weight` to every fragment.
-cudaError_t launch_max_weights(int mode, int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
-                               float* max_weights, float weight_threshold, bool credit_tail, cudaStream_t stream);
+cudaError_t launch_max_weights(const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
+                               const uint32_t* tile_order, FrameStatus* status, float* max_weights, float weight_threshold, bool credit_tail, cudaStream_t stream);
 
 // train.cu: backward pass
 struct GradAccumBuffers {

@@ -90,6 +90,12 @@ __device__ __forceinline__ float3 sh_to_rgb(const float* __restrict__ sh_0, cons
     return make_float3(fmaxf(0.0f, result.x), fmaxf(0.0f, result.y), fmaxf(0.0f, result.z));
 }
 
+struct OutlineThresholds { float max_cutoff_sq, min_alpha_rcp; };
+OutlineThresholds outline_thresholds(int mode) {
+    if (mode == HTGS_MODE_ALPHA_BLEND_FIRST_K) return {ModeTraits<HTGS_MODE_ALPHA_BLEND_FIRST_K>::max_cutoff_sq, ModeTraits<HTGS_MODE_ALPHA_BLEND_FIRST_K>::min_alpha_rcp};
+    return {ModeTraits<HTGS_MODE_HYBRID_BLEND>::max_cutoff_sq, ModeTraits<HTGS_MODE_HYBRID_BLEND>::min_alpha_rcp};      // the other three share them
+}
+
 // Conservative outline of { pixel : the exact per-fragment test can accept }.
 //
 // A fragment is accepted only if rho^2 <= max_cutoff_sq and opacity * exp(-rho^2 / 2) >= min_alpha, i.e.
@@ -100,11 +106,9 @@ __device__ __forceinline__ float3 sh_to_rgb(const float* __restrict__ sh_0, cons
 // the shape matrix is inflated by (0.3 px)^2 and the quadratic form relaxed by 2% to cover the float32
 // rounding of the exact per-fragment evaluation.  An outline that is not a proper ellipse disables culling
 // for the Gaussian ("accept everything"), and L <= 0 rejects everything.
-template <int MODE>
-__device__ __forceinline__ CullRecord make_cull_record(const float4& t1, const float4& t2, const float4& t4, float opacity) {
-    using MT = ModeTraits<MODE>;
+__device__ __forceinline__ CullRecord make_cull_record(const float4& t1, const float4& t2, const float4& t4, float opacity, const OutlineThresholds& thresholds) {
     CullRecord rec = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};   // a = b2 = c = 0: every pixel passes
-    const double level = fmin(double(MT::max_cutoff_sq), 2.0 * log(double(opacity) * double(MT::min_alpha_rcp))) * 1.001 + 1e-4;
+    const double level = fmin(double(thresholds.max_cutoff_sq), 2.0 * log(double(opacity) * double(thresholds.min_alpha_rcp))) * 1.001 + 1e-4;
     if (!(level > 0.0)) { rec.cx = __int_as_float(0x7f800000); return rec; }   // +inf: every comparison fails, nothing passes
     auto conic = [&](const float4& a, const float4& b) {
         return level * (double(a.x) * double(b.x) + double(a.y) * double(b.y) + double(a.z) * double(b.z)) - double(a.w) * double(b.w);
@@ -280,7 +284,7 @@ constexpr int kFinishBlock = 128;
 template <int MODE, bool TRAIN, bool FAST>
 __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
     const float* __restrict__ positions, const float* __restrict__ opacities, const float* __restrict__ sh_0, const float* __restrict__ sh_rest,
-    const float* __restrict__ cam_position_ptr, PrimBuffers out, const FrameStatus* __restrict__ status, int active_sh_bases, int total_sh_bases)
+    const float* __restrict__ cam_position_ptr, PrimBuffers out, const FrameStatus* __restrict__ status, int active_sh_bases, int total_sh_bases, OutlineThresholds thresholds)
 {
     const uint32_t n_visible = status->n_visible;
     const float3 cam_position = make_float3(__ldg(cam_position_ptr), __ldg(cam_position_ptr + 1), __ldg(cam_position_ptr + 2));
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
         if constexpr (FAST) make_fast_record(t1, t2, t4, m3, rgb, opacity, dst, centre);
         else dst[4] = make_float4(rgb.x, rgb.y, rgb.z, opacity);
         if constexpr (TRAIN) out.clamp[gi] = clamp_bits;
-        CullRecord cr = make_cull_record<MODE>(t1, t2, t4, opacity);
+        CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
         if constexpr (FAST) {
             // The fragment evaluation measures from the projected centre, the outline test from the centre of
             // the outline: the record carries the (small) difference, so that outline centre + difference
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
 }
 
 template <int MODE, bool TRAIN, bool FAST>
-cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream) {
+cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim, FrameStatus* status, int outline_mode, cudaStream_t stream) {
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
     if (blocks == 0) return cudaSuccess;
@@ -325,7 +329,7 @@ cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGe
     if (err != cudaSuccess) return err;
     const uint32_t finish_blocks = min((n + kFinishBlock - 1) / kFinishBlock, uint32_t(sm_count_of_current_device()) * 8u);
     preprocess_finish_kernel<MODE, TRAIN, FAST><<<finish_blocks, kFinishBlock, 0, stream>>>(
-        scene.positions, scene.opacities, scene.sh_0, scene.sh_rest, view.cam_position, prim, status, view.active_sh_bases, scene.total_sh_bases);
+        scene.positions, scene.opacities, scene.sh_0, scene.sh_rest, view.cam_position, prim, status, view.active_sh_bases, scene.total_sh_bases, outline_thresholds(outline_mode));
     return cudaGetLastError();
 }
 
@@ -345,18 +349,18 @@ int sm_count_of_current_device() {
 }
 
 cudaError_t launch_preprocess(int mode, bool train, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo,
-                              const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream, bool fast_records) {
+                              const PrimBuffers& prim, FrameStatus* status, cudaStream_t stream, int outline_mode, bool fast_records) {
     if (fast_records) {
         if (train) return cudaErrorInvalidValue;
         switch (mode) {
-            case HTGS_MODE_HYBRID_BLEND: return launch_t<HTGS_MODE_HYBRID_BLEND, false, true>(scene, view, geo, prim, status, stream);
-            case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_t<HTGS_MODE_ALPHA_BLEND_FIRST_K, false, true>(scene, view, geo, prim, status, stream);
-            case HTGS_MODE_OIT_BLEND: return launch_t<HTGS_MODE_OIT_BLEND, false, true>(scene, view, geo, prim, status, stream);
+            case HTGS_MODE_HYBRID_BLEND: return launch_t<HTGS_MODE_HYBRID_BLEND, false, true>(scene, view, geo, prim, status, outline_mode, stream);
+            case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_t<HTGS_MODE_ALPHA_BLEND_FIRST_K, false, true>(scene, view, geo, prim, status, outline_mode, stream);
+            case HTGS_MODE_OIT_BLEND: return launch_t<HTGS_MODE_OIT_BLEND, false, true>(scene, view, geo, prim, status, outline_mode, stream);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (mode) {
-#define HTGS_CASE(M) case M: return train ? launch_t<M, true, false>(scene, view, geo, prim, status, stream) : launch_t<M, false, false>(scene, view, geo, prim, status, stream);
+#define HTGS_CASE(M) case M: return train ? launch_t<M, true, false>(scene, view, geo, prim, status, outline_mode, stream) : launch_t<M, false, false>(scene, view, geo, prim, status, outline_mode, stream);
         HTGS_CASE(HTGS_MODE_HYBRID_BLEND)
         HTGS_CASE(HTGS_MODE_ALPHA_BLEND_FIRST_K)
         HTGS_CASE(HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING)
