@@ -828,6 +828,7 @@ int htgs::backward_with_accum(HtgsContext* ctx, const HtgsScene* scene, const Ht
     const PrimLayout P = carve_primitive_blob(blobs->per_primitive, scene->n_primitives);
     const InstLayout I = carve_instance_blob(blobs->per_instance, plan, n_instances);
     const PixelLayout X = carve_pixel_blob(blobs->per_pixel, view->mode, view->K, geo);
+    const TileLayout T = carve_tile_blob(blobs->per_tile, geo);
     const bool accumulate = (stages & kBackwardAccumulate) != 0;      // the chain rule alone reads the per-Gaussian blob only
     if (!blobs->per_primitive || blobs->per_primitive_bytes < P.bytes ||
         (accumulate && (!blobs->per_instance || blobs->per_instance_bytes < I.bytes || !blobs->per_pixel || blobs->per_pixel_bytes < X.bytes || !blobs->per_tile)))
@@ -848,7 +849,7 @@ int htgs::backward_with_accum(HtgsContext* ctx, const HtgsScene* scene, const Ht
         if ((e = cudaEventRecord(ctx->front_end, ctx->front_stream)) != cudaSuccess) return fail_cuda(e, "front event record");
         outputs_cleared = ctx->front_end;
     }
-    const cudaError_t err = launch_backward(view->mode, view->K, *scene, *view, geo, P.prim, I.inst.prims[plan.final_buffer], static_cast<const uint2*>(blobs->per_tile),
+    const cudaError_t err = launch_backward(view->mode, view->K, *scene, *view, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order,
                                             X.px, grad_image, image, acc, out, outputs_cleared, ctx->sm_count, first, count, stages, stream);
     if (err != cudaSuccess) return fail_cuda(err, "backward");
     return HTGS_OK;

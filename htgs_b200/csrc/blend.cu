@@ -70,46 +70,6 @@ template <int MODE, int K, Buffer BUFFER, BlendTask TASK> struct SmemLayout {
     static constexpr size_t total = bar_off + 2 * 8;
 };
 
-__device__ __forceinline__ float sqrt_approx(float x) { float y; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
-// Pixels of the 8 x 4 block at (x0, y0) that the outline a dx^2 + b2 dx dy + c dy^2 <= 1 about (cx, cy) can touch: bit
-// (row * 8 + column).  A row is cut in an interval; 0.01 pixel is added at both ends, far more than the roundings here and
-// far less than the 0.3 pixel by which the outline was inflated.
-__device__ __forceinline__ uint32_t outline_mask(const float4& c0, float cc, float x0, float y0) {
-    if (c0.z == 0.0f) return c0.x > 1e30f ? 0u : 0xffffffffu;   // nothing can be accepted / no proper ellipse: every pixel is a candidate
-    const float a_rcp = __fdividef(1.0f, c0.z);
-    const float slope = -0.5f * c0.w * a_rcp;                   // centre of the interval per unit of dy
-    const float shrink = slope * slope - cc * a_rcp;            // half width^2 = 1/a + shrink * dy^2
-    const float left = c0.x - x0, dy0 = y0 - c0.y;
-    uint32_t mask = 0;
-    #pragma unroll
-    for (int r = 0; r < kBlockH; ++r) {
-        const float dy = dy0 + float(r);
-        const float half_sq = fmaf(shrink * dy, dy, a_rcp);
-        const float mid = fmaf(slope, dy, left);
-        const float half = half_sq >= 0.0f ? sqrt_approx(half_sq) + 0.01f : -16.0f;
-        const int lo = max(__float2int_ru(mid - half), 0), hi = min(__float2int_rd(mid + half), kBlockW - 1);
-        const uint32_t row = ((2u << (hi & 31)) - 1u) & ~((1u << (lo & 31)) - 1u);       // bits lo..hi
-        if (lo <= hi) mask |= row << (r * kBlockW);
-    }
-    return mask;
-}
-
-// Lane i < 16 holds the pixel mask of survivor i; the result has, in lane = pixel, bit 15 - i set if survivor i can touch it.
-__device__ __forceinline__ uint32_t transpose_masks(uint32_t mask, uint32_t lane) {
-    uint32_t x = __shfl_sync(0xffffffffu, mask, 15u - (lane & 15u)) >> (lane & 16u);     // row 15 - i of a 16 x 16 block per half warp
-    #pragma unroll
-    for (int d = 8; d > 0; d >>= 1) {
-        const uint32_t low = d == 8 ? 0x00ffu : d == 4 ? 0x0f0fu : d == 2 ? 0x3333u : 0x5555u;
-        const bool up = lane & uint32_t(d);
-        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, d);
-        const uint32_t t = __funnelshift_l(y, y, up ? 32u - d : d);
-        const uint32_t keep = up ? ~low : low;
-        x = (x & keep) | (t & ~keep);
-    }
-    return x & 0xffffu;
-}
-
 // The shared per-fragment front end (hybrid_blend/kernels/inference.cuh:137-148).
 struct FragmentFront {
     float3 m, d;

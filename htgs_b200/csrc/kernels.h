@@ -129,7 +129,7 @@ cudaError_t launch_max_weights(const HtgsView& view, const FrameGeometry& geo, c
 
 // train.cu: backward pass
 struct GradAccumBuffers {
-    float4* accum;           // [N][5] float4: dL/dVPMT1, dL/dVPMT2, dL/dVPMT4, (dL/drgb, dL/dopacity), (sum |dL/dposition|, 0, 0, 0)
+    float4* accum;           // [N][5] float4: moments of the rho^2 gradient (3, train.cu), (dL/drgb, dL/dopacity), (sum |dL/dposition|, 0, 0, 0)
 };
 constexpr int kBackwardAccumulate = 1, kBackwardChainRule = 2;
 struct BackwardOutputs {
@@ -142,7 +142,7 @@ struct BackwardOutputs {
 };
 cudaError_t launch_visibility(const uint32_t* n_touched, uint8_t* visible, uint32_t n, cudaStream_t stream);
 cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim,
-                            const uint32_t* prims_sorted, const uint2* tile_ranges, const TrainPixelBuffers& tin, const float* grad_image,
+                            const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order, const TrainPixelBuffers& tin, const float* grad_image,
                             const float* image, const GradAccumBuffers& acc, const BackwardOutputs& out, cudaEvent_t outputs_cleared, int sm_count,
                             uint32_t first, uint32_t count, int stages, cudaStream_t stream);
 // `stages`: kBackwardAccumulate = the per-tile (per-pixel for GLOBAL_ORDERING) pass that accumulates one record per Gaussian,

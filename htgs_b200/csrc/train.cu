@@ -39,99 +39,167 @@ __device__ __forceinline__ void red_add_v4(float4* addr, const float4& v) {
 __device__ __forceinline__ float rcp_approx(float x) { float y; asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f)); return y; }
 
-// Whether the forward pass rejected the fragment for `alpha < min_alpha`.  The forward decides with IEEE arithmetic
-// (1.0f / denominator, expf); the approximate alpha computed here differs from that value by less than 1e-6 of itself
-// (1 ulp reciprocal, 2 ulp exp2, and the rounding of an exponent of magnitude <= 8), so it settles the question unless
-// it lies within 4e-6 of the threshold, and only then is the forward's own arithmetic repeated: the decision is the
-// forward's in every case, the approximations only ever scale gradient terms.
-template <typename MT>
-__device__ __forceinline__ bool rejected_by_forward(float alpha_approx, float opacity, float numerator_rho2, float denominator) {
-    if (fabsf(alpha_approx - MT::min_alpha) < 4e-6f * MT::min_alpha) {
-        const float G = expf(-0.5f * numerator_rho2 * (1.0f / denominator));
-        return fminf(opacity * G, kMaxFragmentAlpha) < MT::min_alpha;
-    }
-    return alpha_approx < MT::min_alpha;
+// The gradient of rho^2 = N / D, N = |m|^2, D = |d|^2, w.r.t. the rows VPMT1, VPMT2, VPMT4 (hybrid_blend/kernels/backward.cuh:258-285), in moments.
+// Along a Gaussian's pixels m and d are affine and N and D quadratic in (x, y) = pixel - centre, the centre of its outline
+// record, and as well in (s, y) with the sheared s = x + shear * y:  m = M0 + s Ms + y My,  d = D0 + s Ds + y Dy  (AffinePlanes).
+// The shear makes Ms and My orthogonal: however long and slanted the ellipse, the terms of m do not cancel.  The rows' gradients
+// are quadratic in (s, y) too, with coefficients that are the Gaussian's alone, so a pair only adds
+//     u = dL/drho^2 / D  and  v = u N / D,  each times  1, s, y, ss, sy, yy
+// to the Gaussian's record, and rows_from_moments applies the coefficients once per Gaussian.  That is 18 instructions per pair
+// instead of 54 for the rows themselves, and offsets from the centre keep the sums well conditioned, where the rows' sums hold products with
+// pixel coordinates that cancel later.
+struct AffinePlanes { float3 M0, Ms, My, D0, Ds, Dy; float4 A, B; float shear; };     // A = VPMT1 - cx VPMT4, B = VPMT2 - cy VPMT4
+__device__ __forceinline__ AffinePlanes affine_planes(const float4& T1, const float4& T2, const float4& T4, float cx, float cy) {
+    AffinePlanes p;
+    p.A = make_float4(fmaf(-cx, T4.x, T1.x), fmaf(-cx, T4.y, T1.y), fmaf(-cx, T4.z, T1.z), fmaf(-cx, T4.w, T1.w));
+    p.B = make_float4(fmaf(-cy, T4.x, T2.x), fmaf(-cy, T4.y, T2.y), fmaf(-cy, T4.z, T2.z), fmaf(-cy, T4.w, T2.w));
+    const float3 a = f3(p.A), b = f3(p.B), n = f3(T4);
+    p.M0 = p.A.w * b - p.B.w * a;
+    p.Ms = p.B.w * n - T4.w * b;
+    p.My = T4.w * a - p.A.w * n;
+    p.D0 = cross(a, b);
+    p.Ds = cross(b, n);
+    p.Dy = cross(n, a);
+    const float ms_sq = dot(p.Ms, p.Ms);
+    p.shear = ms_sq > 0.0f ? __fdividef(dot(p.Ms, p.My), ms_sq) : 0.0f;
+    if (!(fabsf(p.shear) < 1e6f)) p.shear = 0.0f;
+    p.My = p.My - p.shear * p.Ms;
+    p.Dy = p.Dy - p.shear * p.Ds;
+    return p;
 }
 
-struct PairGrad {      // what one (pixel, Gaussian) pair adds to the Gaussian's record
-    float4 dT1, dT2, dT4;
+// What the pair loops evaluate: N and D as quadratics about the centre, and how large rho^2 may be (forward's alpha and cutoff tests).
+struct PairForm {
+    float4 n0, n1, d1;     // n0 = N: 1, s, y, ss   n1 = N: sy, yy, D: 1, s   d1 = D: y, ss, sy, yy
 };
+__device__ __forceinline__ PairForm pair_form(const AffinePlanes& p) {
+    PairForm f;
+    f.n0 = make_float4(dot(p.M0, p.M0), 2.0f * dot(p.M0, p.Ms), 2.0f * dot(p.M0, p.My), dot(p.Ms, p.Ms));
+    f.n1 = make_float4(2.0f * dot(p.Ms, p.My), dot(p.My, p.My), dot(p.D0, p.D0), 2.0f * dot(p.D0, p.Ds));
+    f.d1 = make_float4(2.0f * dot(p.D0, p.Dy), dot(p.Ds, p.Ds), 2.0f * dot(p.Ds, p.Dy), dot(p.Dy, p.Dy));
+    return f;
+}
+__device__ __forceinline__ void evaluate_pair(const PairForm& f, float s, float y, float& numerator, float& denominator) {
+    const float ss = s * s, sy = s * y, yy = y * y;
+    numerator = fmaf(f.n1.y, yy, fmaf(f.n1.x, sy, fmaf(f.n0.w, ss, fmaf(f.n0.z, y, fmaf(f.n0.y, s, f.n0.x)))));
+    denominator = fmaf(f.d1.w, yy, fmaf(f.d1.z, sy, fmaf(f.d1.y, ss, fmaf(f.d1.x, y, fmaf(f.n1.w, s, f.n1.z)))));
+}
 
-// Gradient of rho^2 = |m|^2 / |d|^2 w.r.t. the two planes through the pixel ray, then w.r.t. the rows
-// VPMT1, VPMT2, VPMT4 (hybrid_blend/kernels/backward.cuh:258-285).
-__device__ __forceinline__ PairGrad pair_gradient(const float4& plane_x_diag, const float4& plane_y_diag, const float3& m, const float3& d,
-                                                  float numerator_rho2, float denominator_rcp, float dL_drho2, float pixel_x, float pixel_y) {
-    const float dL_dnum = dL_drho2 * denominator_rcp;
-    const float dL_ddenom = dL_drho2 * -numerator_rho2 * denominator_rcp * denominator_rcp;
-    const float3 dL_dm = dL_dnum * 2.0f * m;
-    const float3 dL_dd = dL_ddenom * 2.0f * d;
-    const float3 nx = f3(plane_x_diag), ny = f3(plane_y_diag);
-    const float4 dpx = make_float4(
-        -plane_y_diag.w * dL_dm.x - plane_y_diag.z * dL_dd.y + plane_y_diag.y * dL_dd.z,
-        -plane_y_diag.w * dL_dm.y + plane_y_diag.z * dL_dd.x - plane_y_diag.x * dL_dd.z,
-        -plane_y_diag.w * dL_dm.z - plane_y_diag.y * dL_dd.x + plane_y_diag.x * dL_dd.y,
-        dot(ny, dL_dm));
-    const float4 dpy = make_float4(
-        plane_x_diag.w * dL_dm.x + plane_x_diag.z * dL_dd.y - plane_x_diag.y * dL_dd.z,
-        plane_x_diag.w * dL_dm.y - plane_x_diag.z * dL_dd.x + plane_x_diag.x * dL_dd.z,
-        plane_x_diag.w * dL_dm.z + plane_x_diag.y * dL_dd.x - plane_x_diag.x * dL_dd.y,
-        -dot(nx, dL_dm));
-    PairGrad g;
-    g.dT1 = dpx;
-    g.dT2 = dpy;
-    g.dT4 = (-pixel_x) * dpx - pixel_y * dpy;
+// Whether the forward pass accepts a fragment is settled by rho^2 unless it lies within kLevelBand of the level where alpha meets
+// its threshold (or rho^2 the cutoff); then the forward's own arithmetic is repeated.  The band is far wider than the
+// difference between the quadratics and the forward's planes (a few 1e-6 of rho^2).
+constexpr float kLevelBand = 5e-5f;
+__device__ __forceinline__ float upper_level(float lower) { return fmaf(lower, 3.0f * kLevelBand, lower) + 4e-6f; }      // beyond it a fragment is certainly rejected
+template <typename MT>
+__device__ __forceinline__ float acceptance_level(float opacity) { return fminf(MT::max_cutoff_sq, 2.0f * __logf(opacity * MT::min_alpha_rcp)); }
+template <typename MT>
+__device__ __noinline__ bool accepted_by_forward(const EvalRecord* rec, float pixel_x, float pixel_y) {
+    const float* r = reinterpret_cast<const float*>(rec);
+    const float4 T1 = ldg4(r), T2 = ldg4(r + 4), T4 = ldg4(r + 8);
+    const float opacity = __ldg(r + 19);
+    const float4 plane_x_diag = T1 - T4 * pixel_x;
+    const float4 plane_y_diag = T2 - T4 * pixel_y;
+    const float3 m = plane_x_diag.w * f3(plane_y_diag) - f3(plane_x_diag) * plane_y_diag.w;
+    const float3 d = cross(f3(plane_x_diag), f3(plane_y_diag));
+    const float numerator_rho2 = dot(m, m), denominator = dot(d, d);
+    const float G = expf(-0.5f * numerator_rho2 * (1.0f / denominator));
+    return !(numerator_rho2 > MT::max_cutoff_sq * denominator) && !(fminf(opacity * G, kMaxFragmentAlpha) < MT::min_alpha);
+}
+
+struct PairMoments { float4 u0, u1, v1; };      // u: 1, s, y, ss | u: sy, yy, v: 1, s | v: y, ss, sy, yy
+__device__ __forceinline__ void add_moments(PairMoments& a, float u, float v, float s, float y) {
+    const float us = u * s, uy = u * y, vs = v * s, vy = v * y;
+    a.u0.x += u; a.u0.y += us; a.u0.z += uy; a.u0.w = fmaf(us, s, a.u0.w);
+    a.u1.x = fmaf(us, y, a.u1.x); a.u1.y = fmaf(uy, y, a.u1.y); a.u1.z += v; a.u1.w += vs;
+    a.v1.x += vy; a.v1.y = fmaf(vs, s, a.v1.y); a.v1.z = fmaf(vs, y, a.v1.z); a.v1.w = fmaf(vy, y, a.v1.w);
+}
+
+// dL/dVPMT1 = sum dX, dL/dVPMT2 = sum dY, and E = sum (x dX + y dY), so that dL/dVPMT4 = -(cx sum dX + cy sum dY + E).  With
+// X = A - x VPMT4, Y = B - y VPMT4, dm = 2 u m and dd = -2 v d:
+//     dX = (Y x dd - Y.w dm, Y . dm),   dY = (X.w dm - X x dd, -X . dm)
+// and the cubic terms of E cancel: x dX + y dY = ((x B - y A) x dd - (x B.w - y A.w) dm, (x B - y A) . dm).
+struct RowGradients { float4 dX, dY, E; };
+__device__ __forceinline__ RowGradients rows_from_moments(const AffinePlanes& p, const float4& T4, const PairMoments& a) {
+    const float3 A = f3(p.A), B = f3(p.B), n = f3(T4);
+    const float u = a.u0.x, us = a.u0.y, uy = a.u0.z, uss = a.u0.w, usy = a.u1.x, uyy = a.u1.y;
+    const float v = a.u1.z, vs = a.u1.w, vy = a.v1.x, vss = a.v1.y, vsy = a.v1.z, vyy = a.v1.w;
+    // sums of u m and v d, and of these times y and x = s - shear * y
+    const float3 m1 = u * p.M0 + us * p.Ms + uy * p.My, my = uy * p.M0 + usy * p.Ms + uyy * p.My;
+    const float3 d1 = v * p.D0 + vs * p.Ds + vy * p.Dy, dy = vy * p.D0 + vsy * p.Ds + vyy * p.Dy;
+    const float3 mx = us * p.M0 + uss * p.Ms + usy * p.My - p.shear * my, dx = vs * p.D0 + vss * p.Ds + vsy * p.Dy - p.shear * dy;
+    RowGradients g;
+    const float3 gx = -(p.B.w * m1 - T4.w * my) - (cross(B, d1) - cross(n, dy));
+    const float3 gy = (p.A.w * m1 - T4.w * mx) + (cross(A, d1) - cross(n, dx));
+    const float3 ge = -(p.B.w * mx - p.A.w * my) - (cross(B, dx) - cross(A, dy));
+    g.dX = make_float4(2.0f * gx.x, 2.0f * gx.y, 2.0f * gx.z, 2.0f * (dot(B, m1) - dot(n, my)));
+    g.dY = make_float4(2.0f * gy.x, 2.0f * gy.y, 2.0f * gy.z, -2.0f * (dot(A, m1) - dot(n, mx)));
+    g.E = make_float4(2.0f * ge.x, 2.0f * ge.y, 2.0f * ge.z, 2.0f * (dot(B, mx) - dot(A, my)));
     return g;
 }
 
+// sum |dL/dposition| needs every pair's own fourth column (dL/dVPMT1.w, dL/dVPMT2.w, dL/dVPMT4.w) = (Y . dm, -X . dm, ...)
 struct CameraCols { float3 c1, c2, c3; };   // columns 1..3 of rows (1,2,4) of VPM
 __device__ __forceinline__ CameraCols load_camera_cols(const float* __restrict__ VPM) {
     const float4 r1 = ldg4(VPM), r2 = ldg4(VPM + 4), r4 = ldg4(VPM + 12);
     return {make_float3(r1.x, r2.x, r4.x), make_float3(r1.y, r2.y, r4.y), make_float3(r1.z, r2.z, r4.z)};
 }
+// Y . m and X . m (3-vectors) as quadratics about the centre; the fourth columns of a pair are 2u times these.
+struct AbsForm { float4 y0, x0, y1x1; };      // Y . m: 1, s, y, sy | X . m: 1, s, y, ss | Y . m: yy, X . m: sy, yy
+__device__ __forceinline__ AbsForm abs_form(const AffinePlanes& p, const float4& T4) {
+    const float3 a = f3(p.A), b = f3(p.B), n = f3(T4);
+    const float nm0 = dot(n, p.M0), nms = dot(n, p.Ms), nmy = dot(n, p.My);
+    return {make_float4(dot(b, p.M0), dot(b, p.Ms), dot(b, p.My) - nm0, -nms), make_float4(dot(a, p.M0), dot(a, p.Ms) - nm0, fmaf(p.shear, nm0, dot(a, p.My)), -nms),
+            make_float4(-nmy, fmaf(p.shear, nms, -nmy), p.shear * nmy, 0.0f)};
+}
+__device__ __forceinline__ float abs_position_gradient(const AbsForm& f, float u, float s, float y, float pixel_x, float pixel_y, const CameraCols& cam) {
+    const float sy = s * y, yy = y * y;
+    const float wx = 2.0f * u * fmaf(f.y1x1.x, yy, fmaf(f.y0.w, sy, fmaf(f.y0.z, y, fmaf(f.y0.y, s, f.y0.x))));
+    const float wy = -2.0f * u * fmaf(f.y1x1.z, yy, fmaf(f.y1x1.y, sy, fmaf(f.x0.w, s * s, fmaf(f.x0.z, y, fmaf(f.x0.y, s, f.x0.x)))));
+    const float wz = -pixel_x * wx - pixel_y * wy;
+    const float3 c4 = make_float3(wx, wy, wz);
+    return fabsf(dot(cam.c1, c4)) + fabsf(dot(cam.c2, c4)) + fabsf(dot(cam.c3, c4));
+}
 
 constexpr int kBwdThreads = 128;       // threads per tile: one staged instance each, and an even share of the batch's pairs
 constexpr int kBwdThreadsLog2 = 7;
-constexpr int kBwdMinBlocks = 5;       // resident CTAs per SM the register budget is held to (shared memory allows as many)
-template <int MODE, int K> struct BwdSmem {
+template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr bool has_core = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
     static constexpr bool has_tail = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_OIT_BLEND);
-    static constexpr int idx_stride = ((K + 3) / 4) * 4 + 4;         // words per pixel row: 16-byte rows, odd multiple of 4 words -> conflict-free uint4 reads
-    static constexpr size_t idx_off = 0;
-    static constexpr size_t idx_bytes = has_core ? size_t(idx_stride) * 64 * 4 : 0;
-    static constexpr size_t cg_off = idx_off + idx_bytes;
+    static constexpr size_t cg_off = 0;
     static constexpr size_t cg_bytes = has_core ? size_t(K) * 64 * 16 : 0;
     static constexpr size_t tc_off = cg_off + cg_bytes;
     static constexpr size_t tc_bytes = has_tail ? 64 * 16 : 0;
     static constexpr size_t ta_off = tc_off + tc_bytes;
     static constexpr size_t ta_bytes = has_tail ? 64 * 4 : 0;
     static constexpr size_t stage_off = (ta_off + ta_bytes + 15) & ~size_t(15);
-    static constexpr size_t stage_bytes = kBwdThreads * (4 * 16 + 8 + 4) + (kBwdThreads + 1) * 4 + 12;
+    static constexpr size_t stage_bytes = kBwdThreads * ((ABS_GRAD ? 8 : 5) * 16 + 8 + 4) + (kBwdThreads + 1) * 4 + 12;
     static constexpr size_t core_off = (stage_off + stage_bytes + 15) & ~size_t(15);     // [NT][64] core entry of each (staged instance, pixel) pair
     static constexpr size_t core_bytes = has_core ? size_t(kBwdThreads) * 64 : 0;
     static constexpr size_t total = core_off + core_bytes;
+    static constexpr int min_blocks = int((227 * 1024) / (total + 1024)) < 5 ? int((227 * 1024) / (total + 1024)) : 5;   // what the register budget is held to
 };
 
-// HYBRID_BLEND / ALPHA_BLEND_FIRST_K / OIT_BLEND: one CTA per 8x8 tile, one thread per Gaussian of a batch of kBwdThreads.
+// HYBRID_BLEND / ALPHA_BLEND_FIRST_K / OIT_BLEND: one CTA per 8x8 tile (long lists first), one thread per Gaussian of a batch of kBwdThreads.
 template <int MODE, int K, bool ABS_GRAD>
-__global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kernel(
-    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
+__global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_blocks)) backward_tile_kernel(
+    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, TrainPixelBuffers tin, const float* __restrict__ grad_image, const float* __restrict__ VPM,
     float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w, uint32_t g_first, uint32_t g_end)
 {
     using MT = ModeTraits<MODE>;
-    using SM = BwdSmem<MODE, K>;
+    using SM = BwdSmem<MODE, K, ABS_GRAD>;
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     extern __shared__ __align__(16) unsigned char smem[];
-    [[maybe_unused]] uint32_t* s_idx = reinterpret_cast<uint32_t*>(smem + SM::idx_off);   // [64 pixels][idx_stride] positions in the tile's list
     [[maybe_unused]] signed char* s_core = reinterpret_cast<signed char*>(smem + SM::core_off);
     [[maybe_unused]] float4* s_cg = reinterpret_cast<float4*>(smem + SM::cg_off);          // [K][64] (W * grad_pixel, A . grad_pixel)
     [[maybe_unused]] float4* s_tc = reinterpret_cast<float4*>(smem + SM::tc_off);          // [64] (full_weight * grad_pixel, common term)
     [[maybe_unused]] float* s_ta = reinterpret_cast<float*>(smem + SM::ta_off);            // [64] term divided by (1 - alpha)
 
     const uint32_t tid = threadIdx.x;
-    const uint32_t tile_x = blockIdx.x, tile_y = blockIdx.y;
-    const uint2 tile_range = tile_ranges[tile_y * grid_w + tile_x];
+    const uint32_t tile = __ldg(tile_order + blockIdx.x);
+    const uint32_t tile_x = tile % grid_w, tile_y = tile / grid_w;
+    const uint2 tile_range = tile_ranges[tile];
     uint2 range = tile_range;
     // A pass over the Gaussians [g_first, g_end) only: a tile's list is ascending in Gaussian index for these modes (instances
     // are emitted in index order and the tile sort is stable), so the pass walks one contiguous piece of it.
@@ -146,26 +214,46 @@ __global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kern
     if (range.x >= range.y) return;
     const uint32_t n_pixels = width * height;
     const uint32_t PP = tin.padded_pixels;
-    constexpr uint32_t NT = kBwdThreads;
-    const uint32_t pix = tid & 63, part = tid >> 6;          // the per-pixel terms are set up by NT / 64 threads per pixel
-    const uint32_t slot = (tile_y * grid_w + tile_x) * 64 + pix;
+    constexpr uint32_t NT = kBwdThreads, kParts = NT / 64;
+    const uint32_t pix = tid & 63, part = tid >> 6;          // the per-pixel terms are set up by kParts threads per pixel
+    const uint32_t slot = tile * 64 + pix;
+    const float x0 = float(tile_x * 8), y0 = float(tile_y * 8);
+    // pixels of the tile that exist in the image, as a 64-bit mask (bit = row * 8 + column)
+    uint64_t inside_mask = 0;
+    {
+        const uint32_t cols = min(8u, width - tile_x * 8), rows = min(8u, height - tile_y * 8);
+        const uint64_t row_bits = (1ull << cols) - 1ull;
+        for (uint32_t r = 0; r < rows; ++r) inside_mask |= row_bits << (8 * r);
+    }
 
-    // Software pipeline of the staging loads: the record and outline of the instance a thread stages in batch b + 1 are
-    // requested while batch b is processed (its index was requested one batch earlier still), so that their latency
-    // overlaps the pair loop instead of sitting between two barriers.  The first indices are requested before the
-    // per-pixel terms are read, so that the two chains of dependent loads at the start of a tile overlap as well.
-    uint32_t g_cur = 0, g_nxt = 0;
-    float4 pT1 = make_float4(0, 0, 0, 0), pT2 = pT1, pT4 = pT1, pRGBA = pT1, pc0 = pT1;
-    float pcc = 0.0f;
-    auto request = [&](uint32_t g) {
-        const float* rec = reinterpret_cast<const float*>(eval + g);
-        pT1 = ldg4(rec); pT2 = ldg4(rec + 4); pT4 = ldg4(rec + 8); pRGBA = ldg4(rec + 16);
-        pc0 = ldg4(reinterpret_cast<const float*>(cull + g));
-        pcc = __ldg(reinterpret_cast<const float*>(cull + g) + 4);
+    // Software pipeline of the staging loads.  While batch b is processed, the outlines of batch b + 1 (requested one batch earlier)
+    // give the pixel masks, the records of those instances that touch a pixel (six in ten) are requested, then the outlines of
+    // batch b + 2 and the indices of batch b + 3.
+    uint32_t g_rec = 0, g_out = 0, g_idx = 0;
+    float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1, outline = rT1;
+    float rcx = 0.0f, rcy = 0.0f, outline_c = 0.0f;
+    uint64_t mask_rec = 0;
+    auto load_index = [&](uint32_t inst) { return inst < range.y ? __ldg(prims_sorted + inst) : 0u; };
+    auto request_outline = [&](uint32_t inst) {
+        if (inst >= range.y) return;
+        outline = ldg4(reinterpret_cast<const float*>(cull + g_out));
+        outline_c = __ldg(reinterpret_cast<const float*>(cull + g_out) + 4);
     };
-    if (range.x + tid < range.y) g_cur = __ldg(prims_sorted + range.x + tid);
-    if (range.x + NT + tid < range.y) g_nxt = __ldg(prims_sorted + range.x + NT + tid);
+    auto request_record = [&](uint32_t inst) {              // of the instance whose outline has arrived
+        mask_rec = 0;
+        if (inst < range.y) mask_rec = (uint64_t(outline_mask(outline, outline_c, x0, y0)) | (uint64_t(outline_mask(outline, outline_c, x0, y0 + 4.0f)) << 32)) & inside_mask;
+        if (mask_rec == 0) return;
+        g_rec = g_out;
+        rcx = outline.x; rcy = outline.y;
+        const float* rec = reinterpret_cast<const float*>(eval + g_rec);
+        rT1 = ldg4(rec); rT2 = ldg4(rec + 4); rT4 = ldg4(rec + 8); rRGBA = ldg4(rec + 16);
+    };
+    g_out = load_index(range.x + tid);
+    g_idx = load_index(range.x + NT + tid);
+    request_outline(range.x + tid);
     // ---- per-pixel terms of this tile (hybrid_blend/kernels/backward.cuh:137-176, oit_blend/kernels/backward.cuh:131-156)
+    // core_pos: this thread's share of the pixel's core entries, as positions in the tile's list
+    [[maybe_unused]] uint32_t core_pos[SM::has_core ? (K + kParts - 1) / kParts : 1];
     {
         const uint32_t px_i = tile_x * 8 + (pix & 7), py_i = tile_y * 8 + (pix >> 3);
         const bool inside = px_i < width && py_i < height;
@@ -176,67 +264,59 @@ __global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kern
         }
         if constexpr (SM::has_core) {
             #pragma unroll
-            for (int k0 = 0; k0 < K; k0 += int(NT / 64)) {
-                const int k = k0 + int(part);
-                if (k >= K) break;
-                uint32_t idx = 0xffffffffu;
-                float4 cg = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (inside) {
-                    idx = tin.idx_core[k * PP + slot];
-                    if (idx != 0xffffffffu) {
+            for (int i = 0; i < int((K + kParts - 1) / kParts); ++i) {
+                const int k = i * int(kParts) + int(part);
+                core_pos[i] = 0xffffffffu;
+                if (k < K && inside) {
+                    core_pos[i] = tin.idx_core[k * PP + slot];
+                    if (core_pos[i] != 0xffffffffu) {
                         const float4 info = tin.info_core[k * PP + slot];
                         const float3 drgb = info.w * grad_pixel;
-                        cg = make_float4(drgb.x, drgb.y, drgb.z, dot(f3(info), grad_pixel));
+                        s_cg[k * 64 + pix] = make_float4(drgb.x, drgb.y, drgb.z, dot(f3(info), grad_pixel));
                     }
                 }
-                s_idx[pix * SM::idx_stride + k] = idx;
-                s_cg[k * 64 + pix] = cg;
             }
         }
         if constexpr (SM::has_tail) {
-            float4 tc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            float ta = 0.0f;
-            if (inside) {
-                const float3 rgb_tail = make_float3(tin.info_tail[slot], tin.info_tail[PP + slot], tin.info_tail[2 * PP + slot]);
-                const float alpha_sum_rcp = tin.info_tail[3 * PP + slot];
-                const float transmittance_tail = tin.info_tail[4 * PP + slot];
-                const float transmittance_core = kHybrid ? tin.info_tail[5 * PP + slot] : 1.0f;
-                const float weight_tail = transmittance_core * alpha_sum_rcp;
-                const float full_weight_tail = weight_tail * (1.0f - transmittance_tail);
-                const float rgb_dot_grad = dot(rgb_tail, grad_pixel);
-                const float3 part = full_weight_tail * grad_pixel;
-                tc = make_float4(part.x, part.y, part.z, -full_weight_tail * alpha_sum_rcp * rgb_dot_grad);
-                ta = weight_tail * transmittance_tail * rgb_dot_grad;
-            }
             if (part == 0) {
+                float4 tc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float ta = 0.0f;
+                if (inside) {
+                    const float3 rgb_tail = make_float3(tin.info_tail[slot], tin.info_tail[PP + slot], tin.info_tail[2 * PP + slot]);
+                    const float alpha_sum_rcp = tin.info_tail[3 * PP + slot];
+                    const float transmittance_tail = tin.info_tail[4 * PP + slot];
+                    const float transmittance_core = kHybrid ? tin.info_tail[5 * PP + slot] : 1.0f;
+                    const float weight_tail = transmittance_core * alpha_sum_rcp;
+                    const float full_weight_tail = weight_tail * (1.0f - transmittance_tail);
+                    const float rgb_dot_grad = dot(rgb_tail, grad_pixel);
+                    const float3 part = full_weight_tail * grad_pixel;
+                    tc = make_float4(part.x, part.y, part.z, -full_weight_tail * alpha_sum_rcp * rgb_dot_grad);
+                    ta = weight_tail * transmittance_tail * rgb_dot_grad;
+                }
                 s_tc[pix] = tc;
                 s_ta[pix] = ta;
             }
         }
     }
-    // pixels of the tile that exist in the image, as a 64-bit mask (bit = row * 8 + column)
-    uint64_t inside_mask = 0;
-    {
-        const uint32_t cols = min(8u, width - tile_x * 8), rows = min(8u, height - tile_y * 8);
-        const uint64_t row_bits = (1ull << cols) - 1ull;
-        for (uint32_t r = 0; r < rows; ++r) inside_mask |= row_bits << (8 * r);
-    }
     [[maybe_unused]] CameraCols cam;
     if constexpr (ABS_GRAD) cam = load_camera_cols(VPM);
-    if (range.x + tid < range.y) request(g_cur);
-    __syncthreads();
+    request_record(range.x + tid);
+    g_out = g_idx;
+    request_outline(range.x + NT + tid);
+    g_idx = load_index(range.x + 2 * NT + tid);
 
     // ---- batches of NT instances; the (Gaussian, pixel) candidate pairs of a batch are split EVENLY over the
     //      NT threads (pairs of one Gaussian are contiguous, so a thread walks a few Gaussians back to back)
-    float4* s_T1 = reinterpret_cast<float4*>(smem + SM::stage_off);
-    float4* s_T2 = s_T1 + NT;
-    float4* s_T4 = s_T2 + NT;
-    float4* s_rgba = s_T4 + NT;
-    unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(s_rgba + NT);
+    float4* s_n0 = reinterpret_cast<float4*>(smem + SM::stage_off);
+    float4* s_n1 = s_n0 + NT;
+    float4* s_d1 = s_n1 + NT;
+    float4* s_rgba = s_d1 + NT;
+    float4* s_pos = s_rgba + NT;         // tile origin - centre, rho^2 below which a fragment is certainly accepted, shear
+    [[maybe_unused]] float4* s_abs = s_pos + NT;    // ABS_GRAD: [3][NT]
+    unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(s_pos + NT * (ABS_GRAD ? 4 : 1));
     uint32_t* s_g = reinterpret_cast<uint32_t*>(s_mask + NT);
     uint32_t* s_off = s_g + NT;          // [NT + 1] exclusive prefix of the per-Gaussian pair counts
     __shared__ uint32_t s_warp_total[NT / 32];
-    const float x0 = float(tile_x * 8), y0 = float(tile_y * 8);
     const uint32_t lane = tid & 31, warp = tid >> 5;
     // The training forward saved, per pixel and core entry, the POSITION of the entry's Gaussian in the tile's list, so the
     // entries that belong to a batch are those within NT of its start, and position - start is the staged slot.
@@ -244,65 +324,51 @@ __global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kern
     // `limit`: staged instances of the batch (entries further down the list belong to a later batch, or - in a pass over a
     // range of Gaussians - to Gaussians beyond the range, whose slots in this batch hold nothing).
     [[maybe_unused]] auto scatter_core_entries = [&](uint32_t batch_pos, uint32_t limit) {
-        const uint4* row = reinterpret_cast<const uint4*>(s_idx + pix * SM::idx_stride);
-        auto put = [&](uint32_t j, int k) {
-            s_core[j * 64 + pix] = (signed char)k;
-            if constexpr (kFirstK) atomicOr(reinterpret_cast<uint32_t*>(s_mask + j) + (pix >> 5), 1u << (pix & 31));
-        };
         #pragma unroll
-        for (int k4 = 0; k4 < (K + 3) / 4; k4 += int(NT / 64)) {
-            const int q = k4 + int(part);
-            if (q >= (K + 3) / 4) break;
-            const uint4 v = row[q];
-            const uint32_t j0 = v.x - batch_pos, j1 = v.y - batch_pos, j2 = v.z - batch_pos, j3 = v.w - batch_pos;
-            if (j0 < limit) put(j0, 4 * q);
-            if (4 * q + 1 < K && j1 < limit) put(j1, 4 * q + 1);
-            if (4 * q + 2 < K && j2 < limit) put(j2, 4 * q + 2);
-            if (4 * q + 3 < K && j3 < limit) put(j3, 4 * q + 3);
+        for (int i = 0; i < int((K + kParts - 1) / kParts); ++i) {
+            const uint32_t j = core_pos[i] - batch_pos;
+            if (j < limit) {
+                s_core[j * 64 + pix] = (signed char)(i * int(kParts) + int(part));
+                if constexpr (kFirstK) atomicOr(reinterpret_cast<uint32_t*>(s_mask + j) + (pix >> 5), 1u << (pix & 31));
+            }
         }
     };
     for (uint32_t batch_begin = range.x; batch_begin < range.y; batch_begin += NT) {
         __syncthreads();                  // previous batch fully consumed
         const uint32_t inst = batch_begin + tid;
-        uint64_t my_mask = 0;
-        const bool valid = inst < range.y;
-        const float4 c0 = pc0;
-        const float cc = pcc;
-        if (valid) {
-            s_T1[tid] = pT1; s_T2[tid] = pT2; s_T4[tid] = pT4; s_rgba[tid] = pRGBA;
-            s_g[tid] = g_cur;
+        uint64_t my_mask = mask_rec;
+        if (my_mask != 0) {
+            const AffinePlanes planes = affine_planes(rT1, rT2, rT4, rcx, rcy);
+            const PairForm form = pair_form(planes);
+            s_n0[tid] = form.n0; s_n1[tid] = form.n1; s_d1[tid] = form.d1; s_rgba[tid] = rRGBA;
+            float level = 0.0f;
+            if constexpr (!kFirstK) level = acceptance_level<MT>(rRGBA.w);
+            const float band = kLevelBand * level + 1e-6f;
+            s_pos[tid] = make_float4(x0 - rcx, y0 - rcy, level - band, planes.shear);
+            if constexpr (ABS_GRAD) {
+                const AbsForm af = abs_form(planes, rT4);
+                s_abs[tid] = af.y0; s_abs[NT + tid] = af.x0; s_abs[2 * NT + tid] = af.y1x1;
+            }
+            s_g[tid] = g_rec;
+            if constexpr (SM::has_core) {      // no pair of my instance is a core entry until the scatter below says so
+                uint4* row = reinterpret_cast<uint4*>(s_core + tid * 64);
+                const uint4 none = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+                row[0] = none; row[1] = none; row[2] = none; row[3] = none;
+            }
         }
-        if constexpr (SM::has_core) {      // no pair of my instance is a core entry until the scatter below says so
-            uint4* row = reinterpret_cast<uint4*>(s_core + tid * 64);
-            const uint4 none = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-            row[0] = none; row[1] = none; row[2] = none; row[3] = none;
-        }
-        // next batch: its index is here, request its data; request the index of the batch after it
-        g_cur = g_nxt;
-        if (inst + NT < range.y) request(g_cur);
-        if (inst + 2 * NT < range.y) g_nxt = __ldg(prims_sorted + inst + 2 * NT);
+        request_record(inst + NT);
+        g_out = g_idx;
+        request_outline(inst + 2 * NT);
+        g_idx = load_index(inst + 3 * NT);
         if constexpr (kFirstK) {
             s_mask[tid] = 0;
             __syncthreads();
-            scatter_core_entries(batch_begin - __ldg(&tile_ranges[blockIdx.y * grid_w + blockIdx.x].x), min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
+            scatter_core_entries(batch_begin - tile_range.x, min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
             __syncthreads();
             my_mask = s_mask[tid];
-        } else if (valid) {
-            const float dx0 = x0 - c0.x, dy0 = y0 - c0.y;
-            #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const float dy = dy0 + float(r);
-                const float b2dy = c0.w * dy, cdy2 = cc * dy * dy;
-                #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float dx = dx0 + float(i);
-                    const float q = dx * (c0.z * dx + b2dy) + cdy2;
-                    if (q <= 1.0f) my_mask |= 1ull << (r * 8 + i);
-                }
-            }
-            my_mask &= inside_mask;
+        } else {
+            s_mask[tid] = my_mask;
         }
-        if constexpr (!kFirstK) s_mask[tid] = my_mask;
         const uint32_t cnt = __popcll(my_mask);
         uint32_t inc = cnt;
         #pragma unroll
@@ -318,7 +384,7 @@ __global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kern
         }
         s_off[tid] = excl;
         if (tid == 0) s_off[NT] = total_pairs;
-        if constexpr (SM::has_core && !kFirstK) scatter_core_entries(batch_begin - __ldg(&tile_ranges[blockIdx.y * grid_w + blockIdx.x].x), min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
+        if constexpr (SM::has_core && !kFirstK) scatter_core_entries(batch_begin - tile_range.x, min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
         __syncthreads();
         if (total_pairs == 0) continue;
         // my share of the pairs
@@ -334,47 +400,43 @@ __global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kern
         }
         uint64_t mask = s_mask[j];
         for (uint32_t skip = lo - s_off[j]; skip > 0; --skip) mask &= mask - 1;     // drop the pairs that belong to the previous thread
-        float4 T1 = s_T1[j], T2 = s_T2[j], T4 = s_T4[j], rgba = s_rgba[j];
-        uint32_t g = s_g[j];
-        float4 aT1 = make_float4(0, 0, 0, 0), aT2 = aT1, aT4 = aT1, aC = aT1;   // aC = (dL/drgb, dL/dopacity)
+        PairForm form{s_n0[j], s_n1[j], s_d1[j]};
+        float4 rgba = s_rgba[j], pos = s_pos[j];
+        PairMoments moments{};
+        float4 aC = make_float4(0, 0, 0, 0);            // (dL/drgb, dL/dopacity)
         [[maybe_unused]] float abs_grad = 0.0f;
         bool touched = false;
         auto flush = [&]() {
             if (touched) {
-                float4* rec = accum + size_t(g) * 5;
-                red_add_v4(rec, aT1); red_add_v4(rec + 1, aT2); red_add_v4(rec + 2, aT4); red_add_v4(rec + 3, aC);
+                float4* rec = accum + size_t(s_g[j]) * 5;
+                red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); red_add_v4(rec + 2, moments.v1); red_add_v4(rec + 3, aC);
                 if constexpr (ABS_GRAD) red_add_v4(rec + 4, make_float4(abs_grad, 0.0f, 0.0f, 0.0f));
             }
-            aT1 = make_float4(0, 0, 0, 0); aT2 = aT1; aT4 = aT1; aC = aT1; abs_grad = 0.0f; touched = false;
+            moments = PairMoments{}; aC = make_float4(0, 0, 0, 0); abs_grad = 0.0f; touched = false;
         };
         for (; remaining > 0; --remaining) {
-            while (mask == 0) {           // next Gaussian of my share (its mask is non-empty somewhere before `hi`)
+            if (mask == 0) {              // next Gaussian of my share (its mask is non-empty somewhere before `hi`)
                 flush();
-                ++j;
-                mask = s_mask[j];
-                T1 = s_T1[j]; T2 = s_T2[j]; T4 = s_T4[j]; rgba = s_rgba[j]; g = s_g[j];
+                do mask = s_mask[++j]; while (mask == 0);
+                form = PairForm{s_n0[j], s_n1[j], s_d1[j]};
+                rgba = s_rgba[j]; pos = s_pos[j];
             }
             const uint32_t p = uint32_t(__ffsll((long long)mask) - 1);
             mask &= mask - 1;
-            const float pixel_x = x0 + float(p & 7), pixel_y = y0 + float(p >> 3);
-            const float4 plane_x_diag = T1 - T4 * pixel_x;
-            const float4 plane_y_diag = T2 - T4 * pixel_y;
-            const float3 nx = f3(plane_x_diag), ny = f3(plane_y_diag);
-            const float3 m = plane_x_diag.w * ny - nx * plane_y_diag.w;
-            const float3 d = cross(nx, ny);
-            const float numerator_rho2 = dot(m, m);
-            const float denominator = dot(d, d);
+            const float y = pos.y + float(p >> 3), s = fmaf(pos.w, y, pos.x + float(p & 7));
+            float numerator_rho2, denominator;
+            evaluate_pair(form, s, y, numerator_rho2, denominator);
             int core_idx = -1;
             if constexpr (SM::has_core) core_idx = s_core[j * 64 + p];
+            const float denominator_rcp = rcp_approx(denominator);
+            const float rho2 = numerator_rho2 * denominator_rcp;
             if constexpr (kFirstK) {
                 if (core_idx < 0) continue;                    // only stored fragments carry gradient (first_k backward.cuh:84-87)
-            } else {
-                if (numerator_rho2 > MT::max_cutoff_sq * denominator) continue;
+            } else if (!(rho2 < pos.z)) {
+                if (rho2 > upper_level(pos.z) || !accepted_by_forward<MT>(eval + s_g[j], x0 + float(p & 7), y0 + float(p >> 3))) continue;
             }
-            const float denominator_rcp = rcp_approx(denominator);
-            const float G = exp_approx(-0.5f * numerator_rho2 * denominator_rcp);
+            const float G = exp_approx(-0.5f * rho2);
             const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
-            if constexpr (!kFirstK) { if (rejected_by_forward<MT>(alpha, rgba.w, numerator_rho2, denominator)) continue; }
             float3 dL_drgb;
             float dL_dalpha;
             if (core_idx >= 0) {
@@ -391,66 +453,50 @@ __global__ void __launch_bounds__(kBwdThreads, kBwdMinBlocks) backward_tile_kern
                 }
             }
             aC.x += dL_drgb.x; aC.y += dL_drgb.y; aC.z += dL_drgb.z;
-            touched = true;
-            if (dL_dalpha == 0.0f) continue;
             aC.w += dL_dalpha * G;
-            const float dL_dG = dL_dalpha * rgba.w;
-            const float dL_drho2 = dL_dG * -0.5f * G;
-            const PairGrad pg = pair_gradient(plane_x_diag, plane_y_diag, m, d, numerator_rho2, denominator_rcp, dL_drho2, pixel_x, pixel_y);
-            aT1 += pg.dT1; aT2 += pg.dT2; aT4 += pg.dT4;
+            touched = true;
+            const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D
+            add_moments(moments, u, u * rho2, s, y);
             if constexpr (ABS_GRAD) {
-                const float3 c4 = make_float3(pg.dT1.w, pg.dT2.w, pg.dT4.w);
-                abs_grad += fabsf(dot(cam.c1, c4)) + fabsf(dot(cam.c2, c4)) + fabsf(dot(cam.c3, c4));
+                abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + float(p & 7), y0 + float(p >> 3), cam);
             }
         }
         flush();
     }
 }
 
-// Sum of 16 per-lane values over the warp in 16 shuffles instead of 80: at every step a lane keeps one half of its
-// values, hands the other half to its partner and adds what the partner hands over.  After the steps with lane bits
-// 4, 3, 2, 1 a lane holds ONE value summed over the 16 lanes that share its bit 0; the last shuffle completes it.
-// On return the lane holds the warp total of v[transpose_reduce_index(lane)].
-__device__ __forceinline__ uint32_t transpose_reduce_index(uint32_t lane) { return (lane >> 1) & 15u; }   // bit 4 -> 8, bit 3 -> 4, bit 2 -> 2, bit 1 -> 1
-__device__ __forceinline__ float transpose_reduce16(const float (&v)[16], uint32_t lane) {
-    float a8[8], a4[4], a2[2];
-    const bool up16 = lane & 16u, up8 = lane & 8u, up4 = lane & 4u, up2 = lane & 2u;
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) a8[i] = (up16 ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, up16 ? v[i] : v[i + 8], 16);
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) a4[i] = (up8 ? a8[i + 4] : a8[i]) + __shfl_xor_sync(0xffffffffu, up8 ? a8[i] : a8[i + 4], 8);
-    #pragma unroll
-    for (int i = 0; i < 2; ++i) a2[i] = (up4 ? a4[i + 2] : a4[i]) + __shfl_xor_sync(0xffffffffu, up4 ? a4[i] : a4[i + 2], 4);
-    float a1 = (up2 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, up2 ? a2[0] : a2[1], 2);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
-    return a1;
-}
-
-// ALPHA_BLEND_GLOBAL_ORDERING: pixel-parallel, front to back in key order, using the final pixel colour so that
+// ALPHA_BLEND_GLOBAL_ORDERING: front to back in key order, using the final pixel colour so that
 // "colour behind" = rgb_pixel - rgb_pixel_new (alpha_blend_global_ordering/kernels/backward.cuh:104-161).
-// One CTA of two warps per 8x8 pixels; the four CTAs of a 16x16 binning tile walk the same list independently (a pixel
-// shares no state with its neighbours) and each stops when ITS pixels are opaque.  Per batch of 64 staged Gaussians a
-// warp first finds, with lane = Gaussian, which of them can touch its 8x4 pixels at all (the conservative outline the
-// forward pass uses) and only walks those; the 16 values a pixel adds to a Gaussian's record are summed over the warp
-// by transpose_reduce16 and added to a shared-memory record per staged Gaussian, flushed once per batch.
-constexpr int kGoBatch = 64;
-constexpr int kGoAccStride = 17;     // 16 values + sum |dL/dposition|; odd stride: rows and columns are both conflict-free
-__global__ void __launch_bounds__(64) backward_global_kernel(
-    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
+// One warp per 8x4 pixels (an eighth of a binning tile; a pixel shares no state with its neighbours), long lists first; it stops
+// when its pixels are opaque.  The list is filtered against the block as in the forward pass and taken in chunks of 16 survivors:
+//  1. lane = survivor: its record becomes the quadratics of N and D (PairForm) in shared memory; the masks are transposed;
+//  2. lane = pixel: walks its own candidates in order and leaves per pair what only the pixel knows - blending weight, dL/dG / opacity,
+//     rho^2, 1 / D - in a table, and a bit for every accepted pair;
+//  3. lane = (survivor, half of the pixels): walks the accepted pairs of its survivor and sums the moments in registers; the
+//     two halves are added and the record goes out with vector reductions.
+// The warp never reduces over pixels (which took 64 instructions per Gaussian and warp, whether one pixel or 32 contributed).
+constexpr int kGoChunk = 16;
+constexpr int kGoQueue = 64;
+template <bool ABS_GRAD>
+__global__ void __launch_bounds__(32) backward_global_kernel(
+    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, const float* __restrict__ grad_image, const float* __restrict__ image, const float* __restrict__ VPM,
-    float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w, bool abs_grad_on)
+    float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w)
 {
     using MT = ModeTraits<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING>;
-    __shared__ float4 s_T1[kGoBatch], s_T2[kGoBatch], s_T4[kGoBatch], s_rgba[kGoBatch], s_c0[kGoBatch];
-    __shared__ float s_cc[kGoBatch];
-    __shared__ uint32_t s_g[kGoBatch];
-    __shared__ float s_acc[kGoBatch * kGoAccStride];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t tile_x = blockIdx.x, tile_y = blockIdx.y;                 // in units of 8 pixels
-    const uint32_t px_i = tile_x * 8 + (tid & 7), py_i = tile_y * 8 + (tid >> 3);
+    constexpr uint32_t kTileX = MT::tile_w / 8, kTileY = MT::tile_h / 4;
+    __shared__ float4 s_pair[kGoChunk][33];              // [survivor][pixel]: weight, dL/dalpha * G, rho^2, 1 / D
+    __shared__ float4 s_n0[kGoChunk], s_n1[kGoChunk], s_d1[kGoChunk], s_rgba[kGoChunk], s_pos[kGoChunk];
+    __shared__ float4 s_grad[32];                        // dL/dpixel
+    __shared__ uint32_t s_g[kGoChunk], s_queue_prim[kGoQueue], s_queue_mask[kGoQueue];
+    const uint32_t lane = threadIdx.x;
+    const uint32_t tile = __ldg(tile_order + blockIdx.x / (kTileX * kTileY)), part = blockIdx.x % (kTileX * kTileY);
+    const uint32_t block_x = (tile % grid_w) * kTileX + part % kTileX, block_y = (tile / grid_w) * kTileY + part / kTileX;
+    if (block_x * 8 >= width || block_y * 4 >= height) return;
+    const uint32_t px_i = block_x * 8 + (lane & 7u), py_i = block_y * 4 + (lane >> 3);
     const bool inside = px_i < width && py_i < height;
-    const float pixel_x = __uint2float_rn(px_i), pixel_y = __uint2float_rn(py_i);
-    const float rect_x0 = float(tile_x * 8), rect_y0 = float(tile_y * 8 + warp * 4);
+    const float x0 = float(block_x * 8), y0 = float(block_y * 4);
+    const float local_x = float(lane & 7u), local_y = float(lane >> 3);
     const uint32_t n_pixels = width * height;
     float3 grad_pixel = make_float3(0, 0, 0), rgb_pixel = make_float3(0, 0, 0);
     if (inside) {
@@ -458,127 +504,154 @@ __global__ void __launch_bounds__(64) backward_global_kernel(
         grad_pixel = make_float3(__ldg(grad_image + pixel_idx), __ldg(grad_image + n_pixels + pixel_idx), __ldg(grad_image + 2 * n_pixels + pixel_idx));
         rgb_pixel = make_float3(__ldg(image + pixel_idx), __ldg(image + n_pixels + pixel_idx), __ldg(image + 2 * n_pixels + pixel_idx));
     }
-    const CameraCols cam = load_camera_cols(VPM);
+    s_grad[lane] = make_float4(grad_pixel.x, grad_pixel.y, grad_pixel.z, 0.0f);
+    [[maybe_unused]] CameraCols cam;
+    if constexpr (ABS_GRAD) cam = load_camera_cols(VPM);
     float3 rgb_pixel_new = make_float3(0, 0, 0);
     float transmittance = 1.0f;
     bool done = !inside;
-    constexpr uint32_t kSplit = MT::tile_w / 8;                               // 8-pixel CTAs per binning tile edge
-    const uint2 range = tile_ranges[(tile_y / kSplit) * grid_w + tile_x / kSplit];
-    const uint32_t out_index = transpose_reduce_index(lane);
-    for (uint32_t batch_begin = range.x; batch_begin < range.y; batch_begin += kGoBatch) {
-        if (__syncthreads_count(done) == 64) break;
-        const uint32_t batch = min(uint32_t(kGoBatch), range.y - batch_begin);
-        if (tid < batch) {
-            const uint32_t g = __ldg(prims_sorted + batch_begin + tid);
-            const float* rec = reinterpret_cast<const float*>(eval + g);
-            s_g[tid] = g;
-            s_T1[tid] = ldg4(rec); s_T2[tid] = ldg4(rec + 4); s_T4[tid] = ldg4(rec + 8); s_rgba[tid] = ldg4(rec + 16);
-            s_c0[tid] = ldg4(reinterpret_cast<const float*>(cull + g));
-            s_cc[tid] = __ldg(reinterpret_cast<const float*>(cull + g) + 4);
-        } else {
-            s_c0[tid] = make_float4(__int_as_float(0x7f800000), 0.0f, 0.0f, 0.0f);   // an outline nothing is inside of
-            s_cc[tid] = 0.0f;
+
+    const uint2 range = tile_ranges[tile];
+    uint32_t next = range.x + lane;
+    uint32_t g_here = 0, g_ahead = 0;
+    float4 outline = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float outline_c = 0.0f;
+    auto request_outline = [&](uint32_t g) {
+        outline = ldg4(reinterpret_cast<const float*>(cull + g));
+        outline_c = __ldg(reinterpret_cast<const float*>(cull + g) + 4);
+    };
+    if (next < range.y) { g_here = __ldg(prims_sorted + next); request_outline(g_here); }
+    if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
+    uint32_t queue_head = 0, queued = 0;
+    auto filter = [&]() {
+        uint32_t mask = 0;
+        if (next < range.y) mask = outline_mask(outline, outline_c, x0, y0);
+        const uint32_t survivors = __ballot_sync(0xffffffffu, mask != 0);
+        if (mask != 0) {
+            const uint32_t at = (queue_head + queued + __popc(survivors & lanemask_lt())) & uint32_t(kGoQueue - 1);
+            s_queue_prim[at] = g_here;
+            s_queue_mask[at] = mask;
         }
-        for (uint32_t i = tid; i < kGoBatch * kGoAccStride; i += 64) s_acc[i] = 0.0f;
-        __syncthreads();
-        // which staged Gaussians can touch this warp's 8x4 pixels (lane = Gaussian)
-        uint64_t todo = 0;
-        #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const float4 c0 = s_c0[half * 32 + lane];
-            const float cc = s_cc[half * 32 + lane];
-            const float dx0 = rect_x0 - c0.x, dy0 = rect_y0 - c0.y;
-            bool touches = false;
-            #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float dy = dy0 + float(r);
-                const float b2dy = c0.w * dy, cdy2 = cc * dy * dy;
-                #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float dx = dx0 + float(i);
-                    const float q = dx * (c0.z * dx + b2dy) + cdy2;
-                    touches |= q <= 1.0f;
-                }
-            }
-            todo |= uint64_t(__ballot_sync(0xffffffffu, touches)) << (32 * half);
+        queued += __popc(survivors);
+        next += 32;
+        g_here = g_ahead;
+        if (next < range.y) request_outline(g_here);
+        if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
+    };
+    // the record of the survivor this lane stages (both half warps hold the same 16)
+    const uint32_t mine = lane & uint32_t(kGoChunk - 1);
+    uint32_t g_mine = 0, mask_mine = 0, count = 0;
+    float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1, centre = rT1;
+    auto take = [&]() {                                  // the next chunk: indices, masks, and requests for its records
+        while (queued < kGoChunk && next - lane < range.y) filter();
+        __syncwarp();
+        count = min(queued, uint32_t(kGoChunk));
+        mask_mine = 0;
+        if (mine < count) {
+            const uint32_t at = (queue_head + mine) & uint32_t(kGoQueue - 1);
+            g_mine = s_queue_prim[at];
+            mask_mine = s_queue_mask[at];
+            const float* rec = reinterpret_cast<const float*>(eval + g_mine);
+            rT1 = ldg4(rec); rT2 = ldg4(rec + 4); rT4 = ldg4(rec + 8); rRGBA = ldg4(rec + 16);
+            centre = ldg4(reinterpret_cast<const float*>(cull + g_mine));
         }
-        while (todo != 0) {
-            if (__all_sync(0xffffffffu, done)) break;
-            const uint32_t j = uint32_t(__ffsll((long long)todo) - 1);
-            todo &= todo - 1;
-            float v[16];
-            #pragma unroll
-            for (int c = 0; c < 16; ++c) v[c] = 0.0f;
-            float v_abs = 0.0f;
-            bool contributes = false;
-            if (!done) {
-                const float4 T1 = s_T1[j], T2 = s_T2[j], T4 = s_T4[j];
-                const float4 plane_x_diag = T1 - T4 * pixel_x;
-                const float4 plane_y_diag = T2 - T4 * pixel_y;
-                const float3 nx = f3(plane_x_diag), ny = f3(plane_y_diag);
-                const float3 m = plane_x_diag.w * ny - nx * plane_y_diag.w;
-                const float3 d = cross(nx, ny);
-                const float numerator_rho2 = dot(m, m);
-                const float denominator = dot(d, d);
-                if (!(numerator_rho2 > MT::max_cutoff_sq * denominator)) {
-                    const float denominator_rcp = rcp_approx(denominator);
-                    const float G = exp_approx(-0.5f * numerator_rho2 * denominator_rcp);
-                    const float4 rgba = s_rgba[j];
-                    const float opacity = rgba.w;
-                    const float alpha = fminf(opacity * G, kMaxFragmentAlpha);
-                    if (!rejected_by_forward<MT>(alpha, opacity, numerator_rho2, denominator)) {
-                        const float blending_weight = transmittance * alpha;
-                        const float3 dL_drgb = blending_weight * grad_pixel;
-                        v[12] = dL_drgb.x; v[13] = dL_drgb.y; v[14] = dL_drgb.z;
-                        contributes = true;
-                        const float3 rgb = f3(rgba);
-                        rgb_pixel_new += blending_weight * rgb;
-                        const float one_minus_alpha = 1.0f - alpha;
-                        const float one_minus_alpha_rcp = rcp_approx(fmaxf(one_minus_alpha, kOneMinusAlphaEps));
-                        const float dL_dalpha = dot(transmittance * rgb - (rgb_pixel - rgb_pixel_new) * one_minus_alpha_rcp, grad_pixel);
-                        if (dL_dalpha != 0.0f) {
-                            v[15] = dL_dalpha * G;
-                            const float dL_dG = dL_dalpha * opacity;
-                            const float dL_drho2 = dL_dG * -0.5f * G;
-                            const PairGrad pg = pair_gradient(plane_x_diag, plane_y_diag, m, d, numerator_rho2, denominator_rcp, dL_drho2, pixel_x, pixel_y);
-                            v[0] = pg.dT1.x; v[1] = pg.dT1.y; v[2] = pg.dT1.z; v[3] = pg.dT1.w;
-                            v[4] = pg.dT2.x; v[5] = pg.dT2.y; v[6] = pg.dT2.z; v[7] = pg.dT2.w;
-                            v[8] = pg.dT4.x; v[9] = pg.dT4.y; v[10] = pg.dT4.z; v[11] = pg.dT4.w;
-                            if (abs_grad_on) {
-                                const float3 c4 = make_float3(pg.dT1.w, pg.dT2.w, pg.dT4.w);
-                                v_abs = fabsf(dot(cam.c1, c4)) + fabsf(dot(cam.c2, c4)) + fabsf(dot(cam.c3, c4));
-                            }
-                        }
-                        transmittance *= one_minus_alpha;
-                        if (transmittance < kTransmittanceThreshold) done = true;
-                    }
-                }
+        queue_head += count;
+        queued -= count;
+        __syncwarp();
+    };
+    take();
+    while (count != 0) {
+        const uint32_t g = g_mine;
+        // ---- 1. lane = survivor ------------------------------------------------------------------------------------
+        [[maybe_unused]] AbsForm af{};
+        float shear = 0.0f;
+        if (mine < count) {
+            const AffinePlanes planes = affine_planes(rT1, rT2, rT4, centre.x, centre.y);
+            if (lane < kGoChunk) {
+                const PairForm form = pair_form(planes);
+                s_n0[mine] = form.n0; s_n1[mine] = form.n1; s_d1[mine] = form.d1; s_rgba[mine] = rRGBA;
+                const float level = acceptance_level<MT>(rRGBA.w);
+                const float band = kLevelBand * level + 1e-6f;
+                s_pos[mine] = make_float4(x0 - centre.x, y0 - centre.y, level - band, planes.shear);
+                s_g[mine] = g;
             }
-            if (__any_sync(0xffffffffu, contributes)) {
-                const float total = transpose_reduce16(v, lane);
-                if ((lane & 1u) == 0 && total != 0.0f) atomicAdd(&s_acc[j * kGoAccStride + out_index], total);
-                if (abs_grad_on) {
-                    #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v_abs += __shfl_xor_sync(0xffffffffu, v_abs, o);
-                    if (lane == 0 && v_abs != 0.0f) atomicAdd(&s_acc[j * kGoAccStride + 16], v_abs);
-                }
-            }
+            shear = planes.shear;
+            if constexpr (ABS_GRAD) af = abs_form(planes, rT4);
         }
-        __syncthreads();
-        if (tid < batch) {
-            const float* a = s_acc + tid * kGoAccStride;
-            bool any = false;
-            #pragma unroll
-            for (int c = 0; c < 17; ++c) any |= a[c] != 0.0f;
-            if (any) {
-                float4* rec = accum + size_t(s_g[tid]) * 5;
-                red_add_v4(rec, make_float4(a[0], a[1], a[2], a[3]));
-                red_add_v4(rec + 1, make_float4(a[4], a[5], a[6], a[7]));
-                red_add_v4(rec + 2, make_float4(a[8], a[9], a[10], a[11]));
-                red_add_v4(rec + 3, make_float4(a[12], a[13], a[14], a[15]));
-                if (abs_grad_on) red_add_v4(rec + 4, make_float4(a[16], 0.0f, 0.0f, 0.0f));
+        const float opacity = rRGBA.w;
+        const float offset_x = x0 - centre.x, offset_y = y0 - centre.y;
+        uint32_t candidates = transpose_masks(lane < kGoChunk ? mask_mine : 0u, lane);      // bit 15 - i: survivor i
+        if (done) candidates = 0;
+        __syncwarp();
+        take();                                          // the records of the next chunk fly while this one is worked on
+        // ---- 2. lane = pixel ------------------------------------------------------------------------------------------
+        uint32_t accepted = 0;
+        while (__any_sync(0xffffffffu, candidates != 0)) {
+            const bool valid = candidates != 0;
+            const uint32_t bit = uint32_t(31 - __clz(int(candidates | 1u)));
+            candidates &= ~(1u << bit);
+            const uint32_t j = uint32_t(kGoChunk - 1) - bit;
+            const float4 pos = s_pos[j];
+            const float y = pos.y + local_y, s = fmaf(pos.w, y, pos.x + local_x);
+            float numerator_rho2, denominator;
+            evaluate_pair(PairForm{s_n0[j], s_n1[j], s_d1[j]}, s, y, numerator_rho2, denominator);
+            const float denominator_rcp = rcp_approx(denominator);
+            const float rho2 = numerator_rho2 * denominator_rcp;
+            bool ok = valid && rho2 < pos.z;
+            if (valid && !ok && !(rho2 > upper_level(pos.z))) ok = accepted_by_forward<MT>(eval + s_g[j], x0 + local_x, y0 + local_y);
+            if (ok) {
+                const float4 rgba = s_rgba[j];
+                const float G = exp_approx(-0.5f * rho2);
+                const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
+                const float blending_weight = transmittance * alpha;
+                const float3 rgb = f3(rgba);
+                rgb_pixel_new += blending_weight * rgb;
+                const float one_minus_alpha = 1.0f - alpha;
+                const float one_minus_alpha_rcp = rcp_approx(fmaxf(one_minus_alpha, kOneMinusAlphaEps));
+                const float dL_dalpha = dot(transmittance * rgb - (rgb_pixel - rgb_pixel_new) * one_minus_alpha_rcp, grad_pixel);
+                s_pair[j][lane] = make_float4(blending_weight, dL_dalpha * G, rho2, denominator_rcp);
+                accepted |= 1u << bit;
+                transmittance *= one_minus_alpha;
+                if (transmittance < kTransmittanceThreshold) { done = true; candidates = 0; }
             }
         }
+        // ---- 3. lane = (survivor, half of the pixels) -----------------------------------------------------------------------
+        // transposing back: bit 15 - i of lane p -> bit p of survivor i, this lane's 16 pixels in the low bits
+        uint32_t pixels = transpose_half(accepted, lane);
+        __syncwarp();
+        PairMoments moments{};
+        float4 aC = make_float4(0, 0, 0, 0);
+        [[maybe_unused]] float abs_grad = 0.0f;
+        const uint32_t first_pixel = lane & 16u;
+        while (__any_sync(0xffffffffu, pixels != 0)) {
+            if (pixels != 0) {
+                const uint32_t p = first_pixel + uint32_t(__ffs(int(pixels)) - 1);
+                pixels &= pixels - 1;
+                const float4 pair = s_pair[mine][p];
+                const float4 grad = s_grad[p];
+                const float y = offset_y + float(p >> 3), s = fmaf(shear, y, offset_x + float(p & 7u));
+                aC.x = fmaf(pair.x, grad.x, aC.x); aC.y = fmaf(pair.x, grad.y, aC.y); aC.z = fmaf(pair.x, grad.z, aC.z);
+                aC.w += pair.y;
+                const float u = -0.5f * opacity * pair.y * pair.w;
+                add_moments(moments, u, u * pair.z, s, y);
+                if constexpr (ABS_GRAD) abs_grad += abs_position_gradient(af, u, s, y, x0 + float(p & 7u), y0 + float(p >> 3), cam);
+            }
+        }
+        auto both_halves = [](float4& v) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, 16); v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+            v.z += __shfl_xor_sync(0xffffffffu, v.z, 16); v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
+        };
+        both_halves(moments.u0); both_halves(moments.u1); both_halves(moments.v1); both_halves(aC);
+        if constexpr (ABS_GRAD) abs_grad += __shfl_xor_sync(0xffffffffu, abs_grad, 16);
+        const uint32_t any = __ballot_sync(0xffffffffu, aC.x != 0.0f || aC.y != 0.0f || aC.z != 0.0f || aC.w != 0.0f);
+        if ((any >> lane) & 1u) {                        // the two half warps share the four or five reductions of a record
+            float4* rec = accum + size_t(g) * 5;
+            if (lane < kGoChunk) { red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); }
+            else { red_add_v4(rec + 2, moments.v1); red_add_v4(rec + 3, aC); }
+            if constexpr (ABS_GRAD) { if (lane < kGoChunk) red_add_v4(rec + 4, make_float4(abs_grad, 0.0f, 0.0f, 0.0f)); }
+        }
+        if (__all_sync(0xffffffffu, done)) break;
+        __syncwarp();
     }
 }
 
@@ -608,7 +681,8 @@ template <bool COMPACT>
 __global__ void __launch_bounds__(256) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ scales, const float* __restrict__ rotations, const float* __restrict__ sh_rest,
     const float* __restrict__ M, const float* __restrict__ VPM, const float* __restrict__ cam_position_ptr,
-    const uint32_t* __restrict__ n_touched, const uint8_t* __restrict__ clamp, const float4* __restrict__ accum, BackwardOutputs out,
+    const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const CullRecord* __restrict__ cull, const uint8_t* __restrict__ clamp,
+    const float4* __restrict__ accum, BackwardOutputs out,
     uint32_t n_primitives, int active_sh_bases, int total_sh_bases, uint32_t g_first, uint32_t g_end)
 {
     const uint32_t idx = g_first + blockIdx.x * 256 + threadIdx.x;
@@ -625,10 +699,18 @@ __global__ void __launch_bounds__(256) preprocess_backward_kernel(
     float4 grad_rotation = make_float4(0, 0, 0, 0);
     float grad_opacity = 0.0f;
     if (kept) {
-    const float4 dT1 = accum[size_t(idx) * 5], dT2 = accum[size_t(idx) * 5 + 1], dT4 = accum[size_t(idx) * 5 + 2], dC = accum[size_t(idx) * 5 + 3];
+    const PairMoments moments{accum[size_t(idx) * 5], accum[size_t(idx) * 5 + 1], accum[size_t(idx) * 5 + 2]};
+    const float4 dC = accum[size_t(idx) * 5 + 3];
+    const float4 T4 = ldg4(reinterpret_cast<const float*>(eval + idx) + 8);
+    float2 centre = __ldg(reinterpret_cast<const float2*>(cull + idx));
+    if (!(fabsf(centre.x) <= FLT_MAX)) centre = make_float2(0.0f, 0.0f);       // nothing of the Gaussian can be accepted: its moments are zero
+    const RowGradients rows = rows_from_moments(affine_planes(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
+                                                              centre.x, centre.y), T4, moments);
+    // dL/dVPMT4 = -(cx dL/dVPMT1 + cy dL/dVPMT2 + E): the products with the centre are moved to the rows of VPM, where they cancel
+    const float4 dT1 = rows.dX, dT2 = rows.dY, dT4 = make_float4(-rows.E.x, -rows.E.y, -rows.E.z, -rows.E.w);
     const float3 c1 = make_float3(dT1.x, dT2.x, dT4.x), c2 = make_float3(dT1.y, dT2.y, dT4.y), c3 = make_float3(dT1.z, dT2.z, dT4.z);
     const float3 c4 = make_float3(dT1.w, dT2.w, dT4.w);
-    const float4 r1 = ldg4(VPM), r2 = ldg4(VPM + 4), r4 = ldg4(VPM + 12);
+    const float4 r4 = ldg4(VPM + 12), r1 = ldg4(VPM) - centre.x * r4, r2 = ldg4(VPM + 4) - centre.y * r4;
     const float3 VPM1 = f3(r1), VPM2 = f3(r2), VPM4 = f3(r4);
     const float3 VPM_c1 = make_float3(r1.x, r2.x, r4.x), VPM_c2 = make_float3(r1.y, r2.y, r4.y), VPM_c3 = make_float3(r1.z, r2.z, r4.z);
 
@@ -738,36 +820,34 @@ __global__ void __launch_bounds__(256) preprocess_backward_kernel(
 }
 
 template <int MODE, int K>
-cudaError_t launch_tile_backward(bool abs_grad, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
+cudaError_t launch_tile_backward(bool abs_grad, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
                                  const TrainPixelBuffers& tin, const float* grad_image, const float* VPM, float4* accum, uint32_t g_first, uint32_t g_end,
                                  cudaStream_t stream) {
-    using SM = BwdSmem<MODE, K>;
-    const dim3 grid(geo.grid_w, geo.grid_h, 1);
-    auto launch = [&](auto kernel) -> cudaError_t {
+    auto launch = [&](auto kernel, size_t smem) -> cudaError_t {
         // both instantiations have the same function-pointer type, so this lambda (and a static in it) is shared by them
         static PerDeviceOnce configured[2];
-        if (SM::total > 48 * 1024) {
-            const cudaError_t err = configured[abs_grad ? 1 : 0].run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SM::total)); });
+        if (smem > 48 * 1024) {
+            const cudaError_t err = configured[abs_grad ? 1 : 0].run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); });
             if (err != cudaSuccess) return err;
         }
-        kernel<<<grid, kBwdThreads, SM::total, stream>>>(tile_ranges, prims_sorted, prim.eval, prim.cull, tin, grad_image, VPM, accum,
+        kernel<<<uint32_t(geo.n_tiles), kBwdThreads, smem, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, tin, grad_image, VPM, accum,
                                                 uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w), g_first, g_end);
         return cudaGetLastError();
     };
-    return abs_grad ? launch(backward_tile_kernel<MODE, K, true>) : launch(backward_tile_kernel<MODE, K, false>);
+    return abs_grad ? launch(backward_tile_kernel<MODE, K, true>, BwdSmem<MODE, K, true>::total) : launch(backward_tile_kernel<MODE, K, false>, BwdSmem<MODE, K, false>::total);
 }
 
 template <int MODE>
 cudaError_t launch_tile_backward_k(int K, bool abs_grad, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted,
-                                   const uint2* tile_ranges, const TrainPixelBuffers& tin, const float* grad_image, const float* VPM, float4* accum,
+                                   const uint2* tile_ranges, const uint32_t* tile_order, const TrainPixelBuffers& tin, const float* grad_image, const float* VPM, float4* accum,
                                    uint32_t g_first, uint32_t g_end, cudaStream_t stream) {
     switch (K) {
-        case 32: return launch_tile_backward<MODE, 32>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, VPM, accum, g_first, g_end, stream);
-        case 16: return launch_tile_backward<MODE, 16>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, VPM, accum, g_first, g_end, stream);
-        case 8: return launch_tile_backward<MODE, 8>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, VPM, accum, g_first, g_end, stream);
-        case 4: return launch_tile_backward<MODE, 4>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, VPM, accum, g_first, g_end, stream);
-        case 2: return launch_tile_backward<MODE, 2>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, VPM, accum, g_first, g_end, stream);
-        default: return launch_tile_backward<MODE, 1>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, VPM, accum, g_first, g_end, stream);
+        case 32: return launch_tile_backward<MODE, 32>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, VPM, accum, g_first, g_end, stream);
+        case 16: return launch_tile_backward<MODE, 16>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, VPM, accum, g_first, g_end, stream);
+        case 8: return launch_tile_backward<MODE, 8>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, VPM, accum, g_first, g_end, stream);
+        case 4: return launch_tile_backward<MODE, 4>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, VPM, accum, g_first, g_end, stream);
+        case 2: return launch_tile_backward<MODE, 2>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, VPM, accum, g_first, g_end, stream);
+        default: return launch_tile_backward<MODE, 1>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, VPM, accum, g_first, g_end, stream);
     }
 }
 
@@ -806,11 +886,11 @@ cudaError_t launch_chain_rule(const HtgsScene& scene, const HtgsView& view, cons
         const cudaError_t err = cudaMemsetAsync(out.compact_rows, 0, sizeof(CompactGradientHeader), stream);
         if (err != cudaSuccess) return err;
         preprocess_backward_kernel<true><<<(count + 255) / 256, 256, 0, stream>>>(scene.positions, scene.scales, scene.rotations, scene.sh_rest, view.M, view.VPM,
-                                                                                  view.cam_position, prim.n_touched, prim.clamp, acc.accum, out, n,
+                                                                                  view.cam_position, prim.n_touched, prim.eval, prim.cull, prim.clamp, acc.accum, out, n,
                                                                                   view.active_sh_bases, scene.total_sh_bases, first, first + count);
     } else {
         preprocess_backward_kernel<false><<<(count + 255) / 256, 256, 0, stream>>>(scene.positions, scene.scales, scene.rotations, scene.sh_rest, view.M, view.VPM,
-                                                                                   view.cam_position, prim.n_touched, prim.clamp, acc.accum, out, n,
+                                                                                   view.cam_position, prim.n_touched, prim.eval, prim.cull, prim.clamp, acc.accum, out, n,
                                                                                    view.active_sh_bases, scene.total_sh_bases, first, first + count);
     }
     return cudaGetLastError();
@@ -818,7 +898,7 @@ cudaError_t launch_chain_rule(const HtgsScene& scene, const HtgsView& view, cons
 }  // namespace
 
 cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim,
-                            const uint32_t* prims_sorted, const uint2* tile_ranges, const TrainPixelBuffers& tin, const float* grad_image,
+                            const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order, const TrainPixelBuffers& tin, const float* grad_image,
                             const float* image, const GradAccumBuffers& acc, const BackwardOutputs& out, cudaEvent_t outputs_cleared, int sm_count,
                             uint32_t first, uint32_t count, int stages, cudaStream_t stream) {
     (void)sm_count;
@@ -841,15 +921,15 @@ cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsV
     const int k = effective_k(mode, K);
     switch (mode) {
         case HTGS_MODE_HYBRID_BLEND:
-            err = launch_tile_backward_k<HTGS_MODE_HYBRID_BLEND>(k, abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
+            err = launch_tile_backward_k<HTGS_MODE_HYBRID_BLEND>(k, abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
         case HTGS_MODE_ALPHA_BLEND_FIRST_K:
-            err = launch_tile_backward_k<HTGS_MODE_ALPHA_BLEND_FIRST_K>(k, abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
+            err = launch_tile_backward_k<HTGS_MODE_ALPHA_BLEND_FIRST_K>(k, abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
         case HTGS_MODE_OIT_BLEND:
-            err = launch_tile_backward<HTGS_MODE_OIT_BLEND, 1>(abs_grad, geo, prim, prims_sorted, tile_ranges, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
+            err = launch_tile_backward<HTGS_MODE_OIT_BLEND, 1>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
         case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: {
-            const dim3 grid((geo.width + 7) / 8, (geo.height + 7) / 8, 1);
-            backward_global_kernel<<<grid, 64, 0, stream>>>(tile_ranges, prims_sorted, prim.eval, prim.cull, grad_image, image, view.VPM, acc.accum,
-                                                             uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w), abs_grad);
+            const auto kernel = abs_grad ? backward_global_kernel<true> : backward_global_kernel<false>;
+            kernel<<<uint32_t(geo.n_tiles) * 8u, 32, 0, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, grad_image, image, view.VPM, acc.accum,
+                                                                  uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w));
             err = cudaGetLastError();
             break;
         }
