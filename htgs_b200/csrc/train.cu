@@ -160,8 +160,9 @@ __device__ __forceinline__ float abs_position_gradient(const AbsForm& f, float u
     return fabsf(dot(cam.c1, c4)) + fabsf(dot(cam.c2, c4)) + fabsf(dot(cam.c3, c4));
 }
 
-constexpr int kBwdThreads = 128;       // threads per tile: one staged instance each, and an even share of the batch's pairs
-constexpr int kBwdThreadsLog2 = 7;
+constexpr int kBwdThreads = 128;       // threads per tile: one staged instance each
+constexpr int kBwdSegments = 4 * kBwdThreads;      // of a batch, at most
+constexpr int kBwdCoreRow = 68;        // bytes per staged instance: 64 pixels, and an odd number of words against bank conflicts
 template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr bool has_core = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
     static constexpr bool has_tail = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_OIT_BLEND);
@@ -172,11 +173,12 @@ template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr size_t ta_off = tc_off + tc_bytes;
     static constexpr size_t ta_bytes = has_tail ? 64 * 4 : 0;
     static constexpr size_t stage_off = (ta_off + ta_bytes + 15) & ~size_t(15);
-    static constexpr size_t stage_bytes = kBwdThreads * ((ABS_GRAD ? 8 : 5) * 16 + 8 + 4) + (kBwdThreads + 1) * 4 + 12;
-    static constexpr size_t core_off = (stage_off + stage_bytes + 15) & ~size_t(15);     // [NT][64] core entry of each (staged instance, pixel) pair
-    static constexpr size_t core_bytes = has_core ? size_t(kBwdThreads) * 64 : 0;
+    static constexpr size_t stage_bytes = kBwdThreads * ((ABS_GRAD ? 8 : 5) * 16 + 4 + (MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K ? 8 : 0)) + kBwdSegments * (4 + 1);
+    static constexpr size_t core_off = (stage_off + stage_bytes + 15) & ~size_t(15);     // [NT][kBwdCoreRow] core entry of each (staged instance, pixel) pair
+    static constexpr size_t core_bytes = has_core ? size_t(kBwdThreads) * kBwdCoreRow : 0;
     static constexpr size_t total = core_off + core_bytes;
-    static constexpr int min_blocks = int((227 * 1024) / (total + 1024)) < 5 ? int((227 * 1024) / (total + 1024)) : 5;   // what the register budget is held to
+    static constexpr int max_blocks = has_core || ABS_GRAD ? 4 : 5;      // five spill the pair loop of the modes with a buffer (1415 against 1366 us)
+    static constexpr int min_blocks = int((227 * 1024) / (total + 1024)) < max_blocks ? int((227 * 1024) / (total + 1024)) : max_blocks;   // what the register budget is held to
 };
 
 // HYBRID_BLEND / ALPHA_BLEND_FIRST_K / OIT_BLEND: one CTA per 8x8 tile (long lists first), one thread per Gaussian of a batch of kBwdThreads.
@@ -263,17 +265,23 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             grad_pixel = make_float3(__ldg(grad_image + pixel_idx), __ldg(grad_image + n_pixels + pixel_idx), __ldg(grad_image + 2 * n_pixels + pixel_idx));
         }
         if constexpr (SM::has_core) {
+            // All loads of a group are in flight together; entries that do not exist are read (their slots do) and dropped.
+            constexpr int kShare = (K + int(kParts) - 1) / int(kParts), kGroup = kShare < 8 ? kShare : 8;
             #pragma unroll
-            for (int i = 0; i < int((K + kParts - 1) / kParts); ++i) {
-                const int k = i * int(kParts) + int(part);
-                core_pos[i] = 0xffffffffu;
-                if (k < K && inside) {
-                    core_pos[i] = tin.idx_core[k * PP + slot];
-                    if (core_pos[i] != 0xffffffffu) {
-                        const float4 info = tin.info_core[k * PP + slot];
-                        const float3 drgb = info.w * grad_pixel;
-                        s_cg[k * 64 + pix] = make_float4(drgb.x, drgb.y, drgb.z, dot(f3(info), grad_pixel));
-                    }
+            for (int i0 = 0; i0 < kShare; i0 += kGroup) {
+                float4 info[kGroup];
+                #pragma unroll
+                for (int i = 0; i < kGroup; ++i) {
+                    const int k = min((i0 + i) * int(kParts) + int(part), K - 1);
+                    core_pos[i0 + i] = __ldg(tin.idx_core + k * PP + slot);
+                    info[i] = __ldg(tin.info_core + k * PP + slot);
+                }
+                #pragma unroll
+                for (int i = 0; i < kGroup; ++i) {
+                    const int k = (i0 + i) * int(kParts) + int(part);
+                    if (k >= K || !inside) core_pos[i0 + i] = 0xffffffffu;
+                    const float3 drgb = info[i].w * grad_pixel;
+                    if (k < K) s_cg[k * 64 + pix] = make_float4(drgb.x, drgb.y, drgb.z, dot(f3(info[i]), grad_pixel));
                 }
             }
         }
@@ -305,17 +313,20 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     request_outline(range.x + NT + tid);
     g_idx = load_index(range.x + 2 * NT + tid);
 
-    // ---- batches of NT instances; the (Gaussian, pixel) candidate pairs of a batch are split EVENLY over the
-    //      NT threads (pairs of one Gaussian are contiguous, so a thread walks a few Gaussians back to back)
+    // ---- batches of NT instances.  A Gaussian's pixels are cut into segments of at most 16 (two rows; four rows if they hold no
+    //      more); a lane takes one segment, sums its record in registers and adds it to the Gaussian's.  All lanes of a warp change
+    //      Gaussians at the same time: with the pairs split evenly over the lanes instead, some lane changed in almost every step,
+    //      and the warp spent a third of its instructions on that (1450 -> SEG_US us at 3 M Gaussians, 1297 x 840, K = 16).
     float4* s_n0 = reinterpret_cast<float4*>(smem + SM::stage_off);
     float4* s_n1 = s_n0 + NT;
     float4* s_d1 = s_n1 + NT;
     float4* s_rgba = s_d1 + NT;
     float4* s_pos = s_rgba + NT;         // tile origin - centre, rho^2 below which a fragment is certainly accepted, shear
     [[maybe_unused]] float4* s_abs = s_pos + NT;    // ABS_GRAD: [3][NT]
-    unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(s_pos + NT * (ABS_GRAD ? 4 : 1));
-    uint32_t* s_g = reinterpret_cast<uint32_t*>(s_mask + NT);
-    uint32_t* s_off = s_g + NT;          // [NT + 1] exclusive prefix of the per-Gaussian pair counts
+    [[maybe_unused]] unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(s_pos + NT * (ABS_GRAD ? 4 : 1));      // FIRST_K
+    uint32_t* s_g = reinterpret_cast<uint32_t*>(s_mask + (kFirstK ? NT : 0));
+    uint32_t* s_segment = s_g + NT;      // pixels of a segment, 32 of the tile's 64
+    unsigned char* s_owner = reinterpret_cast<unsigned char*>(s_segment + kBwdSegments);      // staged instance * 2 + which 32 pixels
     __shared__ uint32_t s_warp_total[NT / 32];
     const uint32_t lane = tid & 31, warp = tid >> 5;
     // The training forward saved, per pixel and core entry, the POSITION of the entry's Gaussian in the tile's list, so the
@@ -328,7 +339,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         for (int i = 0; i < int((K + kParts - 1) / kParts); ++i) {
             const uint32_t j = core_pos[i] - batch_pos;
             if (j < limit) {
-                s_core[j * 64 + pix] = (signed char)(i * int(kParts) + int(part));
+                s_core[j * kBwdCoreRow + pix] = (signed char)(i * int(kParts) + int(part));
                 if constexpr (kFirstK) atomicOr(reinterpret_cast<uint32_t*>(s_mask + j) + (pix >> 5), 1u << (pix & 31));
             }
         }
@@ -351,9 +362,9 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             }
             s_g[tid] = g_rec;
             if constexpr (SM::has_core) {      // no pair of my instance is a core entry until the scatter below says so
-                uint4* row = reinterpret_cast<uint4*>(s_core + tid * 64);
-                const uint4 none = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-                row[0] = none; row[1] = none; row[2] = none; row[3] = none;
+                uint32_t* row = reinterpret_cast<uint32_t*>(s_core + tid * kBwdCoreRow);
+                #pragma unroll
+                for (int i = 0; i < 16; ++i) row[i] = 0xffffffffu;
             }
         }
         request_record(inst + NT);
@@ -366,102 +377,100 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             scatter_core_entries(batch_begin - tile_range.x, min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
             __syncthreads();
             my_mask = s_mask[tid];
-        } else {
-            s_mask[tid] = my_mask;
         }
-        const uint32_t cnt = __popcll(my_mask);
+        // segments with more than 8 pixels come first, so that the lanes of a warp have about equally many steps
+        const uint32_t halves[2] = {uint32_t(my_mask), uint32_t(my_mask >> 32)};
+        uint32_t segments[4], cnt = 0;                   // low half word: long segments, high half word: short ones
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bool split = __popc(halves[h]) > 16;
+            segments[2 * h] = split ? halves[h] & 0xffffu : halves[h];
+            segments[2 * h + 1] = split ? halves[h] & 0xffff0000u : 0u;
+        }
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) cnt += segments[i] == 0 ? 0u : __popc(segments[i]) > 8 ? 1u : 0x10000u;
         uint32_t inc = cnt;
         #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= uint32_t(o)) inc += t; }
         if (lane == 31) s_warp_total[warp] = inc;
         __syncthreads();
-        uint32_t excl = inc - cnt, total_pairs = 0;
+        uint32_t at = inc - cnt, total = 0;
         #pragma unroll
         for (uint32_t w = 0; w < NT / 32; ++w) {
             const uint32_t t = s_warp_total[w];
-            if (w < warp) excl += t;
-            total_pairs += t;
+            if (w < warp) at += t;
+            total += t;
         }
-        s_off[tid] = excl;
-        if (tid == 0) s_off[NT] = total_pairs;
+        const uint32_t n_long = total & 0xffffu, n_segments = n_long + (total >> 16);
+        uint32_t at_long = at & 0xffffu, at_short = n_long + (at >> 16);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (segments[i] == 0) continue;
+            const uint32_t slot_at = __popc(segments[i]) > 8 ? at_long++ : at_short++;
+            s_segment[slot_at] = segments[i];
+            s_owner[slot_at] = (unsigned char)(2 * tid + i / 2);
+        }
         if constexpr (SM::has_core && !kFirstK) scatter_core_entries(batch_begin - tile_range.x, min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
         __syncthreads();
-        if (total_pairs == 0) continue;
-        // my share of the pairs
-        const uint32_t lo = uint32_t((uint64_t(tid) * total_pairs) >> kBwdThreadsLog2), hi = uint32_t((uint64_t(tid + 1) * total_pairs) >> kBwdThreadsLog2);
-        uint32_t remaining = hi - lo;
-        if (remaining == 0) continue;
-        uint32_t j = 0;
-        {
-            uint32_t a = 0, b = NT;      // last j with s_off[j] <= lo
-            #pragma unroll
-            for (int it = 0; it < kBwdThreadsLog2; ++it) { const uint32_t mid = (a + b) >> 1; if (s_off[mid] <= lo) a = mid; else b = mid; }
-            j = a;
-        }
-        uint64_t mask = s_mask[j];
-        for (uint32_t skip = lo - s_off[j]; skip > 0; --skip) mask &= mask - 1;     // drop the pairs that belong to the previous thread
-        PairForm form{s_n0[j], s_n1[j], s_d1[j]};
-        float4 rgba = s_rgba[j], pos = s_pos[j];
-        PairMoments moments{};
-        float4 aC = make_float4(0, 0, 0, 0);            // (dL/drgb, dL/dopacity)
-        [[maybe_unused]] float abs_grad = 0.0f;
-        bool touched = false;
-        auto flush = [&]() {
+        for (uint32_t first = warp * 32; first < n_segments; first += NT) {
+            if (first + lane >= n_segments) continue;
+            uint32_t pixels = s_segment[first + lane];
+            const uint32_t owner = s_owner[first + lane], j = owner >> 1;
+            const float row0 = float((owner & 1u) * 4u);
+            const PairForm form{s_n0[j], s_n1[j], s_d1[j]};
+            const float4 rgba = s_rgba[j], pos = s_pos[j];
+            PairMoments moments{};
+            float4 aC = make_float4(0, 0, 0, 0);            // (dL/drgb, dL/dopacity)
+            [[maybe_unused]] float abs_grad = 0.0f;
+            bool touched = false;
+            while (pixels != 0) {
+                const uint32_t bit = uint32_t(__ffs(int(pixels)) - 1);
+                const uint32_t p = bit + (owner & 1u) * 32u;
+                pixels &= pixels - 1;
+                const float column = float(bit & 7u), row = row0 + float(bit >> 3);
+                const float y = pos.y + row, s = fmaf(pos.w, y, pos.x + column);
+                float numerator_rho2, denominator;
+                evaluate_pair(form, s, y, numerator_rho2, denominator);
+                int core_idx = -1;
+                if constexpr (SM::has_core) core_idx = s_core[j * kBwdCoreRow + p];
+                const float denominator_rcp = rcp_approx(denominator);
+                const float rho2 = numerator_rho2 * denominator_rcp;
+                if constexpr (kFirstK) {
+                    if (core_idx < 0) continue;                    // only stored fragments carry gradient (first_k backward.cuh:84-87)
+                } else if (!(rho2 < pos.z)) {
+                    if (rho2 > upper_level(pos.z) || !accepted_by_forward<MT>(eval + s_g[j], x0 + column, y0 + row)) continue;
+                }
+                const float G = exp_approx(-0.5f * rho2);
+                const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
+                float3 dL_drgb;
+                float dL_dalpha;
+                if (core_idx >= 0) {
+                    const float4 cg = s_cg[core_idx * 64 + p];
+                    dL_drgb = f3(cg);
+                    dL_dalpha = cg.w;
+                } else {
+                    if constexpr (SM::has_tail) {
+                        const float4 tc = s_tc[p];
+                        dL_drgb = f3(tc) * alpha;
+                        dL_dalpha = tc.w + dot(f3(rgba), f3(tc)) + s_ta[p] * rcp_approx(fmaxf(1.0f - alpha, kOneMinusAlphaEps));
+                    } else {
+                        continue;
+                    }
+                }
+                aC.x += dL_drgb.x; aC.y += dL_drgb.y; aC.z += dL_drgb.z;
+                aC.w += dL_dalpha * G;
+                touched = true;
+                const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D
+                add_moments(moments, u, u * rho2, s, y);
+                if constexpr (ABS_GRAD)
+                    abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + column, y0 + row, cam);
+            }
             if (touched) {
                 float4* rec = accum + size_t(s_g[j]) * 5;
                 red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); red_add_v4(rec + 2, moments.v1); red_add_v4(rec + 3, aC);
                 if constexpr (ABS_GRAD) red_add_v4(rec + 4, make_float4(abs_grad, 0.0f, 0.0f, 0.0f));
             }
-            moments = PairMoments{}; aC = make_float4(0, 0, 0, 0); abs_grad = 0.0f; touched = false;
-        };
-        for (; remaining > 0; --remaining) {
-            if (mask == 0) {              // next Gaussian of my share (its mask is non-empty somewhere before `hi`)
-                flush();
-                do mask = s_mask[++j]; while (mask == 0);
-                form = PairForm{s_n0[j], s_n1[j], s_d1[j]};
-                rgba = s_rgba[j]; pos = s_pos[j];
-            }
-            const uint32_t p = uint32_t(__ffsll((long long)mask) - 1);
-            mask &= mask - 1;
-            const float y = pos.y + float(p >> 3), s = fmaf(pos.w, y, pos.x + float(p & 7));
-            float numerator_rho2, denominator;
-            evaluate_pair(form, s, y, numerator_rho2, denominator);
-            int core_idx = -1;
-            if constexpr (SM::has_core) core_idx = s_core[j * 64 + p];
-            const float denominator_rcp = rcp_approx(denominator);
-            const float rho2 = numerator_rho2 * denominator_rcp;
-            if constexpr (kFirstK) {
-                if (core_idx < 0) continue;                    // only stored fragments carry gradient (first_k backward.cuh:84-87)
-            } else if (!(rho2 < pos.z)) {
-                if (rho2 > upper_level(pos.z) || !accepted_by_forward<MT>(eval + s_g[j], x0 + float(p & 7), y0 + float(p >> 3))) continue;
-            }
-            const float G = exp_approx(-0.5f * rho2);
-            const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
-            float3 dL_drgb;
-            float dL_dalpha;
-            if (core_idx >= 0) {
-                const float4 cg = s_cg[core_idx * 64 + p];
-                dL_drgb = f3(cg);
-                dL_dalpha = cg.w;
-            } else {
-                if constexpr (SM::has_tail) {
-                    const float4 tc = s_tc[p];
-                    dL_drgb = f3(tc) * alpha;
-                    dL_dalpha = tc.w + dot(f3(rgba), f3(tc)) + s_ta[p] * rcp_approx(fmaxf(1.0f - alpha, kOneMinusAlphaEps));
-                } else {
-                    continue;
-                }
-            }
-            aC.x += dL_drgb.x; aC.y += dL_drgb.y; aC.z += dL_drgb.z;
-            aC.w += dL_dalpha * G;
-            touched = true;
-            const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D
-            add_moments(moments, u, u * rho2, s, y);
-            if constexpr (ABS_GRAD) {
-                abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + float(p & 7), y0 + float(p >> 3), cam);
-            }
         }
-        flush();
     }
 }
 
