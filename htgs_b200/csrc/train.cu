@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     // ---- batches of NT instances.  A Gaussian's pixels are cut into segments of at most 16 (two rows; four rows if they hold no
     //      more); a lane takes one segment, sums its record in registers and adds it to the Gaussian's.  All lanes of a warp change
     //      Gaussians at the same time: with the pairs split evenly over the lanes instead, some lane changed in almost every step,
-    //      and the warp spent a third of its instructions on that (1450 -> SEG_US us at 3 M Gaussians, 1297 x 840, K = 16).
+    //      and the warp spent a third of its instructions on that (1450 -> 1290 us at 3 M Gaussians, 1297 x 840, K = 16).
     float4* s_n0 = reinterpret_cast<float4*>(smem + SM::stage_off);
     float4* s_n1 = s_n0 + NT;
     float4* s_d1 = s_n1 + NT;

@@ -84,3 +84,34 @@ def test_all_views_in_one_pass_equals_the_loop(n_views):
         for v in range(n_views):
             ref.update_3d_filter(pos_t, torch.from_numpy(w2cs[v]).cuda(), ref_f, ref_m, widths[v], heights[v], fxs[v], fys[v], cxs[v], cys[v], nears[v], 0.15, 0.0007)
         assert torch.equal(one_f, ref_f) and torch.equal(one_m, ref_m.reshape(-1))
+
+
+@pytest.mark.parametrize("n", [1, 511, 1537, 700_001])
+@pytest.mark.parametrize("n_views", [49, 257])
+def test_views_with_points_on_frustum_planes_and_without_a_number(n, n_views):
+    """Tile edges of the one-pass kernel; points on the planes of a frustum, infinite and NaN points, and a view without an area."""
+    import torch
+    tb = harness.ours()
+    rng = np.random.default_rng(n + n_views)
+    positions = (rng.standard_normal((n, 3)) * 3.0).astype(np.float32)
+    w2cs = np.stack([scenes.look_at((4.0 * np.cos(a), 1.5, 4.0 * np.sin(a))).astype(np.float32) for a in np.linspace(0, 2 * np.pi, n_views, endpoint=False)])
+    w2cs[1] = np.eye(4)
+    k = min(n, 300)
+    positions[:k, 2] = rng.uniform(0.5, 4.0, k)
+    positions[:k, 0] = positions[:k, 2] * np.float32(0.65 * 800 / 700)      # the right plane of view 1
+    if n > 400:
+        positions[400] = np.nan
+        positions[401, 0] = np.inf
+    for last_width in (800, 0):
+        widths = [800] * (n_views - 1) + [last_width]
+        start = np.full((n, 1), np.finfo(np.float32).max, np.float32)
+        start[::7] = 0.001
+        pos = torch.from_numpy(positions).cuda()
+        loop_f, loop_m = torch.from_numpy(start).cuda(), torch.zeros(n, dtype=torch.bool, device="cuda")
+        for v in range(n_views):
+            tb.update_3d_filter(pos, torch.from_numpy(w2cs[v]).cuda(), loop_f, loop_m, widths[v], 600, 700.0, 690.0, widths[v] / 2.0, 300.0, 0.2, 0.15, 0.0007)
+        one_f, one_m = torch.from_numpy(start).cuda(), torch.zeros(n, dtype=torch.bool, device="cuda")
+        tb.update_3d_filter_views(pos, torch.from_numpy(w2cs), one_f, one_m, widths, [600] * n_views, [700.0] * n_views, [690.0] * n_views,
+                                  [w / 2.0 for w in widths], [300.0] * n_views, [0.2] * n_views, 0.15, 0.0007)
+        torch.cuda.synchronize()
+        assert torch.equal(one_m, loop_m) and torch.allclose(one_f, loop_f, rtol=0.0, atol=0.0, equal_nan=True)
