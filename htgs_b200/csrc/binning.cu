@@ -121,59 +121,81 @@ template <> struct KeyOps<uint16_t> { static __device__ __forceinline__ uint16_t
 template <> struct KeyOps<uint32_t> { static __device__ __forceinline__ uint32_t make(uint32_t tile, uint32_t) { return tile; } static __device__ __forceinline__ uint32_t tile(uint32_t k) { return k; } };
 template <> struct KeyOps<uint64_t> { static __device__ __forceinline__ uint64_t make(uint32_t tile, uint32_t depth_bits) { return (uint64_t(tile) << 32) | depth_bits; } static __device__ __forceinline__ uint32_t tile(uint64_t k) { return uint32_t(k >> 32); } };
 
-// One block per 256 Gaussians (the blocks of the preprocess kernel).  The block's instances are
-// written cooperatively: slot j of the block belongs to the Gaussian whose in-block exclusive
-// offset is the last one <= j; inside a Gaussian the order is row-major over its tile box
-// (rasterization/src/shared_kernels.cu:21-28), so the emitted stream is identical to the reference's.
+// One block per 256 Gaussians (the blocks of the preprocess kernel).  A warp writes the instances of its 32 Gaussians
+// cooperatively, or the block those of all 256 where one warp would have most of the work: slot j belongs to the Gaussian
+// whose exclusive offset is the last one <= j (five or eight steps of search); inside a Gaussian the order is row-major over
+// its tile box (rasterization/src/shared_kernels.cu:21-28), so the emitted stream is identical to the reference's.  Bound by
+// instructions (the search, the split in row and column by a multiplication).
+// The kernel also clears what the sort and the range kernel count in (`clear`): one launch instead of three.
+struct ClearList { uint4* begin[3]; uint64_t count[3]; uint64_t per_sort_block[3]; };   // 16-byte words: a fixed number, plus so many per sort block of the frame
 template <typename KeyT>
 __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     const uint32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds, const EvalRecord* __restrict__ eval,
     const uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ block_offsets, KeyT* __restrict__ keys, uint32_t* __restrict__ prims,
-    uint32_t n_primitives, uint32_t grid_w, uint32_t capacity, const FrameStatus* __restrict__ status)
+    uint32_t n_primitives, uint32_t grid_w, uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear)
 {
+    const bool overflow = status->overflow;
+    const uint64_t sort_blocks = overflow ? 0 : (uint64_t(status->n_instances) + kSortTile - 1) / kSortTile;
+    #pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const uint64_t words = clear.count[c] + clear.per_sort_block[c] * sort_blocks;
+        for (uint64_t i = blockIdx.x * kPreprocessBlock + threadIdx.x; i < words; i += uint64_t(gridDim.x) * kPreprocessBlock) clear.begin[c][i] = make_uint4(0u, 0u, 0u, 0u);
+    }
     const uint32_t total = block_sums[blockIdx.x];
-    if (total == 0 || status->overflow) return;   // a frame that does not fit its instance buffers is skipped by every later stage
-    __shared__ uint32_t excl[kPreprocessBlock + 1];
-    __shared__ ushort4 box[kPreprocessBlock];
-    __shared__ uint32_t depth_bits[kPreprocessBlock];
+    if (total == 0 || overflow) return;   // a frame that does not fit its instance buffers is skipped by every later stage
+    __shared__ uint32_t excl[kPreprocessBlock];
+    __shared__ uint4 box[kPreprocessBlock];          // x_min | y_min << 16, width, reciprocal of the width (2^32 / width, rounded up; 0: divide), depth bits
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t first = blockIdx.x * kPreprocessBlock;
     const uint32_t idx = first + threadIdx.x;
     const uint32_t cnt = idx < n_primitives ? n_touched[idx] : 0u;
     if (cnt) {
-        box[threadIdx.x] = bounds[idx];
-        if constexpr (sizeof(KeyT) == 8) depth_bits[threadIdx.x] = __float_as_uint(eval[idx].mt3.w);
+        const ushort4 b = bounds[idx];
+        const uint32_t w = uint32_t(b.y) - uint32_t(b.x);
+        const uint32_t rcp = w > 1 && uint64_t(cnt) * w < (1ull << 32) ? 0xffffffffu / w + 1u : 0u;
+        box[threadIdx.x] = make_uint4(uint32_t(b.x) | (uint32_t(b.z) << 16), w, rcp, sizeof(KeyT) == 8 ? __float_as_uint(eval[idx].mt3.w) : 0u);
     }
     const uint32_t inc = warp_inclusive_scan(cnt);
-    if ((threadIdx.x & 31) == 31) warp_tot[threadIdx.x >> 5] = inc;
+    excl[threadIdx.x] = inc - cnt;
+    if (lane == 31) warp_tot[warp] = inc;
     __syncthreads();
-    uint32_t warp_base = 0;
+    uint32_t warp_base = 0, largest = 0;
     #pragma unroll
-    for (int w = 0; w < kPreprocessBlock / 32; ++w) if (w < int(threadIdx.x >> 5)) warp_base += warp_tot[w];
-    excl[threadIdx.x] = warp_base + inc - cnt;
-    if (threadIdx.x == 0) excl[kPreprocessBlock] = total;
-    __syncthreads();
-    const uint32_t base = block_offsets[blockIdx.x];
-    for (uint32_t j = threadIdx.x; j < total; j += kPreprocessBlock) {
-        // upper_bound(excl, j) - 1 over the 256 entries
-        uint32_t lo = 0, hi = kPreprocessBlock;
-        #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (excl[mid] <= j) lo = mid; else hi = mid;
-        }
-        const uint32_t local = j - excl[lo];
-        const ushort4 b = box[lo];
-        const uint32_t w = uint32_t(b.y) - uint32_t(b.x);
-        const uint32_t ly = local / w;
-        const uint32_t lx = local - ly * w;
-        const uint32_t tile = (uint32_t(b.z) + ly) * grid_w + uint32_t(b.x) + lx;
-        const uint64_t dst = uint64_t(base) + j;
+    for (int w = 0; w < kPreprocessBlock / 32; ++w) {
+        const uint32_t t = warp_tot[w];
+        if (w < int(warp)) warp_base += t;
+        largest = max(largest, t);
+    }
+    const uint64_t base = block_offsets[blockIdx.x];
+    auto emit = [&](uint32_t slot, uint32_t local, uint32_t owner) {
+        const uint4 b = box[owner];
+        const uint32_t ly = b.y == 1u ? local : b.z ? __umulhi(local, b.z) : local / b.y;
+        const uint32_t lx = local - ly * b.y;
+        const uint32_t tile = ((b.x >> 16) + ly) * grid_w + (b.x & 0xffffu) + lx;
+        const uint64_t dst = base + slot;
         if (dst < capacity) {
-            uint32_t db = 0;
-            if constexpr (sizeof(KeyT) == 8) db = depth_bits[lo];
-            keys[dst] = KeyOps<KeyT>::make(tile, db);
-            prims[dst] = first + lo;
+            keys[dst] = KeyOps<KeyT>::make(tile, b.w);
+            prims[dst] = first + owner;
+        }
+    };
+    if (largest <= total / 4) {           // the warps have about equally many: each searches its own 32
+        const uint32_t mine = warp_tot[warp];
+        for (uint32_t j = lane; j < mine; j += 32) {
+            uint32_t lo = 32u * warp;
+            #pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1) if (excl[lo + step] <= j) lo += step;
+            emit(warp_base + j, j - excl[lo], lo);
+        }
+    } else {                              // a few Gaussians of many tiles: the whole block writes them
+        __syncthreads();
+        excl[threadIdx.x] += warp_base;
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < total; j += kPreprocessBlock) {
+            uint32_t lo = 0;
+            #pragma unroll
+            for (uint32_t step = kPreprocessBlock / 2; step > 0; step >>= 1) if (excl[lo + step] <= j) lo += step;
+            emit(j, j - excl[lo], lo);
         }
     }
 }
@@ -188,23 +210,28 @@ __device__ __forceinline__ uint32_t digit_of(KeyT k, int shift, uint32_t mask) {
 
 // ---- stable LSD radix sort, one kernel per pass ("onesweep") ------------------------------------------------------------
 // One kernel counts the digits of EVERY pass in a single read of the keys; then each pass is ONE scatter kernel whose sort
-// blocks learn where their digits start from their predecessors through a table of published counts (decoupled look-back)
+// blocks learn where their digits start from their predecessors through tables of published counts (decoupled look-back)
 // instead of a histogram kernel and a scan kernel in front of every scatter.
 //
-// Scratch (zeroed once per frame): per pass a ticket counter, the digit histogram, and one 64-bit word per (sort block, digit):
-// bits 62-63 = state (0 nothing yet, 1 the block's own count, 2 the count summed over the block and all its predecessors),
-// bits 0-61 = the count.  A word is written with one 8-byte store, so state and count can never be seen apart.
+// Scratch (cleared by the emission kernel): per pass a ticket counter, the digit histogram, a word per (sort block, digit) - bit 31:
+// published, below it the block's count - and a 64-bit word per (group of 32 sort blocks, digit): bits 62-63 = state (0 nothing
+// yet, 1 the group's own count, 2 the count summed over the group and all groups before it), below it the count.  A block adds
+// the words of the blocks of its group in front of it and walks back over groups: the blocks of the first wave, which all start
+// together and find no summed count nearby, need a few round trips to L2 instead of one for every 16 blocks in front of them.
 // Blocks take their number from the pass's ticket counter when they start, so a block only ever waits for blocks that are
 // already running; every wait is bounded and reports through the frame status instead of spinning forever.
-constexpr unsigned long long kLookbackAggregate = 1ull << 62, kLookbackPrefix = 2ull << 62, kLookbackValue = (1ull << 62) - 1ull;
+constexpr uint32_t kRowPublished = 1u << 31;
+constexpr unsigned long long kGroupAggregate = 1ull << 62, kGroupPrefix = 2ull << 62, kGroupValue = (1ull << 62) - 1ull;
 constexpr uint32_t kLookbackPolls = 1u << 20;      // about half a second of polling before a block gives up
-constexpr int kLookbackBatch = 8;                 // predecessors read per step of the walk
+constexpr uint32_t kGroup = 32;                    // sort blocks per group
+constexpr int kLookbackBatch = 8;                  // words read per step
 
 struct SortScratch {
-    uint32_t* tickets;                   // [8]
+    uint32_t* tickets;                   // [16]
     uint32_t* digit_hist;                // [8][kMaxRadixBins]
-    unsigned long long* lookback[8];     // per pass [sort_blocks_cap][1 << bits]
-    size_t bytes;
+    unsigned long long* groups[8];       // per pass [ceil(sort_blocks_cap / kGroup)][1 << bits]
+    uint32_t* rows[8];                   // [sort_blocks_cap][row_stride]: the passes' counts of a sort block lie behind one another
+    size_t fixed_bytes, row_stride, bytes;
 };
 __host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32_t sort_blocks_cap) {
     SortScratch sc{};
@@ -212,11 +239,19 @@ __host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32
     size_t off = 0;
     sc.tickets = reinterpret_cast<uint32_t*>(p + off); off += 64;
     sc.digit_hist = reinterpret_cast<uint32_t*>(p + off); off += size_t(8) * kMaxRadixBins * sizeof(uint32_t);
+    const size_t n_groups = (size_t(sort_blocks_cap) + kGroup - 1) / kGroup;
     for (int i = 0; i < plan.n_passes; ++i) {
-        sc.lookback[i] = reinterpret_cast<unsigned long long*>(p + off);
-        off += size_t(sort_blocks_cap) * (size_t(1) << plan.bits[i]) * sizeof(unsigned long long);
+        sc.groups[i] = reinterpret_cast<unsigned long long*>(p + off);
+        off += (n_groups << plan.bits[i]) * sizeof(unsigned long long);
     }
-    sc.bytes = off;
+    off = (off + 15) & ~size_t(15);
+    sc.fixed_bytes = off;
+    for (int i = 0; i < plan.n_passes; ++i) {
+        sc.rows[i] = reinterpret_cast<uint32_t*>(p + off) + sc.row_stride;
+        sc.row_stride += size_t(1) << plan.bits[i];
+    }
+    sc.row_stride = (sc.row_stride + 3) & ~size_t(3);
+    sc.bytes = off + size_t(sort_blocks_cap) * sc.row_stride * sizeof(uint32_t);
     return sc;
 }
 
@@ -286,30 +321,35 @@ __device__ __forceinline__ void block_exclusive_scan_512(uint32_t* vals, uint32_
 }
 
 // One pass: stable scatter.  Warp w of a sort block owns the 512 consecutive keys [w*512, (w+1)*512) of the block's tile
-// and visits them in 16 rounds of 32, so (warp, round, lane) order is input order.  Ranks inside a round come from per-bit
-// warp ballots; per-warp digit counters in shared memory chain the rounds; a scan over warps and digits turns them into
-// positions in the locally sorted tile, which is staged in shared memory and written out as runs.  Where a digit's run
-// starts in the output comes from the pass's digit histogram plus what the preceding sort blocks published.
+// and visits them in 16 rounds of 32, so (warp, round, lane) order is input order.  A warp keeps per digit a count and a mask in
+// shared memory: the lanes of a round OR themselves into the mask of their digit, read mask and count back, and the highest
+// lane of each digit adds the round to the count.  That is 16 instructions for a round; a ballot per digit bit took over 100
+// (225 in the whole kernel, now 138).  A scan over warps and digits turns the counts into positions in the locally sorted
+// tile, which is staged in shared memory (over the masks) and written out as runs.  The Gaussian indices are requested after
+// the ranking, so that they do not hold registers before.
+// Bound by the latency of a block's phases and their barriers.  7.3 M keys of 16 bits, both passes: 189 -> 123 us; 154 M keys of
+// 32 bits: 3.86 -> 2.78 ms; 2.8 M keys of 64 bits, five passes: 294 -> 236 us.  Six blocks per SM instead of four change nothing.
+template <typename KeyT> constexpr int scatter_blocks_per_sm() { return sizeof(KeyT) == 4 ? 5 : 4; }
 template <typename KeyT>
-__global__ void __launch_bounds__(kSortThreads, 3) radix_scatter_kernel(
+__global__ void __launch_bounds__(kSortThreads, scatter_blocks_per_sm<KeyT>()) radix_scatter_kernel(
     const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ prims_in, KeyT* __restrict__ keys_out, uint32_t* __restrict__ prims_out,
-    const uint32_t* __restrict__ digit_hist, unsigned long long* lookback, uint32_t* ticket,
+    const uint32_t* __restrict__ digit_hist, uint32_t* rows, uint32_t row_stride, unsigned long long* groups, uint32_t* ticket,
     FrameStatus* status, uint32_t capacity, int shift, int bits)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint32_t* warp_count = reinterpret_cast<uint32_t*>(smem_raw);                 // [kSortWarps][n_bins]
-    const uint32_t n_bins_layout = 1u << bits;
-    uint32_t* block_excl = warp_count + kSortWarps * n_bins_layout;               // [n_bins]
-    uint32_t* global_base = block_excl + n_bins_layout;                           // [n_bins]
-    uint32_t* digit_base = global_base + n_bins_layout;                           // [n_bins]
-    uint32_t* prims_s = digit_base + n_bins_layout;                               // [kSortTile]
+    const uint32_t n_bins = 1u << bits, mask = n_bins - 1;
+    uint32_t* block_excl = reinterpret_cast<uint32_t*>(smem_raw);                 // [n_bins]
+    uint32_t* global_base = block_excl + n_bins;                                  // [n_bins]
+    uint32_t* digit_base = global_base + n_bins;                                  // [n_bins]
+    uint32_t* shared_region = digit_base + n_bins + (bits == 1 ? 2 : 0);          // 16-byte aligned
+    uint2* table = reinterpret_cast<uint2*>(shared_region);                       // [kSortWarps][n_bins] (mask, count), then:
+    uint32_t* prims_s = shared_region;                                            // [kSortTile]
     KeyT* keys_s = reinterpret_cast<KeyT*>(prims_s + kSortTile);                  // [kSortTile]
     __shared__ uint32_t warp_tot[kSortWarps];
     __shared__ uint32_t s_blk, s_failed;
 
     const uint32_t n = frame_instances(status, capacity);
-    const uint32_t n_blocks = (n + kSortTile - 1) / kSortTile;
-    const uint32_t n_bins = 1u << bits, mask = n_bins - 1;
+    const uint32_t n_blocks = uint32_t((uint64_t(n) + kSortTile - 1) / kSortTile);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // exclusive prefix of the digit totals (same for every sort block)
@@ -320,43 +360,33 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter_kernel(
 
     for (;;) {
         if (threadIdx.x == 0) s_blk = atomicAdd(ticket, 1u);
-        for (uint32_t i = threadIdx.x; i < kSortWarps * n_bins; i += kSortThreads) warp_count[i] = 0;
+        for (uint32_t i = threadIdx.x; i < kSortWarps * n_bins / 2; i += kSortThreads) reinterpret_cast<uint4*>(table)[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
         const uint32_t blk = s_blk;
         if (blk >= n_blocks) break;
         const uint32_t base = blk * kSortTile + warp * (kSortItems * 32);
+        constexpr bool kPacked = sizeof(KeyT) == 2;      // 16-bit keys share a register with their rank
         KeyT key[kSortItems];
-        uint32_t prim[kSortItems];
         uint32_t rank[kSortItems];
+        auto key_of = [&](int r) -> KeyT { return kPacked ? KeyT(rank[r]) : key[r]; };
         #pragma unroll
         for (int r = 0; r < kSortItems; ++r) {
             const uint32_t idx = base + r * 32 + lane;
-            if (idx < n) { key[r] = keys_in[idx]; prim[r] = prims_in[idx]; }
-            else { key[r] = KeyT(0); prim[r] = 0; }
+            key[r] = idx < n ? keys_in[idx] : KeyT(0);
         }
-        uint32_t* my_count = warp_count + warp * n_bins;
+        uint2* mine = table + warp * n_bins;
         #pragma unroll
         for (int r = 0; r < kSortItems; ++r) {
-            const uint32_t idx = base + r * 32 + lane;
-            const bool valid = idx < n;
-            const uint32_t valid_mask = __ballot_sync(0xffffffffu, valid);
-            rank[r] = 0;
-            // lanes holding the same digit: one ballot per digit bit (fixed cost; the hardware match instruction was measured
-            // slower here: 122 / 97 us per pass instead of 85 / 72 us at 7.8 M keys)
-            const uint32_t d = valid ? digit_of(key[r], shift, mask) : 0u;
-            uint32_t peers = valid_mask;
-            for (int b = 0; b < bits; ++b) {
-                const bool bit = (d >> b) & 1u;
-                const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-                peers &= bit ? bal : ~bal;
-            }
-            if (valid) {
-                const int leader = __ffs(peers) - 1;
-                uint32_t old = 0;
-                if (int(lane) == leader) { old = my_count[d]; my_count[d] = old + __popc(peers); }
-                old = __shfl_sync(peers, old, leader);
-                rank[r] = old + __popc(peers & lanemask_lt());
-            }
+            const bool valid = base + r * 32 + lane < n;
+            uint2* cell = mine + digit_of(key[r], shift, mask);
+            if (valid) atomicOr(&cell->x, 1u << lane);
+            __syncwarp();
+            uint2 seen = make_uint2(0u, 0u);
+            if (valid) seen = *cell;
+            rank[r] = seen.y + __popc(seen.x & lanemask_lt());
+            if constexpr (kPacked) rank[r] = (rank[r] << 16) | uint32_t(key[r]);
+            __syncwarp();
+            if (valid && (seen.x >> lane) == 1u) *cell = make_uint2(0u, seen.y + __popc(seen.x));
             __syncwarp();
         }
         __syncthreads();
@@ -364,57 +394,72 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter_kernel(
         for (uint32_t d = threadIdx.x; d < n_bins; d += kSortThreads) {
             uint32_t running = 0;
             #pragma unroll
-            for (int w = 0; w < kSortWarps; ++w) { const uint32_t t = warp_count[w * n_bins + d]; warp_count[w * n_bins + d] = running; running += t; }
+            for (int w = 0; w < kSortWarps; ++w) { const uint32_t t = table[w * n_bins + d].y; table[w * n_bins + d].y = running; running += t; }
             block_excl[d] = running;
-            volatile unsigned long long* mine = lookback + size_t(blk) * n_bins + d;
+            volatile uint32_t* row = rows + d;
+            row[size_t(blk) * row_stride] = kRowPublished | running;
+            const uint32_t group = blk / kGroup, group_first = group * kGroup;
+            const bool closes_group = blk - group_first == kGroup - 1u;
+            uint32_t polls = 0;
             unsigned long long before = 0;          // instances with this digit in the preceding sort blocks
-            if (blk == 0) {
-                *mine = kLookbackPrefix | running;
-            } else {
-                *mine = kLookbackAggregate | running;
-                // Walk back over the predecessors, kLookbackBatch words per step: the loads of a step are independent, so a
-                // long walk (the blocks of the first wave all start together and find no summed count nearby) costs one
-                // memory round trip per batch instead of one per predecessor.
-                uint32_t polls = 0;
-                bool done = false;
-                for (uint32_t p = blk; p > 0 && !done;) {
-                    const uint32_t step = min(uint32_t(kLookbackBatch), p);
-                    unsigned long long v[kLookbackBatch];
-                    #pragma unroll
-                    for (uint32_t i = 0; i < kLookbackBatch; ++i) {
-                        volatile const unsigned long long* theirs = lookback + size_t(p - 1u - (i < step ? i : 0u)) * n_bins + d;
-                        v[i] = *theirs;
-                    }
-                    #pragma unroll
-                    for (uint32_t i = 0; i < kLookbackBatch; ++i) {
-                        if (done || i >= step) continue;
-                        unsigned long long x = v[i];
-                        if ((x >> 62) == 0ull) {
-                            volatile const unsigned long long* theirs = lookback + size_t(p - 1u - i) * n_bins + d;
-                            while ((x >> 62) == 0ull && ++polls < kLookbackPolls) x = *theirs;
-                            if ((x >> 62) == 0ull) { s_failed = 1; done = true; continue; }     // gave up: report, never spin forever
-                        }
-                        before += x & kLookbackValue;
-                        if (x & kLookbackPrefix) done = true;
-                    }
-                    p -= step;
+            bool failed = false;                    // gave up: report, never spin forever
+            for (uint32_t p = group_first; p < blk; p += kLookbackBatch) {
+                uint32_t v[kLookbackBatch];
+                #pragma unroll
+                for (uint32_t i = 0; i < kLookbackBatch; ++i) v[i] = row[size_t(min(p + i, blk - 1u)) * row_stride];
+                #pragma unroll
+                for (uint32_t i = 0; i < kLookbackBatch; ++i) {
+                    if (p + i >= blk) continue;
+                    while (!(v[i] & kRowPublished) && ++polls < kLookbackPolls) v[i] = row[size_t(p + i) * row_stride];
+                    failed |= !(v[i] & kRowPublished);
+                    before += v[i] & ~kRowPublished;
                 }
-                *mine = kLookbackPrefix | ((before + running) & kLookbackValue);
             }
+            volatile unsigned long long* sums = groups + d;
+            if (closes_group) sums[size_t(group) << bits] = kGroupAggregate | (before + running);
+            bool done = false;
+            for (uint32_t p = group; p > 0 && !done;) {
+                const uint32_t step = min(uint32_t(kLookbackBatch), p);
+                unsigned long long v[kLookbackBatch];
+                #pragma unroll
+                for (uint32_t i = 0; i < kLookbackBatch; ++i) v[i] = sums[size_t(p - 1u - (i < step ? i : 0u)) << bits];
+                #pragma unroll
+                for (uint32_t i = 0; i < kLookbackBatch; ++i) {
+                    if (done || i >= step) continue;
+                    while ((v[i] >> 62) == 0ull && ++polls < kLookbackPolls) v[i] = sums[size_t(p - 1u - i) << bits];
+                    if ((v[i] >> 62) == 0ull) { failed = true; done = true; continue; }
+                    before += v[i] & kGroupValue;
+                    if (v[i] & kGroupPrefix) done = true;
+                }
+                p -= step;
+            }
+            if (closes_group) sums[size_t(group) << bits] = kGroupPrefix | ((before + running) & kGroupValue);
+            if (failed) s_failed = 1;
             global_base[d] = digit_base[d] + uint32_t(before);
         }
         __syncthreads();
+        uint32_t prim[kSortItems];
+        #pragma unroll
+        for (int r = 0; r < kSortItems; ++r) {
+            const uint32_t idx = base + r * 32 + lane;
+            prim[r] = idx < n ? __ldg(prims_in + idx) : 0u;
+        }
         block_exclusive_scan_512(block_excl, n_bins, warp_tot);
         const bool failed = s_failed != 0;
         // local stable placement
         #pragma unroll
         for (int r = 0; r < kSortItems; ++r) {
-            const uint32_t idx = base + r * 32 + lane;
-            if (idx < n) {
-                const uint32_t d = digit_of(key[r], shift, mask);
-                const uint32_t lp = block_excl[d] + my_count[d] + rank[r];
-                keys_s[lp] = key[r];
-                prims_s[lp] = prim[r];
+            const uint32_t d = digit_of(key_of(r), shift, mask);
+            rank[r] += (block_excl[d] + mine[d].y) << (kPacked ? 16 : 0);
+        }
+        __syncthreads();                  // the masks and counts are no longer needed
+        for (uint32_t d = threadIdx.x; d < n_bins; d += kSortThreads) global_base[d] -= block_excl[d];
+        #pragma unroll
+        for (int r = 0; r < kSortItems; ++r) {
+            if (base + r * 32 + lane < n) {
+                const uint32_t at = kPacked ? rank[r] >> 16 : rank[r];
+                keys_s[at] = key_of(r);
+                prims_s[at] = prim[r];
             }
         }
         __syncthreads();
@@ -425,8 +470,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter_kernel(
                 const uint32_t j = i * kSortThreads + threadIdx.x;
                 if (j < in_block) {
                     const KeyT k = keys_s[j];
-                    const uint32_t d = digit_of(k, shift, mask);
-                    const uint32_t dst = global_base[d] + (j - block_excl[d]);
+                    const uint32_t dst = global_base[digit_of(k, shift, mask)] + j;
                     keys_out[dst] = k;
                     prims_out[dst] = prims_s[j];
                 }
@@ -438,7 +482,8 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter_kernel(
 }
 
 template <typename KeyT> constexpr size_t scatter_smem_bytes(int bits = kMaxRadixBits) {
-    return (size_t(kSortWarps + 3) * (size_t(1) << bits) + kSortTile) * sizeof(uint32_t) + size_t(kSortTile) * sizeof(KeyT);
+    const size_t n_bins = size_t(1) << bits, table = kSortWarps * n_bins * sizeof(uint2), staging = kSortTile * (sizeof(uint32_t) + sizeof(KeyT));
+    return (3 * n_bins + (bits == 1 ? 2 : 0)) * sizeof(uint32_t) + (table > staging ? table : staging);
 }
 
 // Tiles by the length of their lists, longest first, in half-octave classes: blocks start in this order, so that the long lists do
@@ -541,18 +586,25 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
                                uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
-    cudaError_t err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream);
-    if (err != cudaSuccess) return err;
+    cudaError_t err = cudaSuccess;
     if (prim_blocks == 0 || inst.capacity == 0) {
+        if ((err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream)) != cudaSuccess) return err;
         if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); }
         tile_ranges_kernel<KeyT><<<1, kOrderThreads, 0, stream>>>(static_cast<const KeyT*>(inst.keys[0]), tile_ranges, tile_order, status, 0u, uint32_t(geo.n_tiles));
         if (ev) cudaEventRecord(ev[2], stream);
         if (launches) *launches += 1;
         return cudaGetLastError();
     }
+    const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap);
+    ClearList clear{};      // the buffers are 256-byte aligned and padded to 256 bytes
+    clear.begin[0] = reinterpret_cast<uint4*>(tile_ranges); clear.count[0] = (uint64_t(geo.n_tiles) + 1) / 2;
+    if (plan.n_passes > 0) {
+        clear.begin[1] = reinterpret_cast<uint4*>(sc.tickets); clear.count[1] = sc.fixed_bytes / 16;
+        clear.begin[2] = reinterpret_cast<uint4*>(sc.rows[0]); clear.per_sort_block[2] = sc.row_stride / 4;
+    }
     emit_instances_kernel<KeyT><<<prim_blocks, kPreprocessBlock, 0, stream>>>(
         prim.n_touched, prim.bounds, prim.eval, prim.block_sums, prim.block_offsets, static_cast<KeyT*>(inst.keys[0]), inst.prims[0], n,
-        uint32_t(geo.grid_w), inst.capacity, status);
+        uint32_t(geo.grid_w), inst.capacity, status, clear);
     if (ev) cudaEventRecord(ev[0], stream);
     if (launches) *launches += 1;
     static PerDeviceOnce configured;
@@ -560,8 +612,6 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
     if (err != cudaSuccess) return err;
     int cur = 0;
     if (plan.n_passes > 0) {
-        const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap);
-        if ((err = cudaMemsetAsync(inst.sort_scratch, 0, sc.bytes, stream)) != cudaSuccess) return err;
         PassTable passes{};
         passes.n_passes = plan.n_passes;
         for (int p = 0; p < plan.n_passes; ++p) { passes.shift[p] = plan.shift[p]; passes.bits[p] = plan.bits[p]; }
@@ -572,11 +622,11 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
             KeyT* kin = static_cast<KeyT*>(inst.keys[cur]);
             KeyT* kout = static_cast<KeyT*>(inst.keys[cur ^ 1]);
             const size_t smem = scatter_smem_bytes<KeyT>(plan.bits[p]);
-            const uint32_t resident = uint32_t(std::min<size_t>(3, (227 * 1024) / (smem + 1024)));   // scatter blocks one SM holds (3 by registers)
+            const uint32_t resident = uint32_t(std::min<size_t>(scatter_blocks_per_sm<KeyT>(), (227 * 1024) / (smem + 1024)));
             const uint32_t scatter_grid = std::min<uint32_t>(inst.sort_blocks_cap ? inst.sort_blocks_cap : 1u, uint32_t(sm_count) * resident);
             radix_scatter_kernel<KeyT><<<scatter_grid, kSortThreads, smem, stream>>>(
-                kin, inst.prims[cur], kout, inst.prims[cur ^ 1], sc.digit_hist + size_t(p) * kMaxRadixBins, sc.lookback[p], sc.tickets + p, status,
-                inst.capacity, plan.shift[p], plan.bits[p]);
+                kin, inst.prims[cur], kout, inst.prims[cur ^ 1], sc.digit_hist + size_t(p) * kMaxRadixBins, sc.rows[p],
+                uint32_t(sc.row_stride), sc.groups[p], sc.tickets + p, status, inst.capacity, plan.shift[p], plan.bits[p]);
             cur ^= 1;
             if (launches) *launches += 1;
         }
