@@ -69,6 +69,7 @@ struct FrameLayout {
     InstBuffers inst;
     uint2* tile_ranges;
     uint32_t* tile_order;
+    UnorderedState unordered;
     size_t bytes;
 };
 
@@ -86,8 +87,10 @@ FrameLayout carve_frame(void* blob, int n_primitives, int n_tiles, const SortPla
     L.prim.block_sums = c.take<uint32_t>(prim_blocks + 1);
     L.prim.block_offsets = c.take<uint32_t>(prim_blocks + 1);
     L.prim.visible_list = c.take<uint32_t>(n);
-    L.tile_ranges = c.take<uint2>(size_t(n_tiles));
+    L.tile_ranges = c.take<uint2>(size_t(n_tiles) + kOrderClasses / 2 + 1);
+    L.unordered.counters = reinterpret_cast<uint32_t*>(L.tile_ranges + n_tiles);
     L.tile_order = c.take<uint32_t>(size_t(n_tiles));
+    L.unordered.tile_class = c.take<uint8_t>(size_t(n_tiles));
     const uint64_t cap = instance_capacity > 0xfffffff0ull ? 0xfffffff0ull : instance_capacity;
     L.inst.capacity = uint32_t(cap);
     L.inst.sort_blocks_cap = uint32_t((cap + kSortTile - 1) / kSortTile);
@@ -290,7 +293,7 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
     *launches += (scene.n_primitives > 0 ? 2 : 0) + 1;
     const uint32_t* prims_sorted = L.inst.prims[plan.final_buffer];
     if (f.fast && !ctx->fast_deterministic) {
-        if ((err = launch_bin_unordered(scene, geo, L.prim, L.inst.prims[plan.final_buffer], L.inst.capacity, L.tile_ranges, L.status, ctx->sm_count,
+        if ((err = launch_bin_unordered(scene, geo, L.prim, L.inst.prims[plan.final_buffer], L.inst.capacity, L.tile_ranges, L.tile_order, L.unordered, L.status, ctx->sm_count,
                                         stream, prof ? ev + 3 : nullptr, launches)) != cudaSuccess) return fail_cuda(err, "unordered binning");
     } else if ((err = launch_emit_sort_ranges(view.mode, scene, geo, plan, L.prim, L.inst, L.tile_ranges, L.tile_order, L.status, ctx->sm_count, stream,
                                               prof ? ev + 3 : nullptr, launches)) != cudaSuccess) return fail_cuda(err, "binning");
@@ -303,7 +306,7 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
         if ((err = launch_max_weights(view, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, L.status, f.max_weights, f.weight_threshold, ctx->max_weights_tail_credit,
                                       stream)) != cudaSuccess) return fail_cuda(err, "max weights");
     } else if (f.fast) {
-        if ((err = launch_blend_fast(view.mode, view.K, geo, L.prim, prims_sorted, L.tile_ranges, out.image, out.to_chw, L.status, stream)) != cudaSuccess) return fail_cuda(err, "fast blend");
+        if ((err = launch_blend_fast(view.mode, view.K, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out.image, out.to_chw, L.status, stream)) != cudaSuccess) return fail_cuda(err, "fast blend");
     } else if ((err = launch_blend(view.mode, ctx->collect_stats ? BlendTask::image_with_statistics : BlendTask::image, view, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out, TrainPixelBuffers{}, L.status, stream)) != cudaSuccess) return fail_cuda(err, "blend");
     *launches += 1;
     if (prof) cudaEventRecord(ev[6], stream);

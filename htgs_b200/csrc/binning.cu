@@ -490,13 +490,6 @@ template <typename KeyT> constexpr size_t scatter_smem_bytes(int bits = kMaxRadi
 // not end up as the tail of a launch.  Inside a class the order is that of the image up to a few thousand tiles, which keeps
 // tiles that share Gaussians together in time.  Run by one block of 1024 threads.
 constexpr int kOrderThreads = 1024;
-constexpr int kOrderClasses = 64;
-__device__ __forceinline__ uint32_t order_class(uint2 range) {
-    const uint32_t n = range.y - range.x;
-    if (n < 2) return kOrderClasses - 1;
-    const uint32_t log2n = 31u - __clz(int(n));
-    return uint32_t(kOrderClasses - 1) - min(2u * log2n + ((n >> (log2n - 1)) & 1u) - 1u, uint32_t(kOrderClasses - 1));
-}
 __device__ __forceinline__ void order_tiles(const uint2* ranges, uint32_t* order, uint32_t n_tiles) {
     __shared__ uint32_t start[kOrderClasses];
     constexpr int kUnroll = 4;
@@ -515,7 +508,7 @@ __device__ __forceinline__ void order_tiles(const uint2* ranges, uint32_t* order
             for (int i = 0; i < kUnroll; ++i) {
                 const uint32_t t = base + i * kOrderThreads + threadIdx.x;
                 const bool valid = t < n_tiles;
-                const uint32_t c = order_class(r[i]);
+                const uint32_t c = order_class(r[i].y - r[i].x);
                 // one shared-memory atomic per class and warp
                 const uint32_t same = __match_any_sync(0xffffffffu, valid ? c : 0xffffffffu);
                 const int leader = __ffs(same) - 1;

@@ -6,8 +6,10 @@
 // need (rasterization/src/hybrid_blend/fast_inference.cu: create_instances_cu + cub::DeviceRadixSort::SortPairs +
 // extract_instance_ranges_cu) is replaced by
 //   1. count:  every (Gaussian, tile) instance adds 1 to its tile's counter,
-//   2. scan:   exclusive prefix over the tiles -> begin of every tile's list,
-//   3. place:  every instance takes the next free position of its tile with an atomic and stores the Gaussian index.
+//   2. scan:   every tile's list gets its place (a prefix within 1024 tiles, a shared cursor between them), and the tiles are counted
+//              by list length,
+//   3. place:  every instance takes the next free position of its tile with an atomic and stores the Gaussian index; the tiles are
+//              written down long lists first.
 // A (Gaussian, tile) instance of the Gaussian's tile box is dropped when the conservative outline of the Gaussian (the
 // ellipse the blend kernels test per pixel) does not reach the tile's 8 x 8 pixel square at all: the box of a slanted or
 // round outline has empty corners, and such an instance could only be staged and rejected pixel by pixel.
@@ -54,7 +56,8 @@ __device__ __forceinline__ bool outline_reaches_tile(const float4& c0, float cc,
 template <bool PLACE>
 __global__ void __launch_bounds__(kBinBlock) bin_visible_kernel(
     const uint32_t* __restrict__ visible_list, const uint32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds,
-    const CullRecord* __restrict__ cull, uint2* __restrict__ ranges, uint32_t* __restrict__ prims_sorted, const FrameStatus* __restrict__ status, uint32_t grid_w, uint32_t capacity)
+    const CullRecord* __restrict__ cull, uint2* __restrict__ ranges, uint32_t* __restrict__ prims_sorted, uint32_t* __restrict__ tile_order, UnorderedState state,
+    const FrameStatus* __restrict__ status, uint32_t grid_w, uint32_t n_tiles, uint32_t capacity)
 {
     __shared__ uint32_t excl[kBinBlock + 1];
     __shared__ ushort4 box[kBinBlock];
@@ -63,6 +66,18 @@ __global__ void __launch_bounds__(kBinBlock) bin_visible_kernel(
     __shared__ float outline_c[kBinBlock];
     __shared__ float2 outline_slopes[kBinBlock];
     __shared__ uint32_t warp_tot[kBinBlock / 32];
+    if constexpr (PLACE) {      // scatter the tiles to their class, one atomic per class and warp
+        for (uint32_t t0 = blockIdx.x * kBinBlock; t0 < n_tiles; t0 += gridDim.x * kBinBlock) {
+            const uint32_t t = t0 + threadIdx.x;
+            const uint32_t c = t < n_tiles ? uint32_t(state.tile_class[t]) : 0xffffffffu;
+            const uint32_t same = __match_any_sync(0xffffffffu, c);
+            const int leader = __ffs(same) - 1;
+            uint32_t at = 0;
+            if (t < n_tiles && int(threadIdx.x & 31u) == leader) at = atomicAdd(state.counters + c, uint32_t(__popc(same)));
+            at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & lanemask_lt());
+            if (t < n_tiles) tile_order[at] = t;
+        }
+    }
     if (status->overflow) return;   // the frame is re-run with larger buffers
     const uint32_t n_visible = status->n_visible;
     for (uint32_t first = blockIdx.x * kBinBlock; first < n_visible; first += gridDim.x * kBinBlock) {
@@ -118,51 +133,63 @@ __global__ void __launch_bounds__(kBinBlock) bin_visible_kernel(
     }
 }
 
-// Exclusive prefix over the tile counters: ranges[tile] = (begin, begin).  One block; every thread owns a run of
-// consecutive tiles (sums it, takes its offset from a block scan of the 1024 run totals, writes the run).
-__global__ void __launch_bounds__(1024) scan_tiles_kernel(uint2* __restrict__ ranges, uint32_t n_tiles) {
-    __shared__ uint32_t warp_tot[32];
-    const uint32_t per_thread = (n_tiles + 1023u) / 1024u;
-    const uint32_t begin_tile = min(threadIdx.x * per_thread, n_tiles);
-    const uint32_t end_tile = min(begin_tile + per_thread, n_tiles);
-    uint32_t sum = 0;
-    for (uint32_t t = begin_tile; t < end_tile; ++t) sum += ranges[t].y;
-    const uint32_t inc = warp_inclusive_scan_u32(sum);
-    if ((threadIdx.x & 31) == 31) warp_tot[threadIdx.x >> 5] = inc;
+// ranges[tile] = (begin, begin) from the tile counters.  A block takes 1024 tiles; between blocks the lists lie in the order in
+// which the blocks come, which nothing depends on (one block that scanned all tiles took 100 us at 92 k tiles).  The last block
+// to finish turns the counts of tiles per class into the classes' places in the order.
+__global__ void __launch_bounds__(1024) scan_tiles_kernel(uint2* __restrict__ ranges, UnorderedState state, uint32_t n_tiles) {
+    __shared__ uint32_t warp_tot[32], classes[kOrderClasses], block_begin;
+    __shared__ bool is_last;
+    if (threadIdx.x < kOrderClasses) classes[threadIdx.x] = 0;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const uint32_t t = warp_tot[threadIdx.x];
-        const uint32_t s = warp_inclusive_scan_u32(t);
-        warp_tot[threadIdx.x] = s - t;
+    const uint32_t t = blockIdx.x * 1024u + threadIdx.x;
+    const uint32_t n = t < n_tiles ? ranges[t].y : 0u;
+    const uint32_t inc = warp_inclusive_scan_u32(n);
+    if ((threadIdx.x & 31) == 31) warp_tot[threadIdx.x >> 5] = inc;
+    if (t < n_tiles) {
+        const uint32_t c = order_class(n);
+        state.tile_class[t] = uint8_t(c);
+        atomicAdd(&classes[c], 1u);
     }
     __syncthreads();
-    uint32_t running = warp_tot[threadIdx.x >> 5] + (inc - sum);
-    for (uint32_t t = begin_tile; t < end_tile; ++t) {
-        const uint32_t c = ranges[t].y;
-        ranges[t] = make_uint2(running, running);
-        running += c;
+    if (threadIdx.x < 32) {
+        const uint32_t w = warp_tot[threadIdx.x];
+        const uint32_t s = warp_inclusive_scan_u32(w);
+        warp_tot[threadIdx.x] = s - w;
+        if (threadIdx.x == 31) block_begin = atomicAdd(state.counters + kOrderClasses, s);
+    }
+    if (threadIdx.x < kOrderClasses && classes[threadIdx.x] != 0) atomicAdd(state.counters + threadIdx.x, classes[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    const uint32_t begin = block_begin + warp_tot[threadIdx.x >> 5] + (inc - n);
+    if (t < n_tiles) ranges[t] = make_uint2(begin, begin);
+    if (threadIdx.x == 0) is_last = atomicAdd(state.counters + kOrderClasses + 1, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (is_last && threadIdx.x < 32) {
+        __threadfence();
+        uint32_t* c = state.counters + 2 * threadIdx.x;
+        const uint32_t first = __ldcg(c), second = __ldcg(c + 1);
+        const uint32_t s = warp_inclusive_scan_u32(first + second);
+        c[0] = s - first - second;
+        c[1] = s - second;
     }
 }
 
 }  // namespace
 
 cudaError_t launch_bin_unordered(const HtgsScene& scene, const FrameGeometry& geo, const PrimBuffers& prim, uint32_t* prims_sorted, uint32_t capacity,
-                                 uint2* tile_ranges, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
-    cudaError_t err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream);
+                                 uint2* tile_ranges, uint32_t* tile_order, const UnorderedState& state, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev,
+                                 uint32_t* launches) {
+    cudaError_t err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles) + (kOrderClasses + 2) * sizeof(uint32_t), stream);
     if (err != cudaSuccess) return err;
-    if (scene.n_primitives <= 0 || capacity == 0 || geo.n_tiles == 0) {
-        if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); cudaEventRecord(ev[2], stream); }
-        return cudaSuccess;
-    }
-    const uint32_t max_blocks = (uint32_t(scene.n_primitives) + kBinBlock - 1) / kBinBlock;
-    const uint32_t grid = min(max_blocks, uint32_t(sm_count) * 8u);
-    bin_visible_kernel<false><<<grid, kBinBlock, 0, stream>>>(prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, status,
-                                                              uint32_t(geo.grid_w), capacity);
+    const uint32_t work = max(uint32_t(scene.n_primitives > 0 ? scene.n_primitives : 0), uint32_t(geo.n_tiles));
+    const uint32_t grid = min((work + kBinBlock - 1) / kBinBlock, uint32_t(sm_count) * 8u);
+    bin_visible_kernel<false><<<grid, kBinBlock, 0, stream>>>(prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, tile_order, state, status,
+                                                              uint32_t(geo.grid_w), uint32_t(geo.n_tiles), capacity);
     if (ev) cudaEventRecord(ev[0], stream);
-    scan_tiles_kernel<<<1, 1024, 0, stream>>>(tile_ranges, uint32_t(geo.n_tiles));
+    scan_tiles_kernel<<<(uint32_t(geo.n_tiles) + 1023u) / 1024u, 1024, 0, stream>>>(tile_ranges, state, uint32_t(geo.n_tiles));
     if (ev) cudaEventRecord(ev[1], stream);
-    bin_visible_kernel<true><<<grid, kBinBlock, 0, stream>>>(prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, status,
-                                                             uint32_t(geo.grid_w), capacity);
+    bin_visible_kernel<true><<<grid, kBinBlock, 0, stream>>>(prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, tile_order, state, status,
+                                                             uint32_t(geo.grid_w), uint32_t(geo.n_tiles), capacity);
     if (ev) cudaEventRecord(ev[2], stream);
     if (launches) *launches += 3;
     return cudaGetLastError();

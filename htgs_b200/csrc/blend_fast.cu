@@ -5,8 +5,9 @@
 // about 1e-3 per channel, not bit for bit: this path trades the operation-for-operation evaluation of the
 // exact kernel (blend.cu) for fewer instructions per fragment.
 //
-//  * Staging and candidate masks are those of the exact kernel: one 80-byte bulk asynchronous copy per instance,
-//    outline test with lane = Gaussian, 32 warp ballots per 32 Gaussians, every lane then walks its own mask.
+//  * The organisation is that of the exact kernel (blend.cu): a warp per 8 x 4 pixels filters its tile's list, keeps a window of two
+//    halves of 16 records that its lanes walk independently, and long lists start first.  Against a CTA per 8 x 8 tile with
+//    masks by ballots and a barrier every 64 instances: 944 -> FAST_US us at 3 M Gaussians, 1297 x 840, K = 16.
 //  * Per fragment, rho^2 and depth are ratios of quadratics in (pixel - projected centre) whose coefficients the
 //    preprocess stored per Gaussian (FastRecord): 6 shared-memory loads, 20 multiply-adds, one approximate
 //    reciprocal and one approximate exp2 instead of two plane constructions, two cross products, an IEEE divide
@@ -29,24 +30,25 @@ namespace htgs {
 
 namespace {
 
-constexpr int kFastThreads = 64;     // 8 x 8 pixel tile, one thread per pixel
-constexpr int kFastBatch = 64;       // instances staged per iteration, one per thread
+constexpr int kFastThreads = 32;     // 8 x 4 pixels, one thread per pixel
+constexpr int kFastHalf = 16;        // records per half of the window
+constexpr int kFastQueue = 64;       // survivors of the filter that wait for a place
 
 template <int MODE, int K> struct FastSmem {
     static constexpr bool has_kbuffer = MODE != HTGS_MODE_OIT_BLEND;
     static constexpr bool has_prim = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     static constexpr size_t rec_off = 0;
-    static constexpr size_t rec_bytes = size_t(kFastBatch) * sizeof(FastRecord);
-    static constexpr size_t cull4_off = rec_off + rec_bytes;
-    static constexpr size_t cullc_off = cull4_off + size_t(kFastBatch) * 16;
-    static constexpr size_t ctr_off = cullc_off + size_t(kFastBatch) * 4;      // float2: projected centre relative to the tile origin
-    static constexpr size_t prim_off = ctr_off + size_t(kFastBatch) * 8;        // Gaussian index of every staged instance (FIRST_K)
-    static constexpr size_t bar_off = prim_off + (has_prim ? size_t(kFastBatch) * 4 : 0);
-    static constexpr size_t keys_off = bar_off + 16;
+    static constexpr size_t keys_off = rec_off + 2 * kFastHalf * sizeof(FastRecord);
     static constexpr size_t keys_bytes = has_kbuffer ? size_t(K) * kFastThreads * 4 : 0;     // uint4 [K/4][threads]
     static constexpr size_t pay_off = keys_off + keys_bytes;
     static constexpr size_t pay_bytes = has_kbuffer ? size_t(K) * kFastThreads * 8 : 0;      // 8-byte payload [K][threads]
-    static constexpr size_t total = pay_off + pay_bytes;
+    static constexpr size_t ctr_off = pay_off + pay_bytes;                                   // float2 per record: projected centre relative to the block's origin
+    static constexpr size_t prim_off = ctr_off + 2 * kFastHalf * 8;                          // Gaussian index of every record (FIRST_K)
+    static constexpr size_t queue_ctr_off = prim_off + (has_prim ? 2 * kFastHalf * 4 : 0);
+    static constexpr size_t queue_prim_off = queue_ctr_off + kFastQueue * 8;
+    static constexpr size_t queue_mask_off = queue_prim_off + kFastQueue * 4;
+    static constexpr size_t bar_off = queue_mask_off + kFastQueue * 4;
+    static constexpr size_t total = bar_off + 16;
     static_assert(bar_off % 16 == 0 && keys_off % 16 == 0, "shared-memory sections must stay 16-byte aligned");
 };
 
@@ -121,7 +123,7 @@ __device__ __forceinline__ uint2 core_replace(uint32_t* keys, uint2* pay, uint32
 
 template <int MODE, int K>
 __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
-    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ prims_sorted, const FastRecord* __restrict__ records,
+    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const FastRecord* __restrict__ records,
     const CullRecord* __restrict__ cull, float* __restrict__ image, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
     FrameStatus* status)
 {
@@ -133,23 +135,27 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
     static_assert(kHybrid || kFirstK || kOit, "no relaxed-precision kernel for this mode");
     extern __shared__ __align__(128) unsigned char smem[];
     FastRecord* s_rec = reinterpret_cast<FastRecord*>(smem + SL::rec_off);
-    float4* s_cull4 = reinterpret_cast<float4*>(smem + SL::cull4_off);
-    float* s_cullc = reinterpret_cast<float*>(smem + SL::cullc_off);
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + SL::bar_off);
     float2* s_ctr = reinterpret_cast<float2*>(smem + SL::ctr_off);
     [[maybe_unused]] uint32_t* s_prim = reinterpret_cast<uint32_t*>(smem + SL::prim_off);
+    float2* s_queue_ctr = reinterpret_cast<float2*>(smem + SL::queue_ctr_off);
+    uint32_t* s_queue_prim = reinterpret_cast<uint32_t*>(smem + SL::queue_prim_off);
+    uint32_t* s_queue_mask = reinterpret_cast<uint32_t*>(smem + SL::queue_mask_off);
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + SL::bar_off);
     [[maybe_unused]] uint32_t* keys = reinterpret_cast<uint32_t*>(smem + SL::keys_off);
     [[maybe_unused]] uint2* pay = reinterpret_cast<uint2*>(smem + SL::pay_off);
 
-    const uint32_t tid = threadIdx.x;
-    const uint32_t warp = tid >> 5, lane = tid & 31;
-    const uint32_t tile_x = blockIdx.x, tile_y = blockIdx.y;
+    const uint32_t tid = threadIdx.x, lane = tid;
+    const uint32_t tile = __ldg(tile_order + blockIdx.x / 2), part = blockIdx.x % 2;
+    const uint32_t tile_x = tile % grid_w, block_y = (tile / grid_w) * 2 + part;
+    if (block_y * 4 >= height) return;
     const uint32_t px_i = tile_x * 8 + (tid & 7);
-    const uint32_t py_i = tile_y * 8 + (tid >> 3);
+    const uint32_t py_i = block_y * 4 + (tid >> 3);
     const bool inside = px_i < width && py_i < height;
-    const float local_x = float(tid & 7), local_y = float(tid >> 3);   // pixel position inside the tile
+    const float local_x = float(tid & 7), local_y = float(tid >> 3);   // pixel position inside the block
+    const float block_x0 = float(tile_x * 8), block_y0 = float(block_y * 4);
 
-    if (tid == 0) { mbar_init(s_bar, kFastThreads); mbar_fence_init(); }
+    if (lane < 2) mbar_init(s_bar + lane, 1);
+    mbar_fence_init();
 
     // empty core: the largest keys, carrying their position; zero payloads (FIRST_K: alpha 0, no Gaussian)
     if constexpr (SL::has_kbuffer) {
@@ -167,81 +173,74 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
     float4 tail = make_float4(0.0f, 0.0f, 0.0f, 0.0f);       // HYBRID tail / OIT sums: premultiplied rgb, alpha sum
     float transmittance_tail = 1.0f;
 
-    const uint2 range = tile_ranges[tile_y * grid_w + tile_x];
-    uint32_t phase = 0;
+    const uint2 range = tile_ranges[tile];
     bool wait_failed = false;
-    const float rect_x0 = float(tile_x * 8);
-    const float tile_y0 = float(tile_y * 8);
-    const float rect_y0 = float(tile_y * 8 + warp * 4);
 
-    uint32_t g_next = 0;
-    float4 c0_next = make_float4(__int_as_float(0x7f800000), 0.0f, 0.0f, 0.0f);   // "reject everything"
-    float4 c1_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);                         // c, cx_lo, cy_lo
-    if (range.x + tid < range.y) {
-        g_next = __ldg(prims_sorted + range.x + tid);
-        c0_next = ldg4(reinterpret_cast<const float*>(cull + g_next));
-        c1_next = ldg4(reinterpret_cast<const float*>(cull + g_next) + 4);
-    }
-    __syncthreads();
-
-    for (uint32_t batch_begin = range.x; batch_begin < range.y; batch_begin += kFastBatch) {
-        __syncthreads();
-        // ---- staging: one instance per thread, from the prefetch registers ----------------------------
-        const bool valid_inst = batch_begin + tid < range.y;
-        s_cull4[tid] = c0_next;
-        s_cullc[tid] = c1_next.x;
-        s_ctr[tid] = make_float2((rect_x0 - c0_next.x) - c1_next.y, (tile_y0 - c0_next.y) - c1_next.z);
-        if (valid_inst) {
-            mbar_arrive_expect_tx(s_bar, uint32_t(sizeof(FastRecord)));
-            bulk_copy_g2s(s_rec + tid, records + g_next, uint32_t(sizeof(FastRecord)), s_bar);
-            if constexpr (SL::has_prim) s_prim[tid] = g_next;
-        } else {
-            mbar_arrive(s_bar);
+    uint32_t next = range.x + lane;                      // the instance this lane tests next
+    uint32_t g_here = 0, g_ahead = 0;
+    float4 c0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c1 = c0;      // outline; c, cx_lo, cy_lo
+    auto request_outline = [&](uint32_t g) {
+        c0 = ldg4(reinterpret_cast<const float*>(cull + g));
+        c1 = ldg4(reinterpret_cast<const float*>(cull + g) + 4);
+    };
+    if (next < range.y) { g_here = __ldg(prims_sorted + next); request_outline(g_here); }
+    if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
+    uint32_t queue_head = 0, queued = 0;
+    auto filter = [&]() {
+        uint32_t mask = 0;
+        if (next < range.y) mask = outline_mask(c0, c1.x, block_x0, block_y0);
+        const uint32_t survivors = __ballot_sync(0xffffffffu, mask != 0);
+        if (mask != 0) {
+            const uint32_t at = (queue_head + queued + __popc(survivors & lanemask_lt())) & uint32_t(kFastQueue - 1);
+            s_queue_prim[at] = g_here;
+            s_queue_mask[at] = mask;
+            s_queue_ctr[at] = make_float2((block_x0 - c0.x) - c1.y, (block_y0 - c0.y) - c1.z);
         }
-        const uint32_t inst_next = batch_begin + kFastBatch + tid;
-        const bool valid_next = inst_next < range.y;
-        if (valid_next) g_next = __ldg(prims_sorted + inst_next);
-        __syncthreads();
-        // ---- candidate masks: lane = Gaussian, one ballot per pixel of the warp ------------------------
-        uint64_t cand = 0;
-        #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const uint32_t j = half * 32 + lane;
-            const float4 c0 = s_cull4[j];
-            const float cc = s_cullc[j];
-            const float dx0 = rect_x0 - c0.x, dy0 = rect_y0 - c0.y;
-            uint32_t mine = 0;
-            #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float dy = dy0 + float(r);
-                const float b2dy = c0.w * dy, cdy2 = cc * dy * dy;
-                #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float dx = dx0 + float(i);
-                    const float q = dx * (c0.z * dx + b2dy) + cdy2;
-                    const uint32_t touched = __ballot_sync(0xffffffffu, q <= 1.0f);
-                    if (int(lane) == r * 8 + i) mine = touched;
-                }
+        queued += __popc(survivors);
+        next += 32;
+        g_here = g_ahead;
+        if (next < range.y) request_outline(g_here);
+        if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
+    };
+    while (queued < kFastHalf && next - lane < range.y) filter();
+    __syncwarp();
+
+    uint32_t window = 0;                                 // this pixel's candidates: bits 31..16 the older half, 15..0 the newer half
+    uint32_t phases = 0;                                 // parity of each half's barrier
+    for (uint32_t half = 0;; half ^= 1u) {
+        // ---- replace the half that no lane needs any more -----------------------------------------------------------------
+        const uint32_t count = min(queued, uint32_t(kFastHalf));
+        if (count != 0) {
+            uint32_t g = 0, mask = 0;
+            const uint32_t slot = half * kFastHalf + (uint32_t(kFastHalf) - 1u - (lane & uint32_t(kFastHalf - 1)));
+            if (lane < count) {
+                const uint32_t at = (queue_head + lane) & uint32_t(kFastQueue - 1);
+                g = s_queue_prim[at];
+                mask = s_queue_mask[at];
+                s_ctr[slot] = s_queue_ctr[at];
+                if constexpr (SL::has_prim) s_prim[slot] = g;
             }
-            cand |= uint64_t(mine) << (32 * half);
+            if (lane == 0) mbar_arrive_expect_tx(s_bar + half, count * uint32_t(sizeof(FastRecord)));
+            __syncwarp();
+            if (lane < count) bulk_copy_g2s(s_rec + slot, records + g, uint32_t(sizeof(FastRecord)), s_bar + half);
+            queue_head += count;
+            queued -= count;
+            const uint32_t mine = transpose_masks(mask, lane);
+            if (inside) window |= mine;
+            while (queued < kFastHalf && next - lane < range.y) filter();
+            if (!mbar_wait_bounded(s_bar + half, (phases >> half) & 1u)) wait_failed = true;
+            phases ^= 1u << half;
+            __syncwarp();
+        } else if (!__any_sync(0xffffffffu, window != 0)) {
+            break;
         }
-        if (!inside) cand = 0;
-        if (valid_next) {   // the index prefetched before the barrier has arrived by now
-            c0_next = ldg4(reinterpret_cast<const float*>(cull + g_next));
-            c1_next = ldg4(reinterpret_cast<const float*>(cull + g_next) + 4);
-        } else {
-            c0_next = make_float4(__int_as_float(0x7f800000), 0.0f, 0.0f, 0.0f);
-            c1_next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-        // ---- fragments -----------------------------------------------------------------------------------
-        if (!mbar_wait_bounded(s_bar, phase)) wait_failed = true;
-        phase ^= 1;
-        const uint32_t n_iter = __reduce_max_sync(0xffffffffu, uint32_t(__popcll(cand)));
+        // ---- fragments: until no lane has a candidate of the older half left -------------------------------------------------
+        const uint32_t flip = half * kFastHalf;          // bit j of the window is record j ^ flip
         auto pop_candidate = [&](bool& valid) -> uint32_t {
-            valid = cand != 0;
-            const uint32_t j = valid ? uint32_t(__ffsll((long long)cand) - 1) : 0u;
-            cand &= cand - 1;
-            return j;
+            valid = window != 0;
+            const uint32_t j = uint32_t(31 - __clz(int(window | 1u)));
+            window &= ~(1u << j);
+            return j ^ flip;
         };
         auto evaluate = [&](uint32_t j, float& depth, float4& frag) {
             const float4* rec = reinterpret_cast<const float4*>(s_rec + j);
@@ -281,7 +280,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
                 transmittance_tail *= 1.0f - frag.w;
             }
         };
-        for (uint32_t it = 0; it < n_iter; it += 2) {
+        while (__any_sync(0xffffffffu, window >= 0x10000u)) {
             bool v0, v1;
             const uint32_t j0 = pop_candidate(v0);
             const uint32_t j1 = pop_candidate(v1);
@@ -292,6 +291,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
             if (v0 && !(frag0.w < MT::min_alpha)) commit(j0, depth0, frag0);
             if (v1 && !(frag1.w < MT::min_alpha)) commit(j1, depth1, frag1);
         }
+        window <<= 16;
     }
 
     if (wait_failed) atomicOr(&status->error, 1u);
@@ -368,31 +368,25 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
 }
 
 template <int MODE, int K>
-cudaError_t launch_fast_k(const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, float* image,
+cudaError_t launch_fast_k(const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order, float* image,
                           bool to_chw, FrameStatus* status, cudaStream_t stream) {
     using SL = FastSmem<MODE, K>;
-    static PerDeviceOnce configured;
-    const cudaError_t cfg = configured.run([] {
-        const cudaError_t err = cudaFuncSetAttribute(blend_fast_kernel<MODE, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SL::total));
-        if (err != cudaSuccess) return err;
-        return cudaFuncSetAttribute(blend_fast_kernel<MODE, K>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    });
-    if (cfg != cudaSuccess) return cfg;
+    static_assert(SL::total <= 48 * 1024, "no opt-in for more shared memory needed");
     if (geo.n_tiles == 0) return cudaSuccess;
-    blend_fast_kernel<MODE, K><<<dim3(geo.grid_w, geo.grid_h), kFastThreads, SL::total, stream>>>(
-        tile_ranges, prims_sorted, reinterpret_cast<const FastRecord*>(prim.eval), prim.cull, image, uint32_t(geo.width), uint32_t(geo.height),
+    blend_fast_kernel<MODE, K><<<uint32_t(geo.n_tiles) * 2u, kFastThreads, SL::total, stream>>>(
+        tile_ranges, tile_order, prims_sorted, reinterpret_cast<const FastRecord*>(prim.eval), prim.cull, image, uint32_t(geo.width), uint32_t(geo.height),
         uint32_t(geo.grid_w), to_chw, status);
     return cudaGetLastError();
 }
 
 template <int MODE>
-cudaError_t launch_fast_mode(int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
+cudaError_t launch_fast_mode(int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
                              float* image, bool to_chw, FrameStatus* status, cudaStream_t stream) {
     switch (effective_k(MODE, K)) {
-        case 4: return launch_fast_k<MODE, 4>(geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
-        case 8: return launch_fast_k<MODE, 8>(geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
-        case 16: return launch_fast_k<MODE, 16>(geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
-        case 32: return launch_fast_k<MODE, 32>(geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
+        case 4: return launch_fast_k<MODE, 4>(geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
+        case 8: return launch_fast_k<MODE, 8>(geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
+        case 16: return launch_fast_k<MODE, 16>(geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
+        case 32: return launch_fast_k<MODE, 32>(geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -406,12 +400,12 @@ bool blend_fast_supports(int mode, int K) {
     return k == 4 || k == 8 || k == 16 || k == 32;
 }
 
-cudaError_t launch_blend_fast(int mode, int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
+cudaError_t launch_blend_fast(int mode, int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
                               float* image, bool to_chw, FrameStatus* status, cudaStream_t stream) {
     switch (mode) {
-        case HTGS_MODE_HYBRID_BLEND: return launch_fast_mode<HTGS_MODE_HYBRID_BLEND>(K, geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
-        case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_fast_mode<HTGS_MODE_ALPHA_BLEND_FIRST_K>(K, geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
-        case HTGS_MODE_OIT_BLEND: return launch_fast_k<HTGS_MODE_OIT_BLEND, 4>(geo, prim, prims_sorted, tile_ranges, image, to_chw, status, stream);
+        case HTGS_MODE_HYBRID_BLEND: return launch_fast_mode<HTGS_MODE_HYBRID_BLEND>(K, geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
+        case HTGS_MODE_ALPHA_BLEND_FIRST_K: return launch_fast_mode<HTGS_MODE_ALPHA_BLEND_FIRST_K>(K, geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
+        case HTGS_MODE_OIT_BLEND: return launch_fast_k<HTGS_MODE_OIT_BLEND, 4>(geo, prim, prims_sorted, tile_ranges, tile_order, image, to_chw, status, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -86,8 +86,19 @@ cudaError_t launch_emit_sort_ranges(int mode, const HtgsScene& scene, const Fram
 // binning_unordered.cu: per-tile lists without sort keys (counting sort with atomics; the order inside a list is not
 // defined).  Writes `tile_ranges` and `prims_sorted`; expects `status->n_instances / overflow` from launch_scan_only.
 // `stage_events` (optional): events recorded after the count pass, the tile scan and the placement pass.
+constexpr int kOrderClasses = 64;     // of list lengths, two per octave, longest first
+__device__ __forceinline__ uint32_t order_class(uint32_t n) {
+    if (n < 2) return kOrderClasses - 1;
+    const uint32_t log2n = 31u - __clz(int(n));
+    return uint32_t(kOrderClasses - 1) - min(2u * log2n + ((n >> (log2n - 1)) & 1u) - 1u, uint32_t(kOrderClasses - 1));
+}
+struct UnorderedState {       // `counters` lie behind `tile_ranges`: both are cleared together
+    uint32_t* counters;       // [kOrderClasses + 2] tiles per class of list length (then where the next one goes), end of the lists so far, blocks done
+    uint8_t* tile_class;      // [tiles]
+};
 cudaError_t launch_bin_unordered(const HtgsScene& scene, const FrameGeometry& geo, const PrimBuffers& prim, uint32_t* prims_sorted, uint32_t capacity,
-                                 uint2* tile_ranges, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* stage_events = nullptr,
+                                 uint2* tile_ranges, uint32_t* tile_order, const UnorderedState& state, FrameStatus* status, int sm_count, cudaStream_t stream,
+                                 cudaEvent_t* stage_events = nullptr,
                                  uint32_t* launches = nullptr);
 
 // blend.cu
@@ -118,7 +129,7 @@ cudaError_t launch_blend(int mode, BlendTask task, const HtgsView& view, const F
 // blend_fast.cu: relaxed-precision inference (RGB only) for HYBRID_BLEND, ALPHA_BLEND_FIRST_K and OIT_BLEND.  `supports` tells
 // whether (mode, K) has a fast kernel; these kernels do not depend on the order of a tile's list.
 bool blend_fast_supports(int mode, int K);
-cudaError_t launch_blend_fast(int mode, int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges,
+cudaError_t launch_blend_fast(int mode, int K, const FrameGeometry& geo, const PrimBuffers& prim, const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order,
                               float* image, bool to_chw, FrameStatus* status, cudaStream_t stream);
 
 // weights.cu
