@@ -33,6 +33,7 @@ namespace {
 constexpr int kFastThreads = 32;     // 8 x 4 pixels, one thread per pixel
 constexpr int kFastHalf = 16;        // records per half of the window
 constexpr int kFastQueue = 64;       // survivors of the filter that wait for a place
+constexpr int kFastDense = 20;       // pixels of 32 from which on a record is evaluated by all lanes together
 
 template <int MODE, int K> struct FastSmem {
     static constexpr bool has_kbuffer = MODE != HTGS_MODE_OIT_BLEND;
@@ -47,9 +48,17 @@ template <int MODE, int K> struct FastSmem {
     static constexpr size_t queue_ctr_off = prim_off + (has_prim ? 2 * kFastHalf * 4 : 0);
     static constexpr size_t queue_prim_off = queue_ctr_off + kFastQueue * 8;
     static constexpr size_t queue_mask_off = queue_prim_off + kFastQueue * 4;
-    static constexpr size_t bar_off = queue_mask_off + kFastQueue * 4;
-    static constexpr size_t total = bar_off + 16;
-    static_assert(bar_off % 16 == 0 && keys_off % 16 == 0, "shared-memory sections must stay 16-byte aligned");
+    // the same for dense records: staged, and waiting
+    static constexpr size_t dense_rec_off = queue_mask_off + kFastQueue * 4;
+    static constexpr size_t dense_ctr_off = dense_rec_off + kFastHalf * sizeof(FastRecord);
+    static constexpr size_t dense_mask_off = dense_ctr_off + kFastHalf * 8;
+    static constexpr size_t dense_prim_off = dense_mask_off + kFastHalf * 4;
+    static constexpr size_t dense_queue_ctr_off = dense_prim_off + (has_prim ? kFastHalf * 4 : 0);
+    static constexpr size_t dense_queue_prim_off = dense_queue_ctr_off + kFastQueue * 8;
+    static constexpr size_t dense_queue_mask_off = dense_queue_prim_off + kFastQueue * 4;
+    static constexpr size_t bar_off = dense_queue_mask_off + kFastQueue * 4;
+    static constexpr size_t total = bar_off + 3 * 8;
+    static_assert(bar_off % 8 == 0 && keys_off % 16 == 0 && dense_rec_off % 16 == 0, "shared-memory sections must stay 16-byte aligned");
 };
 
 __device__ __forceinline__ float rcp_approx(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -154,7 +163,11 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
     const float local_x = float(tid & 7), local_y = float(tid >> 3);   // pixel position inside the block
     const float block_x0 = float(tile_x * 8), block_y0 = float(block_y * 4);
 
-    if (lane < 2) mbar_init(s_bar + lane, 1);
+    FastRecord* s_dense = reinterpret_cast<FastRecord*>(smem + SL::dense_rec_off);
+    float2* s_dense_ctr = reinterpret_cast<float2*>(smem + SL::dense_ctr_off);
+    uint32_t* s_dense_mask = reinterpret_cast<uint32_t*>(smem + SL::dense_mask_off);
+    [[maybe_unused]] uint32_t* s_dense_prim = reinterpret_cast<uint32_t*>(smem + SL::dense_prim_off);
+    if (lane < 3) mbar_init(s_bar + lane, 1);
     mbar_fence_init();
 
     // empty core: the largest keys, carrying their position; zero payloads (FIRST_K: alpha 0, no Gaussian)
@@ -185,56 +198,77 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
     };
     if (next < range.y) { g_here = __ldg(prims_sorted + next); request_outline(g_here); }
     if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
-    uint32_t queue_head = 0, queued = 0;
+    // Survivors of the filter wait in two queues: those that touch many of the 32 pixels and the others.
+    uint32_t sparse_head = 0, sparse = 0, dense_head = 0, dense = 0;
     auto filter = [&]() {
         uint32_t mask = 0;
         if (next < range.y) mask = outline_mask(c0, c1.x, block_x0, block_y0);
-        const uint32_t survivors = __ballot_sync(0xffffffffu, mask != 0);
+        const bool is_dense = __popc(mask) >= kFastDense;
+        const uint32_t sparse_lanes = __ballot_sync(0xffffffffu, mask != 0 && !is_dense), dense_lanes = __ballot_sync(0xffffffffu, is_dense);
         if (mask != 0) {
-            const uint32_t at = (queue_head + queued + __popc(survivors & lanemask_lt())) & uint32_t(kFastQueue - 1);
-            s_queue_prim[at] = g_here;
-            s_queue_mask[at] = mask;
-            s_queue_ctr[at] = make_float2((block_x0 - c0.x) - c1.y, (block_y0 - c0.y) - c1.z);
+            const uint32_t at = (is_dense ? dense_head + dense + __popc(dense_lanes & lanemask_lt()) : sparse_head + sparse + __popc(sparse_lanes & lanemask_lt())) & uint32_t(kFastQueue - 1);
+            unsigned char* queue = smem + (is_dense ? SL::dense_queue_ctr_off : SL::queue_ctr_off);     // centres, indices, masks
+            reinterpret_cast<float2*>(queue)[at] = make_float2((block_x0 - c0.x) - c1.y, (block_y0 - c0.y) - c1.z);
+            reinterpret_cast<uint32_t*>(queue + kFastQueue * 8)[at] = g_here;
+            reinterpret_cast<uint32_t*>(queue + kFastQueue * 12)[at] = mask;
         }
-        queued += __popc(survivors);
+        sparse += __popc(sparse_lanes);
+        dense += __popc(dense_lanes);
         next += 32;
         g_here = g_ahead;
         if (next < range.y) request_outline(g_here);
         if (next + 32 < range.y) g_ahead = __ldg(prims_sorted + next + 32);
     };
-    while (queued < kFastHalf && next - lane < range.y) filter();
-    __syncwarp();
+    auto fill_queues = [&]() {
+        while (sparse < kFastHalf && dense < kFastHalf && next - lane < range.y) filter();
+        __syncwarp();
+    };
+    // The next `count` (<= kFastHalf) records of a queue into slots first - lane: index, centre and a copy under way.  Returns the lane's mask.
+    auto stage = [&](size_t queue_off, uint32_t head, uint32_t count, uint32_t slot, FastRecord* rec, float2* ctr, uint32_t* prim, uint64_t* bar) -> uint32_t {
+        uint32_t g = 0, mask = 0;
+        if (lane < count) {
+            const unsigned char* queue = smem + queue_off;
+            const uint32_t at = (head + lane) & uint32_t(kFastQueue - 1);
+            ctr[slot] = reinterpret_cast<const float2*>(queue)[at];
+            g = reinterpret_cast<const uint32_t*>(queue + kFastQueue * 8)[at];
+            mask = reinterpret_cast<const uint32_t*>(queue + kFastQueue * 12)[at];
+            if constexpr (SL::has_prim) prim[slot] = g;
+        }
+        if (lane == 0) mbar_arrive_expect_tx(bar, count * uint32_t(sizeof(FastRecord)));
+        __syncwarp();
+        if (lane < count) bulk_copy_g2s(rec + slot, records + g, uint32_t(sizeof(FastRecord)), bar);
+        return mask;
+    };
 
     uint32_t window = 0;                                 // this pixel's candidates: bits 31..16 the older half, 15..0 the newer half
-    uint32_t phases = 0;                                 // parity of each half's barrier
-    for (uint32_t half = 0;; half ^= 1u) {
-        // ---- replace the half that no lane needs any more -----------------------------------------------------------------
-        const uint32_t count = min(queued, uint32_t(kFastHalf));
-        if (count != 0) {
-            uint32_t g = 0, mask = 0;
+    uint32_t phases = 0;                                 // parity of each barrier
+    uint32_t half = 0;
+    fill_queues();
+    for (;;) {
+        const bool more = next - lane < range.y;
+        const uint32_t n_dense = dense >= kFastHalf || !more ? min(dense, uint32_t(kFastHalf)) : 0u;
+        const uint32_t n_sparse = sparse >= kFastHalf || !more ? min(sparse, uint32_t(kFastHalf)) : 0u;
+        const bool step = n_sparse != 0 || (!more && __any_sync(0xffffffffu, window != 0));
+        if (n_dense == 0 && !step) break;                // only with nothing left: otherwise a queue is full
+        if (n_dense != 0) {
+            const uint32_t mask = stage(SL::dense_queue_ctr_off, dense_head, n_dense, lane, s_dense, s_dense_ctr, s_dense_prim, s_bar + 2);
+            if (lane < n_dense) s_dense_mask[lane] = mask;
+            dense_head += n_dense;
+            dense -= n_dense;
+        }
+        if (n_sparse != 0) {
             const uint32_t slot = half * kFastHalf + (uint32_t(kFastHalf) - 1u - (lane & uint32_t(kFastHalf - 1)));
-            if (lane < count) {
-                const uint32_t at = (queue_head + lane) & uint32_t(kFastQueue - 1);
-                g = s_queue_prim[at];
-                mask = s_queue_mask[at];
-                s_ctr[slot] = s_queue_ctr[at];
-                if constexpr (SL::has_prim) s_prim[slot] = g;
-            }
-            if (lane == 0) mbar_arrive_expect_tx(s_bar + half, count * uint32_t(sizeof(FastRecord)));
-            __syncwarp();
-            if (lane < count) bulk_copy_g2s(s_rec + slot, records + g, uint32_t(sizeof(FastRecord)), s_bar + half);
-            queue_head += count;
-            queued -= count;
-            const uint32_t mine = transpose_masks(mask, lane);
+            const uint32_t mine = transpose_masks(stage(SL::queue_ctr_off, sparse_head, n_sparse, slot, s_rec, s_ctr, s_prim, s_bar + half), lane);
+            sparse_head += n_sparse;
+            sparse -= n_sparse;
             if (inside) window |= mine;
-            while (queued < kFastHalf && next - lane < range.y) filter();
+        }
+        fill_queues();
+        if (n_sparse != 0) {
             if (!mbar_wait_bounded(s_bar + half, (phases >> half) & 1u)) wait_failed = true;
             phases ^= 1u << half;
             __syncwarp();
-        } else if (!__any_sync(0xffffffffu, window != 0)) {
-            break;
         }
-        // ---- fragments: until no lane has a candidate of the older half left -------------------------------------------------
         const uint32_t flip = half * kFastHalf;          // bit j of the window is record j ^ flip
         auto pop_candidate = [&](bool& valid) -> uint32_t {
             valid = window != 0;
@@ -242,9 +276,8 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
             window &= ~(1u << j);
             return j ^ flip;
         };
-        auto evaluate = [&](uint32_t j, float& depth, float4& frag) {
-            const float4* rec = reinterpret_cast<const float4*>(s_rec + j);
-            const float2 ctr = s_ctr[j];
+        auto evaluate = [&](const FastRecord* record, float2 ctr, float& depth, float4& frag) {
+            const float4* rec = reinterpret_cast<const float4*>(record);
             const float4 r0 = rec[0], r1 = rec[1], r3 = rec[3], r4 = rec[4];
             const float dx = local_x + ctr.x, dy = local_y + ctr.y;
             const float xx = dx * dx, xy = dx * dy, yy = dy * dy;
@@ -262,7 +295,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
             if constexpr (kFirstK) frag = make_float4(0.0f, 0.0f, 0.0f, alpha);   // the colour is fetched when the tile is composited
             else frag = make_float4(r3.w * alpha, r4.x * alpha, r4.y * alpha, alpha);
         };
-        auto commit = [&](uint32_t j, float depth, float4 frag) {
+        auto commit = [&](uint32_t prim, float depth, float4 frag) {
             if constexpr (kHybrid) {
                 if (depth < depth_max && frag.w >= MT::min_alpha_core) {
                     frag = unpack_half4(core_replace<K>(keys, pay, tid, depth, pack_half4(frag.x, frag.y, frag.z, frag.w), row_max, kmax));
@@ -272,7 +305,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
                 transmittance_tail *= 1.0f - frag.w;
             } else if constexpr (kFirstK) {
                 if (depth < depth_max) {   // whatever falls out of the buffer is dropped (alpha_blend_first_k/kernels/fast_inference.cuh:147-160)
-                    core_replace<K>(keys, pay, tid, depth, make_uint2(__float_as_uint(frag.w), s_prim[j]), row_max, kmax);
+                    core_replace<K>(keys, pay, tid, depth, make_uint2(__float_as_uint(frag.w), prim), row_max, kmax);
                     depth_max = KeyCodec<K>::decode(kmax);
                 }
             } else {   // oit_blend/kernels/fast_inference.cuh:138-141
@@ -280,18 +313,38 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
                 transmittance_tail *= 1.0f - frag.w;
             }
         };
-        while (__any_sync(0xffffffffu, window >= 0x10000u)) {
-            bool v0, v1;
-            const uint32_t j0 = pop_candidate(v0);
-            const uint32_t j1 = pop_candidate(v1);
-            float depth0, depth1;
-            float4 frag0, frag1;
-            evaluate(j0, depth0, frag0);
-            evaluate(j1, depth1, frag1);
-            if (v0 && !(frag0.w < MT::min_alpha)) commit(j0, depth0, frag0);
-            if (v1 && !(frag1.w < MT::min_alpha)) commit(j1, depth1, frag1);
+        auto prim_of = [&](const uint32_t* prims, uint32_t j) -> uint32_t { return SL::has_prim ? prims[j] : 0u; };
+        if (step) {        // until no lane has a candidate of the older half left
+            while (__any_sync(0xffffffffu, window >= 0x10000u)) {
+                bool v0, v1;
+                const uint32_t j0 = pop_candidate(v0);
+                const uint32_t j1 = pop_candidate(v1);
+                float depth0, depth1;
+                float4 frag0, frag1;
+                evaluate(s_rec + j0, s_ctr[j0], depth0, frag0);
+                evaluate(s_rec + j1, s_ctr[j1], depth1, frag1);
+                if (v0 && !(frag0.w < MT::min_alpha)) commit(prim_of(s_prim, j0), depth0, frag0);
+                if (v1 && !(frag1.w < MT::min_alpha)) commit(prim_of(s_prim, j1), depth1, frag1);
+            }
+            window <<= 16;
+            half ^= 1u;
         }
-        window <<= 16;
+        if (n_dense != 0) {
+            if (!mbar_wait_bounded(s_bar + 2, (phases >> 2) & 1u)) wait_failed = true;
+            phases ^= 4u;
+            __syncwarp();
+            for (uint32_t j = 0; j < n_dense; j += 2) {
+                const uint32_t k = min(j + 1, n_dense - 1);
+                const bool v0 = inside && ((s_dense_mask[j] >> lane) & 1u), v1 = inside && j + 1 < n_dense && ((s_dense_mask[k] >> lane) & 1u);
+                float depth0, depth1;
+                float4 frag0, frag1;
+                evaluate(s_dense + j, s_dense_ctr[j], depth0, frag0);
+                evaluate(s_dense + k, s_dense_ctr[k], depth1, frag1);
+                if (v0 && !(frag0.w < MT::min_alpha)) commit(prim_of(s_dense_prim, j), depth0, frag0);
+                if (v1 && !(frag1.w < MT::min_alpha)) commit(prim_of(s_dense_prim, k), depth1, frag1);
+            }
+            __syncwarp();
+        }
     }
 
     if (wait_failed) atomicOr(&status->error, 1u);
