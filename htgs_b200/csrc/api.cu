@@ -841,19 +841,8 @@ int htgs::backward_with_accum(HtgsContext* ctx, const HtgsScene* scene, const Ht
                         grads->densification_info, grads->densification_info ? grads->densification_rows : 0, grads->use_distance_scaling != 0};
     out.compact_rows = static_cast<float4*>(compact_rows);
     out.compact_capacity = compact_capacity;
-    // The six gradient tensors are only written after the per-tile kernel (2 ms of arithmetic), so they are cleared (0.7 GB at
-    // configuration 2) on the context's side stream meanwhile, ordered after whatever the caller queued before this call.
-    cudaEvent_t outputs_cleared = nullptr;
-    if (ctx->front_priority && count > 0 && accumulate && (!compact_rows || dense_given)) {
-        cudaError_t e;
-        if ((e = cudaEventRecord(ctx->front_begin, stream)) != cudaSuccess) return fail_cuda(e, "front event record");
-        if ((e = cudaStreamWaitEvent(ctx->front_stream, ctx->front_begin, 0)) != cudaSuccess) return fail_cuda(e, "front stream wait");
-        if ((e = clear_backward_outputs(*scene, out, first, count, ctx->front_stream)) != cudaSuccess) return fail_cuda(e, "clearing the gradient tensors");
-        if ((e = cudaEventRecord(ctx->front_end, ctx->front_stream)) != cudaSuccess) return fail_cuda(e, "front event record");
-        outputs_cleared = ctx->front_end;
-    }
     const cudaError_t err = launch_backward(view->mode, view->K, *scene, *view, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order,
-                                            X.px, grad_image, image, acc, out, outputs_cleared, ctx->sm_count, first, count, stages, stream);
+                                            X.px, grad_image, image, acc, out, P.status, ctx->sm_count, first, count, stages, stream);
     if (err != cudaSuccess) return fail_cuda(err, "backward");
     return HTGS_OK;
 }

@@ -154,11 +154,11 @@ struct BackwardOutputs {
 cudaError_t launch_visibility(const uint32_t* n_touched, uint8_t* visible, uint32_t n, cudaStream_t stream);
 cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const PrimBuffers& prim,
                             const uint32_t* prims_sorted, const uint2* tile_ranges, const uint32_t* tile_order, const TrainPixelBuffers& tin, const float* grad_image,
-                            const float* image, const GradAccumBuffers& acc, const BackwardOutputs& out, cudaEvent_t outputs_cleared, int sm_count,
+                            const float* image, const GradAccumBuffers& acc, const BackwardOutputs& out, const FrameStatus* status, int sm_count,
                             uint32_t first, uint32_t count, int stages, cudaStream_t stream);
 // `stages`: kBackwardAccumulate = the per-tile (per-pixel for GLOBAL_ORDERING) pass that accumulates one record per Gaussian,
 // kBackwardChainRule = the per-Gaussian kernel that turns the records into the six gradients; both for a whole backward pass.
-// `outputs_cleared`: event after which rows [first, first + count) of the six tensors are zero, or null to clear them here.
+// `status`: the forward pass's (in the per-Gaussian blob).
 // [first, first + count): the Gaussians whose gradients the call computes (everything else is left untouched); a proper part
 // of the scene is refused (cudaErrorNotSupported) for GLOBAL_ORDERING.
 cudaError_t clear_backward_outputs(const HtgsScene& scene, const BackwardOutputs& out, uint32_t first, uint32_t count, cudaStream_t stream);
