@@ -693,7 +693,7 @@ __device__ __forceinline__ float4 quat_backward(const float4& q, const float (&d
 // the ranks of a multi-GPU trainer send one another instead of the dense rows.
 constexpr int kChainThreads = 128;
 template <bool COMPACT>
-__global__ void __launch_bounds__(kChainThreads) preprocess_backward_kernel(
+__global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ scales, const float* __restrict__ rotations, const float* __restrict__ sh_rest,
     const float* __restrict__ M, const float* __restrict__ VPM, const float* __restrict__ cam_position_ptr,
     const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const CullRecord* __restrict__ cull, const uint8_t* __restrict__ clamp,
