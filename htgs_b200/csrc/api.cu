@@ -147,7 +147,7 @@ struct PendingFrame {
 struct HtgsContext {
     int device = 0;
     int sm_count = 0;
-    FrameStatus* host_status = nullptr;     // pinned
+    FrameStatus* host_status = nullptr;     // pinned: [0] frames and the first half of a training forward, [1] a training forward that is not waited for
     void* workspace = nullptr;              // internal grow-only workspace
     size_t workspace_bytes = 0;
     uint64_t instance_capacity = 0;         // capacity the internal workspace was last carved for
@@ -165,6 +165,10 @@ struct HtgsContext {
     // the frame whose status has not been read yet (htgs_render_async)
     PendingFrame pending{};
     cudaEvent_t frame_done = nullptr;       // recorded after the status copy of a frame
+    // the training forward whose status has not been read yet (htgs_forward_finish_async)
+    bool training_pending = false;
+    cudaEvent_t training_done = nullptr;
+    uint32_t training_visible = 0;          // of the last htgs_forward_begin
     // measurement aids
     bool profiling = false;
     bool collect_stats = false;
@@ -189,8 +193,19 @@ void set_last_error(const char* message) { g_last_error = message ? message : ""
 
 static int finish_frame(HtgsContext* ctx, HtgsFrameInfo* info);
 
-// A call on a context whose previous frame was queued with htgs_render_async checks that frame first.
+static int check_training(HtgsContext* ctx) {
+    if (!ctx->training_pending) return HTGS_OK;
+    ctx->training_pending = false;
+    const cudaError_t err = cudaEventSynchronize(ctx->training_done);
+    if (err != cudaSuccess) return fail_cuda(err, "deferred check of a training forward");
+    if (ctx->host_status[1].error) return fail(HTGS_ERR_DEVICE_FLAG, "deferred check of a training forward: a kernel reported an internal error (bounded wait gave up)");
+    return HTGS_OK;
+}
+
+// A call on a context whose previous frame or training forward was queued without a wait checks it first.
 static int settle_pending(HtgsContext* ctx) {
+    const int training = check_training(ctx);
+    if (training != HTGS_OK) return training;
     if (!ctx->pending.active) return HTGS_OK;
     const int rc = finish_frame(ctx, nullptr);
     if (rc != HTGS_OK) g_last_error = "deferred check of the previous frame: " + g_last_error;
@@ -217,17 +232,18 @@ HtgsContext* htgs_create(int device) {
     ctx->device = device;
     ctx->sm_count = prop.multiProcessorCount;
     int least = 0, greatest = 0;
-    if ((err = cudaHostAlloc(reinterpret_cast<void**>(&ctx->host_status), sizeof(FrameStatus), cudaHostAllocDefault)) != cudaSuccess ||
+    if ((err = cudaHostAlloc(reinterpret_cast<void**>(&ctx->host_status), 2 * sizeof(FrameStatus), cudaHostAllocDefault)) != cudaSuccess ||
         (err = cudaDeviceGetStreamPriorityRange(&least, &greatest)) != cudaSuccess ||
         (err = cudaStreamCreateWithPriority(&ctx->front_stream, cudaStreamNonBlocking, greatest)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->front_begin, cudaEventDisableTiming)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->front_end, cudaEventDisableTiming)) != cudaSuccess ||
-        (err = cudaEventCreateWithFlags(&ctx->frame_done, cudaEventDisableTiming)) != cudaSuccess) {
+        (err = cudaEventCreateWithFlags(&ctx->frame_done, cudaEventDisableTiming)) != cudaSuccess ||
+        (err = cudaEventCreateWithFlags(&ctx->training_done, cudaEventDisableTiming)) != cudaSuccess) {
         fail_cuda(err, "htgs_create: pinned status word, side stream and events");
         htgs_destroy(ctx);
         return nullptr;
     }
-    std::memset(ctx->host_status, 0, sizeof(FrameStatus));
+    std::memset(ctx->host_status, 0, 2 * sizeof(FrameStatus));
     return ctx;
 }
 
@@ -235,6 +251,7 @@ void htgs_destroy(HtgsContext* ctx) {
     if (!ctx) return;
     DeviceGuard guard(ctx->device);
     if (ctx->pending.active) cudaEventSynchronize(ctx->frame_done);
+    if (ctx->training_pending) cudaEventSynchronize(ctx->training_done);
     if (ctx->workspace) cudaFree(ctx->workspace);
     if (ctx->host_path_buf) cudaFree(ctx->host_path_buf);
     if (ctx->host_path_stream) cudaStreamDestroy(ctx->host_path_stream);
@@ -244,6 +261,7 @@ void htgs_destroy(HtgsContext* ctx) {
     if (ctx->front_begin) cudaEventDestroy(ctx->front_begin);
     if (ctx->front_end) cudaEventDestroy(ctx->front_end);
     if (ctx->frame_done) cudaEventDestroy(ctx->frame_done);
+    if (ctx->training_done) cudaEventDestroy(ctx->training_done);
     delete ctx;
 }
 
@@ -705,11 +723,14 @@ int htgs_forward_begin(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
     if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(err, "synchronise");
     if (ctx->host_status->overflow) return fail(HTGS_ERR_INVALID_ARGUMENT, "instance count does not fit 32 bits");
     *n_instances = ctx->host_status->n_instances;
+    ctx->training_visible = ctx->host_status->n_visible;
     return HTGS_OK;
 }
 
-int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
-                        float* image, void* stream_ptr, HtgsFrameInfo* info) {
+}  // extern "C"
+
+static int forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
+                          float* image, void* stream_ptr, HtgsFrameInfo* info, bool wait) {
     if (!ctx || !blobs || !image) return fail(HTGS_ERR_INVALID_ARGUMENT, "null argument");
     int rc = validate(scene, view);
     if (rc != HTGS_OK) return rc;
@@ -733,16 +754,30 @@ int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView
     const BlendOutputs out{image, nullptr, nullptr, true, false, nullptr, 0.0f};
     if ((err = launch_blend(view->mode, BlendTask::training, *view, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order, out, X.px, P.status, stream)) != cudaSuccess)
         return fail_cuda(err, "blend");
-    if ((err = cudaMemcpyAsync(ctx->host_status, P.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
-    if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(err, "synchronise");
-    const FrameStatus st = *ctx->host_status;
+    if ((err = cudaMemcpyAsync(ctx->host_status + 1, P.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
+    if ((err = cudaEventRecord(ctx->training_done, stream)) != cudaSuccess) return fail_cuda(err, "training event record");
+    ctx->training_pending = true;
     if (info) {
         std::memset(info, 0, sizeof(*info));
-        info->n_instances = st.n_instances; info->n_visible = st.n_visible; info->key_bytes = uint32_t(plan.key_bytes); info->end_bit = uint32_t(plan.end_bit);
-        info->device_error = st.error; info->kernel_launches = launches + 4;
+        info->n_instances = n_instances; info->n_visible = ctx->training_visible; info->key_bytes = uint32_t(plan.key_bytes); info->end_bit = uint32_t(plan.end_bit);
+        info->kernel_launches = launches + 4;
     }
-    if (st.error) return fail(HTGS_ERR_DEVICE_FLAG, "a kernel reported an internal error (bounded wait gave up)");
-    return HTGS_OK;
+    if (!wait) return HTGS_OK;
+    rc = check_training(ctx);
+    if (info) info->device_error = ctx->host_status[1].error;
+    return rc;
+}
+
+extern "C" {
+
+int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
+                        float* image, void* stream_ptr, HtgsFrameInfo* info) {
+    return forward_finish(ctx, scene, view, blobs, n_instances, image, stream_ptr, info, true);
+}
+
+int htgs_forward_finish_async(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
+                              float* image, void* stream_ptr, HtgsFrameInfo* info) {
+    return forward_finish(ctx, scene, view, blobs, n_instances, image, stream_ptr, info, false);
 }
 
 size_t htgs_backward_scratch_bytes(const HtgsScene* scene) {
@@ -817,6 +852,7 @@ int htgs::backward_with_accum(HtgsContext* ctx, const HtgsScene* scene, const Ht
     if (rc != HTGS_OK) return rc;
     DeviceGuard guard(ctx->device);
     if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+    if (ctx->training_pending && cudaEventQuery(ctx->training_done) == cudaSuccess && (rc = check_training(ctx)) != HTGS_OK) return rc;
     if (view->mode == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING && !image) return fail(HTGS_ERR_INVALID_ARGUMENT, "ALPHA_BLEND_GLOBAL_ORDERING needs the forward image");
     if (compact_rows && (reinterpret_cast<uintptr_t>(compact_rows) & 15u) != 0) return fail(HTGS_ERR_INVALID_ARGUMENT, "the compact row buffer must be 16-byte aligned");
     const bool dense_given = grads->grad_positions || grads->grad_scales || grads->grad_rotations || grads->grad_opacities || grads->grad_sh_0 || grads->grad_sh_rest;

@@ -222,7 +222,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int, int> forward(
     Tensor per_instance = bytes_on(a.device, pi_bytes);
     HtgsTrainBlobs blobs{per_primitive.data_ptr(), pp_bytes, per_tile.data_ptr(), pt_bytes, per_instance.data_ptr(), pi_bytes, per_pixel.data_ptr(), px_bytes};
     HtgsFrameInfo info{};
-    check(htgs_forward_finish(ctx, &a.scene, &a.view, &blobs, n_instances, image.data_ptr<float>(), stream, &info));
+    check(htgs_forward_finish_async(ctx, &a.scene, &a.view, &blobs, n_instances, image.data_ptr<float>(), stream, &info));
     tls.last_info = info;
     return {image, per_primitive, per_tile, per_instance, per_pixel, int(n_instances), 0};
 }

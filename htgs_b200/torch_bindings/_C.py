@@ -169,7 +169,7 @@ def forward(positions, scales, rotations, opacities, sh_0, sh_rest, M, VPM, cam_
         blobs = _native.HtgsTrainBlobs(per_primitive.data_ptr(), per_primitive.numel(), per_tile.data_ptr(), per_tile.numel(),
                                        per_instance.data_ptr(), per_instance.numel(), per_pixel.data_ptr(), per_pixel.numel())
         info = HtgsFrameInfo()
-        _native.check(lib.htgs_forward_finish(ctx, ctypes.byref(scene), ctypes.byref(view), ctypes.byref(blobs), n_inst.value, image.data_ptr(), stream,
+        _native.check(lib.htgs_forward_finish_async(ctx, ctypes.byref(scene), ctypes.byref(view), ctypes.byref(blobs), n_inst.value, image.data_ptr(), stream,
                                               ctypes.byref(info)))
     _set_info(info)
     return image, per_primitive, per_tile, per_instance, per_pixel, int(n_inst.value), 0

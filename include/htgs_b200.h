@@ -191,6 +191,11 @@ int htgs_forward_begin(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
                        void* stream, uint32_t* n_instances);
 int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
                         float* image, void* stream, HtgsFrameInfo* info);
+/* The same without waiting for the GPU: the call returns when everything is queued, so that the caller can queue the loss and the
+ * backward pass while the forward runs.  Its status is checked by the next call on the context that has to wait anyway, or by
+ * htgs_backward if the forward has finished by then; a device error is reported by that call (HTGS_ERR_DEVICE_FLAG). */
+int htgs_forward_finish_async(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
+                              float* image, void* stream, HtgsFrameInfo* info);
 
 /* Outputs of the backward pass.  Every element of the six gradient tensors is written (zeros for culled
  * Gaussians), so they need not be cleared.  `scratch` (htgs_backward_scratch_bytes) holds the per-Gaussian
