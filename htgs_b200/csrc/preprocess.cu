@@ -175,6 +175,29 @@ __device__ __forceinline__ void make_fast_record(const float4& t1, const float4&
     for (int i = 0; i < 5; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
 }
 
+// The point from which the backward pass measures the pixels of a Gaussian: the centre of the outline, or, where that lies outside the
+// Gaussian's tile box (centres far off the screen belong to long or near Gaussians), the point of the box where the outline's form is
+// smallest.  From a far centre the moments of train.cu would cancel: 5e-5 of a gradient instead of a few 1e-6.
+template <int MODE>
+__device__ __forceinline__ float2 make_moment_centre(const CullRecord& cr, const ushort4& box) {
+    using MT = ModeTraits<MODE>;
+    const float x0 = float(box.x) * MT::tile_w, x1 = float(box.y) * MT::tile_w - 1.0f, y0 = float(box.z) * MT::tile_h, y1 = float(box.w) * MT::tile_h - 1.0f;
+    if (cr.cx >= x0 && cr.cx <= x1 && cr.cy >= y0 && cr.cy <= y1 && cr.a != 0.0f) return make_float2(cr.cx, cr.cy);
+    float2 best = make_float2(0.5f * (x0 + x1), 0.5f * (y0 + y1));
+    if (cr.a == 0.0f || !(fabsf(cr.cx) <= FLT_MAX)) return best;
+    float smallest = FLT_MAX;
+    auto consider = [&](float x, float y) {
+        const float dx = x - cr.cx, dy = y - cr.cy, q = dx * (cr.a * dx + cr.b2 * dy) + cr.c * dy * dy;
+        if (q < smallest) { smallest = q; best = make_float2(x, y); }
+    };
+    const float along_y = -0.5f * cr.b2 / cr.c, along_x = -0.5f * cr.b2 / cr.a;      // where the form is smallest along an edge, per unit of the other coordinate
+    consider(x0, fminf(fmaxf(fmaf(along_y, x0 - cr.cx, cr.cy), y0), y1));
+    consider(x1, fminf(fmaxf(fmaf(along_y, x1 - cr.cx, cr.cy), y0), y1));
+    consider(fminf(fmaxf(fmaf(along_x, y0 - cr.cy, cr.cx), x0), x1), y0);
+    consider(fminf(fmaxf(fmaf(along_x, y1 - cr.cy, cr.cx), x0), x1), y1);
+    return best;
+}
+
 // Pass 1, one thread per Gaussian: culling, tile box, and the rows VPMT1, VPMT2, VPMT4, MT3 (written where the
 // evaluation record lives).  The visible Gaussians of a block are appended to `visible_list` (the order of the list
 // depends on the order in which blocks finish; nothing downstream depends on it).
@@ -300,8 +323,11 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
         [[maybe_unused]] double centre[2] = {0.0, 0.0};
         if constexpr (FAST) make_fast_record(t1, t2, t4, m3, rgb, opacity, dst, centre);
         else dst[4] = make_float4(rgb.x, rgb.y, rgb.z, opacity);
-        if constexpr (TRAIN) out.clamp[gi] = clamp_bits;
         CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
+        if constexpr (TRAIN) {
+            out.clamp[gi] = clamp_bits;
+            out.moment_centre[gi] = make_moment_centre<MODE>(cr, out.bounds[gi]);
+        }
         if constexpr (FAST) {
             // The fragment evaluation measures from the projected centre, the outline test from the centre of
             // the outline: the record carries the (small) difference, so that outline centre + difference

@@ -42,8 +42,8 @@ __device__ __forceinline__ float rcp_approx(float x) { float y; asm("rcp.approx.
 __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f)); return y; }
 
 // The gradient of rho^2 = N / D, N = |m|^2, D = |d|^2, w.r.t. the rows VPMT1, VPMT2, VPMT4 (hybrid_blend/kernels/backward.cuh:258-285), in moments.
-// Along a Gaussian's pixels m and d are affine and N and D quadratic in (x, y) = pixel - centre, the centre of its outline
-// record, and as well in (s, y) with the sheared s = x + shear * y:  m = M0 + s Ms + y My,  d = D0 + s Ds + y Dy  (AffinePlanes).
+// Along a Gaussian's pixels m and d are affine and N and D quadratic in (x, y) = pixel - centre, a point that the
+// preprocess chose (make_moment_centre), and as well in (s, y) with the sheared s = x + shear * y:  m = M0 + s Ms + y My,  d = D0 + s Ds + y Dy  (AffinePlanes).
 // The shear makes Ms and My orthogonal: however long and slanted the ellipse, the terms of m do not cancel.  The rows' gradients
 // are quadratic in (s, y) too, with coefficients that are the Gaussian's alone, so a pair only adds
 //     u = dL/drho^2 / D  and  v = u N / D,  each times  1, s, y, ss, sy, yy
@@ -187,7 +187,7 @@ template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
 template <int MODE, int K, bool ABS_GRAD>
 __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_blocks)) backward_tile_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
-    const CullRecord* __restrict__ cull, TrainPixelBuffers tin, const float* __restrict__ grad_image, const float* __restrict__ VPM,
+    const CullRecord* __restrict__ cull, const float2* __restrict__ moment_centre, TrainPixelBuffers tin, const float* __restrict__ grad_image, const float* __restrict__ VPM,
     float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w, uint32_t g_first, uint32_t g_end)
 {
     using MT = ModeTraits<MODE>;
@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     // batch b + 2 and the indices of batch b + 3.
     uint32_t g_rec = 0, g_out = 0, g_idx = 0;
     float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1, outline = rT1;
-    float rcx = 0.0f, rcy = 0.0f, outline_c = 0.0f;
+    float2 centre = make_float2(0.0f, 0.0f);
+    float outline_c = 0.0f;
     uint64_t mask_rec = 0;
     auto load_index = [&](uint32_t inst) { return inst < range.y ? __ldg(prims_sorted + inst) : 0u; };
     auto request_outline = [&](uint32_t inst) {
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         if (inst < range.y) mask_rec = (uint64_t(outline_mask(outline, outline_c, x0, y0)) | (uint64_t(outline_mask(outline, outline_c, x0, y0 + 4.0f)) << 32)) & inside_mask;
         if (mask_rec == 0) return;
         g_rec = g_out;
-        rcx = outline.x; rcy = outline.y;
+        centre = __ldg(moment_centre + g_rec);
         const float* rec = reinterpret_cast<const float*>(eval + g_rec);
         rT1 = ldg4(rec); rT2 = ldg4(rec + 4); rT4 = ldg4(rec + 8); rRGBA = ldg4(rec + 16);
     };
@@ -351,13 +352,13 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         const uint32_t inst = batch_begin + tid;
         uint64_t my_mask = mask_rec;
         if (my_mask != 0) {
-            const AffinePlanes planes = affine_planes(rT1, rT2, rT4, rcx, rcy);
+            const AffinePlanes planes = affine_planes(rT1, rT2, rT4, centre.x, centre.y);
             const PairForm form = pair_form(planes);
             s_n0[tid] = form.n0; s_n1[tid] = form.n1; s_d1[tid] = form.d1; s_rgba[tid] = rRGBA;
             float level = 0.0f;
             if constexpr (!kFirstK) level = acceptance_level<MT>(rRGBA.w);
             const float band = kLevelBand * level + 1e-6f;
-            s_pos[tid] = make_float4(x0 - rcx, y0 - rcy, level - band, planes.shear);
+            s_pos[tid] = make_float4(x0 - centre.x, y0 - centre.y, level - band, planes.shear);
             if constexpr (ABS_GRAD) {
                 const AbsForm af = abs_form(planes, rT4);
                 s_abs[tid] = af.y0; s_abs[NT + tid] = af.x0; s_abs[2 * NT + tid] = af.y1x1;
@@ -491,7 +492,7 @@ constexpr int kGoQueue = 64;
 template <bool ABS_GRAD>
 __global__ void __launch_bounds__(32) backward_global_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
-    const CullRecord* __restrict__ cull, const float* __restrict__ grad_image, const float* __restrict__ image, const float* __restrict__ VPM,
+    const CullRecord* __restrict__ cull, const float2* __restrict__ moment_centre, const float* __restrict__ grad_image, const float* __restrict__ image, const float* __restrict__ VPM,
     float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w)
 {
     using MT = ModeTraits<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING>;
@@ -552,7 +553,8 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
     // the record of the survivor this lane stages (both half warps hold the same 16)
     const uint32_t mine = lane & uint32_t(kGoChunk - 1);
     uint32_t g_mine = 0, mask_mine = 0, count = 0;
-    float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1, centre = rT1;
+    float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1;
+    float2 centre = make_float2(0.0f, 0.0f);
     auto take = [&]() {                                  // the next chunk: indices, masks, and requests for its records
         while (queued < kGoChunk && next - lane < range.y) filter();
         __syncwarp();
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
             mask_mine = s_queue_mask[at];
             const float* rec = reinterpret_cast<const float*>(eval + g_mine);
             rT1 = ldg4(rec); rT2 = ldg4(rec + 4); rT4 = ldg4(rec + 8); rRGBA = ldg4(rec + 16);
-            centre = ldg4(reinterpret_cast<const float*>(cull + g_mine));
+            centre = __ldg(moment_centre + g_mine);
         }
         queue_head += count;
         queued -= count;
@@ -696,7 +698,7 @@ template <bool COMPACT>
 __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ scales, const float* __restrict__ rotations, const float* __restrict__ sh_rest,
     const float* __restrict__ M, const float* __restrict__ VPM, const float* __restrict__ cam_position_ptr,
-    const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const CullRecord* __restrict__ cull, const uint8_t* __restrict__ clamp,
+    const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const float2* __restrict__ moment_centre, const uint8_t* __restrict__ clamp,
     const float4* __restrict__ accum, BackwardOutputs out,
     uint32_t n_primitives, int active_sh_bases, int total_sh_bases, uint32_t g_first, uint32_t g_end)
 {
@@ -720,8 +722,7 @@ __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const PairMoments moments{accum[size_t(idx) * 5], accum[size_t(idx) * 5 + 1], accum[size_t(idx) * 5 + 2]};
     const float4 dC = accum[size_t(idx) * 5 + 3];
     const float4 T4 = ldg4(reinterpret_cast<const float*>(eval + idx) + 8);
-    float2 centre = __ldg(reinterpret_cast<const float2*>(cull + idx));
-    if (!(fabsf(centre.x) <= FLT_MAX)) centre = make_float2(0.0f, 0.0f);       // nothing of the Gaussian can be accepted: its moments are zero
+    const float2 centre = __ldg(moment_centre + idx);
     const RowGradients rows = rows_from_moments(affine_planes(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
                                                               centre.x, centre.y), T4, moments);
     // dL/dVPMT4 = -(cx dL/dVPMT1 + cy dL/dVPMT2 + E): the products with the centre are moved to the rows of VPM, where they cancel
@@ -871,7 +872,7 @@ cudaError_t launch_tile_backward(bool abs_grad, const FrameGeometry& geo, const 
             const cudaError_t err = configured[abs_grad ? 1 : 0].run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); });
             if (err != cudaSuccess) return err;
         }
-        kernel<<<uint32_t(geo.n_tiles), kBwdThreads, smem, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, tin, grad_image, VPM, accum,
+        kernel<<<uint32_t(geo.n_tiles), kBwdThreads, smem, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, prim.moment_centre, tin, grad_image, VPM, accum,
                                                 uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w), g_first, g_end);
         return cudaGetLastError();
     };
@@ -934,12 +935,12 @@ cudaError_t launch_chain_rule(const HtgsScene& scene, const HtgsView& view, cons
         const cudaError_t err = cudaMemsetAsync(out.compact_rows, 0, sizeof(CompactGradientHeader), stream);
         if (err != cudaSuccess) return err;
         preprocess_backward_kernel<true><<<grid, kChainThreads, 0, stream>>>(scene.positions, scene.scales, scene.rotations, scene.sh_rest, view.M, view.VPM,
-                                                                             view.cam_position, prim.n_touched, prim.eval, prim.cull, prim.clamp, acc.accum, out, n,
+                                                                             view.cam_position, prim.n_touched, prim.eval, prim.moment_centre, prim.clamp, acc.accum, out, n,
                                                                              view.active_sh_bases, scene.total_sh_bases, first, first + count);
     } else {
         const size_t smem = size_t(kChainThreads) * 3 * size_t(scene.total_sh_bases < 15 ? scene.total_sh_bases : 15) * sizeof(float);
         preprocess_backward_kernel<false><<<grid, kChainThreads, smem, stream>>>(scene.positions, scene.scales, scene.rotations, scene.sh_rest, view.M, view.VPM,
-                                                                                 view.cam_position, prim.n_touched, prim.eval, prim.cull, prim.clamp, acc.accum, out, n,
+                                                                                 view.cam_position, prim.n_touched, prim.eval, prim.moment_centre, prim.clamp, acc.accum, out, n,
                                                                                  view.active_sh_bases, scene.total_sh_bases, first, first + count);
     }
     return cudaGetLastError();
@@ -980,7 +981,7 @@ cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsV
             err = launch_tile_backward<HTGS_MODE_OIT_BLEND, 1>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
         case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: {
             const auto kernel = abs_grad ? backward_global_kernel<true> : backward_global_kernel<false>;
-            kernel<<<uint32_t(geo.n_tiles) * 8u, 32, 0, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, grad_image, image, view.VPM, acc.accum,
+            kernel<<<uint32_t(geo.n_tiles) * 8u, 32, 0, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, prim.moment_centre, grad_image, image, view.VPM, acc.accum,
                                                                   uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w));
             err = cudaGetLastError();
             break;
