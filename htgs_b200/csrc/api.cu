@@ -627,7 +627,7 @@ PrimLayout carve_primitive_blob(void* blob, int n_primitives) {
     L.prim.block_sums = c.take<uint32_t>(prim_blocks + 1);
     L.prim.block_offsets = c.take<uint32_t>(prim_blocks + 1);
     L.prim.visible_list = c.take<uint32_t>(n);
-    L.prim.moment_centre = c.take<float2>(n);
+    L.prim.pair = c.take<PairRecord>(n);
     L.bytes = align_up(c.offset);
     return L;
 }

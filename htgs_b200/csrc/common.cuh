@@ -105,6 +105,15 @@ struct __align__(16) FastRecord {
 };
 static_assert(sizeof(FastRecord) == sizeof(EvalRecord), "FastRecord shares the storage of EvalRecord");
 
+// What the backward pass evaluates a pair with (training only).  rho^2 = N / D (both up to a factor that cancels), N = |m|^2 and D = |d|^2
+// quadratic in (s, y): y = pixel_y - cy, s = pixel_x - cx + shear * y.  Computed in float64: a rounding of a coefficient is the
+// same at every pixel and does not average out in a gradient that sums thousands of them.
+struct __align__(16) PairRecord {
+    float4 n0, n1, d1;        // n0 = N: 1, s, y, ss   n1 = N: sy, yy, D: 1, s   d1 = D: y, ss, sy, yy
+    float cx, cy, shear, pad;
+};
+static_assert(sizeof(PairRecord) == 64, "PairRecord must be 64 bytes");
+
 // Device-resident frame status, copied to the host at the end of a call.
 struct FrameStatus {
     unsigned int n_instances;     // total (tile, Gaussian) instances of the frame

@@ -32,7 +32,7 @@ struct PrimBuffers {
     ushort4* bounds;          // [N] x_min,x_max,y_min,y_max in tiles
     EvalRecord* eval;         // [N]
     CullRecord* cull;         // [N]
-    float2* moment_centre;    // [N] point the backward pass measures pixels from (training only, else null)
+    PairRecord* pair;         // [N] (training only, else null)
     uint8_t* clamp;           // [N] bit c set: colour channel c was clamped at 0 (training only, else null)
     uint32_t* block_sums;     // [ceil(N/256)] instances emitted by each block of 256 Gaussians
     uint32_t* block_offsets;  // [ceil(N/256)] exclusive prefix of block_sums

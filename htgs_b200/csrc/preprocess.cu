@@ -198,6 +198,36 @@ __device__ __forceinline__ float2 make_moment_centre(const CullRecord& cr, const
     return best;
 }
 
+// m = M0 + x Mx + y My and d = D0 + x Dx + y Dy about the centre (train.cu: AffinePlanes); the shear makes the two slopes of m orthogonal.
+__device__ __forceinline__ PairRecord make_pair_record(const float4& t1, const float4& t2, const float4& t4, const float2& centre) {
+    struct D3 { double x, y, z; };
+    auto cross3 = [](const D3& a, const D3& b) { return D3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; };
+    auto dot3 = [](const D3& a, const D3& b) { return a.x * b.x + a.y * b.y + a.z * b.z; };
+    auto comb = [](double p, const D3& a, double q, const D3& b) { return D3{p * a.x + q * b.x, p * a.y + q * b.y, p * a.z + q * b.z}; };
+    const double cx = double(centre.x), cy = double(centre.y), w = double(t4.w);
+    const D3 n{double(t4.x), double(t4.y), double(t4.z)};
+    const D3 a{double(t1.x) - cx * n.x, double(t1.y) - cx * n.y, double(t1.z) - cx * n.z};
+    const D3 b{double(t2.x) - cy * n.x, double(t2.y) - cy * n.y, double(t2.z) - cy * n.z};
+    const double aw = double(t1.w) - cx * w, bw = double(t2.w) - cy * w;
+    const D3 m0 = comb(aw, b, -bw, a), ms = comb(bw, n, -w, b);
+    D3 my = comb(w, a, -aw, n);
+    const D3 d0 = cross3(a, b), ds = cross3(b, n);
+    D3 dy = cross3(n, a);
+    const double ms_sq = dot3(ms, ms);
+    float shear = ms_sq > 0.0 ? float(dot3(ms, my) / ms_sq) : 0.0f;
+    if (!(fabsf(shear) < 1e6f)) shear = 0.0f;
+    my = comb(1.0, my, -double(shear), ms);
+    dy = comb(1.0, dy, -double(shear), ds);
+    // N and D grow with the fourth power of sizes in pixels: both are divided by D0
+    const double scale = 1.0 / fmax(dot3(d0, d0), 1e-300);
+    PairRecord r;
+    r.n0 = make_float4(float(scale * dot3(m0, m0)), float(2.0 * scale * dot3(m0, ms)), float(2.0 * scale * dot3(m0, my)), float(scale * dot3(ms, ms)));
+    r.n1 = make_float4(float(2.0 * scale * dot3(ms, my)), float(scale * dot3(my, my)), float(scale * dot3(d0, d0)), float(2.0 * scale * dot3(d0, ds)));
+    r.d1 = make_float4(float(2.0 * scale * dot3(d0, dy)), float(scale * dot3(ds, ds)), float(2.0 * scale * dot3(ds, dy)), float(scale * dot3(dy, dy)));
+    r.cx = centre.x; r.cy = centre.y; r.shear = shear; r.pad = float(scale);
+    return r;
+}
+
 // Pass 1, one thread per Gaussian: culling, tile box, and the rows VPMT1, VPMT2, VPMT4, MT3 (written where the
 // evaluation record lives).  The visible Gaussians of a block are appended to `visible_list` (the order of the list
 // depends on the order in which blocks finish; nothing downstream depends on it).
@@ -326,7 +356,9 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
         CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
         if constexpr (TRAIN) {
             out.clamp[gi] = clamp_bits;
-            out.moment_centre[gi] = make_moment_centre<MODE>(cr, out.bounds[gi]);
+            const PairRecord pair = make_pair_record(t1, t2, t4, make_moment_centre<MODE>(cr, out.bounds[gi]));
+            float4* pdst = reinterpret_cast<float4*>(out.pair + gi);
+            pdst[0] = pair.n0; pdst[1] = pair.n1; pdst[2] = pair.d1; pdst[3] = make_float4(pair.cx, pair.cy, pair.shear, pair.pad);
         }
         if constexpr (FAST) {
             // The fragment evaluation measures from the projected centre, the outline test from the centre of

@@ -43,15 +43,15 @@ __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.
 
 // The gradient of rho^2 = N / D, N = |m|^2, D = |d|^2, w.r.t. the rows VPMT1, VPMT2, VPMT4 (hybrid_blend/kernels/backward.cuh:258-285), in moments.
 // Along a Gaussian's pixels m and d are affine and N and D quadratic in (x, y) = pixel - centre, a point that the
-// preprocess chose (make_moment_centre), and as well in (s, y) with the sheared s = x + shear * y:  m = M0 + s Ms + y My,  d = D0 + s Ds + y Dy  (AffinePlanes).
+// preprocess chose (make_moment_centre; PairRecord has the coefficients), and as well in (s, y) with the sheared s = x + shear * y:  m = M0 + s Ms + y My,  d = D0 + s Ds + y Dy  (AffinePlanes).
 // The shear makes Ms and My orthogonal: however long and slanted the ellipse, the terms of m do not cancel.  The rows' gradients
 // are quadratic in (s, y) too, with coefficients that are the Gaussian's alone, so a pair only adds
-//     u = dL/drho^2 / D  and  v = u N / D,  each times  1, s, y, ss, sy, yy
+//     u = dL/drho^2 / D  (times D at the centre, which the record divides by)  and  v = u N / D,  each times  1, s, y, ss, sy, yy
 // to the Gaussian's record, and rows_from_moments applies the coefficients once per Gaussian.  That is 18 instructions per pair
 // instead of 54 for the rows themselves, and offsets from the centre keep the sums well conditioned, where the rows' sums hold products with
 // pixel coordinates that cancel later.
 struct AffinePlanes { float3 M0, Ms, My, D0, Ds, Dy; float4 A, B; float shear; };     // A = VPMT1 - cx VPMT4, B = VPMT2 - cy VPMT4
-__device__ __forceinline__ AffinePlanes affine_planes(const float4& T1, const float4& T2, const float4& T4, float cx, float cy) {
+__device__ __forceinline__ AffinePlanes affine_planes(const float4& T1, const float4& T2, const float4& T4, float cx, float cy, float shear) {
     AffinePlanes p;
     p.A = make_float4(fmaf(-cx, T4.x, T1.x), fmaf(-cx, T4.y, T1.y), fmaf(-cx, T4.z, T1.z), fmaf(-cx, T4.w, T1.w));
     p.B = make_float4(fmaf(-cy, T4.x, T2.x), fmaf(-cy, T4.y, T2.y), fmaf(-cy, T4.z, T2.z), fmaf(-cy, T4.w, T2.w));
@@ -62,25 +62,13 @@ __device__ __forceinline__ AffinePlanes affine_planes(const float4& T1, const fl
     p.D0 = cross(a, b);
     p.Ds = cross(b, n);
     p.Dy = cross(n, a);
-    const float ms_sq = dot(p.Ms, p.Ms);
-    p.shear = ms_sq > 0.0f ? __fdividef(dot(p.Ms, p.My), ms_sq) : 0.0f;
-    if (!(fabsf(p.shear) < 1e6f)) p.shear = 0.0f;
+    p.shear = shear;
     p.My = p.My - p.shear * p.Ms;
     p.Dy = p.Dy - p.shear * p.Ds;
     return p;
 }
 
-// What the pair loops evaluate: N and D as quadratics about the centre, and how large rho^2 may be (forward's alpha and cutoff tests).
-struct PairForm {
-    float4 n0, n1, d1;     // n0 = N: 1, s, y, ss   n1 = N: sy, yy, D: 1, s   d1 = D: y, ss, sy, yy
-};
-__device__ __forceinline__ PairForm pair_form(const AffinePlanes& p) {
-    PairForm f;
-    f.n0 = make_float4(dot(p.M0, p.M0), 2.0f * dot(p.M0, p.Ms), 2.0f * dot(p.M0, p.My), dot(p.Ms, p.Ms));
-    f.n1 = make_float4(2.0f * dot(p.Ms, p.My), dot(p.My, p.My), dot(p.D0, p.D0), 2.0f * dot(p.D0, p.Ds));
-    f.d1 = make_float4(2.0f * dot(p.D0, p.Dy), dot(p.Ds, p.Ds), 2.0f * dot(p.Ds, p.Dy), dot(p.Dy, p.Dy));
-    return f;
-}
+struct PairForm { float4 n0, n1, d1; };      // of a PairRecord: N and D, both divided by D at the centre
 __device__ __forceinline__ void evaluate_pair(const PairForm& f, float s, float y, float& numerator, float& denominator) {
     const float ss = s * s, sy = s * y, yy = y * y;
     numerator = fmaf(f.n1.y, yy, fmaf(f.n1.x, sy, fmaf(f.n0.w, ss, fmaf(f.n0.z, y, fmaf(f.n0.y, s, f.n0.x)))));
@@ -147,11 +135,15 @@ __device__ __forceinline__ CameraCols load_camera_cols(const float* __restrict__
 }
 // Y . m and X . m (3-vectors) as quadratics about the centre; the fourth columns of a pair are 2u times these.
 struct AbsForm { float4 y0, x0, y1x1; };      // Y . m: 1, s, y, sy | X . m: 1, s, y, ss | Y . m: yy, X . m: sy, yy
-__device__ __forceinline__ AbsForm abs_form(const AffinePlanes& p, const float4& T4) {
+__device__ __forceinline__ AbsForm abs_form(const EvalRecord* rec, const float4& centre_shear_scale) {
+    const float* r = reinterpret_cast<const float*>(rec);
+    const float4 T4 = ldg4(r + 8);
+    const AffinePlanes p = affine_planes(ldg4(r), ldg4(r + 4), T4, centre_shear_scale.x, centre_shear_scale.y, centre_shear_scale.z);
     const float3 a = f3(p.A), b = f3(p.B), n = f3(T4);
+    const float scale = centre_shear_scale.w;
     const float nm0 = dot(n, p.M0), nms = dot(n, p.Ms), nmy = dot(n, p.My);
-    return {make_float4(dot(b, p.M0), dot(b, p.Ms), dot(b, p.My) - nm0, -nms), make_float4(dot(a, p.M0), dot(a, p.Ms) - nm0, fmaf(p.shear, nm0, dot(a, p.My)), -nms),
-            make_float4(-nmy, fmaf(p.shear, nms, -nmy), p.shear * nmy, 0.0f)};
+    return {scale * make_float4(dot(b, p.M0), dot(b, p.Ms), dot(b, p.My) - nm0, -nms), scale * make_float4(dot(a, p.M0), dot(a, p.Ms) - nm0, fmaf(p.shear, nm0, dot(a, p.My)), -nms),
+            scale * make_float4(-nmy, fmaf(p.shear, nms, -nmy), p.shear * nmy, 0.0f)};
 }
 __device__ __forceinline__ float abs_position_gradient(const AbsForm& f, float u, float s, float y, float pixel_x, float pixel_y, const CameraCols& cam) {
     const float sy = s * y, yy = y * y;
@@ -187,7 +179,7 @@ template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
 template <int MODE, int K, bool ABS_GRAD>
 __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_blocks)) backward_tile_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
-    const CullRecord* __restrict__ cull, const float2* __restrict__ moment_centre, TrainPixelBuffers tin, const float* __restrict__ grad_image, const float* __restrict__ VPM,
+    const CullRecord* __restrict__ cull, const PairRecord* __restrict__ pair, TrainPixelBuffers tin, const float* __restrict__ grad_image, const float* __restrict__ VPM,
     float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w, uint32_t g_first, uint32_t g_end)
 {
     using MT = ModeTraits<MODE>;
@@ -234,8 +226,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     // give the pixel masks, the records of those instances that touch a pixel (six in ten) are requested, then the outlines of
     // batch b + 2 and the indices of batch b + 3.
     uint32_t g_rec = 0, g_out = 0, g_idx = 0;
-    float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1, outline = rT1;
-    float2 centre = make_float2(0.0f, 0.0f);
+    float4 rN0 = make_float4(0, 0, 0, 0), rN1 = rN0, rD1 = rN0, rC = rN0, rRGBA = rN0, outline = rN0;     // rC: centre, shear, 1 / D at the centre
     float outline_c = 0.0f;
     uint64_t mask_rec = 0;
     auto load_index = [&](uint32_t inst) { return inst < range.y ? __ldg(prims_sorted + inst) : 0u; };
@@ -249,9 +240,9 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         if (inst < range.y) mask_rec = (uint64_t(outline_mask(outline, outline_c, x0, y0)) | (uint64_t(outline_mask(outline, outline_c, x0, y0 + 4.0f)) << 32)) & inside_mask;
         if (mask_rec == 0) return;
         g_rec = g_out;
-        centre = __ldg(moment_centre + g_rec);
-        const float* rec = reinterpret_cast<const float*>(eval + g_rec);
-        rT1 = ldg4(rec); rT2 = ldg4(rec + 4); rT4 = ldg4(rec + 8); rRGBA = ldg4(rec + 16);
+        const float* rec = reinterpret_cast<const float*>(pair + g_rec);
+        rN0 = ldg4(rec); rN1 = ldg4(rec + 4); rD1 = ldg4(rec + 8); rC = ldg4(rec + 12);
+        rRGBA = ldg4(reinterpret_cast<const float*>(eval + g_rec) + 16);
     };
     g_out = load_index(range.x + tid);
     g_idx = load_index(range.x + NT + tid);
@@ -352,15 +343,13 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         const uint32_t inst = batch_begin + tid;
         uint64_t my_mask = mask_rec;
         if (my_mask != 0) {
-            const AffinePlanes planes = affine_planes(rT1, rT2, rT4, centre.x, centre.y);
-            const PairForm form = pair_form(planes);
-            s_n0[tid] = form.n0; s_n1[tid] = form.n1; s_d1[tid] = form.d1; s_rgba[tid] = rRGBA;
+            s_n0[tid] = rN0; s_n1[tid] = rN1; s_d1[tid] = rD1; s_rgba[tid] = rRGBA;
             float level = 0.0f;
             if constexpr (!kFirstK) level = acceptance_level<MT>(rRGBA.w);
             const float band = kLevelBand * level + 1e-6f;
-            s_pos[tid] = make_float4(x0 - centre.x, y0 - centre.y, level - band, planes.shear);
+            s_pos[tid] = make_float4(x0 - rC.x, y0 - rC.y, level - band, rC.z);
             if constexpr (ABS_GRAD) {
-                const AbsForm af = abs_form(planes, rT4);
+                const AbsForm af = abs_form(eval + g_rec, rC);
                 s_abs[tid] = af.y0; s_abs[NT + tid] = af.x0; s_abs[2 * NT + tid] = af.y1x1;
             }
             s_g[tid] = g_rec;
@@ -463,7 +452,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
                 aC.x += dL_drgb.x; aC.y += dL_drgb.y; aC.z += dL_drgb.z;
                 aC.w += dL_dalpha * G;
                 touched = true;
-                const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D
+                const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D, times D at the centre
                 add_moments(moments, u, u * rho2, s, y);
                 if constexpr (ABS_GRAD)
                     abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + column, y0 + row, cam);
@@ -492,7 +481,7 @@ constexpr int kGoQueue = 64;
 template <bool ABS_GRAD>
 __global__ void __launch_bounds__(32) backward_global_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
-    const CullRecord* __restrict__ cull, const float2* __restrict__ moment_centre, const float* __restrict__ grad_image, const float* __restrict__ image, const float* __restrict__ VPM,
+    const CullRecord* __restrict__ cull, const PairRecord* __restrict__ pair, const float* __restrict__ grad_image, const float* __restrict__ image, const float* __restrict__ VPM,
     float4* __restrict__ accum, uint32_t width, uint32_t height, uint32_t grid_w)
 {
     using MT = ModeTraits<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING>;
@@ -553,8 +542,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
     // the record of the survivor this lane stages (both half warps hold the same 16)
     const uint32_t mine = lane & uint32_t(kGoChunk - 1);
     uint32_t g_mine = 0, mask_mine = 0, count = 0;
-    float4 rT1 = make_float4(0, 0, 0, 0), rT2 = rT1, rT4 = rT1, rRGBA = rT1;
-    float2 centre = make_float2(0.0f, 0.0f);
+    float4 rN0 = make_float4(0, 0, 0, 0), rN1 = rN0, rD1 = rN0, rC = rN0, rRGBA = rN0;
     auto take = [&]() {                                  // the next chunk: indices, masks, and requests for its records
         while (queued < kGoChunk && next - lane < range.y) filter();
         __syncwarp();
@@ -564,9 +552,9 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
             const uint32_t at = (queue_head + mine) & uint32_t(kGoQueue - 1);
             g_mine = s_queue_prim[at];
             mask_mine = s_queue_mask[at];
-            const float* rec = reinterpret_cast<const float*>(eval + g_mine);
-            rT1 = ldg4(rec); rT2 = ldg4(rec + 4); rT4 = ldg4(rec + 8); rRGBA = ldg4(rec + 16);
-            centre = __ldg(moment_centre + g_mine);
+            const float* rec = reinterpret_cast<const float*>(pair + g_mine);
+            rN0 = ldg4(rec); rN1 = ldg4(rec + 4); rD1 = ldg4(rec + 8); rC = ldg4(rec + 12);
+            rRGBA = ldg4(reinterpret_cast<const float*>(eval + g_mine) + 16);
         }
         queue_head += count;
         queued -= count;
@@ -577,22 +565,18 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
         const uint32_t g = g_mine;
         // ---- 1. lane = survivor ------------------------------------------------------------------------------------
         [[maybe_unused]] AbsForm af{};
-        float shear = 0.0f;
         if (mine < count) {
-            const AffinePlanes planes = affine_planes(rT1, rT2, rT4, centre.x, centre.y);
             if (lane < kGoChunk) {
-                const PairForm form = pair_form(planes);
-                s_n0[mine] = form.n0; s_n1[mine] = form.n1; s_d1[mine] = form.d1; s_rgba[mine] = rRGBA;
+                s_n0[mine] = rN0; s_n1[mine] = rN1; s_d1[mine] = rD1; s_rgba[mine] = rRGBA;
                 const float level = acceptance_level<MT>(rRGBA.w);
                 const float band = kLevelBand * level + 1e-6f;
-                s_pos[mine] = make_float4(x0 - centre.x, y0 - centre.y, level - band, planes.shear);
+                s_pos[mine] = make_float4(x0 - rC.x, y0 - rC.y, level - band, rC.z);
                 s_g[mine] = g;
             }
-            shear = planes.shear;
-            if constexpr (ABS_GRAD) af = abs_form(planes, rT4);
+            if constexpr (ABS_GRAD) af = abs_form(eval + g, rC);
         }
         const float opacity = rRGBA.w;
-        const float offset_x = x0 - centre.x, offset_y = y0 - centre.y;
+        const float offset_x = x0 - rC.x, offset_y = y0 - rC.y, shear = rC.z;
         uint32_t candidates = transpose_masks(lane < kGoChunk ? mask_mine : 0u, lane);      // bit 15 - i: survivor i
         if (done) candidates = 0;
         __syncwarp();
@@ -698,7 +682,7 @@ template <bool COMPACT>
 __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ scales, const float* __restrict__ rotations, const float* __restrict__ sh_rest,
     const float* __restrict__ M, const float* __restrict__ VPM, const float* __restrict__ cam_position_ptr,
-    const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const float2* __restrict__ moment_centre, const uint8_t* __restrict__ clamp,
+    const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const PairRecord* __restrict__ pair, const uint8_t* __restrict__ clamp,
     const float4* __restrict__ accum, BackwardOutputs out,
     uint32_t n_primitives, int active_sh_bases, int total_sh_bases, uint32_t g_first, uint32_t g_end)
 {
@@ -719,12 +703,12 @@ __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     float4 grad_rotation = make_float4(0, 0, 0, 0);
     float grad_opacity = 0.0f;
     if (kept) {
-    const PairMoments moments{accum[size_t(idx) * 5], accum[size_t(idx) * 5 + 1], accum[size_t(idx) * 5 + 2]};
     const float4 dC = accum[size_t(idx) * 5 + 3];
     const float4 T4 = ldg4(reinterpret_cast<const float*>(eval + idx) + 8);
-    const float2 centre = __ldg(moment_centre + idx);
+    const float4 centre = ldg4(&pair[idx].cx);       // and shear, 1 / D at the centre
+    const PairMoments moments{centre.w * accum[size_t(idx) * 5], centre.w * accum[size_t(idx) * 5 + 1], centre.w * accum[size_t(idx) * 5 + 2]};
     const RowGradients rows = rows_from_moments(affine_planes(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
-                                                              centre.x, centre.y), T4, moments);
+                                                              centre.x, centre.y, centre.z), T4, moments);
     // dL/dVPMT4 = -(cx dL/dVPMT1 + cy dL/dVPMT2 + E): the products with the centre are moved to the rows of VPM, where they cancel
     const float4 dT1 = rows.dX, dT2 = rows.dY, dT4 = make_float4(-rows.E.x, -rows.E.y, -rows.E.z, -rows.E.w);
     const float3 c1 = make_float3(dT1.x, dT2.x, dT4.x), c2 = make_float3(dT1.y, dT2.y, dT4.y), c3 = make_float3(dT1.z, dT2.z, dT4.z);
@@ -872,7 +856,7 @@ cudaError_t launch_tile_backward(bool abs_grad, const FrameGeometry& geo, const 
             const cudaError_t err = configured[abs_grad ? 1 : 0].run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); });
             if (err != cudaSuccess) return err;
         }
-        kernel<<<uint32_t(geo.n_tiles), kBwdThreads, smem, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, prim.moment_centre, tin, grad_image, VPM, accum,
+        kernel<<<uint32_t(geo.n_tiles), kBwdThreads, smem, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, prim.pair, tin, grad_image, VPM, accum,
                                                 uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w), g_first, g_end);
         return cudaGetLastError();
     };
@@ -935,12 +919,12 @@ cudaError_t launch_chain_rule(const HtgsScene& scene, const HtgsView& view, cons
         const cudaError_t err = cudaMemsetAsync(out.compact_rows, 0, sizeof(CompactGradientHeader), stream);
         if (err != cudaSuccess) return err;
         preprocess_backward_kernel<true><<<grid, kChainThreads, 0, stream>>>(scene.positions, scene.scales, scene.rotations, scene.sh_rest, view.M, view.VPM,
-                                                                             view.cam_position, prim.n_touched, prim.eval, prim.moment_centre, prim.clamp, acc.accum, out, n,
+                                                                             view.cam_position, prim.n_touched, prim.eval, prim.pair, prim.clamp, acc.accum, out, n,
                                                                              view.active_sh_bases, scene.total_sh_bases, first, first + count);
     } else {
         const size_t smem = size_t(kChainThreads) * 3 * size_t(scene.total_sh_bases < 15 ? scene.total_sh_bases : 15) * sizeof(float);
         preprocess_backward_kernel<false><<<grid, kChainThreads, smem, stream>>>(scene.positions, scene.scales, scene.rotations, scene.sh_rest, view.M, view.VPM,
-                                                                                 view.cam_position, prim.n_touched, prim.eval, prim.moment_centre, prim.clamp, acc.accum, out, n,
+                                                                                 view.cam_position, prim.n_touched, prim.eval, prim.pair, prim.clamp, acc.accum, out, n,
                                                                                  view.active_sh_bases, scene.total_sh_bases, first, first + count);
     }
     return cudaGetLastError();
@@ -981,7 +965,7 @@ cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsV
             err = launch_tile_backward<HTGS_MODE_OIT_BLEND, 1>(abs_grad, geo, prim, prims_sorted, tile_ranges, tile_order, tin, grad_image, view.VPM, acc.accum, g_first, g_end, stream); break;
         case HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING: {
             const auto kernel = abs_grad ? backward_global_kernel<true> : backward_global_kernel<false>;
-            kernel<<<uint32_t(geo.n_tiles) * 8u, 32, 0, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, prim.moment_centre, grad_image, image, view.VPM, acc.accum,
+            kernel<<<uint32_t(geo.n_tiles) * 8u, 32, 0, stream>>>(tile_ranges, tile_order, prims_sorted, prim.eval, prim.cull, prim.pair, grad_image, image, view.VPM, acc.accum,
                                                                   uint32_t(geo.width), uint32_t(geo.height), uint32_t(geo.grid_w));
             err = cudaGetLastError();
             break;
