@@ -7,7 +7,7 @@
 //
 //  * The organisation is that of the exact kernel (blend.cu): a warp per 8 x 4 pixels filters its tile's list, keeps a window of two
 //    halves of 16 records that its lanes walk independently, and long lists start first.  Against a CTA per 8 x 8 tile with
-//    masks by ballots and a barrier every 64 instances: 944 -> FAST_US us at 3 M Gaussians, 1297 x 840, K = 16.
+//    masks by ballots and a barrier every 64 instances: 944 -> 820 us at 3 M Gaussians, 1297 x 840, K = 16.
 //  * Per fragment, rho^2 and depth are ratios of quadratics in (pixel - projected centre) whose coefficients the
 //    preprocess stored per Gaussian (FastRecord): 6 shared-memory loads, 20 multiply-adds, one approximate
 //    reciprocal and one approximate exp2 instead of two plane constructions, two cross products, an IEEE divide
@@ -43,7 +43,7 @@ template <int MODE, int K> struct FastSmem {
     static constexpr size_t keys_bytes = has_kbuffer ? size_t(K) * kFastThreads * 4 : 0;     // uint4 [K/4][threads]
     static constexpr size_t pay_off = keys_off + keys_bytes;
     static constexpr size_t pay_bytes = has_kbuffer ? size_t(K) * kFastThreads * 8 : 0;      // 8-byte payload [K][threads]
-    static constexpr size_t ctr_off = pay_off + pay_bytes;                                   // float2 per record: projected centre relative to the block's origin
+    static constexpr size_t ctr_off = pay_off + pay_bytes;                                   // float2 per record: projected centre relative to the tile's origin
     static constexpr size_t prim_off = ctr_off + 2 * kFastHalf * 8;                          // Gaussian index of every record (FIRST_K)
     static constexpr size_t queue_ctr_off = prim_off + (has_prim ? 2 * kFastHalf * 4 : 0);
     static constexpr size_t queue_prim_off = queue_ctr_off + kFastQueue * 8;
@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
     const uint32_t px_i = tile_x * 8 + (tid & 7);
     const uint32_t py_i = block_y * 4 + (tid >> 3);
     const bool inside = px_i < width && py_i < height;
-    const float local_x = float(tid & 7), local_y = float(tid >> 3);   // pixel position inside the block
+    // fragments are measured from the tile's origin (not the block's), so that both blocks of a tile round alike
+    const float local_x = float(tid & 7), local_y = float((tid >> 3) + 4 * part), tile_y0 = float((tile / grid_w) * 8);
     const float block_x0 = float(tile_x * 8), block_y0 = float(block_y * 4);
 
     FastRecord* s_dense = reinterpret_cast<FastRecord*>(smem + SL::dense_rec_off);
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
         if (mask != 0) {
             const uint32_t at = (is_dense ? dense_head + dense + __popc(dense_lanes & lanemask_lt()) : sparse_head + sparse + __popc(sparse_lanes & lanemask_lt())) & uint32_t(kFastQueue - 1);
             unsigned char* queue = smem + (is_dense ? SL::dense_queue_ctr_off : SL::queue_ctr_off);     // centres, indices, masks
-            reinterpret_cast<float2*>(queue)[at] = make_float2((block_x0 - c0.x) - c1.y, (block_y0 - c0.y) - c1.z);
+            reinterpret_cast<float2*>(queue)[at] = make_float2((block_x0 - c0.x) - c1.y, (tile_y0 - c0.y) - c1.z);
             reinterpret_cast<uint32_t*>(queue + kFastQueue * 8)[at] = g_here;
             reinterpret_cast<uint32_t*>(queue + kFastQueue * 12)[at] = mask;
         }
