@@ -10,15 +10,13 @@
 //
 // The chain rule is the reference's: gradients flow through alpha = opacity * G and the colour only
 // (not through depth, thresholds, the min(.,1) clamp or the bounds).  The organisation is new:
-//  * every mode accumulates the same per-Gaussian record of five float4 (dL/dVPMT1, dL/dVPMT2, dL/dVPMT4,
-//    (dL/drgb, dL/dopacity), (sum |dL/dposition|, -, -, -)) with 16-byte vector reductions
-//    (red.global.add.v4.f32): 4-5 per (Gaussian, tile) instead of 15-17 scalar atomics, and one
-//    per-Gaussian kernel turns the record into the six output gradients (the reference repeats the
-//    scale / rotation chain rule per fragment in two of its modes);
-//  * HYBRID / FIRST_K / OIT: one thread per Gaussian of a tile batch first builds the 64-bit mask of
-//    tile pixels its conservative outline can touch (3 flops per pixel); the (Gaussian, pixel) pairs of the
-//    batch are then split evenly over the threads.  The forward pass saves core entries as positions in the
-//    tile's list, so which pairs are core entries is a table filled once per batch, not a search per pair;
+//  * every mode accumulates the same per-Gaussian record of five float4 with 16-byte vector reductions
+//    (red.global.add.v4.f32) instead of 15-17 scalar atomics: 12 moments that stand for dL/dVPMT1, dL/dVPMT2, dL/dVPMT4 (below),
+//    (dL/drgb, dL/dopacity) and sum |dL/dposition|.  One per-Gaussian kernel turns the record into the six output gradients
+//    (the reference repeats the scale / rotation chain rule per fragment in two of its modes);
+//  * HYBRID / FIRST_K / OIT: the (Gaussian, pixel) candidates of a batch are cut into segments of at most 16 pixels of one
+//    Gaussian, one segment per lane.  The forward pass saves core entries as positions in the tile's list, so which pairs
+//    are core entries is a table filled once per batch, not a search per pair;
 //  * GLOBAL_ORDERING needs the running transmittance per pixel, so it stays pixel-parallel, in independent
 //    8x8-pixel CTAs; a warp only walks the staged Gaussians whose outline reaches its pixels, and the 32
 //    pixel contributions to one Gaussian are summed with a transposing shuffle reduction into a
