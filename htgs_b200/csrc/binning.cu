@@ -75,6 +75,7 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanRun = 16;            // values per thread and round: 16384 block sums (4.2 M Gaussians) per round
 __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uint32_t* __restrict__ block_sums, uint32_t* __restrict__ block_offsets,
                                                                      uint32_t n_blocks, uint32_t capacity, FrameStatus* status) {
+    grid_dependency();
     __shared__ unsigned long long warp_tot[kScanThreads / 32];
     __shared__ unsigned long long carry_s;
     if (threadIdx.x == 0) carry_s = 0ull;
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     const uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ block_offsets, KeyT* __restrict__ keys, uint32_t* __restrict__ prims,
     uint32_t n_primitives, uint32_t grid_w, uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear)
 {
+    grid_dependency();
     const bool overflow = status->overflow;
     const uint64_t sort_blocks = overflow ? 0 : (uint64_t(status->n_instances) + kSortTile - 1) / kSortTile;
     #pragma unroll
@@ -263,6 +265,7 @@ struct PassTable { int n_passes; int shift[8]; int bits[8]; };
 template <typename KeyT>
 __global__ void __launch_bounds__(256) radix_histogram_all_kernel(const KeyT* __restrict__ keys, uint32_t* __restrict__ digit_hist,
                                                                    const FrameStatus* status, uint32_t capacity, const __grid_constant__ PassTable passes) {
+    grid_dependency();
     constexpr uint32_t kRun = 16 / sizeof(KeyT);
     __shared__ uint32_t hist[8 * kMaxRadixBins];
     const uint32_t n = frame_instances(status, capacity);
@@ -336,6 +339,7 @@ __global__ void __launch_bounds__(kSortThreads, scatter_blocks_per_sm<KeyT>()) r
     const uint32_t* __restrict__ digit_hist, uint32_t* rows, uint32_t row_stride, unsigned long long* groups, uint32_t* ticket,
     FrameStatus* status, uint32_t capacity, int shift, int bits)
 {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t n_bins = 1u << bits, mask = n_bins - 1;
     uint32_t* block_excl = reinterpret_cast<uint32_t*>(smem_raw);                 // [n_bins]
@@ -537,6 +541,7 @@ __device__ __forceinline__ void order_tiles(const uint2* ranges, uint32_t* order
 template <typename KeyT>
 __global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* __restrict__ keys, uint2* __restrict__ ranges, uint32_t* __restrict__ order,
                                                                     FrameStatus* status, uint32_t capacity, uint32_t n_tiles) {
+    grid_dependency();
     constexpr uint32_t kRangeRun = 16 / sizeof(KeyT);            // 8 / 4 / 2 keys per 16-byte load
     const uint32_t n = frame_instances(status, capacity);
     const uint32_t n_runs = (n + kRangeRun - 1) / kRangeRun;
@@ -583,7 +588,7 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
     if (prim_blocks == 0 || inst.capacity == 0) {
         if ((err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream)) != cudaSuccess) return err;
         if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); }
-        tile_ranges_kernel<KeyT><<<1, kOrderThreads, 0, stream>>>(static_cast<const KeyT*>(inst.keys[0]), tile_ranges, tile_order, status, 0u, uint32_t(geo.n_tiles));
+        launch_after(tile_ranges_kernel<KeyT>, 1, kOrderThreads, 0, stream, static_cast<const KeyT*>(inst.keys[0]), tile_ranges, tile_order, status, 0u, uint32_t(geo.n_tiles));
         if (ev) cudaEventRecord(ev[2], stream);
         if (launches) *launches += 1;
         return cudaGetLastError();
@@ -595,7 +600,7 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
         clear.begin[1] = reinterpret_cast<uint4*>(sc.tickets); clear.count[1] = sc.fixed_bytes / 16;
         clear.begin[2] = reinterpret_cast<uint4*>(sc.rows[0]); clear.per_sort_block[2] = sc.row_stride / 4;
     }
-    emit_instances_kernel<KeyT><<<prim_blocks, kPreprocessBlock, 0, stream>>>(
+    launch_after(emit_instances_kernel<KeyT>, prim_blocks, kPreprocessBlock, 0, stream,
         prim.n_touched, prim.bounds, prim.eval, prim.block_sums, prim.block_offsets, static_cast<KeyT*>(inst.keys[0]), inst.prims[0], n,
         uint32_t(geo.grid_w), inst.capacity, status, clear);
     if (ev) cudaEventRecord(ev[0], stream);
@@ -609,7 +614,7 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
         passes.n_passes = plan.n_passes;
         for (int p = 0; p < plan.n_passes; ++p) { passes.shift[p] = plan.shift[p]; passes.bits[p] = plan.bits[p]; }
         const uint32_t hist_grid = std::min<uint32_t>(inst.sort_blocks_cap ? inst.sort_blocks_cap : 1u, uint32_t(sm_count) * 8u);
-        radix_histogram_all_kernel<KeyT><<<hist_grid, 256, 0, stream>>>(static_cast<const KeyT*>(inst.keys[0]), sc.digit_hist, status, inst.capacity, passes);
+        launch_after(radix_histogram_all_kernel<KeyT>, hist_grid, 256, 0, stream, static_cast<const KeyT*>(inst.keys[0]), sc.digit_hist, status, inst.capacity, passes);
         if (launches) *launches += 1;
         for (int p = 0; p < plan.n_passes; ++p) {
             KeyT* kin = static_cast<KeyT*>(inst.keys[cur]);
@@ -617,7 +622,7 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
             const size_t smem = scatter_smem_bytes<KeyT>(plan.bits[p]);
             const uint32_t resident = uint32_t(std::min<size_t>(scatter_blocks_per_sm<KeyT>(), (227 * 1024) / (smem + 1024)));
             const uint32_t scatter_grid = std::min<uint32_t>(inst.sort_blocks_cap ? inst.sort_blocks_cap : 1u, uint32_t(sm_count) * resident);
-            radix_scatter_kernel<KeyT><<<scatter_grid, kSortThreads, smem, stream>>>(
+            launch_after(radix_scatter_kernel<KeyT>, scatter_grid, kSortThreads, smem, stream,
                 kin, inst.prims[cur], kout, inst.prims[cur ^ 1], sc.digit_hist + size_t(p) * kMaxRadixBins, sc.rows[p],
                 uint32_t(sc.row_stride), sc.groups[p], sc.tickets + p, status, inst.capacity, plan.shift[p], plan.bits[p]);
             cur ^= 1;
@@ -625,7 +630,7 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
         }
     }
     if (ev) cudaEventRecord(ev[1], stream);
-    tile_ranges_kernel<KeyT><<<uint32_t(sm_count), kOrderThreads, 0, stream>>>(static_cast<const KeyT*>(inst.keys[cur]), tile_ranges, tile_order, status, inst.capacity,
+    launch_after(tile_ranges_kernel<KeyT>, uint32_t(sm_count), kOrderThreads, 0, stream, static_cast<const KeyT*>(inst.keys[cur]), tile_ranges, tile_order, status, inst.capacity,
                                                                                 uint32_t(geo.n_tiles));
     if (ev) cudaEventRecord(ev[2], stream);
     if (launches) *launches += 1;
@@ -639,7 +644,7 @@ size_t sort_scratch_bytes(const SortPlan& plan, uint32_t sort_blocks_cap) { retu
 cudaError_t launch_scan_only(const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream) {
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
-    scan_block_sums_kernel<<<1, kScanThreads, 0, stream>>>(prim.block_sums, prim.block_offsets, prim_blocks, capacity, status);
+    launch_after(scan_block_sums_kernel, 1, kScanThreads, 0, stream, prim.block_sums, prim.block_offsets, prim_blocks, capacity, status);
     return cudaGetLastError();
 }
 

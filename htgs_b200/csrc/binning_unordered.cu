@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(kBinBlock) bin_visible_kernel(
     const CullRecord* __restrict__ cull, uint2* __restrict__ ranges, uint32_t* __restrict__ prims_sorted, uint32_t* __restrict__ tile_order, UnorderedState state,
     const FrameStatus* __restrict__ status, uint32_t grid_w, uint32_t n_tiles, uint32_t capacity)
 {
+    grid_dependency();
     __shared__ uint32_t excl[kBinBlock + 1];
     __shared__ ushort4 box[kBinBlock];
     __shared__ uint32_t owner[kBinBlock];
@@ -137,6 +138,7 @@ __global__ void __launch_bounds__(kBinBlock) bin_visible_kernel(
 // which the blocks come, which nothing depends on (one block that scanned all tiles took 100 us at 92 k tiles).  The last block
 // to finish turns the counts of tiles per class into the classes' places in the order.
 __global__ void __launch_bounds__(1024) scan_tiles_kernel(uint2* __restrict__ ranges, UnorderedState state, uint32_t n_tiles) {
+    grid_dependency();
     __shared__ uint32_t warp_tot[32], classes[kOrderClasses], block_begin;
     __shared__ bool is_last;
     if (threadIdx.x < kOrderClasses) classes[threadIdx.x] = 0;
@@ -183,12 +185,12 @@ cudaError_t launch_bin_unordered(const HtgsScene& scene, const FrameGeometry& ge
     if (err != cudaSuccess) return err;
     const uint32_t work = max(uint32_t(scene.n_primitives > 0 ? scene.n_primitives : 0), uint32_t(geo.n_tiles));
     const uint32_t grid = min((work + kBinBlock - 1) / kBinBlock, uint32_t(sm_count) * 8u);
-    bin_visible_kernel<false><<<grid, kBinBlock, 0, stream>>>(prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, tile_order, state, status,
+    launch_after(bin_visible_kernel<false>, grid, kBinBlock, 0, stream, prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, tile_order, state, status,
                                                               uint32_t(geo.grid_w), uint32_t(geo.n_tiles), capacity);
     if (ev) cudaEventRecord(ev[0], stream);
-    scan_tiles_kernel<<<(uint32_t(geo.n_tiles) + 1023u) / 1024u, 1024, 0, stream>>>(tile_ranges, state, uint32_t(geo.n_tiles));
+    launch_after(scan_tiles_kernel, (uint32_t(geo.n_tiles) + 1023u) / 1024u, 1024, 0, stream, tile_ranges, state, uint32_t(geo.n_tiles));
     if (ev) cudaEventRecord(ev[1], stream);
-    bin_visible_kernel<true><<<grid, kBinBlock, 0, stream>>>(prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, tile_order, state, status,
+    launch_after(bin_visible_kernel<true>, grid, kBinBlock, 0, stream, prim.visible_list, prim.n_touched, prim.bounds, prim.cull, tile_ranges, prims_sorted, tile_order, state, status,
                                                              uint32_t(geo.grid_w), uint32_t(geo.n_tiles), capacity);
     if (ev) cudaEventRecord(ev[2], stream);
     if (launches) *launches += 3;

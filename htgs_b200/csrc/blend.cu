@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(32) blend_kernel(
     unsigned int* __restrict__ max_weights, float weight_threshold, TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
     bool use_median_depth, int32_t key_base, FrameStatus* status)
 {
+    cudaGridDependencySynchronize();      // no launch_after kernel follows
     using MT = ModeTraits<MODE>;
     using SL = SmemLayout<MODE, K, BUFFER, TASK>;
     constexpr bool TRAIN = TASK == BlendTask::training, STATS = TASK == BlendTask::image_with_statistics, WEIGHTS = TASK == BlendTask::max_weights;
@@ -602,10 +603,9 @@ cudaError_t launch_task(const BlendLaunch& l, int32_t key_base) {
         if (err != cudaSuccess) return err;
     }
     const uint32_t grid = uint32_t(l.geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
-    kernel<<<grid, 32, SL::total, l.stream>>>(l.tile_ranges, l.tile_order, l.prims_sorted, l.prim.eval, l.prim.cull, l.out.image, l.out.depth, l.out.alpha,
+    return launch_after(kernel, grid, 32, SL::total, l.stream, l.tile_ranges, l.tile_order, l.prims_sorted, l.prim.eval, l.prim.cull, l.out.image, l.out.depth, l.out.alpha,
                                               reinterpret_cast<unsigned int*>(l.out.max_weights), l.out.weight_threshold, l.tout, uint32_t(l.geo.width),
                                               uint32_t(l.geo.height), uint32_t(l.geo.grid_w), l.out.to_chw, l.out.use_median_depth, key_base, l.status);
-    return cudaGetLastError();
 }
 
 template <int MODE, int K, Buffer BUFFER>

