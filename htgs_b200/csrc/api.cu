@@ -168,6 +168,7 @@ struct HtgsContext {
     // the training forward whose status has not been read yet (htgs_forward_finish_async)
     bool training_pending = false;
     cudaEvent_t training_done = nullptr;
+    cudaEvent_t training_counted = nullptr; // the instance count of a training forward has reached host_status[0]
     uint32_t training_visible = 0;          // of the last htgs_forward_begin
     // measurement aids
     bool profiling = false;
@@ -238,7 +239,8 @@ HtgsContext* htgs_create(int device) {
         (err = cudaEventCreateWithFlags(&ctx->front_begin, cudaEventDisableTiming)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->front_end, cudaEventDisableTiming)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->frame_done, cudaEventDisableTiming)) != cudaSuccess ||
-        (err = cudaEventCreateWithFlags(&ctx->training_done, cudaEventDisableTiming)) != cudaSuccess) {
+        (err = cudaEventCreateWithFlags(&ctx->training_done, cudaEventDisableTiming)) != cudaSuccess ||
+        (err = cudaEventCreateWithFlags(&ctx->training_counted, cudaEventDisableTiming)) != cudaSuccess) {
         fail_cuda(err, "htgs_create: pinned status word, side stream and events");
         htgs_destroy(ctx);
         return nullptr;
@@ -262,6 +264,7 @@ void htgs_destroy(HtgsContext* ctx) {
     if (ctx->front_end) cudaEventDestroy(ctx->front_end);
     if (ctx->frame_done) cudaEventDestroy(ctx->frame_done);
     if (ctx->training_done) cudaEventDestroy(ctx->training_done);
+    if (ctx->training_counted) cudaEventDestroy(ctx->training_counted);
     delete ctx;
 }
 
@@ -639,10 +642,11 @@ InstLayout carve_instance_blob(void* blob, const SortPlan& plan, uint64_t capaci
     const uint64_t cap = capacity > 0xfffffff0ull ? 0xfffffff0ull : capacity;
     L.inst.capacity = uint32_t(cap);
     L.inst.sort_blocks_cap = uint32_t((cap + kSortTile - 1) / kSortTile);
+    // the sorted indices, all that the backward pass reads, come first: it finds them whatever capacity the forward pass had
+    L.inst.prims[plan.final_buffer] = c.take<uint32_t>(size_t(cap));
+    L.inst.prims[plan.final_buffer ^ 1] = c.take<uint32_t>(size_t(cap));
     L.inst.keys[0] = c.take_bytes<void>(size_t(cap) * plan.key_bytes);
     L.inst.keys[1] = c.take_bytes<void>(size_t(cap) * plan.key_bytes);
-    L.inst.prims[0] = c.take<uint32_t>(size_t(cap));
-    L.inst.prims[1] = c.take<uint32_t>(size_t(cap));
     L.inst.sort_scratch = c.take_bytes<void>(sort_scratch_bytes(plan, L.inst.sort_blocks_cap));
     L.bytes = align_up(c.offset);
     return L;
@@ -704,31 +708,45 @@ size_t htgs_forward_instance_bytes(const HtgsView* view, uint64_t n_instances) {
     return carve_instance_blob(nullptr, make_sort_plan(view->mode, geo.n_tiles), n_instances).bytes;
 }
 
-int htgs_forward_begin(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, void* per_primitive, size_t per_primitive_bytes,
-                       void* stream_ptr, uint32_t* n_instances) {
-    if (!ctx || !n_instances) return fail(HTGS_ERR_INVALID_ARGUMENT, "null argument");
+}  // extern "C"
+
+// Queues preprocess, prefix sum and the copy of the status to host_status[0]; more than `capacity` instances set the overflow flag.
+static int forward_front(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, void* per_primitive, size_t per_primitive_bytes,
+                         uint32_t capacity, cudaStream_t stream) {
     int rc = validate(scene, view);
     if (rc != HTGS_OK) return rc;
-    DeviceGuard guard(ctx->device);
-    if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
     if ((rc = settle_pending(ctx)) != HTGS_OK) return rc;
     const PrimLayout L = carve_primitive_blob(per_primitive, scene->n_primitives);
     if (!per_primitive || per_primitive_bytes < L.bytes) return fail(HTGS_ERR_WORKSPACE_TOO_SMALL, "per-primitive blob too small");
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     const FrameGeometry geo = make_geometry(view->mode, view->width, view->height);
     cudaError_t err;
     if ((err = cudaMemsetAsync(L.status, 0, sizeof(FrameStatus), stream)) != cudaSuccess) return fail_cuda(err, "status reset");
     if ((err = launch_preprocess(view->mode, true, *scene, *view, geo, L.prim, L.status, stream, view->mode)) != cudaSuccess) return fail_cuda(err, "preprocess");
-    if ((err = launch_scan_only(*scene, L.prim, 0xfffffff0u, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
+    if ((err = launch_scan_only(*scene, L.prim, capacity, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
-    if ((err = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(err, "synchronise");
-    if (ctx->host_status->overflow) return fail(HTGS_ERR_INVALID_ARGUMENT, "instance count does not fit 32 bits");
-    *n_instances = ctx->host_status->n_instances;
-    ctx->training_visible = ctx->host_status->n_visible;
     return HTGS_OK;
 }
 
-}  // extern "C"
+static constexpr uint32_t kMostInstances = 0xfffffff0u;
+
+static int forward_counted(HtgsContext* ctx, uint32_t* n_instances) {
+    *n_instances = ctx->host_status->n_instances;
+    ctx->training_visible = ctx->host_status->n_visible;
+    return *n_instances > kMostInstances ? fail(HTGS_ERR_INVALID_ARGUMENT, "instance count does not fit 32 bits") : HTGS_OK;
+}
+
+extern "C" int htgs_forward_begin(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, void* per_primitive, size_t per_primitive_bytes,
+                                  void* stream_ptr, uint32_t* n_instances) {
+    if (!ctx || !n_instances) return fail(HTGS_ERR_INVALID_ARGUMENT, "null argument");
+    DeviceGuard guard(ctx->device);
+    if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    const int rc = forward_front(ctx, scene, view, per_primitive, per_primitive_bytes, kMostInstances, stream);
+    if (rc != HTGS_OK) return rc;
+    const cudaError_t err = cudaStreamSynchronize(stream);
+    if (err != cudaSuccess) return fail_cuda(err, "synchronise");
+    return forward_counted(ctx, n_instances);
+}
 
 static int forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
                           float* image, void* stream_ptr, HtgsFrameInfo* info, bool wait) {
@@ -779,6 +797,24 @@ int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView
 int htgs_forward_finish_async(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
                               float* image, void* stream_ptr, HtgsFrameInfo* info) {
     return forward_finish(ctx, scene, view, blobs, n_instances, image, stream_ptr, info, false);
+}
+
+int htgs_forward_ahead(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t capacity,
+                       float* image, void* stream_ptr, uint32_t* n_instances, HtgsFrameInfo* info) {
+    if (!ctx || !blobs || !image || !n_instances) return fail(HTGS_ERR_INVALID_ARGUMENT, "null argument");
+    DeviceGuard guard(ctx->device);
+    if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+    if (capacity > kMostInstances) capacity = kMostInstances;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    int rc = forward_front(ctx, scene, view, blobs->per_primitive, blobs->per_primitive_bytes, capacity, stream);
+    if (rc != HTGS_OK) return rc;
+    cudaError_t err = cudaEventRecord(ctx->training_counted, stream);
+    if (err != cudaSuccess) return fail_cuda(err, "training event record");
+    if ((rc = forward_finish(ctx, scene, view, blobs, capacity, image, stream_ptr, info, false)) != HTGS_OK) return rc;
+    if ((err = cudaEventSynchronize(ctx->training_counted)) != cudaSuccess) return fail_cuda(err, "synchronise");
+    if ((rc = forward_counted(ctx, n_instances)) != HTGS_OK) return rc;
+    if (info) { info->n_instances = *n_instances; info->n_visible = ctx->training_visible; }
+    return *n_instances > capacity ? fail(HTGS_ERR_WORKSPACE_TOO_SMALL, "the per-instance blob holds fewer instances than the view has") : HTGS_OK;
 }
 
 size_t htgs_backward_scratch_bytes(const HtgsScene* scene) {

@@ -192,6 +192,25 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int, int> forward(
     const c10::cuda::CUDAStream torch_stream = c10::cuda::getCurrentCUDAStream(a.device.index());
     cudaStream_t stream = torch_stream.stream();
     uint32_t n_instances = 0;
+    // The previous forward of this thread saw the same scene size and image: its capacity is the guess for this view, and the whole
+    // forward is queued before the call waits for the count (a training step of 100 k Gaussians at 649 x 420: 467 -> 446 us).  Not when the visible rows are asked for, which others wait for while the forward runs.
+    struct Guess { int device = -1; int64_t n = 0; int width = 0, height = 0, mode = 0; uint64_t capacity = 0; };
+    static thread_local Guess guess;
+    if (guess.capacity && guess.device == a.device.index() && guess.n == a.n && guess.width == width && guess.height == height &&
+        guess.mode == rasterizer_mode && !g_track_visibility.load()) {
+        const size_t bytes = htgs_forward_instance_bytes(&a.view, guess.capacity);
+        Tensor per_instance = bytes_on(a.device, bytes);
+        HtgsTrainBlobs blobs{per_primitive.data_ptr(), pp_bytes, per_tile.data_ptr(), pt_bytes, per_instance.data_ptr(), bytes, per_pixel.data_ptr(), px_bytes};
+        HtgsFrameInfo info{};
+        const int rc = htgs_forward_ahead(ctx, &a.scene, &a.view, &blobs, uint32_t(guess.capacity), image.data_ptr<float>(), stream, &n_instances, &info);
+        if (rc != HTGS_ERR_WORKSPACE_TOO_SMALL) check(rc);
+        // a far smaller view gives the next one a smaller blob
+        if (guess.capacity > 4 * htgs_forward_instance_capacity(n_instances)) guess.capacity = 0;
+        if (rc == HTGS_OK) {
+            tls.last_info = info;
+            return {image, per_primitive, per_tile, per_instance, per_pixel, int(n_instances), 0};
+        }
+    }
     check(htgs_forward_begin(ctx, &a.scene, &a.view, per_primitive.data_ptr(), pp_bytes, stream, &n_instances));
     if (g_track_visibility.load()) {   // before the rest of the forward is queued: the list is final and the stream is idle here
         Tensor visible = torch::empty({a.n}, torch::TensorOptions().dtype(torch::kBool).device(a.device));
@@ -218,6 +237,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int, int> forward(
         while (before < capacity && !seen.compare_exchange_weak(before, capacity)) {}
         if (before > capacity && before <= 4 * capacity) capacity = before;
     }
+    guess = capacity <= 0xfffffff0ull ? Guess{a.device.index(), a.n, width, height, rasterizer_mode, capacity} : Guess{};
     const size_t pi_bytes = htgs_forward_instance_bytes(&a.view, capacity);
     Tensor per_instance = bytes_on(a.device, pi_bytes);
     HtgsTrainBlobs blobs{per_primitive.data_ptr(), pp_bytes, per_tile.data_ptr(), pt_bytes, per_instance.data_ptr(), pi_bytes, per_pixel.data_ptr(), px_bytes};

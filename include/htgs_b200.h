@@ -197,6 +197,14 @@ int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView
 int htgs_forward_finish_async(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
                               float* image, void* stream, HtgsFrameInfo* info);
 
+/* Both halves in one call, for a caller that has a guess of the instance count (the previous view's): everything is queued for a
+ * per-instance blob of htgs_forward_instance_bytes(view, capacity) bytes before the call waits for the count, so the GPU does not
+ * idle between the halves.  A view with more instances than `capacity` returns HTGS_ERR_WORKSPACE_TOO_SMALL with its count in
+ * *n_instances and leaves blobs and image without meaning; repeat with a larger blob.  The status is checked as after
+ * htgs_forward_finish_async. */
+int htgs_forward_ahead(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t capacity,
+                       float* image, void* stream, uint32_t* n_instances, HtgsFrameInfo* info);
+
 /* Outputs of the backward pass.  Every element of the six gradient tensors is written (zeros for culled
  * Gaussians), so they need not be cleared.  `scratch` (htgs_backward_scratch_bytes) holds the per-Gaussian
  * accumulation records and is cleared by the call.  `densification_info` ([rows,N], rows 2 or 3) is

@@ -1,0 +1,43 @@
+"""GPU: a training forward that is queued before its instance count is known (htgs_forward_ahead).
+
+The guess is the previous forward's capacity; a view that exceeds it, one that needs a fraction of it and one without instances have to
+give what the forward in two halves gives, which tracking the visible rows selects.
+"""
+import pytest
+
+import harness
+from htgs_b200 import scenes
+from htgs_b200.torch_bindings import rasterization
+
+pytestmark = pytest.mark.gpu
+
+
+def step(tb, scene, mode, factor, behind):
+    import torch
+    tensors = harness.scene_tensors(scene)
+    tensors[1] = tensors[1] * factor
+    if behind:
+        tensors[0] = tensors[0] - torch.tensor([0.0, 0.0, 100.0], device="cuda")
+    tensors = [t.detach().clone().requires_grad_() for t in tensors]
+    image = tb.diff_rasterize(*tensors, torch.empty(0, device="cuda"), harness.settings_for(tb, scene, scene.views[0], mode, 8), False)
+    image.square().sum().backward()
+    return image.detach(), [t.grad for t in tensors]
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_views_above_and_below_the_guess(mode):
+    import torch
+    tb = harness.ours()
+    scene = scenes.tiny_scene(n=3000, size=256, seed=11, mode=mode, K=8, sh_degree=1)
+    cases = [(0.05, False), (3.0, False), (0.05, False), (1.0, True), (1.0, False), (1.0, False)]
+    got = [step(tb, scene, mode, *c) for c in cases]
+    rasterization.track_training_visibility(True)
+    try:
+        want = [step(tb, scene, mode, *c) for c in cases]
+    finally:
+        rasterization.track_training_visibility(False)
+    for (image, grads), (image_w, grads_w) in zip(got, want):
+        assert torch.equal(image, image_w)
+        for a, b in zip(grads, grads_w):
+            assert torch.allclose(a, b, rtol=1e-4, atol=1e-5 * float(b.abs().max()))
+    assert float(want[1][0].max()) > 0.0 and not float(want[3][0].abs().max()) > 0.0
