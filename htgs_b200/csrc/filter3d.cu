@@ -50,7 +50,7 @@ struct __align__(16) FilterView {
     float near_plane, pad[3];
 };
 template <int VIEWS> struct FilterViewBatch { FilterView view[VIEWS]; float largest_entry, largest_offset; };   // by value: up to 28 KB of kernel parameters
-constexpr int kFewViews = 48, kManyViews = 256;
+constexpr int kFewestViews = 32, kFewViews = 48, kManyViews = 256;      // kFewestViews: kernel parameters of less than 4 KB, whose launch is the cheapest
 
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
@@ -203,10 +203,10 @@ extern "C" int htgs_update_3d_filter_views(const float* positions, const HtgsFil
     }
     if (n_points == 0) return HTGS_OK;
     // two points to a thread where more would leave SMs without a full set of threads
-    const bool many_points = uint32_t(n_points) >= uint32_t(htgs::sm_count_of_current_device()) * 4096u;
+    const bool many_points = n_views > kFewViews && uint32_t(n_points) >= uint32_t(htgs::sm_count_of_current_device()) * 4096u;
     for (int32_t first = 0; first < n_views;) {
         const int32_t left = n_views - first, count = std::min<int32_t>(left, left > kFewViews ? kManyViews : kFewViews);
-        const auto launch = count <= kFewViews ? launch_views<kFewViews, 1> : many_points ? launch_views<kManyViews, 3> : launch_views<kManyViews, 1>;
+        const auto launch = count <= kFewestViews ? launch_views<kFewestViews, 1> : count <= kFewViews ? launch_views<kFewViews, 1> : many_points ? launch_views<kManyViews, 3> : launch_views<kManyViews, 1>;
         const cudaError_t err = launch(positions, views + first, count, filter_3d, visibility_mask, uint32_t(n_points), clipping_tolerance, distance2filter,
                                        static_cast<cudaStream_t>(stream));
         if (err != cudaSuccess) {

@@ -87,9 +87,9 @@ def test_all_views_in_one_pass_equals_the_loop(n_views):
 
 
 @pytest.mark.parametrize("n", [1, 511, 1537, 700_001])
-@pytest.mark.parametrize("n_views", [49, 257])
+@pytest.mark.parametrize("n_views", [32, 33, 49, 257])
 def test_views_with_points_on_frustum_planes_and_without_a_number(n, n_views):
-    """Tile edges of the one-pass kernel; points on the planes of a frustum, infinite and NaN points, and a view without an area."""
+    """Tile edges of the one-pass kernel, edges of its view batches; points on the planes of a frustum, infinite and NaN points, and a view without an area."""
     import torch
     tb = harness.ours()
     rng = np.random.default_rng(n + n_views)
