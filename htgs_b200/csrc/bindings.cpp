@@ -193,7 +193,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int, int> forward(
     cudaStream_t stream = torch_stream.stream();
     uint32_t n_instances = 0;
     // The previous forward of this thread saw the same scene size and image: its capacity is the guess for this view, and the whole
-    // forward is queued before the call waits for the count (a training step of 100 k Gaussians at 649 x 420: 467 -> 446 us).  Not when the visible rows are asked for, which others wait for while the forward runs.
+    // forward is queued before the call waits for the count (a training step of 100 k Gaussians at 649 x 420: 467 -> 446 us).
+    // Not when the visible rows are asked for, which others wait for while the forward runs.
     struct Guess { int device = -1; int64_t n = 0; int width = 0, height = 0, mode = 0; uint64_t capacity = 0; };
     static thread_local Guess guess;
     if (guess.capacity && guess.device == a.device.index() && guess.n == a.n && guess.width == width && guess.height == height &&
