@@ -621,6 +621,196 @@ void max_weights_image(int mode, const BlendIn<R>& in, R weight_threshold, R* ma
     }
 }
 
+// ----------------------------------------------------------------------------
+// gradients in float64, with the discrete decisions of the K-buffer given from outside
+// R/include/hybrid_blend/kernels/backward.cuh:104-331, alpha_blend_first_k :88-206, alpha_blend_global_ordering :78-251,
+// oit_blend :104-290; per-Gaussian chain rule hybrid_blend/kernels/backward.cuh:10-102, R/include/kernel_utils.cuh:44-61, 190-281.
+// `core_pos` [K][n_tiles * 64]: position in the tile's list of the Gaussian of each core entry that carries weight, front to back,
+// 0xffffffff = none (HYBRID_BLEND, ALPHA_BLEND_FIRST_K), or null.  Which fragments the K-buffer holds hangs on comparisons of depths; with
+// them taken from the run under test, what is left of a difference is rounding.  Null: the chain is run here, in float64.
+// ----------------------------------------------------------------------------
+inline void atomic_add(double* at, double v) {
+    int64_t seen = __atomic_load_n(reinterpret_cast<int64_t*>(at), __ATOMIC_RELAXED), want;
+    do {
+        double sum;
+        std::memcpy(&sum, &seen, 8);
+        sum += v;
+        std::memcpy(&want, &sum, 8);
+    } while (!__atomic_compare_exchange_n(reinterpret_cast<int64_t*>(at), &seen, want, true, __ATOMIC_RELAXED, __ATOMIC_RELAXED));
+}
+
+struct PixelFragment { int64_t g; double alpha; Fragment<double> fr; };
+
+// per Gaussian: dL/dVPMT1 (4), dL/dVPMT2 (4), dL/dVPMT4 (4), dL/drgb (3), dL/dopacity, sum |dL/dposition|
+constexpr int kRowGrads = 17;
+void add_fragment_gradient(const BlendIn<double>& in, const PixelFragment& f, double px, double py, const double drgb[3], double dalpha, const Camera<double>& cam, double* grads) {
+    const double opacity = in.rgba[4 * f.g + 3];
+    const double drho2 = -0.5 * dalpha * opacity * f.fr.G, u = drho2 / f.fr.denom, v = u * f.fr.rho2_num / f.fr.denom;
+    const Vec3<double> X = xyz(f.fr.plane_x), Y = xyz(f.fr.plane_y);
+    const Vec3<double> dm = scale3(f.fr.m, 2.0 * u), dd = scale3(f.fr.d, -2.0 * v);
+    const Vec3<double> cX = cross3(Y, dd), cY = cross3(dd, X);
+    const double xw = f.fr.plane_x.w, yw = f.fr.plane_y.w;
+    const double dX[4] = {cX.x - yw * dm.x, cX.y - yw * dm.y, cX.z - yw * dm.z, dot3(Y, dm)};
+    const double dY[4] = {cY.x + xw * dm.x, cY.y + xw * dm.y, cY.z + xw * dm.z, -dot3(X, dm)};
+    double* a = grads + kRowGrads * f.g;
+    for (int i = 0; i < 4; ++i) { atomic_add(a + i, dX[i]); atomic_add(a + 4 + i, dY[i]); atomic_add(a + 8 + i, -px * dX[i] - py * dY[i]); }
+    for (int c = 0; c < 3; ++c) atomic_add(a + 12 + c, drgb[c]);
+    atomic_add(a + 15, dalpha * f.fr.G);
+    const double c4[3] = {dX[3], dY[3], -px * dX[3] - py * dY[3]};
+    const Vec4<double>&r1 = cam.VPM[0], &r2 = cam.VPM[1], &r4 = cam.VPM[3];
+    atomic_add(a + 16, std::fabs(r1.x * c4[0] + r2.x * c4[1] + r4.x * c4[2]) + std::fabs(r1.y * c4[0] + r2.y * c4[1] + r4.y * c4[2]) +
+                           std::fabs(r1.z * c4[0] + r2.z * c4[1] + r4.z * c4[2]));
+}
+
+void backward_pixel(int mode, const BlendIn<double>& in, const ModeConstants& mc, int tile, int px_i, int py_i, const uint32_t* core_pos, int64_t padded, int64_t slot,
+                    const double g[3], const Camera<double>& cam, double* grads) {
+    const double px = px_i, py = py_i;
+    const uint32_t begin = in.ranges[2 * tile], end = in.ranges[2 * tile + 1];
+    auto evaluate = [&](uint32_t it, PixelFragment& f, bool core = false) -> bool {
+        f.g = in.prim_idx[it];
+        fragment_planes(in.vpmt1 + 4 * f.g, in.vpmt2 + 4 * f.g, in.vpmt4 + 4 * f.g, px, py, f.fr);
+        if (!core && f.fr.rho2_num > double(mc.max_cutoff_sq) * f.fr.denom) return false;
+        f.fr.G = std::exp(-0.5 * f.fr.rho2_num / f.fr.denom);
+        f.alpha = std::min(in.rgba[4 * f.g + 3] * f.fr.G, 1.0);
+        return !(f.alpha < double(mc.min_alpha));
+    };
+    auto colour = [&](const PixelFragment& f) { return in.rgba + 4 * f.g; };
+    if (mode == 2) {
+        std::vector<PixelFragment> hit;
+        double t = 1.0;
+        for (uint32_t it = begin; it < end; ++it) {
+            PixelFragment f;
+            if (!evaluate(it, f)) continue;
+            hit.push_back(f);
+            t *= 1.0 - f.alpha;
+            if (t < double(kTransmittanceThreshold)) break;
+        }
+        double behind[3] = {0, 0, 0};
+        std::vector<double> before(hit.size());
+        t = 1.0;
+        for (size_t i = 0; i < hit.size(); ++i) { before[i] = t; t *= 1.0 - hit[i].alpha; }
+        for (size_t i = hit.size(); i-- > 0;) {
+            const double *c = colour(hit[i]), w = before[i] * hit[i].alpha, rcp = 1.0 / std::max(1.0 - hit[i].alpha, double(kOneMinusAlphaEps));
+            double drgb[3], dalpha = 0;
+            for (int k = 0; k < 3; ++k) { drgb[k] = w * g[k]; dalpha += (before[i] * c[k] - behind[k] * rcp) * g[k]; }
+            add_fragment_gradient(in, hit[i], px, py, drgb, dalpha, cam, grads);
+            for (int k = 0; k < 3; ++k) behind[k] += w * c[k];
+        }
+        return;
+    }
+    std::vector<PixelFragment> core, tail;
+    std::vector<uint32_t> stored;
+    std::vector<uint32_t> own(size_t(in.K), UINT32_MAX);      // without decisions from outside: the insertion chain of the forward pass
+    if (mode != 3 && !core_pos) {
+        std::vector<double> kd(size_t(in.K), double(FLT_MAX)), ka(size_t(in.K), 0.0);
+        for (uint32_t it = begin; it < end; ++it) {
+            PixelFragment f;
+            if (!evaluate(it, f) || (mode == 0 && f.alpha < double(mc.min_alpha_core))) continue;
+            f.fr.denom_rcp = 1.0 / f.fr.denom;
+            double depth = fragment_depth(in.mt3 + 4 * f.g, f.fr), alpha = f.alpha;
+            uint32_t pos = it - begin;
+            for (int k = 0; k < in.K; ++k)
+                if (depth < kd[k]) { std::swap(depth, kd[k]); std::swap(pos, own[k]); std::swap(alpha, ka[k]); }
+        }
+        double t = 1.0;
+        for (int k = 0; k < in.K; ++k) { if (t < double(kTransmittanceThreshold)) own[k] = UINT32_MAX; t *= 1.0 - ka[k]; }
+    }
+    if (mode != 3)
+        for (int k = 0; k < in.K; ++k) {
+            const uint32_t pos = core_pos ? core_pos[k * padded + slot] : own[k];
+            if (pos == UINT32_MAX) continue;
+            PixelFragment f;
+            evaluate(begin + pos, f, true);
+            core.push_back(f);
+            stored.push_back(pos);
+        }
+    double t_core = 1.0;
+    for (const PixelFragment& f : core) t_core *= 1.0 - f.alpha;
+    if (mode == 0 && t_core < double(kTransmittanceThreshold)) t_core = 0.0;
+    double tail_rgb[3] = {0, 0, 0}, alpha_sum = 0, t_tail = 1.0;
+    if (mode != 1)
+        for (uint32_t it = begin; it < end; ++it) {
+            if (std::find(stored.begin(), stored.end(), it - begin) != stored.end()) continue;
+            PixelFragment f;
+            if (!evaluate(it, f)) continue;
+            tail.push_back(f);
+            for (int k = 0; k < 3; ++k) tail_rgb[k] += f.alpha * colour(f)[k];
+            alpha_sum += f.alpha;
+            t_tail *= 1.0 - f.alpha;
+        }
+    const bool has_tail = mode != 1 && alpha_sum >= double(mc.min_alpha);
+    const double weight = has_tail ? t_core / alpha_sum : 0.0, full = weight * (1.0 - t_tail);
+    double behind[3];
+    for (int k = 0; k < 3; ++k) behind[k] = full * tail_rgb[k];
+    std::vector<double> before(core.size());
+    double t = 1.0;
+    for (size_t i = 0; i < core.size(); ++i) { before[i] = t; t *= 1.0 - core[i].alpha; }
+    for (size_t i = core.size(); i-- > 0;) {
+        const double *c = colour(core[i]), w = before[i] * core[i].alpha, rcp = 1.0 / std::max(1.0 - core[i].alpha, double(kOneMinusAlphaEps));
+        double drgb[3], dalpha = 0;
+        for (int k = 0; k < 3; ++k) { drgb[k] = w * g[k]; dalpha += (before[i] * c[k] - behind[k] * rcp) * g[k]; }
+        add_fragment_gradient(in, core[i], px, py, drgb, dalpha, cam, grads);
+        for (int k = 0; k < 3; ++k) behind[k] += w * c[k];
+    }
+    if (!has_tail || full == 0.0) return;
+    double tail_dot = 0;
+    for (int k = 0; k < 3; ++k) tail_dot += tail_rgb[k] * g[k];
+    for (const PixelFragment& f : tail) {
+        const double* c = colour(f);
+        double drgb[3], dalpha = -full / alpha_sum * tail_dot + weight * t_tail * tail_dot / std::max(1.0 - f.alpha, double(kOneMinusAlphaEps));
+        for (int k = 0; k < 3; ++k) { drgb[k] = full * g[k] * f.alpha; dalpha += full * g[k] * c[k]; }
+        add_fragment_gradient(in, f, px, py, drgb, dalpha, cam, grads);
+    }
+}
+
+void chain_rule(int64_t i, const float* positions, const float* scales, const float* rotations, const float* sh_rest, const Camera<double>& cam, int active_sh, int total_sh,
+                const uint8_t* clamp, int64_t n, const double* a, double* d_pos, double* d_scale, double* d_rot, double* d_op, double* d_sh0, double* d_rest) {
+    const Vec4<double>* rows[3] = {&cam.VPM[0], &cam.VPM[1], &cam.VPM[3]};
+    const double q[4] = {rotations[4 * i], rotations[4 * i + 1], rotations[4 * i + 2], rotations[4 * i + 3]}, r = q[0], x = q[1], y = q[2], z = q[3];
+    const double R[3][3] = {{1 - 2 * (y * y + z * z), 2 * (x * y - r * z), 2 * (x * z + r * y)},
+                            {2 * (x * y + r * z), 1 - 2 * (x * x + z * z), 2 * (y * z - r * x)},
+                            {2 * (x * z - r * y), 2 * (y * z + r * x), 1 - 2 * (x * x + y * y)}};
+    double dR[3][3];
+    for (int c = 0; c < 3; ++c) {
+        d_pos[3 * i + c] = 0; d_scale[3 * i + c] = 0;
+        double col[3] = {0, 0, 0};     // sum over the rows of VPM (x, y, z) * dL/dT[row][c]
+        for (int k = 0; k < 3; ++k) { col[0] += rows[k]->x * a[4 * k + c]; col[1] += rows[k]->y * a[4 * k + c]; col[2] += rows[k]->z * a[4 * k + c]; }
+        for (int j = 0; j < 3; ++j) { d_scale[3 * i + c] += col[j] * R[j][c]; dR[j][c] = col[j] * double(scales[3 * i + c]); }
+    }
+    for (int k = 0; k < 3; ++k) { d_pos[3 * i] += rows[k]->x * a[4 * k + 3]; d_pos[3 * i + 1] += rows[k]->y * a[4 * k + 3]; d_pos[3 * i + 2] += rows[k]->z * a[4 * k + 3]; }
+    // dR/dq, quaternion taken as given
+    d_rot[4 * i] = 2 * (-z * dR[0][1] + y * dR[0][2] + z * dR[1][0] - x * dR[1][2] - y * dR[2][0] + x * dR[2][1]);
+    d_rot[4 * i + 1] = 2 * (y * dR[0][1] + z * dR[0][2] + y * dR[1][0] - 2 * x * dR[1][1] - r * dR[1][2] + z * dR[2][0] + r * dR[2][1] - 2 * x * dR[2][2]);
+    d_rot[4 * i + 2] = 2 * (-2 * y * dR[0][0] + x * dR[0][1] + r * dR[0][2] + x * dR[1][0] + z * dR[1][2] - r * dR[2][0] + z * dR[2][1] - 2 * y * dR[2][2]);
+    d_rot[4 * i + 3] = 2 * (-2 * z * dR[0][0] - r * dR[0][1] + x * dR[0][2] + r * dR[1][0] - 2 * z * dR[1][1] + y * dR[1][2] + x * dR[2][0] + y * dR[2][1]);
+    d_op[i] = a[15];
+    double rgb[3];
+    for (int c = 0; c < 3; ++c) { rgb[c] = clamp[c * n + i] ? 0.0 : a[12 + c]; d_sh0[3 * i + c] = double(0.28209479177387814f) * rgb[c]; }
+    for (int b = 0; b < 3 * total_sh; ++b) d_rest[int64_t(i) * 3 * total_sh + b] = 0;
+    if (active_sh <= 1) return;
+    // basis functions of the direction and their derivatives with respect to it
+    const double raw[3] = {double(positions[3 * i]) - cam.cam.x, double(positions[3 * i + 1]) - cam.cam.y, double(positions[3 * i + 2]) - cam.cam.z};
+    const double len = std::sqrt(raw[0] * raw[0] + raw[1] * raw[1] + raw[2] * raw[2]), dx = raw[0] / len, dy = raw[1] / len, dz = raw[2] / len;
+    const double xx = dx * dx, yy = dy * dy, zz = dz * dz, c1 = 0.48860251190291987f, c2 = 1.0925484305920792f, c3 = 0.59004358992664352f, c4 = 0.45704579946446572f;
+    const double k20 = 0.94617469575755997f, k21 = 0.31539156525251999f, k22 = 0.54627421529603959f, k31 = 2.8906114426405538f, k33 = 0.3731763325901154f, k35 = 1.4453057213202769f;
+    const double basis[15] = {-c1 * dy, c1 * dz, -c1 * dx, c2 * dx * dy, -c2 * dy * dz, k20 * zz - k21, -c2 * dx * dz, k22 * (xx - yy), c3 * dy * (-3 * xx + yy), k31 * dx * dy * dz,
+                              c4 * dy * (1 - 5 * zz), k33 * dz * (5 * zz - 3), c4 * dx * (1 - 5 * zz), k35 * dz * (xx - yy), c3 * dx * (-xx + 3 * yy)};
+    const double slope[15][3] = {{0, -c1, 0}, {0, 0, c1}, {-c1, 0, 0}, {c2 * dy, c2 * dx, 0}, {0, -c2 * dz, -c2 * dy}, {0, 0, 2 * k20 * dz}, {-c2 * dz, 0, -c2 * dx},
+                                 {2 * k22 * dx, -2 * k22 * dy, 0}, {-6 * c3 * dx * dy, 3 * c3 * (yy - xx), 0}, {k31 * dy * dz, k31 * dx * dz, k31 * dx * dy},
+                                 {0, c4 * (1 - 5 * zz), -10 * c4 * dy * dz}, {0, 0, k33 * (15 * zz - 3)}, {c4 * (1 - 5 * zz), 0, -10 * c4 * dx * dz},
+                                 {2 * k35 * dx * dz, -2 * k35 * dy * dz, k35 * (xx - yy)}, {3 * c3 * (yy - xx), 6 * c3 * dx * dy, 0}};
+    double gdir[3] = {0, 0, 0};
+    for (int b = 0; b < active_sh - 1; ++b) {
+        const float* k = sh_rest + (int64_t(i) * total_sh + b) * 3;
+        double* out = d_rest + (int64_t(i) * total_sh + b) * 3;
+        double along = 0;
+        for (int c = 0; c < 3; ++c) { out[c] = basis[b] * rgb[c]; along += double(k[c]) * rgb[c]; }
+        for (int c = 0; c < 3; ++c) gdir[c] += slope[b][c] * along;
+    }
+    const double radial = dx * gdir[0] + dy * gdir[1] + dz * gdir[2], dir[3] = {dx, dy, dz};
+    for (int c = 0; c < 3; ++c) d_pos[3 * i + c] += (gdir[c] - dir[c] * radial) / len;
+}
+
 }  // namespace
 
 // ----------------------------------------------------------------------------
@@ -709,6 +899,34 @@ int64_t htgs_oracle_render_f64(SCENE_ARGS, int64_t n, int mode, int K, int activ
                                int n_threads) {
     return run_render<double>(SCENE_PASS, n, mode, K, active_sh, total_sh, width, height, near_plane, far_plane, scale_modifier, to_chw,
                               use_median_depth, image, depth, alpha, n_threads);
+}
+
+// Gradients of the image with respect to the six input tensors, in float64, for a binned scene (see backward_pixel).  `vpmt1` .. `rgba` are the
+// per-Gaussian rows to start from (float64: computed from the inputs, or rounded ones widened again); rows of Gaussians in no list get zeros.
+// `abs_position` [N]: sum over the pixels of the 1-norm of dL/dposition.
+void htgs_oracle_backward_f64(SCENE_ARGS, int64_t n, int mode, int K, int active_sh, int total_sh, int width, int height, const uint32_t* ranges, const uint32_t* prim_idx,
+                              const double* vpmt1, const double* vpmt2, const double* vpmt4, const double* mt3, const double* rgba, const uint8_t* clamp,
+                              const uint32_t* core_pos, const double* grad_image, double* d_pos, double* d_scale, double* d_rot, double* d_op, double* d_sh0, double* d_rest,
+                              double* abs_position, int n_threads) {
+    (void)opacities; (void)sh_0;
+    const ModeConstants mc = mode_constants(mode);
+    const Camera<double> cam = load_camera<double>(M, VPM, cam_position);
+    BlendIn<double> in{ranges, prim_idx, vpmt1, vpmt2, vpmt4, mt3, rgba, width, height, (width + mc.tile_w - 1) / mc.tile_w, (height + mc.tile_h - 1) / mc.tile_h, K, false};
+    std::vector<double> grads(size_t(n) * kRowGrads, 0.0);
+    const int64_t n_tiles = int64_t(in.grid_w) * in.grid_h, n_pixels = int64_t(width) * height;
+    parallel_for(n_tiles, n_threads, [&](int64_t tile) {
+        for (int p = 0; p < mc.tile_w * mc.tile_h; ++p) {
+            const int px = int(tile % in.grid_w) * mc.tile_w + p % mc.tile_w, py = int(tile / in.grid_w) * mc.tile_h + p / mc.tile_w;
+            if (px >= width || py >= height) continue;
+            const int64_t at = int64_t(py) * width + px;
+            const double g[3] = {grad_image[at], grad_image[n_pixels + at], grad_image[2 * n_pixels + at]};
+            backward_pixel(mode, in, mc, int(tile), px, py, core_pos, n_tiles * 64, tile * 64 + p, g, cam, grads.data());
+        }
+    });
+    parallel_for(n, n_threads, [&](int64_t i) {
+        chain_rule(i, positions, scales, rotations, sh_rest, cam, active_sh, total_sh, clamp, n, grads.data() + kRowGrads * i, d_pos, d_scale, d_rot, d_op, d_sh0, d_rest);
+        abs_position[i] = grads[kRowGrads * i + 16];
+    });
 }
 
 }  // extern "C"

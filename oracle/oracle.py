@@ -153,6 +153,25 @@ def render(scene, view, mode: Optional[int] = None, K: Optional[int] = None, sca
     return image, depth, alpha, int(n_inst)
 
 
+def backward(scene, view, mode: int, K: int, ranges, prim_idx, grad_image, pre: dict, core_positions=None, n_threads: int = 0):
+    """Gradients of the training image with respect to the six input tensors in float64 (htgs_oracle.cpp: backward_pixel), plus the sum
+    over pixels of |dL/dposition| (1-norm).  `pre`: preprocess(..., dtype=np.float64, with_clamp=True), or its rows rounded and widened
+    again.  `core_positions` [K, tiles * 64]: the K-buffer's decisions, taken from the run under test (None: made here, in float64)."""
+    n, h, w = scene.n, view.height, view.width
+    keep, ptrs = _scene_ptrs(scene, view)
+    total_sh = int(scene.sh_rest.shape[1])
+    out = [np.zeros((n, 3)), np.zeros((n, 3)), np.zeros((n, 4)), np.zeros((n, 1)), np.zeros((n, 1, 3)), np.zeros((n, total_sh, 3)), np.zeros(n)]
+    ranges, prim_idx = np.ascontiguousarray(ranges, np.uint32), np.ascontiguousarray(prim_idx, np.uint32)
+    core = None if core_positions is None else np.ascontiguousarray(core_positions, np.uint32)
+    grad = np.ascontiguousarray(grad_image, np.float64)
+    assert grad.shape == (3, h, w)
+    lib().htgs_oracle_backward_f64(*ptrs, ctypes.c_int64(n), int(mode), int(K), int(scene.active_sh_bases), total_sh, int(w), int(h), _p(ranges), _p(prim_idx),
+                                   _p(pre["vpmt1"]), _p(pre["vpmt2"]), _p(pre["vpmt4"]), _p(pre["mt3"]), _p(pre["rgba"]), _p(pre["clamp"]), _p(core), _p(grad),
+                                   *(_p(a) for a in out), int(n_threads or hardware_threads()))
+    del keep
+    return out
+
+
 def update_3d_filter(positions, w2c, filter_3d, visibility_mask, width, height, focal_x, focal_y, center_x, center_y, near_plane,
                      clipping_tolerance, distance2filter):
     """numpy restatement of the 3D-filter update (filter3d/src/filter3d_kernels.cu:6-35, filter3d/src/filter3d_api.cu:23-33).
