@@ -88,8 +88,12 @@ __device__ __forceinline__ FragmentFront fragment_front(const float4& VPMT1, con
     return f;
 }
 
+// HYBRID_BLEND with unsorted keys is held to the registers that leave the warps which shared memory admits (K = 16: 22, K = 32: 14).  Without
+// a bound the calls of the tie handling make the compiler spend 93 to 96 registers on some forms and spill others to 72.
+constexpr int blend_min_blocks(int mode, int K, bool chain) { return mode != HTGS_MODE_HYBRID_BLEND || chain || K < 8 ? 0 : K >= 32 ? 20 : 24; }
+
 template <int MODE, int K, Buffer BUFFER, BlendTask TASK>
-__global__ void __launch_bounds__(32) blend_kernel(
+__global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER == Buffer::chain)) blend_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, float* __restrict__ image, float* __restrict__ depth_out, float* __restrict__ alpha_out,
     unsigned int* __restrict__ max_weights, float weight_threshold, TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,

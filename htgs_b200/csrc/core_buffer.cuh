@@ -10,6 +10,7 @@
 //
 // Both buffers announce the entry that the next insertion will push out (`last`), so that the caller can fetch what it needs of
 // it long before it falls out; `replace` says whether the announced one is what fell out (it is, but for ties in depth).
+// Exact copies of a Gaussian, which densification by cloning makes, are tied in depth at every pixel.
 #pragma once
 
 #include "common.cuh"
@@ -57,6 +58,7 @@ struct UnsortedCore {
     int32_t base;
     uint32_t row_max[kRows];
     uint32_t kmax;
+    uint32_t settled;        // depth key of the last depth whose entries have been put in order where they lie (settle_ties)
     float depth_limit;       // a fragment enters if it is nearer than this
     uint32_t order[K];       // after finish(): keys in ascending order
 
@@ -79,6 +81,7 @@ struct UnsortedCore {
             for (int c = 0; c < 3 * K; ++c) rgb[c * THREADS] = 0.0f;
         }
         kmax = kEmpty + K - 1;
+        settled = 0xffffffffu;               // no depth: depth keys have kPosBits fewer bits
         depth_limit = decode(kmax);
     }
 
@@ -114,15 +117,17 @@ struct UnsortedCore {
         if constexpr (kRows % 2 == 0) top = max(top, row_max[kRows - 1]);
         kmax = top;
         depth_limit = decode(top);
-        if ((top ^ old) < uint32_t(K) && old < kEmpty) {
-            const uint32_t other = resolve_tie(keys, pay, c, old >> kPosBits, payload.y, evicted.y);
-            if (other < uint32_t(K)) {
-                const uint2 t = pay[other * THREADS];
-                pay[other * THREADS] = evicted;
-                evicted = t;
-                if constexpr (COLOUR) swap_colour(other, colour);
-                return false;
-            }
+        if ((top ^ old) < uint32_t(K) && old < kEmpty && (old >> kPosBits) != settled) {
+            // others of the depth stay: back into the slot with what was announced, and what the chain drops lies there afterwards
+            settled = old >> kPosBits;
+            const uint32_t announced = evicted.y;
+            pay[c * THREADS] = evicted;
+            if constexpr (COLOUR) swap_colour(c, colour);
+            settle_ties(keys, pay, c, settled);
+            if constexpr (COLOUR) swap_colour(c, colour);
+            evicted = pay[c * THREADS];
+            pay[c * THREADS] = payload;
+            return evicted.y == announced;
         }
         return true;
     }
@@ -151,17 +156,7 @@ struct UnsortedCore {
         bool tie = false;
         #pragma unroll
         for (int k = 0; k + 1 < K; ++k) tie |= (order[k] ^ order[k + 1]) < uint32_t(K) && order[k] < kEmpty;
-        if (tie) {
-            #pragma unroll
-            for (int q = 0; q < kRows; ++q)
-                *reinterpret_cast<uint4*>(keys + q * (THREADS * 4)) = make_uint4(order[4 * q], order[4 * q + 1], order[4 * q + 2], order[4 * q + 3]);
-            order_ties(keys, pay);
-            #pragma unroll
-            for (int q = 0; q < kRows; ++q) {
-                const uint4 row = *reinterpret_cast<const uint4*>(keys + q * (THREADS * 4));
-                order[4 * q] = row.x; order[4 * q + 1] = row.y; order[4 * q + 2] = row.z; order[4 * q + 3] = row.w;
-            }
-        }
+        if (tie) order_ties(keys, pay, settled);
     }
 
     // After finish(): entry k from the front; false if there is none.
@@ -180,43 +175,95 @@ private:
     }
     static __device__ __forceinline__ uint32_t key_at(const uint32_t* keys, uint32_t i) { return keys[(i >> 2) * (THREADS * 4) + (i & 3u)]; }
 
-    // How the chain orders two entries of equal depth: the one that arrived later goes behind the other one, and every later
-    // insertion in front of them rotates them by one (the carried entry passes entries of its own depth).  Nothing nearer than an
-    // entry falls out before it does, so the insertions in front of it are all still in the buffer and can be counted.
-    // True if the entry that arrived first comes first.  (Three or more entries of one depth at one pixel: pairs are ordered by the
-    // same rule, which need not be the chain's order.)
-    static __device__ __forceinline__ bool arrival_order(const uint32_t* keys, const uint2* pay, uint32_t depth_key, uint32_t later_word, uint32_t newest_word) {
-        uint32_t rotations = 0;
-        for (uint32_t i = 0; i < uint32_t(K); ++i) {
-            const uint32_t key = key_at(keys, i);
-            const uint32_t word = pay[(key & uint32_t(K - 1)) * THREADS].y;
-            if ((key >> kPosBits) < depth_key && word > later_word && word != newest_word) ++rotations;
+    static __device__ __forceinline__ uint32_t slot_key(const uint32_t* keys, uint32_t slot) { return keys[(slot >> 2) * (THREADS * 4) + (slot & 3u)]; }
+    static __device__ __forceinline__ void exchange(uint2* pay, uint32_t a, uint32_t b) {
+        const uint2 t = pay[a * THREADS];
+        pay[a * THREADS] = pay[b * THREADS];
+        pay[b * THREADS] = t;
+        if constexpr (COLOUR) {
+            float* rgb = reinterpret_cast<float*>(pay - threadIdx.x + K * THREADS) + threadIdx.x;
+            #pragma unroll 1
+            for (uint32_t i = 0; i < 3; ++i) {
+                const float x = rgb[(3 * a + i) * THREADS];
+                rgb[(3 * a + i) * THREADS] = rgb[(3 * b + i) * THREADS];
+                rgb[(3 * b + i) * THREADS] = x;
+            }
         }
-        return (rotations & 1u) == 0;
     }
 
-    // The new entry (`newest_word`, stored at c) pushed out an entry that has the same depth as another one that stayed.
-    // Returns the position of the other one if that is the one that has to fall out, else K.
-    static __device__ __noinline__ uint32_t resolve_tie(const uint32_t* keys, const uint2* pay, uint32_t c, uint32_t depth_key, uint32_t newest_word, uint32_t evicted_word) {
-        for (uint32_t i = 0; i < uint32_t(K); ++i) {
-            if (i == c || (key_at(keys, i) >> kPosBits) != depth_key) continue;
-            const uint32_t other_word = pay[i * THREADS].y;
-            const bool evicted_first = evicted_word < other_word;    // who arrived first
-            const bool in_arrival_order = arrival_order(keys, pay, depth_key, max(evicted_word, other_word), newest_word);
-            return evicted_first == in_arrival_order ? uint32_t(K) : i;   // the one in front falls out
+    // How the chain orders entries of exactly equal depth: a new one goes behind those that are there, and every later insertion in front
+    // of them carries the first one past the others, to their end - or out of a full buffer, if no entry is farther.  Nothing nearer
+    // than an entry falls out before it does, so the insertions in front are all still in the buffer, and as long as none of the tied
+    // entries has fallen out their order can be replayed from the words, which ascend in the order of arrival.  That is done when the
+    // first of them falls out (replace) or at the end (finish).  Once one has fallen out the order of the others is fixed: the depth is the
+    // buffer's limit, so nothing is added to it, and every insertion takes away the first.
+
+    // Exchanges the payloads of the entries of depth `depth_key` so that descending slots hold them in the chain's order, which is the order
+    // in which their keys make them fall out.  Slot c counts as one of them, whatever its key (K: there is no such slot).
+    static __device__ __noinline__ void settle_ties(const uint32_t* keys, uint2* pay, uint32_t c, uint32_t depth_key) {
+        uint32_t words[K], n = 0;
+        #pragma unroll 1
+        for (uint32_t slot = 0; slot < uint32_t(K); ++slot) {         // in the order of arrival
+            if (slot != c && (slot_key(keys, slot) >> kPosBits) != depth_key) continue;
+            const uint32_t word = pay[slot * THREADS].y;
+            uint32_t i = n++;
+            #pragma unroll 1
+            for (; i > 0 && words[i - 1] > word; --i) words[i] = words[i - 1];
+            words[i] = word;
         }
-        return uint32_t(K);
+        auto in_front_after = [&](uint32_t word) {                    // insertions in front of the depth since `word` arrived
+            uint32_t count = 0;
+            #pragma unroll 1
+            for (uint32_t slot = 0; slot < uint32_t(K); ++slot)
+                if (slot != c && (slot_key(keys, slot) >> kPosBits) < depth_key && pay[slot * THREADS].y > word) ++count;
+            return count;
+        };
+        #pragma unroll 1
+        for (uint32_t size = 2; size <= n; ++size) {                  // the first `size` that arrived, in the chain's order until the next one arrives
+            uint32_t turns = in_front_after(words[size - 1]);
+            if (size < n) turns -= in_front_after(words[size]);
+            #pragma unroll 1
+            for (turns %= size; turns > 0; --turns) {
+                const uint32_t first = words[0];
+                #pragma unroll 1
+                for (uint32_t i = 1; i < size; ++i) words[i - 1] = words[i];
+                words[size - 1] = first;
+            }
+        }
+        uint32_t place = 0;
+        #pragma unroll 1
+        for (uint32_t slot = K; slot-- > 0 && place < n;) {
+            if (slot != c && (slot_key(keys, slot) >> kPosBits) != depth_key) continue;
+            const uint32_t word = words[place++];
+            uint32_t other = slot;
+            #pragma unroll 1
+            while (other > 0 && pay[other * THREADS].y != word) --other;
+            if (other != slot) exchange(pay, slot, other);
+        }
     }
 
-    static __device__ __noinline__ void order_ties(uint32_t* keys, const uint2* pay) {
-        for (uint32_t k = 0; k + 1 < uint32_t(K); ++k) {
-            const uint32_t a = key_at(keys, k), b = key_at(keys, k + 1);
-            if ((a >> kPosBits) != (b >> kPosBits) || b >= kEmpty) continue;
-            const uint32_t wa = pay[(a & uint32_t(K - 1)) * THREADS].y, wb = pay[(b & uint32_t(K - 1)) * THREADS].y;
-            const bool in_arrival_order = arrival_order(keys, pay, a >> kPosBits, max(wa, wb), kNoEntry);
-            if ((wa < wb) != in_arrival_order) {
-                keys[(k >> 2) * (THREADS * 4) + (k & 3u)] = b;
-                keys[((k + 1) >> 2) * (THREADS * 4) + ((k + 1) & 3u)] = a;
+    // At the end: payloads of equal depth in the chain's order by ascending slot, as keys in ascending order name them.
+    static __device__ __noinline__ void order_ties(const uint32_t* keys, uint2* pay, uint32_t settled) {
+        #pragma unroll 1
+        for (uint32_t first = 0; first < uint32_t(K); ++first) {
+            const uint32_t key = slot_key(keys, first), depth_key = key >> kPosBits;
+            if (key >= kEmpty) continue;
+            uint32_t low = first, high = K;
+            auto tied = [&](uint32_t slot) { return (slot_key(keys, slot) >> kPosBits) == depth_key; };
+            bool seen = false;
+            #pragma unroll 1
+            for (uint32_t slot = 0; slot < first; ++slot) seen |= tied(slot);
+            if (seen) continue;
+            if (depth_key != settled) settle_ties(keys, pay, K, depth_key);
+            #pragma unroll 1
+            for (;;) {                                                // reverses them
+                #pragma unroll 1
+                do --high; while (high > low && !tied(high));
+                if (high <= low) break;
+                exchange(pay, low, high);
+                #pragma unroll 1
+                do ++low; while (low < high && !tied(low));
+                if (low >= high) break;
             }
         }
     }

@@ -58,3 +58,40 @@ def test_training_forward_and_gradients_agree_between_the_two_forms(mode, K):
     assert torch.equal(outs[0][0], outs[1][0])
     for a, b in zip(outs[0][1], outs[1][1]):
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-5 * float(b.abs().max()))
+
+
+def scene_with_copies(n, size, K, mode, copies, seed):
+    """Every Gaussian `copies` times, at random places of the list: between two copies of one Gaussian others arrive in front of and
+    behind them.  Colours and opacities differ."""
+    scene = scenes.tiny_scene(n=n, size=size, seed=seed, mode=mode, K=K, sh_degree=1)
+    of = np.random.default_rng(seed).permutation(n) // copies
+    for a in (scene.positions, scene.scales, scene.rotations):
+        a[:] = a[of]
+    scene.scales *= 1.5
+    scene.opacities[:] = np.clip(scene.opacities, 0.1, 0.6)
+    return scene, scene.views[0]
+
+
+@pytest.mark.parametrize("mode,K", [(0, 4), (0, 8), (0, 16), (0, 32), (1, 4), (1, 8), (1, 16), (1, 32)])
+@pytest.mark.parametrize("copies", [3, 4, 7])
+def test_three_and_more_entries_of_one_depth(mode, K, copies):
+    # 64 x 64 pixels run the form that keeps colours, 512 x 512 the other one
+    for size, n in ((64, 3000), (512, 6000)):
+        scene, view = scene_with_copies(n, size, K, mode, copies, seed=31 + copies)
+        for median in (False, True):
+            got = render(scene, view, mode, K, 0.2, 100.0, median)
+            want = render(scene, view, mode, K, 0.2, 3e38, median)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("mode,K", [(0, 8), (1, 16)])
+def test_training_forward_with_three_entries_of_one_depth(mode, K):
+    import torch
+    tb = harness.ours()
+    scene, view = scene_with_copies(4000, 160, K, mode, 3, seed=6)
+    images = []
+    for near, far in ((0.2, 100.0), (0.2, 3e38)):
+        wide = scenes.make_view(view.M, view.width, view.height, 256.0, 256.0, view.width / 2.0, view.height / 2.0, near, far)
+        with torch.no_grad():
+            images.append(tb.diff_rasterize(*harness.scene_tensors(scene), torch.empty(0, device="cuda"), harness.settings_for(tb, scene, wide, mode, K), False))
+    assert torch.equal(*images)
