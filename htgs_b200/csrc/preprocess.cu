@@ -175,26 +175,30 @@ __device__ __forceinline__ void make_fast_record(const float4& t1, const float4&
     for (int i = 0; i < 5; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
 }
 
-// The point from which the backward pass measures the pixels of a Gaussian: the centre of the outline, or, where that lies outside the
-// Gaussian's tile box (centres far off the screen belong to long or near Gaussians), the point of the box where the outline's form is
-// smallest.  From a far centre the moments of train.cu would cancel: 5e-5 of a gradient instead of a few 1e-6.
+// The point from which the backward pass measures the pixels of a Gaussian: its projected centre, where m = 0 and its weight is largest, or,
+// where that lies outside the tile box (long or near Gaussians), the point of the box where |m|^2, with its slopes at the projected
+// centre, is smallest.  From a point off the weight the moments of train.cu cancel (from the centre of the outline, which perspective
+// moves away from the projected centre: up to 3e-5 of the position gradient of a Gaussian of 2000 tiles, from here 1e-6).
 template <int MODE>
-__device__ __forceinline__ float2 make_moment_centre(const CullRecord& cr, const ushort4& box) {
+__device__ __forceinline__ float2 make_moment_centre(const float4& t1, const float4& t2, const float4& t4, const ushort4& box) {
     using MT = ModeTraits<MODE>;
     const float x0 = float(box.x) * MT::tile_w, x1 = float(box.y) * MT::tile_w - 1.0f, y0 = float(box.z) * MT::tile_h, y1 = float(box.w) * MT::tile_h - 1.0f;
-    if (cr.cx >= x0 && cr.cx <= x1 && cr.cy >= y0 && cr.cy <= y1 && cr.a != 0.0f) return make_float2(cr.cx, cr.cy);
+    const float cx = t1.w / t4.w, cy = t2.w / t4.w;
+    if (cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1) return make_float2(cx, cy);
+    // m = (y - cy) a - (x - cx) b there, up to the depth: |m|^2 = xx dx^2 + xy dx dy + yy dy^2
+    const float3 a = f3(t1) - cx * f3(t4), b = f3(t2) - cy * f3(t4);
+    const float xx = dot(b, b), xy = -2.0f * dot(a, b), yy = dot(a, a);
     float2 best = make_float2(0.5f * (x0 + x1), 0.5f * (y0 + y1));
-    if (cr.a == 0.0f || !(fabsf(cr.cx) <= FLT_MAX)) return best;
     float smallest = FLT_MAX;
     auto consider = [&](float x, float y) {
-        const float dx = x - cr.cx, dy = y - cr.cy, q = dx * (cr.a * dx + cr.b2 * dy) + cr.c * dy * dy;
+        const float dx = x - cx, dy = y - cy, q = dx * (xx * dx + xy * dy) + yy * dy * dy;
         if (q < smallest) { smallest = q; best = make_float2(x, y); }
     };
-    const float along_y = -0.5f * cr.b2 / cr.c, along_x = -0.5f * cr.b2 / cr.a;      // where the form is smallest along an edge, per unit of the other coordinate
-    consider(x0, fminf(fmaxf(fmaf(along_y, x0 - cr.cx, cr.cy), y0), y1));
-    consider(x1, fminf(fmaxf(fmaf(along_y, x1 - cr.cx, cr.cy), y0), y1));
-    consider(fminf(fmaxf(fmaf(along_x, y0 - cr.cy, cr.cx), x0), x1), y0);
-    consider(fminf(fmaxf(fmaf(along_x, y1 - cr.cy, cr.cx), x0), x1), y1);
+    const float along_y = -0.5f * xy / yy, along_x = -0.5f * xy / xx;      // where the form is smallest along an edge, per unit of the other coordinate
+    consider(x0, fminf(fmaxf(fmaf(along_y, x0 - cx, cy), y0), y1));
+    consider(x1, fminf(fmaxf(fmaf(along_y, x1 - cx, cy), y0), y1));
+    consider(fminf(fmaxf(fmaf(along_x, y0 - cy, cx), x0), x1), y0);
+    consider(fminf(fmaxf(fmaf(along_x, y1 - cy, cx), x0), x1), y1);
     return best;
 }
 
@@ -357,7 +361,7 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
         CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
         if constexpr (TRAIN) {
             out.clamp[gi] = clamp_bits;
-            const PairRecord pair = make_pair_record(t1, t2, t4, make_moment_centre<MODE>(cr, out.bounds[gi]));
+            const PairRecord pair = make_pair_record(t1, t2, t4, make_moment_centre<MODE>(t1, t2, t4, out.bounds[gi]));
             float4* pdst = reinterpret_cast<float4*>(out.pair + gi);
             pdst[0] = pair.n0; pdst[1] = pair.n1; pdst[2] = pair.d1; pdst[3] = make_float4(pair.cx, pair.cy, pair.shear, pair.pad);
         }

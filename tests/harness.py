@@ -93,6 +93,34 @@ def our_intermediates(device_index: int, n_primitives: int, n_instances: int):
     return out
 
 
+def training_blobs(scene, view, mode, K, blobs, n_instances):
+    """What the oracle needs of the four blobs of a training forward (per Gaussian, per tile, per instance, per pixel): the rows as the
+    forward rounded them, widened to float64, the tile ranges, the sorted list, and the core entries' positions (None without a K-buffer)."""
+    from oracle import oracle
+    per_primitive, per_tile, per_instance, per_pixel = blobs
+    n = scene.n
+    grid_w, grid_h = oracle.grid_of(view, mode)
+    n_tiles = grid_w * grid_h
+    at = 0
+
+    def section(count, dtype):          # csrc/api.cu: carve_primitive_blob
+        nonlocal at
+        begin = (at + 255) // 256 * 256
+        at = begin + count * np.dtype(dtype).itemsize
+        return per_primitive[begin:at].view(dtype)
+
+    section(20, np.uint32)              # FrameStatus
+    kept = section(n, np.uint32) != 0
+    section(4 * n, np.uint16)
+    records = section(20 * n, np.float32).reshape(n, 5, 4).astype(np.float64)
+    rows = {name: np.where(kept[:, None], records[:, i], 0.0) for i, name in enumerate(("vpmt1", "vpmt2", "vpmt4", "mt3", "rgba"))}
+    rows["clamp"] = oracle.preprocess(scene, view, mode, dtype=np.float64, with_clamp=True)["clamp"]
+    ranges = per_tile[:8 * n_tiles].view(np.uint32).reshape(n_tiles, 2)
+    prims = per_instance[:4 * n_instances].view(np.uint32)
+    core = per_pixel[:4 * K * n_tiles * 64].view(np.uint32).reshape(K, n_tiles * 64) if mode in (0, 1) else None
+    return rows, ranges, prims, core
+
+
 # ----------------------------------------------------------------------------------------------
 # parsers for the reference's scratch blobs (layouts: rasterization/include/*/buffer_utils.h;
 # every section starts on a 128-byte boundary of the absolute address, torch allocations are
