@@ -403,9 +403,9 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         if constexpr (SM::has_core && !kFirstK) scatter_core_entries(batch_begin - tile_range.x, min(NT, range.y - batch_begin));   // the forward's stored core positions count from the start of the tile's list
         __syncthreads();
         for (uint32_t first = warp * 32; first < n_segments; first += NT) {
-            if (first + lane >= n_segments) continue;
-            uint32_t pixels = s_segment[first + lane];
-            const uint32_t owner = s_owner[first + lane], j = owner >> 1;
+            const bool has_segment = first + lane < n_segments;
+            uint32_t pixels = has_segment ? s_segment[first + lane] : 0u;
+            const uint32_t owner = s_owner[min(first + lane, n_segments - 1u)], j = owner >> 1;
             const float row0 = float((owner & 1u) * 4u);
             const PairForm form{s_n0[j], s_n1[j], s_d1[j]};
             const float4 rgba = s_rgba[j], pos = s_pos[j];
@@ -455,7 +455,29 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
                 if constexpr (ABS_GRAD)
                     abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + column, y0 + row, cam);
             }
-            if (touched) {
+            // The segments of a Gaussian (at most four) lie side by side, but for the border between long and short ones: they are added up
+            // before they go out, since it is the number of additions to a record that its rounding grows with.
+            const uint32_t key = has_segment ? j : ~lane;
+            const bool join_1 = __shfl_down_sync(0xffffffffu, key, 1) == key && lane < 31;
+            const uint32_t joined_1 = __ballot_sync(0xffffffffu, join_1), joined_2 = joined_1 & (joined_1 >> 1);      // with the next lane, with the next but one
+            auto join = [&](float& x, int o, bool take) { const float t = __shfl_down_sync(0xffffffffu, x, o); if (take) x += t; };
+            auto join_all = [&](int o, bool take) {
+                join(moments.u0.x, o, take); join(moments.u0.y, o, take); join(moments.u0.z, o, take); join(moments.u0.w, o, take);
+                join(moments.u1.x, o, take); join(moments.u1.y, o, take); join(moments.u1.z, o, take); join(moments.u1.w, o, take);
+                join(moments.v1.x, o, take); join(moments.v1.y, o, take); join(moments.v1.z, o, take); join(moments.v1.w, o, take);
+                join(aC.x, o, take); join(aC.y, o, take); join(aC.z, o, take); join(aC.w, o, take);
+                if constexpr (ABS_GRAD) join(abs_grad, o, take);
+            };
+            uint32_t out = __ballot_sync(0xffffffffu, touched);
+            if (joined_1 != 0) {
+                join_all(1, join_1);
+                out |= joined_1 & (out >> 1);
+            }
+            if (joined_2 != 0) {
+                join_all(2, (joined_2 >> lane) & 1u);
+                out |= joined_2 & (out >> 2);
+            }
+            if (((out & ~(joined_1 << 1)) >> lane) & 1u) {
                 float4* rec = accum + size_t(s_g[j]) * 5;
                 red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); red_add_v4(rec + 2, moments.v1); red_add_v4(rec + 3, aC);
                 if constexpr (ABS_GRAD) red_add_v4(rec + 4, make_float4(abs_grad, 0.0f, 0.0f, 0.0f));
