@@ -45,7 +45,9 @@ __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.
 // The shear makes Ms and My orthogonal: however long and slanted the ellipse, the terms of m do not cancel.  The rows' gradients
 // are quadratic in (s, y) too, with coefficients that are the Gaussian's alone, so a pair only adds
 //     u = dL/drho^2 / D  (times D at the centre, which the record divides by)  and  v = u N / D,  each times  1, s, y, ss, sy, yy
-// to the Gaussian's record, and rows_from_moments applies the coefficients once per Gaussian.  That is 18 instructions per pair
+// to the Gaussian's record, and rows_from_moments applies the coefficients once per Gaussian.  Of the sum of v, which the rows of a scale
+// all but cancel against the second moments of u, only v - u N is added up, which vanishes with the perspective: u N follows from the
+// moments of u (a third to a half of the rounding of grad_scales).  That is 18 instructions per pair
 // instead of 54 for the rows themselves, and offsets from the centre keep the sums well conditioned, where the rows' sums hold products with
 // pixel coordinates that cancel later.
 struct AffinePlanes { float3 M0, Ms, My, D0, Ds, Dy; float4 A, B; float shear; };     // A = VPMT1 - cx VPMT4, B = VPMT2 - cy VPMT4
@@ -94,11 +96,11 @@ __device__ __noinline__ bool accepted_by_forward(const EvalRecord* rec, float pi
     return !(numerator_rho2 > MT::max_cutoff_sq * denominator) && !(fminf(opacity * G, kMaxFragmentAlpha) < MT::min_alpha);
 }
 
-struct PairMoments { float4 u0, u1, v1; };      // u: 1, s, y, ss | u: sy, yy, v: 1, s | v: y, ss, sy, yy
-__device__ __forceinline__ void add_moments(PairMoments& a, float u, float v, float s, float y) {
+struct PairMoments { float4 u0, u1, v1; };      // u: 1, s, y, ss | u: sy, yy, v: 1 (less u N), s | v: y, ss, sy, yy
+__device__ __forceinline__ void add_moments(PairMoments& a, float u, float v, float uN, float s, float y) {
     const float us = u * s, uy = u * y, vs = v * s, vy = v * y;
     a.u0.x += u; a.u0.y += us; a.u0.z += uy; a.u0.w = fmaf(us, s, a.u0.w);
-    a.u1.x = fmaf(us, y, a.u1.x); a.u1.y = fmaf(uy, y, a.u1.y); a.u1.z += v; a.u1.w += vs;
+    a.u1.x = fmaf(us, y, a.u1.x); a.u1.y = fmaf(uy, y, a.u1.y); a.u1.z += v - uN; a.u1.w += vs;
     a.v1.x += vy; a.v1.y = fmaf(vs, s, a.v1.y); a.v1.z = fmaf(vs, y, a.v1.z); a.v1.w = fmaf(vy, y, a.v1.w);
 }
 
@@ -107,10 +109,11 @@ __device__ __forceinline__ void add_moments(PairMoments& a, float u, float v, fl
 //     dX = (Y x dd - Y.w dm, Y . dm),   dY = (X.w dm - X x dd, -X . dm)
 // and the cubic terms of E cancel: x dX + y dY = ((x B - y A) x dd - (x B.w - y A.w) dm, (x B - y A) . dm).
 struct RowGradients { float4 dX, dY, E; };
-__device__ __forceinline__ RowGradients rows_from_moments(const AffinePlanes& p, const float4& T4, const PairMoments& a) {
+__device__ __forceinline__ RowGradients rows_from_moments(const AffinePlanes& p, const float4& T4, const float4& n0, const float4& n1, const PairMoments& a) {
     const float3 A = f3(p.A), B = f3(p.B), n = f3(T4);
     const float u = a.u0.x, us = a.u0.y, uy = a.u0.z, uss = a.u0.w, usy = a.u1.x, uyy = a.u1.y;
-    const float v = a.u1.z, vs = a.u1.w, vy = a.v1.x, vss = a.v1.y, vsy = a.v1.z, vyy = a.v1.w;
+    // the sum of v from that of v - u N; n0, n1: N as the pairs saw it
+    const float v = a.u1.z + fmaf(n1.y, uyy, fmaf(n1.x, usy, fmaf(n0.w, uss, fmaf(n0.z, uy, fmaf(n0.y, us, n0.x * u))))), vs = a.u1.w, vy = a.v1.x, vss = a.v1.y, vsy = a.v1.z, vyy = a.v1.w;
     // sums of u m and v d, and of these times y and x = s - shear * y
     const float3 m1 = u * p.M0 + us * p.Ms + uy * p.My, my = uy * p.M0 + usy * p.Ms + uyy * p.My;
     const float3 d1 = v * p.D0 + vs * p.Ds + vy * p.Dy, dy = vy * p.D0 + vsy * p.Ds + vyy * p.Dy;
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
                 aC.w += dL_dalpha * G;
                 touched = true;
                 const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D, times D at the centre
-                add_moments(moments, u, u * rho2, s, y);
+                add_moments(moments, u, u * rho2, u * numerator_rho2, s, y);
                 if constexpr (ABS_GRAD)
                     abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + column, y0 + row, cam);
             }
@@ -649,8 +652,8 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
                 const float y = offset_y + float(p >> 3), s = fmaf(shear, y, offset_x + float(p & 7u));
                 aC.x = fmaf(pair.x, grad.x, aC.x); aC.y = fmaf(pair.x, grad.y, aC.y); aC.z = fmaf(pair.x, grad.z, aC.z);
                 aC.w += pair.y;
-                const float u = -0.5f * opacity * pair.y * pair.w;
-                add_moments(moments, u, u * pair.z, s, y);
+                const float dL_drho2 = -0.5f * opacity * pair.y, u = dL_drho2 * pair.w;
+                add_moments(moments, u, u * pair.z, dL_drho2 * pair.z, s, y);
                 if constexpr (ABS_GRAD) abs_grad += abs_position_gradient(af, u, s, y, x0 + float(p & 7u), y0 + float(p >> 3), cam);
             }
         }
@@ -728,7 +731,7 @@ __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const float4 centre = ldg4(&pair[idx].cx);       // and shear, 1 / D at the centre
     const PairMoments moments{centre.w * accum[size_t(idx) * 5], centre.w * accum[size_t(idx) * 5 + 1], centre.w * accum[size_t(idx) * 5 + 2]};
     const RowGradients rows = rows_from_moments(affine_planes(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
-                                                              centre.x, centre.y, centre.z), T4, moments);
+                                                              centre.x, centre.y, centre.z), T4, ldg4(&pair[idx].n0.x), ldg4(&pair[idx].n1.x), moments);
     // dL/dVPMT4 = -(cx dL/dVPMT1 + cy dL/dVPMT2 + E): the products with the centre are moved to the rows of VPM, where they cancel
     const float4 dT1 = rows.dX, dT2 = rows.dY, dT4 = make_float4(-rows.E.x, -rows.E.y, -rows.E.z, -rows.E.w);
     const float3 c1 = make_float3(dT1.x, dT2.x, dT4.x), c2 = make_float3(dT1.y, dT2.y, dT4.y), c3 = make_float3(dT1.z, dT2.z, dT4.z);
