@@ -638,6 +638,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
         // ---- 3. lane = (survivor, half of the pixels) -----------------------------------------------------------------------
         // transposing back: bit 15 - i of lane p -> bit p of survivor i, this lane's 16 pixels in the low bits
         uint32_t pixels = transpose_half(accepted, lane);
+        const uint32_t halves = __ballot_sync(0xffffffffu, pixels != 0), any = halves | (halves >> 16) | (halves << 16);     // survivors with an accepted pair
         __syncwarp();
         PairMoments moments{};
         float4 aC = make_float4(0, 0, 0, 0);
@@ -663,7 +664,6 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
         };
         both_halves(moments.u0); both_halves(moments.u1); both_halves(moments.v1); both_halves(aC);
         if constexpr (ABS_GRAD) abs_grad += __shfl_xor_sync(0xffffffffu, abs_grad, 16);
-        const uint32_t any = __ballot_sync(0xffffffffu, aC.x != 0.0f || aC.y != 0.0f || aC.z != 0.0f || aC.w != 0.0f);
         if ((any >> lane) & 1u) {                        // the two half warps share the four or five reductions of a record
             float4* rec = accum + size_t(g) * 5;
             if (lane < kGoChunk) { red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); }

@@ -4,6 +4,7 @@ import pytest
 
 import harness
 from htgs_b200 import scenes
+from test_oracle_backward import gradients
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +41,31 @@ def test_sums_over_many_tiles(oracle_lib, mode, K, seed):
     want = oracle_lib.backward(scene, view, mode, K, ranges, prims, weights, rows, core)
     for leaf, grad, name in zip(leaves[:4], want, ("positions", "scales", "rotations", "opacities")):
         assert np.linalg.norm(leaf.grad.cpu().numpy() - grad) <= 3e-6 * np.linalg.norm(grad), name
+
+
+def mirrored_pair_scene():
+    """One Gaussian on the optical axis of an 8 x 8 image: pixels 3 and 4 of a row lie symmetrically about it."""
+    scene = scenes.tiny_scene(n=1, size=8, seed=1, sh_degree=0)
+    scene.positions[:] = (0.0, 0.0, 4.0)
+    scene.scales[:] = 0.8
+    scene.rotations[:] = (1.0, 0.0, 0.0, 0.0)
+    scene.opacities[:] = 0.5
+    scene.sh_0[:] = 0.5
+    return scene, scene.views[0]
+
+
+@pytest.mark.parametrize("mode,K", [(0, 4), (1, 4), (2, 1), (3, 1)])
+def test_opposite_gradients_of_a_mirrored_pair(oracle_lib, mode, K):
+    """The gradients of colour and opacity cancel, that of the position does not."""
+    import torch
+    tb = harness.ours()
+    scene, view = mirrored_pair_scene()
+    weights = np.zeros((3, 8, 8))
+    weights[:, 2, 3], weights[:, 2, 4] = 1.0, -1.0
+    leaves = [t.requires_grad_() for t in harness.scene_tensors(scene)]
+    image = tb.diff_rasterize(*leaves, torch.empty(0, device="cuda"), harness.settings_for(tb, scene, view, mode, K), False)
+    image.backward(torch.from_numpy(weights).float().cuda())
+    want = gradients(oracle_lib, scene, view, mode, K, weights)
+    assert abs(want[0][0, 0]) > 0.1
+    for leaf, grad in zip(leaves[:5], want):         # a few dozen float32 operations on numbers of this size
+        assert np.abs(leaf.grad.cpu().numpy() - grad).max() <= 1e-5 * abs(want[0][0, 0])
