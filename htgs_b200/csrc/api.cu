@@ -329,7 +329,8 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
     } else if (f.fast) {
         if ((err = launch_blend_fast(view.mode, view.K, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out.image, out.to_chw, L.status, stream)) != cudaSuccess) return fail_cuda(err, "fast blend");
     } else if ((err = launch_blend(view.mode, ctx->collect_stats ? BlendTask::image_with_statistics : BlendTask::image, view, geo, L.prim, prims_sorted, L.tile_ranges, L.tile_order, out, TrainPixelBuffers{}, L.status, stream)) != cudaSuccess) return fail_cuda(err, "blend");
-    *launches += 1;
+    const bool one_form = f.fast || (f.max_weights && (outline_mode == HTGS_MODE_HYBRID_BLEND || outline_mode == HTGS_MODE_OIT_BLEND));
+    *launches += one_form ? 1 : 2;     // blend kernels are launched in two forms (blend.cu)
     if (prof) cudaEventRecord(ev[6], stream);
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
     if ((err = cudaEventRecord(ctx->frame_done, stream)) != cudaSuccess) return fail_cuda(err, "frame event record");
@@ -779,7 +780,7 @@ static int forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsVi
     if (info) {
         std::memset(info, 0, sizeof(*info));
         info->n_instances = n_instances; info->n_visible = ctx->training_visible; info->key_bytes = uint32_t(plan.key_bytes); info->end_bit = uint32_t(plan.end_bit);
-        info->kernel_launches = launches + 4;
+        info->kernel_launches = launches + 5;
     }
     if (!wait) return HTGS_OK;
     rc = check_training(ctx);

@@ -49,7 +49,10 @@ constexpr int kHalf = 16;                        // records per half of the wind
 constexpr int kQueue = 64;                       // survivors of the filter that wait for a place: fewer than kHalf before a step of 32
 
 // The unsorted buffer from four entries on, where the depth range allows it (core_key_window); the chain otherwise.
-enum class Buffer { chain, keys, keys_and_colours };
+// `dividing` is the chain in a kernel that divides where the others take reciprocal_rn: every blend is launched in that form too, and
+// FrameStatus::divide tells which of the two launches has to do with the frame (the other one costs 2 us, 1 us behind a large frame).
+// A branch in the loop instead cost the frame 2 to 4 %, two copies of the loop 1 to 2 %.
+enum class Buffer { chain, keys, keys_and_colours, dividing };
 template <int K, Buffer BUFFER> struct CoreOf { using type = SortedCore<K, 32>; };
 template <int K> struct CoreOf<K, Buffer::keys> { using type = UnsortedCore<K, 32, false>; };
 template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = UnsortedCore<K, 32, true>; };
@@ -88,18 +91,23 @@ __device__ __forceinline__ FragmentFront fragment_front(const float4& VPMT1, con
     return f;
 }
 
-// HYBRID_BLEND with unsorted keys is held to the registers that leave the warps which shared memory admits (K = 16: 22, K = 32: 14).  Without
-// a bound the calls of the tie handling make the compiler spend 93 to 96 registers on some forms and spill others to 72.
-constexpr int blend_min_blocks(int mode, int K, bool chain) { return mode != HTGS_MODE_HYBRID_BLEND || chain || K < 8 ? 0 : K >= 32 ? 20 : 24; }
+// Warps per SM that forms with unsorted keys leave registers for: those that shared memory admits (K = 16: 22, K = 32: 14), fewer where that
+// would spill (K = 8: 31).  Without a bound the calls of the tie handling make the compiler spend 93 to 96 registers on some and spill others to 64 or 72.
+constexpr int blend_min_blocks(int mode, int K, Buffer buffer) {
+    if ((buffer != Buffer::keys && buffer != Buffer::keys_and_colours) || K < 8) return 0;
+    return mode == HTGS_MODE_HYBRID_BLEND ? (K >= 32 ? 20 : 24) : K >= 32 ? 14 : K >= 16 ? 22 : 28;
+}
 
 template <int MODE, int K, Buffer BUFFER, BlendTask TASK>
-__global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER == Buffer::chain)) blend_kernel(
+__global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_kernel(
     const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, float* __restrict__ image, float* __restrict__ depth_out, float* __restrict__ alpha_out,
     unsigned int* __restrict__ max_weights, float weight_threshold, TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
     bool use_median_depth, int32_t key_base, FrameStatus* status)
 {
-    cudaGridDependencySynchronize();      // no launch_after kernel follows
+    cudaGridDependencySynchronize();
+    constexpr bool kDivide = BUFFER == Buffer::dividing;
+    if ((__ldg(&status->divide) != 0) != kDivide) return;
     using MT = ModeTraits<MODE>;
     using SL = SmemLayout<MODE, K, BUFFER, TASK>;
     constexpr bool TRAIN = TASK == BlendTask::training, STATS = TASK == BlendTask::image_with_statistics, WEIGHTS = TASK == BlendTask::max_weights;
@@ -230,7 +238,7 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER == Buffer
                     const float numerator_rho2 = fr.numerator_rho2;
                     const float denominator = fr.denominator;
                     const bool inside_cutoff = !(numerator_rho2 > MT::max_cutoff_sq * denominator);
-                    const float denominator_rcp = reciprocal_rn(denominator);
+                    const float denominator_rcp = kDivide ? 1.0f / denominator : reciprocal_rn(denominator);
                     const float4 rgba_in = rec[4];
                     const float G = expf(-0.5f * numerator_rho2 * denominator_rcp);
                     const float alpha = fminf(rgba_in.w * G, kMaxFragmentAlpha);
@@ -295,7 +303,7 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER == Buffer
                     const float numerator_rho2 = fr.numerator_rho2;
                     const float denominator = fr.denominator;
                     const bool inside_cutoff = !(numerator_rho2 > MT::max_cutoff_sq * denominator);
-                    const float denominator_rcp = reciprocal_rn(denominator);
+                    const float denominator_rcp = kDivide ? 1.0f / denominator : reciprocal_rn(denominator);
                     rgba_in = rec[4];
                     const float G = expf(-0.5f * numerator_rho2 * denominator_rcp);
                     alpha = fminf(rgba_in.w * G, kMaxFragmentAlpha);
@@ -607,9 +615,11 @@ cudaError_t launch_task(const BlendLaunch& l, int32_t key_base) {
         if (err != cudaSuccess) return err;
     }
     const uint32_t grid = uint32_t(l.geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
-    return launch_after(kernel, grid, 32, SL::total, l.stream, l.tile_ranges, l.tile_order, l.prims_sorted, l.prim.eval, l.prim.cull, l.out.image, l.out.depth, l.out.alpha,
+    const cudaError_t err = launch_after(kernel, grid, 32, SL::total, l.stream, l.tile_ranges, l.tile_order, l.prims_sorted, l.prim.eval, l.prim.cull, l.out.image, l.out.depth, l.out.alpha,
                                               reinterpret_cast<unsigned int*>(l.out.max_weights), l.out.weight_threshold, l.tout, uint32_t(l.geo.width),
                                               uint32_t(l.geo.height), uint32_t(l.geo.grid_w), l.out.to_chw, l.out.use_median_depth, key_base, l.status);
+    if constexpr (BUFFER == Buffer::dividing) return err;
+    else return err != cudaSuccess ? err : launch_task<MODE, K, Buffer::dividing, TASK>(l, 0);
 }
 
 template <int MODE, int K, Buffer BUFFER>

@@ -126,7 +126,7 @@ struct FrameStatus {
     unsigned long long warp_trips_inserting;// ... of which at least one lane inserted into its K-buffer (the insertion chain ran)
     unsigned long long lane_insertions;     // ... and the lanes that inserted
     unsigned int range_blocks_done;         // blocks of the tile-range kernel that have finished; the last one orders the tiles
-    unsigned int reserved[1];
+    unsigned int divide;                    // 1 if a visible Gaussian's |d|^2 may lie outside the range of reciprocal_rn
 };
 
 // ---------------------------------------------------------------------------
@@ -158,15 +158,15 @@ __device__ __forceinline__ void operator+=(float4& a, const float4& b) { a.x += 
 __device__ __forceinline__ float3 normalize(const float3& v) { const float inv_len = rsqrtf(dot(v, v)); return v * inv_len; }
 __device__ __forceinline__ float length(const float3& v) { return sqrtf(dot(v, v)); }
 
-// 1 / x rounded to nearest, without a branch: the hardware approximation (within one unit in the last place) and one Newton step with
-// the residual in a fused multiply-add (Markstein, IBM J. Res. Dev. 34(1), 1990).  Compared with 1.0f / x on
-// the GPU for all 2^23 mantissas at twelve exponents: no difference.  Below the normal range it gives infinity, as 1 / 0 does.
-// The compiler's quotient takes a branch; without it the blend kernels run 10 % faster.
+// 1 / x rounded to nearest: the hardware approximation (within one unit in the last place) and one Newton step with the residual in a
+// fused multiply-add (Markstein, IBM J. Res. Dev. 34(1), 1990).  Equal to 1.0f / x for 2^-126 <= x <= 2^126, where x and 1 / x are
+// normal numbers (tests/test_gpu_reciprocal.py compares all of them), and not for other x: frames that hold a Gaussian whose
+// denominators may be such a number divide instead (FrameStatus::divide).  The compiler's quotient takes a branch, which keeps two
+// evaluations from being interleaved; without it the blend kernels run 10 % faster.
 __device__ __forceinline__ float reciprocal_rn(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    const float refined = __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
-    return fabsf(y) <= FLT_MAX ? refined : y;
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
 }
 
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }

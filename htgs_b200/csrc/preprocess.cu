@@ -334,6 +334,19 @@ __global__ void __launch_bounds__(kPreprocessBlock) preprocess_cull_kernel(
     }
 }
 
+// Whether |d|^2 = |(T1 - x T4) x (T2 - y T4)|^2 stays between 2^-100 and 2^100 at every pixel of the box.  d is the cofactor matrix of the rows
+// times (x, y, 1), so |d| is at least the product of the two smaller singular values of the rows, |det| over the largest one.  Holds for
+// Gaussians of 1e-9 to 1e5 units at a focal length of 1000 pixels; whatever overflows, underflows or is not a number does not hold.
+template <int MODE>
+__device__ __forceinline__ bool denominator_in_range(const float4& t1, const float4& t2, const float4& t4, const ushort4& box) {
+    using MT = ModeTraits<MODE>;
+    const float3 a = f3(t1), b = f3(t2), n = f3(t4);
+    const float aa = dot(a, a), bb = dot(b, b), nn = dot(n, n), det = dot(n, cross(a, b));
+    const float x = float(box.y) * MT::tile_w, y = float(box.w) * MT::tile_h;
+    const float largest = (sqrtf(aa) + x * sqrtf(nn)) * (sqrtf(bb) + y * sqrtf(nn));      // >= |d|
+    return det * det > 0x1p-100f * (aa + bb + nn) && largest < 0x1p50f;
+}
+
 // Pass 2, one thread per VISIBLE Gaussian (grid-stride over the list): colour from the SH coefficients, the
 // remaining parts of the evaluation record, the conservative outline.  Runs with full warps whatever the
 // fraction of Gaussians that survived culling.
@@ -341,7 +354,7 @@ constexpr int kFinishBlock = 128;
 template <int MODE, bool TRAIN, bool FAST>
 __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
     const float* __restrict__ positions, const float* __restrict__ opacities, const float* __restrict__ sh_0, const float* __restrict__ sh_rest,
-    const float* __restrict__ cam_position_ptr, PrimBuffers out, const FrameStatus* __restrict__ status, int active_sh_bases, int total_sh_bases, OutlineThresholds thresholds)
+    const float* __restrict__ cam_position_ptr, PrimBuffers out, FrameStatus* status, int active_sh_bases, int total_sh_bases, OutlineThresholds thresholds)
 {
     grid_dependency();
     const uint32_t n_visible = status->n_visible;
@@ -358,6 +371,7 @@ __global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
         [[maybe_unused]] double centre[2] = {0.0, 0.0};
         if constexpr (FAST) make_fast_record(t1, t2, t4, m3, rgb, opacity, dst, centre);
         else dst[4] = make_float4(rgb.x, rgb.y, rgb.z, opacity);
+        if constexpr (!FAST) { if (!denominator_in_range<MODE>(t1, t2, t4, out.bounds[gi])) atomicOr(&status->divide, 1u); }
         CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
         if constexpr (TRAIN) {
             out.clamp[gi] = clamp_bits;
