@@ -140,6 +140,9 @@ def lib():
                                                   ctypes.c_uint32, ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(HtgsFrameInfo)]
                 l.htgs_forward_finish_async.argtypes = l.htgs_forward_finish.argtypes
                 l.htgs_forward_ahead.argtypes = l.htgs_forward_finish.argtypes[:7] + [ctypes.POINTER(ctypes.c_uint32), ctypes.POINTER(HtgsFrameInfo)]
+                l.htgs_forward_wait.argtypes = [ctypes.c_void_p]
+                l.htgs_forward_check_begin.argtypes = [ctypes.c_void_p, ctypes.POINTER(HtgsTrainBlobs), ctypes.c_void_p]
+                l.htgs_forward_check_end.argtypes = [ctypes.c_void_p]
                 l.htgs_backward_scratch_bytes.restype = ctypes.c_size_t
                 l.htgs_backward_scratch_bytes.argtypes = [ctypes.POINTER(HtgsScene)]
                 l.htgs_backward.argtypes = [ctypes.c_void_p, ctypes.POINTER(HtgsScene), ctypes.POINTER(HtgsView), ctypes.POINTER(HtgsTrainBlobs),

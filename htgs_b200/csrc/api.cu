@@ -147,7 +147,7 @@ struct PendingFrame {
 struct HtgsContext {
     int device = 0;
     int sm_count = 0;
-    FrameStatus* host_status = nullptr;     // pinned: [0] frames and the first half of a training forward, [1] a training forward that is not waited for
+    FrameStatus* host_status = nullptr;     // pinned: [0] frames and the first half of a training forward, [1] a training forward that is not waited for, [2] a blob's (htgs_forward_check_begin)
     void* workspace = nullptr;              // internal grow-only workspace
     size_t workspace_bytes = 0;
     uint64_t instance_capacity = 0;         // capacity the internal workspace was last carved for
@@ -170,6 +170,8 @@ struct HtgsContext {
     cudaEvent_t training_done = nullptr;
     cudaEvent_t training_counted = nullptr; // the instance count of a training forward has reached host_status[0]
     uint32_t training_visible = 0;          // of the last htgs_forward_begin
+    bool blob_check_pending = false;        // between htgs_forward_check_begin and _end
+    cudaEvent_t blob_checked = nullptr;     // the blob's status has reached host_status[2]
     // measurement aids
     bool profiling = false;
     bool collect_stats = false;
@@ -233,19 +235,20 @@ HtgsContext* htgs_create(int device) {
     ctx->device = device;
     ctx->sm_count = prop.multiProcessorCount;
     int least = 0, greatest = 0;
-    if ((err = cudaHostAlloc(reinterpret_cast<void**>(&ctx->host_status), 2 * sizeof(FrameStatus), cudaHostAllocDefault)) != cudaSuccess ||
+    if ((err = cudaHostAlloc(reinterpret_cast<void**>(&ctx->host_status), 3 * sizeof(FrameStatus), cudaHostAllocDefault)) != cudaSuccess ||
         (err = cudaDeviceGetStreamPriorityRange(&least, &greatest)) != cudaSuccess ||
         (err = cudaStreamCreateWithPriority(&ctx->front_stream, cudaStreamNonBlocking, greatest)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->front_begin, cudaEventDisableTiming)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->front_end, cudaEventDisableTiming)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->frame_done, cudaEventDisableTiming)) != cudaSuccess ||
         (err = cudaEventCreateWithFlags(&ctx->training_done, cudaEventDisableTiming)) != cudaSuccess ||
-        (err = cudaEventCreateWithFlags(&ctx->training_counted, cudaEventDisableTiming)) != cudaSuccess) {
+        (err = cudaEventCreateWithFlags(&ctx->training_counted, cudaEventDisableTiming)) != cudaSuccess ||
+        (err = cudaEventCreateWithFlags(&ctx->blob_checked, cudaEventDisableTiming)) != cudaSuccess) {
         fail_cuda(err, "htgs_create: pinned status word, side stream and events");
         htgs_destroy(ctx);
         return nullptr;
     }
-    std::memset(ctx->host_status, 0, 2 * sizeof(FrameStatus));
+    std::memset(ctx->host_status, 0, 3 * sizeof(FrameStatus));
     return ctx;
 }
 
@@ -254,6 +257,7 @@ void htgs_destroy(HtgsContext* ctx) {
     DeviceGuard guard(ctx->device);
     if (ctx->pending.active) cudaEventSynchronize(ctx->frame_done);
     if (ctx->training_pending) cudaEventSynchronize(ctx->training_done);
+    if (ctx->blob_check_pending) cudaEventSynchronize(ctx->blob_checked);
     if (ctx->workspace) cudaFree(ctx->workspace);
     if (ctx->host_path_buf) cudaFree(ctx->host_path_buf);
     if (ctx->host_path_stream) cudaStreamDestroy(ctx->host_path_stream);
@@ -265,6 +269,7 @@ void htgs_destroy(HtgsContext* ctx) {
     if (ctx->frame_done) cudaEventDestroy(ctx->frame_done);
     if (ctx->training_done) cudaEventDestroy(ctx->training_done);
     if (ctx->training_counted) cudaEventDestroy(ctx->training_counted);
+    if (ctx->blob_checked) cudaEventDestroy(ctx->blob_checked);
     delete ctx;
 }
 
@@ -816,6 +821,53 @@ int htgs_forward_ahead(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
     if ((rc = forward_counted(ctx, n_instances)) != HTGS_OK) return rc;
     if (info) { info->n_instances = *n_instances; info->n_visible = ctx->training_visible; }
     return *n_instances > capacity ? fail(HTGS_ERR_WORKSPACE_TOO_SMALL, "the per-instance blob holds fewer instances than the view has") : HTGS_OK;
+}
+
+int htgs_forward_wait(HtgsContext* ctx) {
+    if (!ctx) return fail(HTGS_ERR_INVALID_ARGUMENT, "context must not be null");
+    DeviceGuard guard(ctx->device);
+    if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+    return check_training(ctx);
+}
+
+int htgs_forward_check_begin(HtgsContext* ctx, const HtgsTrainBlobs* blobs, void* stream_ptr) {
+    if (!ctx || !blobs) return fail(HTGS_ERR_INVALID_ARGUMENT, "null argument");
+    if (!blobs->per_primitive || blobs->per_primitive_bytes < sizeof(FrameStatus)) return fail(HTGS_ERR_WORKSPACE_TOO_SMALL, "the per-Gaussian forward blob is missing or too small");
+    DeviceGuard guard(ctx->device);
+    if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    cudaError_t err;
+    if (ctx->blob_check_pending) {       // the read of a check that was never ended may still be on its way
+        ctx->blob_check_pending = false;
+        if ((err = cudaEventSynchronize(ctx->blob_checked)) != cudaSuccess) return fail_cuda(err, "forward check");
+    }
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if ((err = cudaStreamIsCapturing(stream, &capture)) != cudaSuccess) return fail_cuda(err, "forward check");
+    if (capture != cudaStreamCaptureStatusNone) return HTGS_OK;
+    const FrameStatus* status = carve_primitive_blob(blobs->per_primitive, 0).status;      // comes first, however many Gaussians
+    if ((err = cudaMemcpyAsync(ctx->host_status + 2, status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "forward check");
+    if ((err = cudaEventRecord(ctx->blob_checked, stream)) != cudaSuccess) return fail_cuda(err, "forward check");
+    ctx->blob_check_pending = true;
+    return HTGS_OK;
+}
+
+int htgs_forward_check_end(HtgsContext* ctx) {
+    if (!ctx) return fail(HTGS_ERR_INVALID_ARGUMENT, "context must not be null");
+    if (!ctx->blob_check_pending) return HTGS_OK;
+    ctx->blob_check_pending = false;
+    DeviceGuard guard(ctx->device);
+    if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+    const cudaError_t err = cudaEventSynchronize(ctx->blob_checked);
+    if (err != cudaSuccess) return fail_cuda(err, "check of the training forward");
+    return htgs_check_status(ctx->host_status + 2);
+}
+
+int htgs_check_status(const void* host_status) {
+    static_assert(sizeof(FrameStatus) == HTGS_STATUS_BYTES, "the status comes first in the per-Gaussian blob");
+    FrameStatus status;
+    if (!host_status) return fail(HTGS_ERR_INVALID_ARGUMENT, "null argument");
+    std::memcpy(&status, host_status, sizeof(status));
+    return status.error ? fail(HTGS_ERR_DEVICE_FLAG, "check of the training forward: a kernel reported an internal error (bounded wait gave up)") : HTGS_OK;
 }
 
 size_t htgs_backward_scratch_bytes(const HtgsScene* scene) {

@@ -44,6 +44,7 @@ def frame_results(device=None):
     """Waits for and checks every frame this host thread queued with deferred checks (on `device`, or on all devices);
     raises what the blocking call would have raised.  Returns the HtgsFrameInfo of each context that was checked."""
     index = None if device is None else _device_index(torch.device(device))
+    check_training_forwards(-1 if index is None else index)
     infos = []
     for ctx in _native.contexts_of_thread(index):
         if ctx not in _queued:
@@ -55,6 +56,12 @@ def frame_results(device=None):
         infos.append(info)
         _set_info(info)
     return infos
+
+
+def check_training_forwards(device_index=-1):
+    """Waits for the training forwards of this host thread whose status nothing has checked yet; raises if one failed."""
+    for ctx in _native.contexts_of_thread(None if device_index < 0 else device_index):
+        _native.check(_native.lib().htgs_forward_wait(ctx))
 
 
 def _check_inputs(positions, scales, rotations, opacities, sh_0, sh_rest, M, VPM, cam_position):
@@ -300,6 +307,9 @@ def backward(densification_info, grad_image, image, positions, scales, rotations
         image_ptr = image.contiguous().data_ptr() if image.numel() else None
         stream = torch.cuda.current_stream(device).cuda_stream
         outs = (grad_positions, grad_scales, grad_rotations, grad_opacities, grad_sh_0, grad_sh_rest)
+        # The forward's status, read through its blob (autograd calls this on a thread whose context did not queue the forward) and
+        # waited for once the first part of the pass has been queued.
+        _native.check(lib.htgs_forward_check_begin(ctx, ctypes.byref(blobs), stream))
         if compact is not None:
             capacity = int(compact.capacity(n))
             rows = compact.buffer(lib.htgs_compact_rows_bytes(capacity), device)
@@ -310,6 +320,7 @@ def backward(densification_info, grad_image, image, positions, scales, rotations
                                              densification_info.data_ptr() if rows_d else None, rows_d, int(bool(use_distance_scaling)))
             _native.check(lib.htgs_backward_compact(ctx, ctypes.byref(scene), ctypes.byref(view), ctypes.byref(blobs), int(n_instances), grad_image.data_ptr(),
                                                     image_ptr, ctypes.byref(no_dense if one_pass else grads), rows.data_ptr(), capacity, stream))
+            _native.check(lib.htgs_forward_check_end(ctx))
             parts = compact.exchange(rows, capacity)
             if one_pass:
                 addresses = (ctypes.c_void_p * len(parts))(*[int(address) for address, _, _ in parts])
@@ -324,6 +335,7 @@ def backward(densification_info, grad_image, image, positions, scales, rotations
         if ranges is None:
             _native.check(lib.htgs_backward(ctx, ctypes.byref(scene), ctypes.byref(view), ctypes.byref(blobs), int(n_instances), grad_image.data_ptr(),
                                             image_ptr, ctypes.byref(grads), stream))
+            _native.check(lib.htgs_forward_check_end(ctx))
         else:
             covered = 0
             if not split_pass:
@@ -339,6 +351,8 @@ def backward(densification_info, grad_image, image, positions, scales, rotations
                 else:
                     _native.check(lib.htgs_backward_finish_range(ctx, ctypes.byref(scene), ctypes.byref(view), ctypes.byref(blobs), ctypes.byref(grads),
                                                                  int(first), int(count), stream))
+                if k == 0:
+                    _native.check(lib.htgs_forward_check_end(ctx))
                 if after_range is not None:
                     after_range(k, int(first), int(count), outs)
             if covered != n:

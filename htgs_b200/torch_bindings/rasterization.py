@@ -107,7 +107,8 @@ def deferred_checks() -> bool:
 
 
 def frame_results(device=None):
-    """Waits for and checks the frames queued with deferred checks by this host thread; see `set_deferred_checks`.
+    """Waits for and checks the frames queued with deferred checks by this host thread (see `set_deferred_checks`), and its training
+    forwards that nothing has checked yet (a backward pass checks the forward it belongs to).
     Returns one frame-statistics object per CUDA stream that had a frame queued."""
     _mark()
     if _via_pybind:
@@ -172,7 +173,10 @@ class _Rasterize(torch.autograd.Function):
 
 def diff_rasterize(positions, scales, rotations, opacities, sh_0, sh_rest, densification_info, settings: RasterizerSettings,
                    use_distance_scaling: bool) -> torch.Tensor:
-    return _Rasterize.apply(positions, scales, rotations, opacities, sh_0, sh_rest, densification_info, settings, use_distance_scaling)
+    image = _Rasterize.apply(positions, scales, rotations, opacities, sh_0, sh_rest, densification_info, settings, use_distance_scaling)
+    if not image.requires_grad:      # the backward pass checks the forward's status; here there will be none
+        _impl.check_training_forwards(image.device.index)
+    return image
 
 
 def rasterize(positions, scales, rotations, opacities, sh_0, sh_rest, settings: RasterizerSettings, to_chw: bool,

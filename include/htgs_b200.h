@@ -192,8 +192,9 @@ int htgs_forward_begin(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
 int htgs_forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
                         float* image, void* stream, HtgsFrameInfo* info);
 /* The same without waiting for the GPU: the call returns when everything is queued, so that the caller can queue the loss and the
- * backward pass while the forward runs.  Its status is checked by the next call on the context that has to wait anyway, or by
- * htgs_backward if the forward has finished by then; a device error is reported by that call (HTGS_ERR_DEVICE_FLAG). */
+ * backward pass while the forward runs.  Its status is checked by htgs_forward_wait or by the next call on the context that has to wait
+ * anyway, or by htgs_backward on the same context if the forward has finished by then; a device error is reported by that call
+ * (HTGS_ERR_DEVICE_FLAG). */
 int htgs_forward_finish_async(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t n_instances,
                               float* image, void* stream, HtgsFrameInfo* info);
 
@@ -204,6 +205,19 @@ int htgs_forward_finish_async(HtgsContext* ctx, const HtgsScene* scene, const Ht
  * htgs_forward_finish_async. */
 int htgs_forward_ahead(HtgsContext* ctx, const HtgsScene* scene, const HtgsView* view, const HtgsTrainBlobs* blobs, uint32_t capacity,
                        float* image, void* stream, uint32_t* n_instances, HtgsFrameInfo* info);
+
+/* Waits for the training forward that the context queued without a wait, if its status has not been checked yet, and returns it. */
+int htgs_forward_wait(HtgsContext* ctx);
+
+/* The status of a forward through its per-Gaussian blob, whichever context or thread queued it (a backward pass often runs on a thread of
+ * its own): _begin queues the read of the status word on `stream`, _end waits for that read, not for what was queued behind it, and
+ * returns HTGS_ERR_DEVICE_FLAG if the forward failed.  With htgs_backward between the two the GPU does not idle and no gradient of a
+ * failed forward goes unnoticed.  On a stream that is being captured both do nothing. */
+int htgs_forward_check_begin(HtgsContext* ctx, const HtgsTrainBlobs* blobs, void* stream);
+int htgs_forward_check_end(HtgsContext* ctx);
+/* The same for a caller that copies the first HTGS_STATUS_BYTES of the per-Gaussian blob to the host itself: what _end returns for them. */
+#define HTGS_STATUS_BYTES 64
+int htgs_check_status(const void* host_status);
 
 /* Outputs of the backward pass.  Every element of the six gradient tensors is written (zeros for culled
  * Gaussians), so they need not be cleared.  `scratch` (htgs_backward_scratch_bytes) holds the per-Gaussian
