@@ -122,11 +122,11 @@ template <> struct KeyOps<uint16_t> { static __device__ __forceinline__ uint16_t
 template <> struct KeyOps<uint32_t> { static __device__ __forceinline__ uint32_t make(uint32_t tile, uint32_t) { return tile; } static __device__ __forceinline__ uint32_t tile(uint32_t k) { return k; } };
 template <> struct KeyOps<uint64_t> { static __device__ __forceinline__ uint64_t make(uint32_t tile, uint32_t depth_bits) { return (uint64_t(tile) << 32) | depth_bits; } static __device__ __forceinline__ uint32_t tile(uint64_t k) { return uint32_t(k >> 32); } };
 
-// One block per 256 Gaussians (the blocks of the preprocess kernel).  A warp writes the instances of its 32 Gaussians
-// cooperatively, or the block those of all 256 where one warp would have most of the work: slot j belongs to the Gaussian
-// whose exclusive offset is the last one <= j (five or eight steps of search); inside a Gaussian the order is row-major over
+// One block per 256 Gaussians (the blocks of the preprocess kernel), which writes their instances cooperatively: slot j belongs to
+// the Gaussian whose exclusive offset is the last one <= j (eight steps of search); inside a Gaussian the order is row-major over
 // its tile box (rasterization/src/shared_kernels.cu:21-28), so the emitted stream is identical to the reference's.  Bound by
-// instructions (the search, the split in row and column by a multiplication).
+// instructions (the search, the split in row and column by a multiplication).  7.3 M instances: 49 us, 154 M: 493 us.  A search per
+// warp (five steps) where the warps have about equal work gave 51 and 504 us, always 88 and 715: one warp often has most of them.
 // The kernel also clears what the sort and the range kernel count in (`clear`): one launch instead of three.
 struct ClearList { uint4* begin[3]; uint64_t count[3]; uint64_t per_sort_block[3]; };   // 16-byte words: a fixed number, plus so many per sort block of the frame
 template <typename KeyT>
@@ -162,13 +162,10 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     excl[threadIdx.x] = inc - cnt;
     if (lane == 31) warp_tot[warp] = inc;
     __syncthreads();
-    uint32_t warp_base = 0, largest = 0;
+    uint32_t warp_base = 0;
     #pragma unroll
-    for (int w = 0; w < kPreprocessBlock / 32; ++w) {
-        const uint32_t t = warp_tot[w];
-        if (w < int(warp)) warp_base += t;
-        largest = max(largest, t);
-    }
+    for (int w = 0; w < kPreprocessBlock / 32; ++w)
+        if (w < int(warp)) warp_base += warp_tot[w];
     const uint64_t base = block_offsets[blockIdx.x];
     auto emit = [&](uint32_t slot, uint32_t local, uint32_t owner) {
         const uint4 b = box[owner];
@@ -181,24 +178,14 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
             prims[dst] = first + owner;
         }
     };
-    if (largest <= total / 4) {           // the warps have about equally many: each searches its own 32
-        const uint32_t mine = warp_tot[warp];
-        for (uint32_t j = lane; j < mine; j += 32) {
-            uint32_t lo = 32u * warp;
-            #pragma unroll
-            for (uint32_t step = 16; step > 0; step >>= 1) if (excl[lo + step] <= j) lo += step;
-            emit(warp_base + j, j - excl[lo], lo);
-        }
-    } else {                              // a few Gaussians of many tiles: the whole block writes them
-        __syncthreads();
-        excl[threadIdx.x] += warp_base;
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < total; j += kPreprocessBlock) {
-            uint32_t lo = 0;
-            #pragma unroll
-            for (uint32_t step = kPreprocessBlock / 2; step > 0; step >>= 1) if (excl[lo + step] <= j) lo += step;
-            emit(j, j - excl[lo], lo);
-        }
+    __syncthreads();
+    excl[threadIdx.x] += warp_base;
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < total; j += kPreprocessBlock) {
+        uint32_t lo = 0;
+        #pragma unroll
+        for (uint32_t step = kPreprocessBlock / 2; step > 0; step >>= 1) if (excl[lo + step] <= j) lo += step;
+        emit(j, j - excl[lo], lo);
     }
 }
 
