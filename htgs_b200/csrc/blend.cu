@@ -50,7 +50,8 @@ constexpr int kQueue = 64;                       // survivors of the filter that
 
 // The unsorted buffer from four entries on, where the depth range allows it (core_key_window); the chain otherwise.
 // `dividing` is the chain in a kernel that divides where the others take reciprocal_rn: every blend is launched in that form too, and
-// FrameStatus::divide tells which of the two launches has to do with the frame (the other one costs 2 us, 1 us behind a large frame).
+// FrameStatus::divide tells which of the two launches has to do with the frame.  The other one returns at once: 1184 CTAs (all 34230 of a
+// frame of 1297 x 840 took 22 us).
 // A branch in the loop instead cost the frame 2 to 4 %, two copies of the loop 1 to 2 %.
 enum class Buffer { chain, keys, keys_and_colours, dividing };
 template <int K, Buffer BUFFER> struct CoreOf { using type = SortedCore<K, 32>; };
@@ -91,23 +92,15 @@ __device__ __forceinline__ FragmentFront fragment_front(const float4& VPMT1, con
     return f;
 }
 
-// Warps per SM that forms with unsorted keys leave registers for: those that shared memory admits (K = 16: 22, K = 32: 14), fewer where that
-// would spill (K = 8: 31).  Without a bound the calls of the tie handling make the compiler spend 93 to 96 registers on some and spill others to 64 or 72.
-constexpr int blend_min_blocks(int mode, int K, Buffer buffer) {
-    if ((buffer != Buffer::keys && buffer != Buffer::keys_and_colours) || K < 8) return 0;
-    return mode == HTGS_MODE_HYBRID_BLEND ? (K >= 32 ? 20 : 24) : K >= 32 ? 14 : K >= 16 ? 22 : 28;
-}
-
+// One block of 8 x 4 pixels.  `phases`: the parities of the two halves' barriers, which the caller has initialised.  False if a wait gave up.
 template <int MODE, int K, Buffer BUFFER, BlendTask TASK>
-__global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_kernel(
-    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
+__device__ __forceinline__ bool blend_block(
+    uint32_t block, uint32_t& phases, unsigned char* smem, const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
     const CullRecord* __restrict__ cull, float* __restrict__ image, float* __restrict__ depth_out, float* __restrict__ alpha_out,
     unsigned int* __restrict__ max_weights, float weight_threshold, TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
     bool use_median_depth, int32_t key_base, FrameStatus* status)
 {
-    cudaGridDependencySynchronize();
     constexpr bool kDivide = BUFFER == Buffer::dividing;
-    if ((__ldg(&status->divide) != 0) != kDivide) return;
     using MT = ModeTraits<MODE>;
     using SL = SmemLayout<MODE, K, BUFFER, TASK>;
     constexpr bool TRAIN = TASK == BlendTask::training, STATS = TASK == BlendTask::image_with_statistics, WEIGHTS = TASK == BlendTask::max_weights;
@@ -115,7 +108,6 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
     constexpr uint32_t kTileX = MT::tile_w / kBlockW, kTileY = MT::tile_h / kBlockH;     // blocks per binning tile
-    extern __shared__ __align__(128) unsigned char smem[];
     EvalRecord* s_record = reinterpret_cast<EvalRecord*>(smem + SL::record_off);
     uint32_t* s_queue_prim = reinterpret_cast<uint32_t*>(smem + SL::queue_prim_off);
     uint32_t* s_queue_mask = reinterpret_cast<uint32_t*>(smem + SL::queue_mask_off);
@@ -124,18 +116,15 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + SL::bar_off);
 
     const uint32_t lane = threadIdx.x;
-    const uint32_t tile = __ldg(tile_order + blockIdx.x / (kTileX * kTileY)), part = blockIdx.x % (kTileX * kTileY);
+    const uint32_t tile = __ldg(tile_order + block / (kTileX * kTileY)), part = block % (kTileX * kTileY);
     const uint32_t block_x = (tile % grid_w) * kTileX + part % kTileX, block_y = (tile / grid_w) * kTileY + part / kTileX;
-    if (block_x * kBlockW >= width || block_y * kBlockH >= height) return;       // a ragged edge leaves blocks without pixels
+    if (block_x * kBlockW >= width || block_y * kBlockH >= height) return true;       // a ragged edge leaves blocks without pixels
     const uint32_t px_i = block_x * kBlockW + (lane & 7u);
     const uint32_t py_i = block_y * kBlockH + (lane >> 3);
     const bool inside = px_i < width && py_i < height;
     const float pixel_x = __uint2float_rn(px_i);
     const float pixel_y = __uint2float_rn(py_i);
     const float block_x0 = float(block_x * kBlockW), block_y0 = float(block_y * kBlockH);
-
-    if (lane < 2) mbar_init(s_bar + lane, 1);
-    mbar_fence_init();
 
     // ---- per-pixel state -------------------------------------------------------------------
     [[maybe_unused]] typename SL::Core core;
@@ -191,7 +180,6 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
     __syncwarp();
 
     uint32_t window = 0;                                 // this pixel's candidates: bits 31..16 the older half, 15..0 the newer half
-    uint32_t phases = 0;                                 // parity of each half's barrier
     for (uint32_t half = 0;; half ^= 1u) {
         // ---- 2. replace the half that no lane needs any more ----------------------------------------------------------
         const uint32_t count = min(queued, uint32_t(kHalf));
@@ -370,7 +358,7 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
             atomicAdd(&status->lane_insertions, (unsigned long long)ins);
         }
     }
-    if (!inside) return;
+    if (!inside) return !wait_failed;
     if constexpr (SL::has_kbuffer) core.finish();
 
     const uint32_t pixel_idx = width * py_i + px_i;
@@ -392,7 +380,6 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
                 if (stored && !(blending_weight < weight_threshold)) raise_weight(max_weights, payload.y, blending_weight);
             }
         }
-        return;
     } else if constexpr (TRAIN) {
         // ---- training forward: unclamped CHW image + what the backward pass needs per pixel ------------
         const uint32_t slot_base = tile * 64u + part * 32u + lane;   // tile-major pixel slot (modes with 8 x 8 tiles)
@@ -506,7 +493,7 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
         image[pixel_idx] = rgb_pixel.x;
         image[n_pixels + pixel_idx] = rgb_pixel.y;
         image[2 * n_pixels + pixel_idx] = rgb_pixel.z;
-        return;
+        return !wait_failed;
     } else {
     // ---- inference compositing ----------------------------------------------------------------------
     float3 rgb_pixel = make_float3(0.0f, 0.0f, 0.0f);
@@ -590,6 +577,42 @@ __global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_k
     if (depth_out) depth_out[pixel_idx] = depth_pixel;
     if (alpha_out) alpha_out[pixel_idx] = alpha_pixel;
     }
+    return !wait_failed;
+}
+
+// Warps per SM that forms with unsorted keys leave registers for: those that shared memory admits (K = 16: 22, K = 32: 14), fewer where that
+// would spill (K = 8: 31).  Without a bound the calls of the tie handling make the compiler spend 93 to 96 registers on some and spill others to 64 or 72.
+constexpr int blend_min_blocks(int mode, int K, Buffer buffer) {
+    if ((buffer != Buffer::keys && buffer != Buffer::keys_and_colours) || K < 8) return 0;
+    return mode == HTGS_MODE_HYBRID_BLEND ? (K >= 32 ? 20 : 24) : K >= 32 ? 14 : K >= 16 ? 22 : 28;
+}
+
+template <int MODE, int K, Buffer BUFFER, BlendTask TASK>
+__global__ void __launch_bounds__(32, blend_min_blocks(MODE, K, BUFFER)) blend_kernel(
+    const uint2* __restrict__ tile_ranges, const uint32_t* __restrict__ tile_order, const uint32_t* __restrict__ prims_sorted, const EvalRecord* __restrict__ eval,
+    const CullRecord* __restrict__ cull, float* __restrict__ image, float* __restrict__ depth_out, float* __restrict__ alpha_out,
+    unsigned int* __restrict__ max_weights, float weight_threshold, TrainPixelBuffers tout, uint32_t width, uint32_t height, uint32_t grid_w, bool to_chw,
+    bool use_median_depth, int32_t key_base, FrameStatus* status, uint32_t n_blocks)
+{
+    cudaGridDependencySynchronize();
+    if ((__ldg(&status->divide) != 0) != (BUFFER == Buffer::dividing)) return;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + SmemLayout<MODE, K, BUFFER, TASK>::bar_off);
+    if (threadIdx.x < 2) mbar_init(s_bar + threadIdx.x, 1);
+    mbar_fence_init();
+    uint32_t phases = 0;
+    auto one = [&](uint32_t block) {
+        return blend_block<MODE, K, BUFFER, TASK>(block, phases, smem, tile_ranges, tile_order, prims_sorted, eval, cull, image, depth_out, alpha_out, max_weights, weight_threshold,
+                                                  tout, width, height, grid_w, to_chw, use_median_depth, key_base, status);
+    };
+    if constexpr (BUFFER != Buffer::dividing) {
+        one(blockIdx.x);
+    } else {       // a small grid, since it mostly has nothing to do
+        for (uint32_t block = blockIdx.x; block < n_blocks; block += gridDim.x) {
+            if (!__all_sync(0xffffffffu, one(block))) return;      // the barriers' state is not known any more; the status has the error
+            __syncwarp();
+        }
+    }
 }
 
 struct BlendLaunch {
@@ -614,10 +637,11 @@ cudaError_t launch_task(const BlendLaunch& l, int32_t key_base) {
         const cudaError_t err = configured.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SL::total)); });
         if (err != cudaSuccess) return err;
     }
-    const uint32_t grid = uint32_t(l.geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
+    const uint32_t blocks = uint32_t(l.geo.n_tiles) * uint32_t((MT::tile_w / kBlockW) * (MT::tile_h / kBlockH));
+    const uint32_t grid = BUFFER == Buffer::dividing ? std::min(blocks, uint32_t(sm_count_of_current_device()) * 8u) : blocks;
     const cudaError_t err = launch_after(kernel, grid, 32, SL::total, l.stream, l.tile_ranges, l.tile_order, l.prims_sorted, l.prim.eval, l.prim.cull, l.out.image, l.out.depth, l.out.alpha,
                                               reinterpret_cast<unsigned int*>(l.out.max_weights), l.out.weight_threshold, l.tout, uint32_t(l.geo.width),
-                                              uint32_t(l.geo.height), uint32_t(l.geo.grid_w), l.out.to_chw, l.out.use_median_depth, key_base, l.status);
+                                              uint32_t(l.geo.height), uint32_t(l.geo.grid_w), l.out.to_chw, l.out.use_median_depth, key_base, l.status, blocks);
     if constexpr (BUFFER == Buffer::dividing) return err;
     else return err != cudaSuccess ? err : launch_task<MODE, K, Buffer::dividing, TASK>(l, 0);
 }

@@ -76,3 +76,26 @@ def test_frames_beyond_the_reciprocals_range(oracle_lib, mode, K, scale, depth):
     with torch.no_grad():
         image = tb.diff_rasterize(*harness.scene_tensors(scene), torch.empty(0, device="cuda"), settings, False)
     assert np.abs(image.cpu().numpy() - want)[near].max() <= 1e-6
+
+
+@pytest.mark.parametrize("mode,K", [(0, 2), (0, 8), (0, 16), (0, 32), (1, 16), (2, 1), (3, 1)])
+def test_dividing_form_equals_the_others(mode, K):
+    """A Gaussian of no extent that meets no pixel centre makes the whole frame divide (5120 blocks of pixels, more than the grid of that form)."""
+    import torch
+    tb = harness.ours()
+    images = []
+    for extent in (0.02, 1e-12):
+        scene = scenes.tiny_scene(n=6000, size=640, seed=9, mode=mode, K=K, sh_degree=1)
+        scene.positions[17] = (0.30001, 0.20001, 3.0)
+        scene.scales[17], scene.opacities[17] = extent, 1e-3 if extent > 1e-3 else 0.9      # neither shows
+        view = scene.views[0]
+        view.height = 512
+        settings = harness.settings_for(tb, scene, view, mode, K)
+        outputs = list(tb.rasterize(*harness.scene_tensors(scene), settings, True, False))
+        with torch.no_grad():
+            outputs.append(tb.diff_rasterize(*harness.scene_tensors(scene), torch.empty(0, device="cuda"), settings, False))
+        weights = torch.zeros((scene.n, 1), device="cuda")
+        tb.update_max_weights(weights, *harness.scene_tensors(scene)[:4], settings, 0.01)
+        images.append(outputs + [weights])
+    for a, b in zip(*images):
+        assert torch.equal(a, b)
