@@ -17,10 +17,9 @@
 //  * HYBRID / FIRST_K / OIT: the (Gaussian, pixel) candidates of a batch are cut into segments of at most 16 pixels of one
 //    Gaussian, one segment per lane.  The forward pass saves core entries as positions in the tile's list, so which pairs
 //    are core entries is a table filled once per batch, not a search per pair;
-//  * GLOBAL_ORDERING needs the running transmittance per pixel, so it stays pixel-parallel, in independent
-//    8x8-pixel CTAs; a warp only walks the staged Gaussians whose outline reaches its pixels, and the 32
-//    pixel contributions to one Gaussian are summed with a transposing shuffle reduction into a
-//    shared-memory record per staged Gaussian, flushed with vector reductions once per batch.
+//  * GLOBAL_ORDERING needs the running transmittance per pixel: one warp per 8x4 pixels walks the Gaussians that reach them, lane =
+//    pixel, and leaves what only the pixel knows of a pair in a table; then lane = Gaussian sums the pairs of the table and
+//    adds a record per Gaussian and warp.
 #include "kernels.h"
 
 #include <algorithm>
@@ -51,20 +50,28 @@ __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.
 // instead of 54 for the rows themselves, and offsets from the centre keep the sums well conditioned, where the rows' sums hold products with
 // pixel coordinates that cancel later.
 struct AffinePlanes { float3 M0, Ms, My, D0, Ds, Dy; float4 A, B; float shear; };     // A = VPMT1 - cx VPMT4, B = VPMT2 - cy VPMT4
+// In double where sums are turned into rows: for a Gaussian a hundred times as long as thick the sheared My is a hundredth of its terms
+// (in float32 the gradients of rotations lost 1e-5 of their norm by it).
+template <typename Real>
 __device__ __forceinline__ AffinePlanes affine_planes(const float4& T1, const float4& T2, const float4& T4, float cx, float cy, float shear) {
+    struct R3 { Real x, y, z; };
+    auto comb = [](Real p, const R3& a, Real q, const R3& b) { return R3{p * a.x + q * b.x, p * a.y + q * b.y, p * a.z + q * b.z}; };
+    auto cross3 = [](const R3& a, const R3& b) { return R3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; };
+    auto narrow = [](const R3& a) { return make_float3(float(a.x), float(a.y), float(a.z)); };
+    const Real x = cx, y = cy, w = T4.w, sh = shear;
+    const R3 n{T4.x, T4.y, T4.z}, a{T1.x - x * n.x, T1.y - x * n.y, T1.z - x * n.z}, b{T2.x - y * n.x, T2.y - y * n.y, T2.z - y * n.z};
+    const Real aw = T1.w - x * w, bw = T2.w - y * w;
+    const R3 ms = comb(bw, n, -w, b), ds = cross3(b, n);
     AffinePlanes p;
-    p.A = make_float4(fmaf(-cx, T4.x, T1.x), fmaf(-cx, T4.y, T1.y), fmaf(-cx, T4.z, T1.z), fmaf(-cx, T4.w, T1.w));
-    p.B = make_float4(fmaf(-cy, T4.x, T2.x), fmaf(-cy, T4.y, T2.y), fmaf(-cy, T4.z, T2.z), fmaf(-cy, T4.w, T2.w));
-    const float3 a = f3(p.A), b = f3(p.B), n = f3(T4);
-    p.M0 = p.A.w * b - p.B.w * a;
-    p.Ms = p.B.w * n - T4.w * b;
-    p.My = T4.w * a - p.A.w * n;
-    p.D0 = cross(a, b);
-    p.Ds = cross(b, n);
-    p.Dy = cross(n, a);
+    p.A = make_float4(float(a.x), float(a.y), float(a.z), float(aw));
+    p.B = make_float4(float(b.x), float(b.y), float(b.z), float(bw));
+    p.M0 = narrow(comb(aw, b, -bw, a));
+    p.D0 = narrow(cross3(a, b));
+    p.Ms = narrow(ms);
+    p.Ds = narrow(ds);
+    p.My = narrow(comb(Real(1), comb(w, a, -aw, n), -sh, ms));
+    p.Dy = narrow(comb(Real(1), cross3(n, a), -sh, ds));
     p.shear = shear;
-    p.My = p.My - p.shear * p.Ms;
-    p.Dy = p.Dy - p.shear * p.Ds;
     return p;
 }
 
@@ -139,7 +146,7 @@ struct AbsForm { float4 y0, x0, y1x1; };      // Y . m: 1, s, y, sy | X . m: 1, 
 __device__ __forceinline__ AbsForm abs_form(const EvalRecord* rec, const float4& centre_shear_scale) {
     const float* r = reinterpret_cast<const float*>(rec);
     const float4 T4 = ldg4(r + 8);
-    const AffinePlanes p = affine_planes(ldg4(r), ldg4(r + 4), T4, centre_shear_scale.x, centre_shear_scale.y, centre_shear_scale.z);
+    const AffinePlanes p = affine_planes<float>(ldg4(r), ldg4(r + 4), T4, centre_shear_scale.x, centre_shear_scale.y, centre_shear_scale.z);
     const float3 a = f3(p.A), b = f3(p.B), n = f3(T4);
     const float scale = centre_shear_scale.w;
     const float nm0 = dot(n, p.M0), nms = dot(n, p.Ms), nmy = dot(n, p.My);
@@ -692,13 +699,13 @@ __device__ __forceinline__ float4 quat_backward(const float4& q, const float (&d
 // (hybrid_blend/kernels/backward.cuh:10-102; SH part kernel_utils.cuh:190-281).  Every output element is
 // defined after the call: the rows of Gaussians that the view culled are written as zeros.  What bounds it is the store of the rows
 // (236 bytes per Gaussian at SH degree 3): a warp collects its 32 rows of grad_sh_rest in shared memory and stores them as
-// one block of 16-byte words.  3 M Gaussians: 260 us, against 219 us for rows stored in place after 0.7 GB of memsets, which
+// one block of 16-byte words.  3 M Gaussians: 248 us, against 219 us for rows stored in place after 0.7 GB of memsets, which
 // ran beside the per-tile kernel and slowed it down.
 //
 // COMPACT: instead of the six dense rows (59 floats at SH degree 3) the kernel appends one 64-byte record per Gaussian the view
-// kept to `out.compact_rows` (common.cuh: CompactGradientRow): the gradients of position, scale, rotation and opacity and the
+// kept to `out.compact_rows` (common.cuh: compact gradient rows): the gradients of position, scale, rotation and opacity and the
 // clamp-masked colour gradient.  The rows of grad_sh_0 / grad_sh_rest are (basis function of the view direction) x (colour
-// gradient), so whoever knows the camera position can rebuild them (expand_compact_row below and exchange.cu); this is what
+// gradient), so whoever knows the camera position can rebuild them (sh_rest_gradient_rows, exchange.cu); this is what
 // the ranks of a multi-GPU trainer send one another instead of the dense rows.
 constexpr int kChainThreads = 128;
 template <bool COMPACT>
@@ -730,7 +737,7 @@ __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const float4 T4 = ldg4(reinterpret_cast<const float*>(eval + idx) + 8);
     const float4 centre = ldg4(&pair[idx].cx);       // and shear, 1 / D at the centre
     const PairMoments moments{centre.w * accum[size_t(idx) * 5], centre.w * accum[size_t(idx) * 5 + 1], centre.w * accum[size_t(idx) * 5 + 2]};
-    const RowGradients rows = rows_from_moments(affine_planes(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
+    const RowGradients rows = rows_from_moments(affine_planes<double>(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
                                                               centre.x, centre.y, centre.z), T4, ldg4(&pair[idx].n0.x), ldg4(&pair[idx].n1.x), moments);
     // dL/dVPMT4 = -(cx dL/dVPMT1 + cy dL/dVPMT2 + E): the products with the centre are moved to the rows of VPM, where they cancel
     const float4 dT1 = rows.dX, dT2 = rows.dY, dT4 = make_float4(-rows.E.x, -rows.E.y, -rows.E.z, -rows.E.w);
@@ -968,7 +975,7 @@ cudaError_t launch_backward(int mode, int K, const HtgsScene& scene, const HtgsV
     if (!whole && mode == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING) return cudaErrorNotSupported;
     const uint32_t g_first = whole ? 0u : first, g_end = whole ? 0xffffffffu : first + count;
     cudaError_t err = cudaSuccess;
-    if (whole) {       // only the records of Gaussians that the view kept are ever added to or read (one in six: 15 us instead of 45 at 3 M)
+    if (whole) {       // only the records of Gaussians that the view kept are ever added to or read (one in six: 35 us at 3 M, a memset of all 45)
         clear_records_kernel<<<std::min<uint32_t>((n + 63) / 64, uint32_t(sm_count) * 8u), 256, 0, stream>>>(acc.accum, prim.visible_list, status);
         err = cudaGetLastError();
     } else {

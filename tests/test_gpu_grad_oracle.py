@@ -23,14 +23,26 @@ def tilted_scene(seed):
     return scene, scene.views[0]
 
 
+def needle_scene(seed):
+    """Gaussians a hundred times as long as thick, at all angles."""
+    scene = scenes.tiny_scene(n=16, size=768, seed=seed, sh_degree=0)
+    rng = np.random.default_rng(seed)
+    scene.positions[:, 2] = rng.uniform(3.0, 6.0, scene.n)
+    scene.positions[:, :2] = rng.uniform(-0.3, 0.3, (scene.n, 2)) * scene.positions[:, 2:]
+    scene.scales[:] = (0.005, 0.5, 0.005)
+    scene.opacities[:] = rng.uniform(0.5, 0.9, (scene.n, 1))
+    return scene, scene.views[0]
+
+
 @pytest.mark.parametrize("mode,K", [(0, 16), (0, 32), (1, 8), (2, 1), (3, 1)])
 @pytest.mark.parametrize("seed", [0, 1, 2, 3])
-def test_sums_over_many_tiles(oracle_lib, mode, K, seed):
+@pytest.mark.parametrize("make_scene", [tilted_scene, needle_scene])
+def test_sums_over_many_tiles(oracle_lib, mode, K, seed, make_scene):
     """Against float64 sums over the same rounded rows and core entries: what is left is the rounding of the pairs and of the sums.  A Gaussian has
     up to 3000 partial sums, added in no fixed order: roundings of 2^-25 on average give sqrt(3000) * 2^-25 = 1.6e-6 of a sum."""
     import torch
     tb = harness.ours()
-    scene, view = tilted_scene(seed)
+    scene, view = make_scene(seed)
     leaves = [t.requires_grad_() for t in harness.scene_tensors(scene)]
     image = tb.diff_rasterize(*leaves, torch.empty(0, device="cuda"), harness.settings_for(tb, scene, view, mode, K), False)
     weights = np.random.default_rng(7 + seed).choice([-1.0, 1.0], image.shape)       # signs, as an L1 loss gives them
