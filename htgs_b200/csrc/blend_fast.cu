@@ -33,7 +33,9 @@ namespace {
 constexpr int kFastThreads = 32;     // 8 x 4 pixels, one thread per pixel
 constexpr int kFastHalf = 16;        // records per half of the window
 constexpr int kFastQueue = 64;       // survivors of the filter that wait for a place
-constexpr int kFastDense = 20;       // pixels of 32 from which on a record is evaluated by all lanes together
+// pixels of 32 from which on a record is evaluated by all lanes together.  12: 1030 us, 16: 1022, 20: 1015, 24: 1012, 28: 1017 (3 M Gaussians, 1297 x 840, K = 16; 0.5 M, 3127 x
+// 1880: 1745, 1748, 1740, 1726, 1733): lanes that walk their own records read each one's rows again, all together they also evaluate where it does not reach.
+constexpr int kFastDense = 20;
 
 template <int MODE, int K> struct FastSmem {
     static constexpr bool has_kbuffer = MODE != HTGS_MODE_OIT_BLEND;

@@ -123,7 +123,7 @@ struct FrameStatus {
     unsigned long long candidate_pairs;     // statistics mode of the blend kernels
     unsigned long long accepted_fragments;  // statistics mode of the blend kernels
     unsigned long long warp_trips;          // statistics mode, HYBRID_BLEND: warp-level evaluations of one candidate per lane
-    unsigned long long warp_trips_inserting;// ... of which at least one lane inserted into its K-buffer (the insertion chain ran)
+    unsigned long long warp_trips_inserting;// ... of which at least one lane inserted into its K-buffer
     unsigned long long lane_insertions;     // ... and the lanes that inserted
     unsigned int range_blocks_done;         // blocks of the tile-range kernel that have finished; the last one orders the tiles
     unsigned int divide;                    // 1 if a visible Gaussian's |d|^2 may lie outside the range of reciprocal_rn
@@ -233,9 +233,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }

@@ -50,7 +50,9 @@ struct __align__(16) FilterView {
     float near_plane, pad[3];
 };
 template <int VIEWS> struct FilterViewBatch { FilterView view[VIEWS]; float largest_entry, largest_offset; };   // by value: up to 28 KB of kernel parameters
-constexpr int kFewestViews = 32, kFewViews = 48, kManyViews = 256;      // kFewestViews: kernel parameters of less than 4 KB, whose launch is the cheapest
+// Sizes of the kernel's parameter block: 3.6 KB, 5.4 KB and 29 KB.  A launch costs more the larger it is, most of all beyond 4 KB; 40 views take 36 us
+// with room for 48 and 47 us with room for 256 (16 k points; 300 k: 37 and 51, 3 M: 123 and 126).
+constexpr int kFewestViews = 32, kFewViews = 48, kManyViews = 256;
 
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }

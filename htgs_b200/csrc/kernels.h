@@ -28,8 +28,9 @@ struct PerDeviceOnce {
 };
 
 // Launch behind the previous kernel of the stream without the gap between two kernels (programmatic dependent launch).  The kernel has
-// to begin with grid_dependency().  A small frame is ten short kernels: 300 k Gaussians, 501 x 333, 192 -> 180 us per call; 16 k
-// Gaussians, 256 x 256, 318 -> 308 us; 1.5 M, 980 x 545, GLOBAL_ORDERING 715 -> 703 us.
+// to begin with grid_dependency().  A small frame is ten short kernels: 300 k Gaussians, 501 x 333, 199 -> 186 us per call; 16 k
+// Gaussians, 256 x 256, 315 -> 304 us; 1.5 M, 980 x 545, GLOBAL_ORDERING 715 -> 703 us.  (A blend kernel that follows a wait for another stream, as
+// a frame's does by default, gains nothing by it; a training forward's does.)
 template <typename... Params, typename... Args>
 cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchAttribute attribute{};

@@ -18,6 +18,6 @@ def update_3d_filter(positions: torch.Tensor, w2c: torch.Tensor, filter_3d: torc
 def update_3d_filter_views(positions: torch.Tensor, w2cs, filter_3d: torch.Tensor, visibility_mask: torch.Tensor, widths, heights, focal_xs, focal_ys,
                            center_xs, center_ys, near_planes, clipping_tolerance: float, distance2filter: float) -> None:
     """The loop over a dataset's views (Model.py:126-145 of the reference) as one call: same result, bit for bit, as
-    `update_3d_filter` once per view, with the positions read once per 48 views."""
+    `update_3d_filter` once per view, with the positions read once per 256 views."""
     return _C.update_3d_filter_views_cuda(positions, w2cs, filter_3d, visibility_mask, widths, heights, focal_xs, focal_ys, center_xs, center_ys,
                                           near_planes, clipping_tolerance, distance2filter)

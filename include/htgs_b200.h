@@ -85,7 +85,7 @@ typedef struct HtgsFrameInfo {
     uint64_t candidate_pairs;    /* statistics mode only: (pixel, Gaussian) pairs that passed the outline test */
     uint64_t accepted_fragments; /* statistics mode only: fragments accepted by the exact test */
     uint64_t warp_trips;           /* statistics mode, HYBRID_BLEND: warp-level evaluations of one candidate per lane */
-    uint64_t warp_trips_inserting; /* ... in which at least one lane inserted into its K-buffer (the insertion chain ran) */
+    uint64_t warp_trips_inserting; /* ... in which at least one lane inserted into its K-buffer */
     uint64_t lane_insertions;      /* ... and the number of lanes that inserted */
 } HtgsFrameInfo;
 
@@ -411,7 +411,7 @@ int htgs_update_3d_filter(const float* positions, const float* w2c, float* filte
 /*
  * The same update for several views in one pass over the points (no counterpart in the reference, whose caller loops over
  * the views, Model.py:126-145): equal, bit for bit, to calling htgs_update_3d_filter once per view in order, but the
- * positions are read once per 48 views instead of once per view.  `views` is a HOST array (camera parameters travel as
+ * positions are read once per 256 views instead of once per view.  `views` is a HOST array (camera parameters travel as
  * kernel arguments); every other pointer is a device pointer.  Stream-ordered, no host synchronisation, no allocation.
  */
 typedef struct HtgsFilterView {
