@@ -46,7 +46,7 @@ __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.
 //     u = dL/drho^2 / D  (times D at the centre, which the record divides by)  and  v = u N / D,  each times  1, s, y, ss, sy, yy
 // to the Gaussian's record, and rows_from_moments applies the coefficients once per Gaussian.  Of the sum of v, which the rows of a scale
 // all but cancel against the second moments of u, only v - u N is added up, which vanishes with the perspective: u N follows from the
-// moments of u (a third to a half of the rounding of grad_scales).  That is 18 instructions per pair
+// moments of u (a third to a half of the rounding of grad_scales).  That is 19 instructions per pair
 // instead of 54 for the rows themselves, and offsets from the centre keep the sums well conditioned, where the rows' sums hold products with
 // pixel coordinates that cancel later.
 struct AffinePlanes { float3 M0, Ms, My, D0, Ds, Dy; float4 A, B; float shear; };     // A = VPMT1 - cx VPMT4, B = VPMT2 - cy VPMT4
