@@ -51,15 +51,13 @@ __device__ __forceinline__ float4 row_times_T(const float4& row, const float3& u
 }
 
 // rasterization/include/kernel_utils.cuh:140-188
+// `c`: the Gaussian's coefficients beyond the first band, in shared memory.
 template <bool TRAIN>
-__device__ __forceinline__ float3 sh_to_rgb(const float* __restrict__ sh_0, const float* __restrict__ sh_rest, const float3& position,
-                                            const float3& cam_position, uint32_t idx, int active_sh_bases, int total_sh_bases,
+__device__ __forceinline__ float3 sh_to_rgb(const float3& dc, const float* c, const float3& position, const float3& cam_position, int active_sh_bases,
                                             uint8_t* clamp_bits) {
-    const float3 dc = make_float3(__ldg(sh_0 + 3 * size_t(idx)), __ldg(sh_0 + 3 * size_t(idx) + 1), __ldg(sh_0 + 3 * size_t(idx) + 2));
     float3 result = 0.5f + 0.28209479177387814f * dc;
     if (active_sh_bases > 1) {
-        const float* c = sh_rest + size_t(idx) * size_t(total_sh_bases) * 3;
-        auto coef = [&](int i) { return make_float3(__ldg(c + 3 * i), __ldg(c + 3 * i + 1), __ldg(c + 3 * i + 2)); };
+        auto coef = [&](int i) { return make_float3(c[3 * i], c[3 * i + 1], c[3 * i + 2]); };
         const float3 dir = normalize(position - cam_position);
         const float x = dir.x, y = dir.y, z = dir.z;
         result = result + (-0.48860251190291987f * y) * coef(0)
@@ -302,6 +300,7 @@ __global__ void __launch_bounds__(kPreprocessBlock) preprocess_cull_kernel(
                         dst[0] = T1; dst[1] = T2; dst[2] = T4;
                         if constexpr (MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING) dst[3] = make_float4(0.0f, 0.0f, 0.0f, z);
                         else dst[3] = make_float4(dot3_pinned_alt(f3(M3), u), dot3_pinned(f3(M3), v), dot3_pinned(f3(M3), w), z);
+                        dst[4] = make_float4(position.x, position.y, position.z, opacity);      // until the finish pass puts the colour there
                     }
                 }
             }
@@ -347,50 +346,111 @@ __device__ __forceinline__ bool denominator_in_range(const float4& t1, const flo
     return det * det > 0x1p-100f * (aa + bb + nn) && largest < 0x1p50f;
 }
 
-// Pass 2, one thread per VISIBLE Gaussian (grid-stride over the list): colour from the SH coefficients, the
+// Pass 2, one lane per VISIBLE Gaussian (grid-stride over the list, a warp at a time): colour from the SH coefficients, the
 // remaining parts of the evaluation record, the conservative outline.  Runs with full warps whatever the
 // fraction of Gaussians that survived culling.
+//
+// The visible Gaussians are scattered, so a lane's inputs share no cache line with its neighbours', and a warp's load of one float
+// costs the L1 a look-up per lane, for 45 coefficients, 16 floats of the rows, position and opacity.  So each lane fetches its
+// inputs with two bulk copies, the record (in which the cull pass left position and opacity too) and the 16-byte aligned window around
+// its row of coefficients, and reads them from shared memory; strides of 80 and, at degree 3, 208 bytes spread the lanes over the
+// banks.  What bounds it now is DRAM (53 % of its throughput at 600 bytes in 64-byte pieces per Gaussian) and the latency of the float64 chains.
+// Loads by lane -> copies, 3 M Gaussians, 1297 x 840: 88 -> 73 us, training 107 -> 88, relaxed precision 94 -> 79, 1.5 M in GLOBAL_ORDERING 82 -> 65.
 constexpr int kFinishBlock = 128;
+constexpr int kFinishWarps = kFinishBlock / 32;
+struct FinishLayout {               // of a warp's part of shared memory: 32 windows, 32 records
+    uint32_t window_bytes;          // copied around a row of coefficients (0: degree 0, or no colour wanted)
+    uint32_t window_stride;
+};
+inline FinishLayout finish_layout(int active_sh_bases, bool colour) {
+    if (!colour || active_sh_bases <= 1) return {0, 0};
+    const uint32_t bytes = (12u * uint32_t(active_sh_bases - 1) + 12u + 15u) & ~15u;      // a row starts up to 12 bytes behind a 16-byte boundary
+    return {bytes, (bytes / 16u) % 2u ? bytes : bytes + 16u};                             // an odd number of 16-byte words
+}
+constexpr int finish_blocks_per_sm(bool train, bool fast) { return train || fast ? 5 : 6; }
 template <int MODE, bool TRAIN, bool FAST>
-__global__ void __launch_bounds__(kFinishBlock) preprocess_finish_kernel(
-    const float* __restrict__ positions, const float* __restrict__ opacities, const float* __restrict__ sh_0, const float* __restrict__ sh_rest,
-    const float* __restrict__ cam_position_ptr, PrimBuffers out, FrameStatus* status, int active_sh_bases, int total_sh_bases, OutlineThresholds thresholds)
+__global__ void __launch_bounds__(kFinishBlock, finish_blocks_per_sm(TRAIN, FAST)) preprocess_finish_kernel(
+    const float* __restrict__ sh_0, const float* __restrict__ sh_rest, const float* __restrict__ cam_position_ptr, PrimBuffers out, FrameStatus* status,
+    uint32_t n_primitives, int active_sh_bases, int total_sh_bases, OutlineThresholds thresholds, FinishLayout layout)
 {
     grid_dependency();
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t s_bar[kFinishWarps];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint64_t* bar = s_bar + warp;
+    if (lane == 0) mbar_init(bar, 1);
+    mbar_fence_init();
+    __syncwarp();
+    unsigned char* my_window = smem + warp * (32u * (layout.window_stride + sizeof(EvalRecord))) + lane * layout.window_stride;
+    float4* my_record = reinterpret_cast<float4*>(smem + warp * (32u * (layout.window_stride + sizeof(EvalRecord))) + 32u * layout.window_stride) + lane * 5u;
     const uint32_t n_visible = status->n_visible;
     const float3 cam_position = make_float3(__ldg(cam_position_ptr), __ldg(cam_position_ptr + 1), __ldg(cam_position_ptr + 2));
-    for (uint32_t i = blockIdx.x * kFinishBlock + threadIdx.x; i < n_visible; i += gridDim.x * kFinishBlock) {
-        const uint32_t gi = out.visible_list[i];
+    const size_t row_bytes = size_t(total_sh_bases) * 12u;
+    const uintptr_t sh_begin = reinterpret_cast<uintptr_t>(sh_rest), sh_end = sh_begin + size_t(n_primitives) * row_bytes;
+    const uint32_t step = gridDim.x * kFinishBlock;
+    uint32_t i = blockIdx.x * kFinishBlock + threadIdx.x;
+    uint32_t gi_next = i < n_visible ? out.visible_list[i] : 0u;
+    for (uint32_t parity = 0; i - lane < n_visible; i += step, parity ^= 1u) {
+        const bool valid = i < n_visible;
+        const uint32_t gi = gi_next;
         float4* dst = reinterpret_cast<float4*>(out.eval + gi);
-        const float4 t1 = dst[0], t2 = dst[1], t4 = dst[2], m3 = dst[3];
-        const float3 position = make_float3(__ldg(positions + 3 * size_t(gi)), __ldg(positions + 3 * size_t(gi) + 1), __ldg(positions + 3 * size_t(gi) + 2));
-        const float opacity = __ldg(opacities + gi);
-        uint8_t clamp_bits = 0;
-        const float3 rgb = sh_0 ? sh_to_rgb<TRAIN>(sh_0, sh_rest, position, cam_position, gi, active_sh_bases, total_sh_bases, &clamp_bits)
-                                : make_float3(0.0f, 0.0f, 0.0f);   // colour-less callers (update_max_weights)
-        [[maybe_unused]] double centre[2] = {0.0, 0.0};
-        if constexpr (FAST) make_fast_record(t1, t2, t4, m3, rgb, opacity, dst, centre);
-        else dst[4] = make_float4(rgb.x, rgb.y, rgb.z, opacity);
-        if constexpr (!FAST) { if (!denominator_in_range<MODE>(t1, t2, t4, out.bounds[gi])) atomicOr(&status->divide, 1u); }
-        CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
-        if constexpr (TRAIN) {
-            out.clamp[gi] = clamp_bits;
-            const PairRecord pair = make_pair_record(t1, t2, t4, make_moment_centre<MODE>(t1, t2, t4, out.bounds[gi]));
-            float4* pdst = reinterpret_cast<float4*>(out.pair + gi);
-            pdst[0] = pair.n0; pdst[1] = pair.n1; pdst[2] = pair.d1; pdst[3] = make_float4(pair.cx, pair.cy, pair.shear, pair.pad);
+        // the window may reach beyond the ends of the tensor: at the first and last row, if these do not lie on 16-byte boundaries
+        const uintptr_t row = sh_begin + size_t(gi) * row_bytes, window = row & ~uintptr_t(15);
+        const bool whole = valid && layout.window_bytes != 0 && window >= sh_begin && window + layout.window_bytes <= sh_end;
+        const uint32_t n_valid = __popc(__ballot_sync(0xffffffffu, valid)), n_whole = __popc(__ballot_sync(0xffffffffu, whole));
+        if (lane == 0) mbar_arrive_expect_tx(bar, n_valid * uint32_t(sizeof(EvalRecord)) + n_whole * layout.window_bytes);
+        __syncwarp();
+        if (valid) bulk_copy_g2s(my_record, dst, uint32_t(sizeof(EvalRecord)), bar);
+        if (whole) bulk_copy_g2s(my_window, reinterpret_cast<const void*>(window), layout.window_bytes, bar);
+        float* coefficients = reinterpret_cast<float*>(my_window + (row & 15u));
+        if (valid && !whole && layout.window_bytes != 0) {
+            const float* from = sh_rest + size_t(gi) * size_t(total_sh_bases) * 3;
+            for (int c = 0; c < 3 * (active_sh_bases - 1); ++c) coefficients[c] = __ldg(from + c);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // in front of the copy that the next round puts here
         }
-        if constexpr (FAST) {
-            // The fragment evaluation measures from the projected centre, the outline test from the centre of
-            // the outline: the record carries the (small) difference, so that outline centre + difference
-            // gives the projected centre to better than float32 resolution at the pixel's magnitude.
-            cr.r = float(centre[0] - double(cr.cx));
-            cr.g = float(centre[1] - double(cr.cy));
-        } else {
-            cr.r = rgb.x; cr.g = rgb.y; cr.b = rgb.z;
+        float3 dc = make_float3(0.0f, 0.0f, 0.0f);
+        ushort4 box = make_ushort4(0, 0, 0, 0);
+        if (valid) {
+            if (sh_0) dc = make_float3(__ldg(sh_0 + 3 * size_t(gi)), __ldg(sh_0 + 3 * size_t(gi) + 1), __ldg(sh_0 + 3 * size_t(gi) + 2));
+            if constexpr (!FAST) box = out.bounds[gi];
         }
-        float4* cdst = reinterpret_cast<float4*>(out.cull + gi);
-        cdst[0] = make_float4(cr.cx, cr.cy, cr.a, cr.b2);
-        cdst[1] = make_float4(cr.c, cr.r, cr.g, cr.b);
+        gi_next = i + step < n_visible ? out.visible_list[i + step] : 0u;
+        if (!mbar_wait_bounded(bar, parity)) {
+            atomicOr(&status->error, 1u);
+            return;
+        }
+        if (valid) {
+            const float4 t1 = my_record[0], t2 = my_record[1], t4 = my_record[2], m3 = my_record[3], centre_opacity = my_record[4];
+            const float3 position = f3(centre_opacity);
+            const float opacity = centre_opacity.w;
+            uint8_t clamp_bits = 0;
+            const float3 rgb = sh_0 ? sh_to_rgb<TRAIN>(dc, coefficients, position, cam_position, active_sh_bases, &clamp_bits)
+                                    : make_float3(0.0f, 0.0f, 0.0f);   // colour-less callers (update_max_weights)
+            [[maybe_unused]] double centre[2] = {0.0, 0.0};
+            if constexpr (FAST) make_fast_record(t1, t2, t4, m3, rgb, opacity, dst, centre);
+            else dst[4] = make_float4(rgb.x, rgb.y, rgb.z, opacity);
+            if constexpr (!FAST) { if (!denominator_in_range<MODE>(t1, t2, t4, box)) atomicOr(&status->divide, 1u); }
+            CullRecord cr = make_cull_record(t1, t2, t4, opacity, thresholds);
+            if constexpr (TRAIN) {
+                out.clamp[gi] = clamp_bits;
+                const PairRecord pair = make_pair_record(t1, t2, t4, make_moment_centre<MODE>(t1, t2, t4, box));
+                float4* pdst = reinterpret_cast<float4*>(out.pair + gi);
+                pdst[0] = pair.n0; pdst[1] = pair.n1; pdst[2] = pair.d1; pdst[3] = make_float4(pair.cx, pair.cy, pair.shear, pair.pad);
+            }
+            if constexpr (FAST) {
+                // The fragment evaluation measures from the projected centre, the outline test from the centre of
+                // the outline: the record carries the (small) difference, so that outline centre + difference
+                // gives the projected centre to better than float32 resolution at the pixel's magnitude.
+                cr.r = float(centre[0] - double(cr.cx));
+                cr.g = float(centre[1] - double(cr.cy));
+            } else {
+                cr.r = rgb.x; cr.g = rgb.y; cr.b = rgb.z;
+            }
+            float4* cdst = reinterpret_cast<float4*>(out.cull + gi);
+            cdst[0] = make_float4(cr.cx, cr.cy, cr.a, cr.b2);
+            cdst[1] = make_float4(cr.c, cr.r, cr.g, cr.b);
+        }
+        __syncwarp();
     }
 }
 
@@ -404,9 +464,10 @@ cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGe
         uint32_t(geo.grid_h), view.near_plane, view.far_plane, view.scale_modifier);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    const uint32_t finish_blocks = min((n + kFinishBlock - 1) / kFinishBlock, uint32_t(sm_count_of_current_device()) * 8u);
-    launch_after(preprocess_finish_kernel<MODE, TRAIN, FAST>, finish_blocks, kFinishBlock, 0, stream,
-        scene.positions, scene.opacities, scene.sh_0, scene.sh_rest, view.cam_position, prim, status, view.active_sh_bases, scene.total_sh_bases, outline_thresholds(outline_mode));
+    const FinishLayout layout = finish_layout(view.active_sh_bases, scene.sh_0 != nullptr);
+    const uint32_t finish_blocks = min((n + kFinishBlock - 1) / kFinishBlock, uint32_t(sm_count_of_current_device()) * uint32_t(finish_blocks_per_sm(TRAIN, FAST)));
+    launch_after(preprocess_finish_kernel<MODE, TRAIN, FAST>, finish_blocks, kFinishBlock, size_t(kFinishBlock) * (layout.window_stride + sizeof(EvalRecord)), stream,
+        scene.sh_0, scene.sh_rest, view.cam_position, prim, status, n, view.active_sh_bases, scene.total_sh_bases, outline_thresholds(outline_mode), layout);
     return cudaGetLastError();
 }
 
