@@ -175,24 +175,30 @@ __device__ __forceinline__ float sqrt_approx(float x) { float y; asm("sqrt.appro
 
 // Pixels of the 8 x 4 block at (x0, y0) that the outline a dx^2 + b2 dx dy + c dy^2 <= 1 about (cx, cy) can touch: bit
 // (row * 8 + column).  A row is cut in an interval; 0.01 pixel is added at both ends, far more than the roundings here and
-// far less than the 0.3 pixel by which the outline was inflated.
+// far less than the 0.3 pixel by which the outline was inflated.  Lengths along the row are in units of the block's width, so that the clamp to
+// the block is the additions' saturation; a row that the outline does not reach has the root of a negative number, which the
+// saturation turns into 0 at both ends.  The ends are rounded to whole pixels by adding 1.5 * 2^23, whose low bits then are the
+// shift counts.  About 70 instructions, five of them on the pipe for roots and conversions (rounding by conversions: 100 and 13).  3 M Gaussians, 1297 x
+// 840: max_weights 449 -> 438 us, backward tiles 995 -> 980, blend 866 -> 856; 1.5 M in GLOBAL_ORDERING: blend 268 -> 257.
 __device__ __forceinline__ uint32_t outline_mask(const float4& c0, float cc, float x0, float y0) {
-    if (c0.z == 0.0f) return c0.x > 1e30f ? 0u : 0xffffffffu;   // nothing can be accepted / no proper ellipse: every pixel is a candidate
-    const float a_rcp = __fdividef(1.0f, c0.z);
-    const float slope = -0.5f * c0.w * a_rcp;                   // centre of the interval per unit of dy
-    const float shrink = slope * slope - cc * a_rcp;            // half width^2 = 1/a + shrink * dy^2
-    const float left = c0.x - x0, dy0 = y0 - c0.y;
+    float a_rcp;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a_rcp) : "f"(c0.z));
+    const float slope = (-0.0625f * c0.w) * a_rcp;                             // centre of the interval per unit of dy
+    const float width = 0.015625f * a_rcp;
+    const float shrink = fmaf(slope, slope, -cc * width);                      // half width^2 = 1/a + shrink * dy^2
+    const float middle = fmaf(c0.x - x0, 0.125f, 0.0625f), dy0 = y0 - c0.y;    // half a pixel further, for the rounding
     uint32_t mask = 0;
     #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 3; r >= 0; --r) {
         const float dy = dy0 + float(r);
-        const float half_sq = fmaf(shrink * dy, dy, a_rcp);
-        const float mid = fmaf(slope, dy, left);
-        const float half = half_sq >= 0.0f ? sqrt_approx(half_sq) + 0.01f : -16.0f;
-        const int lo = max(__float2int_ru(mid - half), 0), hi = min(__float2int_rd(mid + half), 7);
-        const uint32_t row = ((2u << (hi & 31)) - 1u) & ~((1u << (lo & 31)) - 1u);       // bits lo..hi
-        if (lo <= hi) mask |= row << (r * 8);
+        const float half = sqrt_approx(fmaf(shrink * dy, dy, width)) + 0.00125f;
+        const float mid = fmaf(slope, dy, middle);
+        const float begin = fmaf(__saturatef(mid - half), 8.0f, 12582912.0f), end = fmaf(__saturatef(mid + half), 8.0f, 12582912.0f);
+        // bits begin .. end - 1 (the shifts take their count modulo 32)
+        const uint32_t row = __funnelshift_l(0u, 1u, __float_as_uint(end)) - __funnelshift_l(0u, 1u, __float_as_uint(begin));
+        mask = mask * 256u + row;
     }
+    if (c0.z == 0.0f) mask = c0.x > 1e30f ? 0u : 0xffffffffu;   // nothing can be accepted / no proper ellipse: every pixel is a candidate
     return mask;
 }
 
