@@ -20,20 +20,20 @@
 //     brings one, an mbarrier per half tracks them, and the next instances are filtered while they fly.  The masks of a
 //     half are transposed (16 x 32 bits, shuffles), so that lane = pixel holds the bits of its own candidates: the
 //     older half in the upper 16 bits of a word, the newer one below.
-//  3. Exact pass.  Every lane walks the bits of its own word from the top; almost every step of every lane is an accepted
-//     fragment.  A half is replaced when no lane has a bit of it left; lanes that are ahead work on the newer half
+//  3. Exact pass.  Every lane walks the bits of its own word from the top, two or three candidates per trip; almost every one is
+//     an accepted fragment.  A half is replaced when no lane has a bit of it left; lanes that are ahead work on the newer half
 //     meanwhile, so lanes wait for the pixel with the most fragments only over a tile, not over every batch of 64 (lanes busy
 //     per step: 0.92 instead of 0.83 at 1297 x 840, 3 M Gaussians).
 //  4. K-buffer (core_buffer.cuh).  The K nearest core fragments lie unsorted in shared memory, 12 bytes each; an insertion
-//     overwrites the one that falls out and costs the same for every K.  The colour of the entry that will fall out next is
-//     fetched from its record right after the insertion before, so that it has arrived when it is needed.
+//     overwrites the one that falls out and costs the same for every K, or takes the next empty place, which costs a quarter of that.
+//     The colour of the entry that will fall out next is fetched from its record right after the insertion before, so that it has
+//     arrived when it is needed.
 //
 // Blocks start in the order of `tile_order`, long lists first: the last blocks of a launch are short ones.
 //
-// What bounds it: instruction issue (1.0e9 warp instructions at 3 M Gaussians, 1297 x 840, K = 16, 7.3 M instances; 65 % of the
-// issue slots), at the 22 warps per SM that the K-buffers leave (K = 32: 14).  Measured against the form with one CTA of 64 pixels,
-// candidate masks by ballots and the chain in registers: K = 16 at that size 1660 -> 1185 us, K = 32 at 4K with 8 M Gaussians
-// 46.6 -> 34.9 ms, training forward 1813 -> 1370 us, GLOBAL_ORDERING (1.5 M, 980 x 545) 351 -> 262 us.
+// What bounds it: instruction issue (74 % of the issue slots at 1.5 M Gaussians, 1297 x 840, K = 16; a fifth of the instructions are
+// insertions, a quarter filter, window and compositing), at the 22 warps per SM that the K-buffers leave (K = 32: 14).  3 M
+// Gaussians, 1297 x 840, K = 16: 788 us; 8 M, 4K, K = 32: 27.8 ms.
 #include <algorithm>
 #include <type_traits>
 
@@ -57,7 +57,11 @@ enum class Buffer { chain, keys, keys_and_colours, dividing };
 template <int K, Buffer BUFFER> struct CoreOf { using type = SortedCore<K, 32>; };
 template <int K> struct CoreOf<K, Buffer::keys> { using type = UnsortedCore<K, 32, false>; };
 template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = UnsortedCore<K, 32, true>; };
-struct NoCore { static constexpr bool keeps_colour = false; static constexpr size_t smem_bytes = 0; };
+// HYBRID_BLEND with the unsorted buffer: candidates that a lane evaluates per trip, of which one may enter the buffer.  With K = 32 the 14 warps
+// that shared memory leaves have registers for a third one, which hides more latency than its repeated evaluations cost; with K = 16 the
+// registers do not suffice (1297 x 840, 3 M Gaussians: two 803 us, three 857; 4K, K = 32: two 29.9 ms, three 28.7, four 31.5).
+constexpr int candidates_per_trip(int K) { return K >= 32 ? 3 : 2; }
+struct NoCore { static constexpr bool keeps_colour = false, unsorted = false; static constexpr size_t smem_bytes = 0; };
 
 template <int MODE, int K, Buffer BUFFER, BlendTask TASK> struct SmemLayout {
     static constexpr bool has_kbuffer = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
@@ -107,6 +111,8 @@ __device__ __forceinline__ bool blend_block(
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
+    constexpr bool kMerged = kHybrid && SL::Core::unsorted;
+    constexpr int kPerTrip = candidates_per_trip(K);
     constexpr uint32_t kTileX = MT::tile_w / kBlockW, kTileY = MT::tile_h / kBlockH;     // blocks per binning tile
     EvalRecord* s_record = reinterpret_cast<EvalRecord*>(smem + SL::record_off);
     uint32_t* s_queue_prim = reinterpret_cast<uint32_t*>(smem + SL::queue_prim_off);
@@ -215,69 +221,115 @@ __device__ __forceinline__ bool blend_block(
             window &= ~(1u << j);
             return j ^ flip;
         };
+        [[maybe_unused]] auto evaluate = [&](bool valid, uint32_t j, float& depth, float& alpha) -> bool {       // HYBRID
+            const float4* rec = reinterpret_cast<const float4*>(s_record + j);
+            const FragmentFront fr = fragment_front(rec[0], rec[1], rec[2], pixel_x, pixel_y);
+            const float numerator_rho2 = fr.numerator_rho2;
+            const float denominator = fr.denominator;
+            const bool inside_cutoff = !(numerator_rho2 > MT::max_cutoff_sq * denominator);
+            const float denominator_rcp = kDivide ? 1.0f / denominator : reciprocal_rn(denominator);
+            const float G = expf(-0.5f * numerator_rho2 * denominator_rcp);
+            alpha = fminf(rec[4].w * G, kMaxFragmentAlpha);
+            const float3 eval_point_diag = cross(fr.d, fr.m) * denominator_rcp;
+            const float4 MT3 = rec[3];
+            depth = dot(f3(MT3), eval_point_diag) + MT3.w;
+            return valid && inside_cutoff && !(alpha < MT::min_alpha);
+        };
+        [[maybe_unused]] auto add_to_tail = [&](float depth, const float4& frag) {
+            if constexpr (STATS) ++stat_accepted;
+            if constexpr (TRAIN) {
+                acc += make_float4(frag.x * frag.w, frag.y * frag.w, frag.z * frag.w, frag.w);
+            } else {       // premultiplied colours are rounded before they are summed (inference.cuh:158)
+                acc += make_float4(__fmul_rn(frag.x, frag.w), __fmul_rn(frag.y, frag.w), __fmul_rn(frag.z, frag.w), frag.w);
+                if (!use_median_depth) acc_depth += depth * frag.w;
+            }
+            transmittance *= 1.0f - frag.w;
+        };
         while (__any_sync(0xffffffffu, window >= 0x10000u)) {
-            if constexpr (kHybrid) {
-                // Two candidates per trip: their evaluations are independent instruction streams (the compiler
-                // interleaves them), which hides the latency of the divide / expf / dot chains; the buffer
-                // and tail updates then happen strictly in list order.
-                auto evaluate = [&](bool valid, uint32_t j, float& depth, float4& frag) -> bool {
-                    const float4* rec = reinterpret_cast<const float4*>(s_record + j);
-                    const FragmentFront fr = fragment_front(rec[0], rec[1], rec[2], pixel_x, pixel_y);
-                    const float numerator_rho2 = fr.numerator_rho2;
-                    const float denominator = fr.denominator;
-                    const bool inside_cutoff = !(numerator_rho2 > MT::max_cutoff_sq * denominator);
-                    const float denominator_rcp = kDivide ? 1.0f / denominator : reciprocal_rn(denominator);
-                    const float4 rgba_in = rec[4];
-                    const float G = expf(-0.5f * numerator_rho2 * denominator_rcp);
-                    const float alpha = fminf(rgba_in.w * G, kMaxFragmentAlpha);
-                    const float3 eval_point_diag = cross(fr.d, fr.m) * denominator_rcp;
-                    const float4 MT3 = rec[3];
-                    depth = dot(f3(MT3), eval_point_diag) + MT3.w;
-                    frag = make_float4(rgba_in.x, rgba_in.y, rgba_in.z, alpha);
-                    return valid && inside_cutoff && !(alpha < MT::min_alpha);
-                };
-                auto commit = [&](float depth, float4 frag, uint32_t j) {
-                    if constexpr (STATS) ++stat_accepted;
-                    if (depth < core.limit() && frag.w >= MT::min_alpha_core) {
+            if constexpr (kMerged) {
+                // A lane takes kPerTrip candidates; their evaluations are independent instruction streams.  One of them may enter the buffer: the
+                // warp runs an insertion (a third of a trip's instructions) whenever one lane has one to do, and with one insertion per
+                // candidate (9 lanes of 32 at a time) that was four times for every five candidates.  A second one of a lane, and what comes
+                // behind it, goes back into the window.  The tail's sums stay in list order: what falls out takes the place of what entered.
+                // 3 M Gaussians, 1297 x 840, K = 16: 866 -> 787 us, training forward 1026 -> 894; 4K, K = 32: 33.7 -> 27.8 ms.  (FIRST_K, where
+                // every candidate enters until the buffer is full, gets slower: 262 -> 292 us.)
+                const uint32_t before = window;
+                uint32_t j[kPerTrip], bit[kPerTrip];
+                float depth[kPerTrip], alpha[kPerTrip];
+                bool counts[kPerTrip];
+                #pragma unroll
+                for (int i = 0; i < kPerTrip; ++i) {
+                    bool valid;
+                    j[i] = pop_candidate(valid);
+                    bit[i] = j[i] ^ flip;
+                    counts[i] = evaluate(valid, j[i], depth[i], alpha[i]);
+                }
+                const float limit = core.limit();
+                bool enters = false, stopped = false, is_entering[kPerTrip];
+                float in_depth = 0.0f, in_alpha = 0.0f;
+                uint32_t in_j = 0, stop_bit = 0;
+                #pragma unroll
+                for (int i = 0; i < kPerTrip; ++i) {
+                    const bool nearer = counts[i] && depth[i] < limit && alpha[i] >= MT::min_alpha_core;
+                    is_entering[i] = nearer && !enters;
+                    if (is_entering[i]) { in_depth = depth[i]; in_alpha = alpha[i]; in_j = j[i]; }
+                    if (nearer && enters && !stopped) { stopped = true; stop_bit = bit[i]; }
+                    enters |= nearer;
+                    counts[i] = counts[i] && !stopped;
+                }
+                if (stopped) window = before & ((2u << stop_bit) - 1u);
+                if constexpr (STATS) { stat_trips += kPerTrip; stat_trips_inserting += __any_sync(0xffffffffu, enters) ? 1 : 0; stat_insertions += enters ? 1 : 0; }
+                float4 evicted = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (enters) {
+                    const uint2 payload = make_uint2(__float_as_uint(in_alpha), s_word[in_j]);   // training: what the backward pass looks up
+                    // what falls out is a fragment, or nothing (alpha 0; its colour does not matter)
+                    if constexpr (SL::Core::keeps_colour) {
+                        float3 rgb = f3(reinterpret_cast<const float4*>(s_record + in_j)[4]);
+                        core.insert(in_depth, payload, last, rgb);
+                        evicted = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(last.x));
+                    } else {
+                        if (!core.insert(in_depth, payload, last, last_rgb)) last_rgb = colour_of(last.y);
+                        evicted = make_float4(last_rgb.x, last_rgb.y, last_rgb.z, __uint_as_float(last.x));
+                        if (core.last(last)) last_rgb = colour_of(last.y);
+                    }
+                }
+                #pragma unroll
+                for (int i = 0; i < kPerTrip; ++i) {
+                    if (counts[i]) {
+                        const float4 rgba = reinterpret_cast<const float4*>(s_record + j[i])[4];
+                        add_to_tail(is_entering[i] ? limit : depth[i], is_entering[i] ? evicted : make_float4(rgba.x, rgba.y, rgba.z, alpha[i]));
+                    }
+                }
+            } else if constexpr (kHybrid) {
+                // Two candidates per trip, as above; the buffer and tail updates happen strictly in list order.
+                auto commit = [&](float depth, float alpha, uint32_t j) {
+                    const float4 rgba = reinterpret_cast<const float4*>(s_record + j)[4];
+                    float4 frag = make_float4(rgba.x, rgba.y, rgba.z, alpha);
+                    if (depth < core.limit() && alpha >= MT::min_alpha_core) {
                         const float limit = core.limit();
-                        const uint2 payload = make_uint2(__float_as_uint(frag.w), s_word[j]);   // training: what the backward pass looks up
-                        // what falls out is a fragment, or nothing (alpha 0; its colour does not matter)
-                        if constexpr (SL::Core::keeps_colour) {
-                            float3 rgb = f3(frag);
-                            core.replace(depth, payload, last, rgb);
-                            frag = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(last.x));
-                        } else {
-                            if (!core.replace(depth, payload, last, last_rgb)) last_rgb = colour_of(last.y);
-                            frag = make_float4(last_rgb.x, last_rgb.y, last_rgb.z, __uint_as_float(last.x));
-                            if (core.last(last)) last_rgb = colour_of(last.y);
-                        }
+                        if (!core.replace(depth, make_uint2(__float_as_uint(alpha), s_word[j]), last, last_rgb)) last_rgb = colour_of(last.y);
+                        frag = make_float4(last_rgb.x, last_rgb.y, last_rgb.z, __uint_as_float(last.x));
+                        if (core.last(last)) last_rgb = colour_of(last.y);
                         depth = limit;
                     }
-                    if constexpr (TRAIN) {
-                        acc += make_float4(frag.x * frag.w, frag.y * frag.w, frag.z * frag.w, frag.w);
-                    } else {       // premultiplied colours are rounded before they are summed (inference.cuh:158)
-                        acc += make_float4(__fmul_rn(frag.x, frag.w), __fmul_rn(frag.y, frag.w), __fmul_rn(frag.z, frag.w), frag.w);
-                        if (!use_median_depth) acc_depth += depth * frag.w;
-                    }
-                    transmittance *= 1.0f - frag.w;
+                    add_to_tail(depth, frag);
                 };
                 bool v0, v1;
                 const uint32_t j0 = pop_candidate(v0);
                 const uint32_t j1 = pop_candidate(v1);
-                float depth0, depth1;
-                float4 frag0, frag1;
-                const bool ok0 = evaluate(v0, j0, depth0, frag0);
-                const bool ok1 = evaluate(v1, j1, depth1, frag1);
+                float depth0, depth1, alpha0, alpha1;
+                const bool ok0 = evaluate(v0, j0, depth0, alpha0);
+                const bool ok1 = evaluate(v1, j1, depth1, alpha1);
                 if constexpr (STATS) {   // how often a lane of the warp inserts
-                    const bool in0 = ok0 && depth0 < core.limit() && frag0.w >= MT::min_alpha_core;
+                    const bool in0 = ok0 && depth0 < core.limit() && alpha0 >= MT::min_alpha_core;
                     stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in0) ? 1 : 0; stat_insertions += in0 ? 1 : 0;
                 }
-                if (ok0) commit(depth0, frag0, j0);
+                if (ok0) commit(depth0, alpha0, j0);
                 if constexpr (STATS) {
-                    const bool in1 = ok1 && depth1 < core.limit() && frag1.w >= MT::min_alpha_core;
+                    const bool in1 = ok1 && depth1 < core.limit() && alpha1 >= MT::min_alpha_core;
                     stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in1) ? 1 : 0; stat_insertions += in1 ? 1 : 0;
                 }
-                if (ok1) commit(depth1, frag1, j1);
+                if (ok1) commit(depth1, alpha1, j1);
             } else {
                 // The other three modes use the same two-candidates-per-trip shape: both evaluations (divide, expf, depth) are
                 // independent instruction streams; the state updates happen in list order.  A fragment counts iff it passes
@@ -308,8 +360,12 @@ __device__ __forceinline__ bool blend_block(
                     if constexpr (kFirstK) {
                         if (depth >= core.limit()) return;
                         if constexpr (STATS) ++stat_accepted;
+                        const uint2 payload = make_uint2(__float_as_uint(alpha), s_word[j]);
+                        if constexpr (SL::Core::unsorted) {
+                            if (core.filling()) { core.append(depth, payload, last_rgb); return; }
+                        }
                         core.last(last);
-                        core.replace(depth, make_uint2(__float_as_uint(alpha), s_word[j]), last, last_rgb);   // what falls out is dropped
+                        core.replace(depth, payload, last, last_rgb);   // what falls out is dropped
                     } else if constexpr (kGlobal) {
                         if (done) return;
                         if constexpr (STATS) ++stat_accepted;

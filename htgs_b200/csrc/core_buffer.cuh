@@ -47,7 +47,7 @@ template <int K, int THREADS, bool COLOUR>
 struct UnsortedCore {
     static_assert(K >= 4, "rows of four keys");
     static constexpr int kPosBits = core_pos_bits(K), kRows = K / 4;
-    static constexpr bool keeps_colour = COLOUR;
+    static constexpr bool keeps_colour = COLOUR, unsorted = true;
     static constexpr size_t smem_bytes = size_t(K) * THREADS * (COLOUR ? 24 : 12);
     static constexpr uint32_t kEmpty = 0xffffffffu & ~uint32_t(K - 1);
     static constexpr int32_t kRelLimit = int32_t((1u << (32 - kPosBits)) - 2u);   // one below an empty entry
@@ -89,8 +89,39 @@ struct UnsortedCore {
 
     // The entry that falls out next; false if it is an empty one.
     __device__ __forceinline__ bool last(uint2& payload) const {
+        if (filling()) return false;
         payload = pay[(kmax & uint32_t(K - 1)) * THREADS];
         return payload.y != kNoEntry;
+    }
+
+    // While there are empty entries nothing falls out, and the rows' maxima do not matter: a new entry takes the last empty place.
+    __device__ __forceinline__ bool filling() const { return kmax >= kEmpty; }
+    __device__ __forceinline__ void append(float depth, uint2 payload, float3& colour) {
+        const uint32_t c = kmax & uint32_t(K - 1);
+        pay[c * THREADS] = payload;
+        if constexpr (COLOUR) swap_colour(c, colour);
+        const int32_t rel = min(max(__float_as_int(depth) - base, 0), kRelLimit);
+        keys[(c >> 2) * (THREADS * 4) + (c & 3u)] = uint32_t(rel) * uint32_t(K) + c;
+        --kmax;
+        if (c == 0) {
+            #pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const uint4 row = *reinterpret_cast<const uint4*>(keys + i * (THREADS * 4));
+                row_max[i] = max(__vimax3_u32(row.x, row.y, row.z), row.w);
+            }
+            kmax = row_max[0];
+            #pragma unroll
+            for (int i = 1; i < kRows; ++i) kmax = max(kmax, row_max[i]);
+            depth_limit = decode(kmax);
+        }
+    }
+
+    // One or the other.  `evicted` and `colour` of an empty entry are zero, as the caller set them in the beginning.
+    __device__ __forceinline__ bool insert(float depth, uint2 payload, uint2& evicted, float3& colour) {
+        if (!filling()) return replace(depth, payload, evicted, colour);
+        append(depth, payload, colour);
+        if constexpr (COLOUR) { colour = make_float3(0.0f, 0.0f, 0.0f); evicted = make_uint2(0u, kNoEntry); }
+        return true;
     }
 
     // Puts (depth, payload) in place of the last entry.  `evicted` holds the last entry's payload (from last()); if a tie in depth makes
@@ -276,7 +307,7 @@ private:
 // numbers travel as floats (0..K are exact): one add and two multiply-adds per level on the FMA pipes.
 template <int K, int THREADS>
 struct SortedCore {
-    static constexpr bool keeps_colour = false;
+    static constexpr bool keeps_colour = false, unsorted = false;
     static constexpr size_t smem_bytes = size_t(K + 1) * THREADS * 8;
     uint2* pay;              // [K + 1][THREADS]
     float kd[K];

@@ -95,3 +95,31 @@ def test_training_forward_with_three_entries_of_one_depth(mode, K):
         with torch.no_grad():
             images.append(tb.diff_rasterize(*harness.scene_tensors(scene), torch.empty(0, device="cuda"), harness.settings_for(tb, scene, wide, mode, K), False))
     assert torch.equal(*images)
+
+
+@pytest.mark.parametrize("mode,K", [(0, 4), (0, 8), (0, 16), (0, 32), (1, 4), (1, 16), (1, 32)])
+@pytest.mark.parametrize("order", ["front first", "back first", "mixed", "one depth"])
+def test_buffer_filled_to_the_last_entry(mode, K, order):
+    # every pixel sees the same Gaussians, one short of a full buffer to one more, and all of them enter: the step from an empty place
+    # to an entry that falls out; 64 x 64 pixels run the form that keeps colours, 512 x 512 the other one
+    for size in (64, 512):
+        for n in (K - 1, K, K + 1, 2 * K + 1):
+            scene = scenes.tiny_scene(n=n, size=size, seed=n, mode=mode, K=K, sh_degree=1)
+            depth = np.linspace(2.0, 4.0, n)
+            if order == "back first":
+                depth = depth[::-1]
+            elif order == "mixed":
+                depth = np.random.default_rng(n).permutation(depth)
+            elif order == "one depth":
+                depth[:] = 3.0
+            scene.positions[:] = 0.0
+            scene.positions[:, 2] = depth
+            scene.scales[:] = 1.0 if order == "one depth" else 0.2 * depth[:, None]
+            scene.scales[:, 2] = 1e-3
+            scene.rotations[:] = np.array([1.0, 0.0, 0.0, 0.0], dtype=np.float32)
+            scene.opacities[:] = np.random.default_rng(K).uniform(0.2, 0.5, scene.opacities.shape)
+            for median in (False, True):
+                got = render(scene, scene.views[0], mode, K, 0.2, 100.0, median)
+                want = render(scene, scene.views[0], mode, K, 0.2, 3e38, median)
+                assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+                assert got[0].max() > 0.0
