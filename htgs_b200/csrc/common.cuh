@@ -109,8 +109,8 @@ static_assert(sizeof(FastRecord) == sizeof(EvalRecord), "FastRecord shares the s
 // quadratic in (s, y): y = pixel_y - cy, s = pixel_x - cx + shear * y.  Computed in float64: a rounding of a coefficient is the
 // same at every pixel and does not average out in a gradient that sums thousands of them.
 struct __align__(16) PairRecord {
-    float4 n0, n1, d1;        // n0 = N: 1, s, y, ss   n1 = N: sy, yy, D: 1, s   d1 = D: y, ss, sy, yy
-    float cx, cy, shear, pad;
+    float4 q0, q1, q2;        // coefficients of N and D side by side: q0 = those of 1 and s, q1 = y and ss, q2 = sy and yy
+    float cx, cy, shear, scale;     // scale: what N and D were multiplied by (1 / D at the centre)
 };
 static_assert(sizeof(PairRecord) == 64, "PairRecord must be 64 bytes");
 
@@ -168,6 +168,16 @@ __device__ __forceinline__ float reciprocal_rn(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
 }
+
+// Two floats in one register pair: one instruction for two rounded operations (two of them take the FMA pipe as long as four single ones would, but half
+// the issue slots).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 unpack2(f32x2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
 
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 

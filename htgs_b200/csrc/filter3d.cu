@@ -11,6 +11,8 @@
 #include "kernels.h"
 
 
+using namespace htgs;
+
 namespace {
 
 __global__ void __launch_bounds__(256) update_3d_filter_kernel(const float* __restrict__ positions, const float* __restrict__ w2c, float* __restrict__ filter_3d,
@@ -53,13 +55,6 @@ template <int VIEWS> struct FilterViewBatch { FilterView view[VIEWS]; float larg
 // Sizes of the kernel's parameter block: 3.6 KB, 5.4 KB and 29 KB.  A launch costs more the larger it is, most of all beyond 4 KB; 40 views take 36 us
 // with room for 48 and 47 us with room for 256 (16 k points; 300 k: 37 and 51, 3 M: 123 and 126).
 constexpr int kFewestViews = 32, kFewViews = 48, kManyViews = 256;
-
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ float2 unpack2(f32x2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 __device__ __forceinline__ float view_depth(const FilterView& v, const float3& p) { return htgs::dot(make_float3(v.r3[0], v.r3[1], v.r3[2]), p) + v.r3[3]; }
 __device__ __forceinline__ bool in_view(const FilterView& v, const float3& p, float z) {      // as update_3d_filter_kernel tests it

@@ -46,7 +46,7 @@ __device__ __forceinline__ float exp_approx(float x) { float y; asm("ex2.approx.
 //     u = dL/drho^2 / D  (times D at the centre, which the record divides by)  and  v = u N / D,  each times  1, s, y, ss, sy, yy
 // to the Gaussian's record, and rows_from_moments applies the coefficients once per Gaussian.  Of the sum of v, which the rows of a scale
 // all but cancel against the second moments of u, only v - u N is added up, which vanishes with the perspective: u N follows from the
-// moments of u (a third to a half of the rounding of grad_scales).  That is 19 instructions per pair
+// moments of u (a third to a half of the rounding of grad_scales).  That is 13 instructions per pair
 // instead of 54 for the rows themselves, and offsets from the centre keep the sums well conditioned, where the rows' sums hold products with
 // pixel coordinates that cancel later.
 struct AffinePlanes { float3 M0, Ms, My, D0, Ds, Dy; float4 A, B; float shear; };     // A = VPMT1 - cx VPMT4, B = VPMT2 - cy VPMT4
@@ -75,11 +75,15 @@ __device__ __forceinline__ AffinePlanes affine_planes(const float4& T1, const fl
     return p;
 }
 
-struct PairForm { float4 n0, n1, d1; };      // of a PairRecord: N and D, both divided by D at the centre
+// N and D of a PairRecord at (s, y), side by side in one register pair.
+struct PairForm { float4 q0, q1, q2; };
+__device__ __forceinline__ f32x2 low2(const float4& v) { return pack2(v.x, v.y); }
+__device__ __forceinline__ f32x2 high2(const float4& v) { return pack2(v.z, v.w); }
 __device__ __forceinline__ void evaluate_pair(const PairForm& f, float s, float y, float& numerator, float& denominator) {
-    const float ss = s * s, sy = s * y, yy = y * y;
-    numerator = fmaf(f.n1.y, yy, fmaf(f.n1.x, sy, fmaf(f.n0.w, ss, fmaf(f.n0.z, y, fmaf(f.n0.y, s, f.n0.x)))));
-    denominator = fmaf(f.d1.w, yy, fmaf(f.d1.z, sy, fmaf(f.d1.y, ss, fmaf(f.d1.x, y, fmaf(f.n1.w, s, f.n1.z)))));
+    const f32x2 s2 = pack2(s, s), y2 = pack2(y, y);
+    const float2 v = unpack2(fma2(high2(f.q2), mul2(y2, y2), fma2(low2(f.q2), mul2(s2, y2), fma2(high2(f.q1), mul2(s2, s2), fma2(low2(f.q1), y2, fma2(high2(f.q0), s2, low2(f.q0)))))));
+    numerator = v.x;
+    denominator = v.y;
 }
 
 // Whether the forward pass accepts a fragment is settled by rho^2 unless it lies within kLevelBand of the level where alpha meets
@@ -103,12 +107,25 @@ __device__ __noinline__ bool accepted_by_forward(const EvalRecord* rec, float pi
     return !(numerator_rho2 > MT::max_cutoff_sq * denominator) && !(fminf(opacity * G, kMaxFragmentAlpha) < MT::min_alpha);
 }
 
-struct PairMoments { float4 u0, u1, v1; };      // u: 1, s, y, ss | u: sy, yy, v: 1 (less u N), s | v: y, ss, sy, yy
+// Sums over pairs, as pairs of registers: a pair of pixel offsets (s, y) serves both factors of a product.  13 instructions (single ones: 19).
+struct PairMoments {
+    f32x2 uv;                       // u, v - u N
+    f32x2 u1, u2, v1, v2;           // us, uy | uss, uyy | vs, vy | vss, vyy
+    float usy, vsy;
+    __device__ __forceinline__ float4 row(int i) const {      // as they lie in the Gaussian's record
+        const float2 a = unpack2(i == 0 ? uv : i == 1 ? u2 : v2), b = i == 2 ? make_float2(usy, vsy) : unpack2(i == 0 ? u1 : v1);
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+};
 __device__ __forceinline__ void add_moments(PairMoments& a, float u, float v, float uN, float s, float y) {
-    const float us = u * s, uy = u * y, vs = v * s, vy = v * y;
-    a.u0.x += u; a.u0.y += us; a.u0.z += uy; a.u0.w = fmaf(us, s, a.u0.w);
-    a.u1.x = fmaf(us, y, a.u1.x); a.u1.y = fmaf(uy, y, a.u1.y); a.u1.z += v - uN; a.u1.w += vs;
-    a.v1.x += vy; a.v1.y = fmaf(vs, s, a.v1.y); a.v1.z = fmaf(vs, y, a.v1.z); a.v1.w = fmaf(vy, y, a.v1.w);
+    const f32x2 sy = pack2(s, y), us_uy = mul2(pack2(u, u), sy), vs_vy = mul2(pack2(v, v), sy);
+    a.uv = add2(a.uv, pack2(u, v - uN));
+    a.u1 = add2(a.u1, us_uy);
+    a.u2 = fma2(us_uy, sy, a.u2);
+    a.v1 = add2(a.v1, vs_vy);
+    a.v2 = fma2(vs_vy, sy, a.v2);
+    a.usy = fmaf(unpack2(us_uy).x, y, a.usy);
+    a.vsy = fmaf(unpack2(vs_vy).x, y, a.vsy);
 }
 
 // dL/dVPMT1 = sum dX, dL/dVPMT2 = sum dY, and E = sum (x dX + y dY), so that dL/dVPMT4 = -(cx sum dX + cy sum dY + E).  With
@@ -116,11 +133,11 @@ __device__ __forceinline__ void add_moments(PairMoments& a, float u, float v, fl
 //     dX = (Y x dd - Y.w dm, Y . dm),   dY = (X.w dm - X x dd, -X . dm)
 // and the cubic terms of E cancel: x dX + y dY = ((x B - y A) x dd - (x B.w - y A.w) dm, (x B - y A) . dm).
 struct RowGradients { float4 dX, dY, E; };
-__device__ __forceinline__ RowGradients rows_from_moments(const AffinePlanes& p, const float4& T4, const float4& n0, const float4& n1, const PairMoments& a) {
+__device__ __forceinline__ RowGradients rows_from_moments(const AffinePlanes& p, const float4& T4, const PairForm& f, const float4& r0, const float4& r1, const float4& r2) {
     const float3 A = f3(p.A), B = f3(p.B), n = f3(T4);
-    const float u = a.u0.x, us = a.u0.y, uy = a.u0.z, uss = a.u0.w, usy = a.u1.x, uyy = a.u1.y;
-    // the sum of v from that of v - u N; n0, n1: N as the pairs saw it
-    const float v = a.u1.z + fmaf(n1.y, uyy, fmaf(n1.x, usy, fmaf(n0.w, uss, fmaf(n0.z, uy, fmaf(n0.y, us, n0.x * u))))), vs = a.u1.w, vy = a.v1.x, vss = a.v1.y, vsy = a.v1.z, vyy = a.v1.w;
+    const float u = r0.x, us = r0.z, uy = r0.w, uss = r1.x, uyy = r1.y, usy = r2.z;      // PairMoments::row
+    // the sum of v from that of v - u N; N as the pairs saw it
+    const float v = r0.y + fmaf(f.q2.z, uyy, fmaf(f.q2.x, usy, fmaf(f.q1.z, uss, fmaf(f.q1.x, uy, fmaf(f.q0.z, us, f.q0.x * u))))), vs = r1.z, vy = r1.w, vss = r2.x, vsy = r2.w, vyy = r2.y;
     // sums of u m and v d, and of these times y and x = s - shear * y
     const float3 m1 = u * p.M0 + us * p.Ms + uy * p.My, my = uy * p.M0 + usy * p.Ms + uyy * p.My;
     const float3 d1 = v * p.D0 + vs * p.Ds + vy * p.Dy, dy = vy * p.D0 + vsy * p.Ds + vyy * p.Dy;
@@ -162,12 +179,15 @@ __device__ __forceinline__ float abs_position_gradient(const AbsForm& f, float u
     return fabsf(dot(cam.c1, c4)) + fabsf(dot(cam.c2, c4)) + fabsf(dot(cam.c3, c4));
 }
 
+__device__ __forceinline__ float small_int_to_float(uint32_t i) { return __uint_as_float(0x4b000000u | i) - 8388608.0f; }      // i < 2^23; off the pipe of the conversions
+
 constexpr int kBwdThreads = 128;       // threads per tile: one staged instance each
 constexpr int kBwdSegments = 4 * kBwdThreads;      // of a batch, at most
 constexpr int kBwdCoreRow = 68;        // bytes per staged instance: 64 pixels, and an odd number of words against bank conflicts
 template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr bool has_core = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K);
     static constexpr bool has_tail = (MODE == HTGS_MODE_HYBRID_BLEND || MODE == HTGS_MODE_OIT_BLEND);
+    static constexpr int core_rows = has_core ? K : 0;
     static constexpr size_t cg_off = 0;
     static constexpr size_t cg_bytes = has_core ? size_t(K) * 64 * 16 : 0;
     static constexpr size_t tc_off = cg_off + cg_bytes;
@@ -179,7 +199,7 @@ template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr size_t core_off = (stage_off + stage_bytes + 15) & ~size_t(15);     // [NT][kBwdCoreRow] core entry of each (staged instance, pixel) pair
     static constexpr size_t core_bytes = has_core ? size_t(kBwdThreads) * kBwdCoreRow : 0;
     static constexpr size_t total = core_off + core_bytes;
-    static constexpr int max_blocks = has_core || ABS_GRAD ? 4 : 5;      // five spill the pair loop of the modes with a buffer (1415 against 1366 us)
+    static constexpr int max_blocks = 4;      // five spill the pair loop
     static constexpr int min_blocks = int((227 * 1024) / (total + 1024)) < max_blocks ? int((227 * 1024) / (total + 1024)) : max_blocks;   // what the register budget is held to
 };
 
@@ -195,8 +215,9 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     extern __shared__ __align__(16) unsigned char smem[];
-    [[maybe_unused]] signed char* s_core = reinterpret_cast<signed char*>(smem + SM::core_off);
-    [[maybe_unused]] float4* s_cg = reinterpret_cast<float4*>(smem + SM::cg_off);          // [K][64] (W * grad_pixel, A . grad_pixel)
+    constexpr uint32_t kNotCore = kFirstK ? 0xffu : uint32_t(SM::core_rows);      // in s_core: not a core entry
+    [[maybe_unused]] unsigned char* s_core = smem + SM::core_off;
+    float4* s_terms = reinterpret_cast<float4*>(smem + SM::cg_off);                        // [K][64] (W * grad_pixel, A . grad_pixel), then s_tc
     [[maybe_unused]] float4* s_tc = reinterpret_cast<float4*>(smem + SM::tc_off);          // [64] (full_weight * grad_pixel, common term)
     [[maybe_unused]] float* s_ta = reinterpret_cast<float*>(smem + SM::ta_off);            // [64] term divided by (1 - alpha)
 
@@ -234,7 +255,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     // give the pixel masks, the records of those instances that touch a pixel (six in ten) are requested, then the outlines of
     // batch b + 2 and the indices of batch b + 3.
     uint32_t g_rec = 0, g_out = 0, g_idx = 0;
-    float4 rN0 = make_float4(0, 0, 0, 0), rN1 = rN0, rD1 = rN0, rC = rN0, rRGBA = rN0, outline = rN0;     // rC: centre, shear, 1 / D at the centre
+    float4 rQ0 = make_float4(0, 0, 0, 0), rQ1 = rQ0, rQ2 = rQ0, rC = rQ0, rRGBA = rQ0, outline = rQ0;     // rC: centre, shear, 1 / D at the centre
     float outline_c = 0.0f;
     uint64_t mask_rec = 0;
     auto load_index = [&](uint32_t inst) { return inst < range.y ? __ldg(prims_sorted + inst) : 0u; };
@@ -249,7 +270,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         if (mask_rec == 0) return;
         g_rec = g_out;
         const float* rec = reinterpret_cast<const float*>(pair + g_rec);
-        rN0 = ldg4(rec); rN1 = ldg4(rec + 4); rD1 = ldg4(rec + 8); rC = ldg4(rec + 12);
+        rQ0 = ldg4(rec); rQ1 = ldg4(rec + 4); rQ2 = ldg4(rec + 8); rC = ldg4(rec + 12);
         rRGBA = ldg4(reinterpret_cast<const float*>(eval + g_rec) + 16);
     };
     g_out = load_index(range.x + tid);
@@ -283,7 +304,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
                     const int k = (i0 + i) * int(kParts) + int(part);
                     if (k >= K || !inside) core_pos[i0 + i] = 0xffffffffu;
                     const float3 drgb = info[i].w * grad_pixel;
-                    if (k < K) s_cg[k * 64 + pix] = make_float4(drgb.x, drgb.y, drgb.z, dot(f3(info[i]), grad_pixel));
+                    if (k < K) s_terms[k * 64 + pix] = make_float4(drgb.x, drgb.y, drgb.z, dot(f3(info[i]), grad_pixel));
                 }
             }
         }
@@ -319,10 +340,10 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
     //      more); a lane takes one segment, sums its record in registers and adds it to the Gaussian's.  All lanes of a warp change
     //      Gaussians at the same time: with the pairs split evenly over the lanes instead, some lane changed in almost every step,
     //      and the warp spent a third of its instructions on that (1450 -> 1290 us at 3 M Gaussians, 1297 x 840, K = 16).
-    float4* s_n0 = reinterpret_cast<float4*>(smem + SM::stage_off);
-    float4* s_n1 = s_n0 + NT;
-    float4* s_d1 = s_n1 + NT;
-    float4* s_rgba = s_d1 + NT;
+    float4* s_q0 = reinterpret_cast<float4*>(smem + SM::stage_off);
+    float4* s_q1 = s_q0 + NT;
+    float4* s_q2 = s_q1 + NT;
+    float4* s_rgba = s_q2 + NT;
     float4* s_pos = s_rgba + NT;         // tile origin - centre, rho^2 below which a fragment is certainly accepted, shear
     [[maybe_unused]] float4* s_abs = s_pos + NT;    // ABS_GRAD: [3][NT]
     [[maybe_unused]] unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(s_pos + NT * (ABS_GRAD ? 4 : 1));      // FIRST_K
@@ -341,7 +362,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         for (int i = 0; i < int((K + kParts - 1) / kParts); ++i) {
             const uint32_t j = core_pos[i] - batch_pos;
             if (j < limit) {
-                s_core[j * kBwdCoreRow + pix] = (signed char)(i * int(kParts) + int(part));
+                s_core[j * kBwdCoreRow + pix] = (unsigned char)(i * int(kParts) + int(part));
                 if constexpr (kFirstK) atomicOr(reinterpret_cast<uint32_t*>(s_mask + j) + (pix >> 5), 1u << (pix & 31));
             }
         }
@@ -351,7 +372,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
         const uint32_t inst = batch_begin + tid;
         uint64_t my_mask = mask_rec;
         if (my_mask != 0) {
-            s_n0[tid] = rN0; s_n1[tid] = rN1; s_d1[tid] = rD1; s_rgba[tid] = rRGBA;
+            s_q0[tid] = rQ0; s_q1[tid] = rQ1; s_q2[tid] = rQ2; s_rgba[tid] = rRGBA;
             float level = 0.0f;
             if constexpr (!kFirstK) level = acceptance_level<MT>(rRGBA.w);
             const float band = kLevelBand * level + 1e-6f;
@@ -364,7 +385,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             if constexpr (SM::has_core) {      // no pair of my instance is a core entry until the scatter below says so
                 uint32_t* row = reinterpret_cast<uint32_t*>(s_core + tid * kBwdCoreRow);
                 #pragma unroll
-                for (int i = 0; i < 16; ++i) row[i] = 0xffffffffu;
+                for (int i = 0; i < 16; ++i) row[i] = kNotCore * 0x01010101u;
             }
         }
         request_record(inst + NT);
@@ -417,53 +438,71 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             uint32_t pixels = has_segment ? s_segment[first + lane] : 0u;
             const uint32_t owner = s_owner[min(first + lane, n_segments - 1u)], j = owner >> 1;
             const float row0 = float((owner & 1u) * 4u);
-            const PairForm form{s_n0[j], s_n1[j], s_d1[j]};
+            const PairForm form{s_q0[j], s_q1[j], s_q2[j]};
             const float4 rgba = s_rgba[j], pos = s_pos[j];
             PairMoments moments{};
-            float4 aC = make_float4(0, 0, 0, 0);            // (dL/drgb, dL/dopacity)
+            f32x2 aC_rg = pack2(0.0f, 0.0f);                // dL/drgb and dL/dopacity
+            float aC_b = 0.0f, aC_opacity = 0.0f;
             [[maybe_unused]] float abs_grad = 0.0f;
             bool touched = false;
-            while (pixels != 0) {
-                const uint32_t bit = uint32_t(__ffs(int(pixels)) - 1);
-                const uint32_t p = bit + (owner & 1u) * 32u;
-                pixels &= pixels - 1;
-                const float column = float(bit & 7u), row = row0 + float(bit >> 3);
-                const float y = pos.y + row, s = fmaf(pos.w, y, pos.x + column);
-                float numerator_rho2, denominator;
-                evaluate_pair(form, s, y, numerator_rho2, denominator);
-                int core_idx = -1;
-                if constexpr (SM::has_core) core_idx = s_core[j * kBwdCoreRow + p];
-                const float denominator_rcp = rcp_approx(denominator);
-                const float rho2 = numerator_rho2 * denominator_rcp;
+            const uint32_t first_pixel = (owner & 1u) * 32u;
+            // Two pairs per trip, without a branch behind the test: independent instruction streams, which the 14 warps of an SM that registers
+            // and shared memory leave need (they issue on half of the cycles).  3 M Gaussians, 1297 x 840, K = 16: one pair with single
+            // instructions and branches for core and tail 980 us; packed, one row of terms for both 917; two pairs 873; without the branch 865.
+            // OIT 233 -> 226, FIRST_K 123 -> 111 (0.5 M, 800 x 600).
+            struct Pair { float s, y, rho2, numerator, denominator_rcp, column, row; uint32_t terms, p; bool ok; };
+            auto look = [&](uint32_t bit, bool valid) -> Pair {
+                Pair r;
+                r.p = bit + first_pixel;
+                r.column = small_int_to_float(bit & 7u); r.row = row0 + small_int_to_float(bit >> 3);
+                r.y = pos.y + r.row; r.s = fmaf(pos.w, r.y, pos.x + r.column);
+                float denominator;
+                evaluate_pair(form, r.s, r.y, r.numerator, denominator);
+                // the row of the pixel's terms: a core entry's, or that of the tail behind them
+                r.terms = 0;
+                if constexpr (SM::has_core) r.terms = s_core[j * kBwdCoreRow + r.p];
+                r.denominator_rcp = rcp_approx(denominator);
+                r.rho2 = r.numerator * r.denominator_rcp;
                 if constexpr (kFirstK) {
-                    if (core_idx < 0) continue;                    // only stored fragments carry gradient (first_k backward.cuh:84-87)
-                } else if (!(rho2 < pos.z)) {
-                    if (rho2 > upper_level(pos.z) || !accepted_by_forward<MT>(eval + s_g[j], x0 + column, y0 + row)) continue;
-                }
-                const float G = exp_approx(-0.5f * rho2);
-                const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
-                float3 dL_drgb;
-                float dL_dalpha;
-                if (core_idx >= 0) {
-                    const float4 cg = s_cg[core_idx * 64 + p];
-                    dL_drgb = f3(cg);
-                    dL_dalpha = cg.w;
+                    r.ok = valid && r.terms != kNotCore;           // only stored fragments carry gradient (first_k backward.cuh:84-87)
+                    r.terms = r.ok ? r.terms : 0u;
                 } else {
-                    if constexpr (SM::has_tail) {
-                        const float4 tc = s_tc[p];
-                        dL_drgb = f3(tc) * alpha;
-                        dL_dalpha = tc.w + dot(f3(rgba), f3(tc)) + s_ta[p] * rcp_approx(fmaxf(1.0f - alpha, kOneMinusAlphaEps));
-                    } else {
-                        continue;
-                    }
+                    r.ok = valid && r.rho2 < pos.z;
+                    if (valid && !r.ok && !(r.rho2 > upper_level(pos.z))) r.ok = accepted_by_forward<MT>(eval + s_g[j], x0 + r.column, y0 + r.row);
                 }
-                aC.x += dL_drgb.x; aC.y += dL_drgb.y; aC.z += dL_drgb.z;
-                aC.w += dL_dalpha * G;
-                touched = true;
-                const float u = -0.5f * dL_dalpha * rgba.w * G * denominator_rcp;      // dL/drho^2 / D, times D at the centre
-                add_moments(moments, u, u * rho2, u * numerator_rho2, s, y);
+                return r;
+            };
+            auto add = [&](Pair r) {                     // of a pair that is not accepted only zeros
+                const float G = r.ok ? exp_approx(-0.5f * r.rho2) : 0.0f;
+                if (!r.ok) r.rho2 = r.numerator = r.denominator_rcp = 0.0f;
+                const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
+                const float4 term = s_terms[r.terms * 64 + r.p];
+                float dL_dalpha = term.w, scale = 1.0f;
+                if constexpr (SM::has_tail) {            // both, since in almost every step some lanes have the one and some the other
+                    const float tail_dL_dalpha = term.w + dot(f3(rgba), f3(term)) + s_ta[r.p] * rcp_approx(fmaxf(1.0f - alpha, kOneMinusAlphaEps));
+                    const bool core = r.terms < uint32_t(SM::core_rows);
+                    scale = core ? 1.0f : alpha;
+                    dL_dalpha = core ? dL_dalpha : tail_dL_dalpha;
+                }
+                scale = r.ok ? scale : 0.0f;
+                aC_rg = fma2(low2(term), pack2(scale, scale), aC_rg);
+                aC_b = fmaf(term.z, scale, aC_b);
+                aC_opacity = fmaf(dL_dalpha, G, aC_opacity);
+                touched |= r.ok;
+                const float u = -0.5f * dL_dalpha * rgba.w * G * r.denominator_rcp;      // dL/drho^2 / D, times D at the centre
+                add_moments(moments, u, u * r.rho2, u * r.numerator, r.s, r.y);
                 if constexpr (ABS_GRAD)
-                    abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, s, y, x0 + column, y0 + row, cam);
+                    abs_grad += abs_position_gradient(AbsForm{s_abs[j], s_abs[NT + j], s_abs[2 * NT + j]}, u, r.s, r.y, x0 + r.column, y0 + r.row, cam);
+            };
+            while (pixels != 0) {
+                const uint32_t bit0 = uint32_t(__ffs(int(pixels)) - 1);
+                pixels &= pixels - 1;
+                const bool second = pixels != 0;
+                const uint32_t bit1 = second ? uint32_t(__ffs(int(pixels)) - 1) : bit0;
+                pixels &= pixels - 1;
+                const Pair a = look(bit0, true), b = look(bit1, second);
+                add(a);
+                add(b);
             }
             // The segments of a Gaussian (at most four) lie side by side, but for the border between long and short ones: they are added up
             // before they go out, since it is the number of additions to a record that its rounding grows with.
@@ -471,11 +510,11 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             const bool join_1 = __shfl_down_sync(0xffffffffu, key, 1) == key && lane < 31;
             const uint32_t joined_1 = __ballot_sync(0xffffffffu, join_1), joined_2 = joined_1 & (joined_1 >> 1);      // with the next lane, with the next but one
             auto join = [&](float& x, int o, bool take) { const float t = __shfl_down_sync(0xffffffffu, x, o); if (take) x += t; };
+            auto join2 = [&](f32x2& x, int o, bool take) { const f32x2 t = __shfl_down_sync(0xffffffffu, x, o); if (take) x = add2(x, t); };
             auto join_all = [&](int o, bool take) {
-                join(moments.u0.x, o, take); join(moments.u0.y, o, take); join(moments.u0.z, o, take); join(moments.u0.w, o, take);
-                join(moments.u1.x, o, take); join(moments.u1.y, o, take); join(moments.u1.z, o, take); join(moments.u1.w, o, take);
-                join(moments.v1.x, o, take); join(moments.v1.y, o, take); join(moments.v1.z, o, take); join(moments.v1.w, o, take);
-                join(aC.x, o, take); join(aC.y, o, take); join(aC.z, o, take); join(aC.w, o, take);
+                join2(moments.uv, o, take); join2(moments.u1, o, take); join2(moments.u2, o, take); join2(moments.v1, o, take); join2(moments.v2, o, take);
+                join(moments.usy, o, take); join(moments.vsy, o, take);
+                join2(aC_rg, o, take); join(aC_b, o, take); join(aC_opacity, o, take);
                 if constexpr (ABS_GRAD) join(abs_grad, o, take);
             };
             uint32_t out = __ballot_sync(0xffffffffu, touched);
@@ -489,7 +528,8 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             }
             if (((out & ~(joined_1 << 1)) >> lane) & 1u) {
                 float4* rec = accum + size_t(s_g[j]) * 5;
-                red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); red_add_v4(rec + 2, moments.v1); red_add_v4(rec + 3, aC);
+                red_add_v4(rec, moments.row(0)); red_add_v4(rec + 1, moments.row(1)); red_add_v4(rec + 2, moments.row(2));
+                red_add_v4(rec + 3, make_float4(unpack2(aC_rg).x, unpack2(aC_rg).y, aC_b, aC_opacity));
                 if constexpr (ABS_GRAD) red_add_v4(rec + 4, make_float4(abs_grad, 0.0f, 0.0f, 0.0f));
             }
         }
@@ -517,7 +557,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
     using MT = ModeTraits<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING>;
     constexpr uint32_t kTileX = MT::tile_w / 8, kTileY = MT::tile_h / 4;
     __shared__ float4 s_pair[kGoChunk][33];              // [survivor][pixel]: weight, dL/dalpha * G, rho^2, 1 / D
-    __shared__ float4 s_n0[kGoChunk], s_n1[kGoChunk], s_d1[kGoChunk], s_rgba[kGoChunk], s_pos[kGoChunk];
+    __shared__ float4 s_q0[kGoChunk], s_q1[kGoChunk], s_q2[kGoChunk], s_rgba[kGoChunk], s_pos[kGoChunk];
     __shared__ float4 s_grad[32];                        // dL/dpixel
     __shared__ uint32_t s_g[kGoChunk], s_queue_prim[kGoQueue], s_queue_mask[kGoQueue];
     const uint32_t lane = threadIdx.x;
@@ -572,7 +612,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
     // the record of the survivor this lane stages (both half warps hold the same 16)
     const uint32_t mine = lane & uint32_t(kGoChunk - 1);
     uint32_t g_mine = 0, mask_mine = 0, count = 0;
-    float4 rN0 = make_float4(0, 0, 0, 0), rN1 = rN0, rD1 = rN0, rC = rN0, rRGBA = rN0;
+    float4 rQ0 = make_float4(0, 0, 0, 0), rQ1 = rQ0, rQ2 = rQ0, rC = rQ0, rRGBA = rQ0;
     auto take = [&]() {                                  // the next chunk: indices, masks, and requests for its records
         while (queued < kGoChunk && next - lane < range.y) filter();
         __syncwarp();
@@ -583,7 +623,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
             g_mine = s_queue_prim[at];
             mask_mine = s_queue_mask[at];
             const float* rec = reinterpret_cast<const float*>(pair + g_mine);
-            rN0 = ldg4(rec); rN1 = ldg4(rec + 4); rD1 = ldg4(rec + 8); rC = ldg4(rec + 12);
+            rQ0 = ldg4(rec); rQ1 = ldg4(rec + 4); rQ2 = ldg4(rec + 8); rC = ldg4(rec + 12);
             rRGBA = ldg4(reinterpret_cast<const float*>(eval + g_mine) + 16);
         }
         queue_head += count;
@@ -597,7 +637,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
         [[maybe_unused]] AbsForm af{};
         if (mine < count) {
             if (lane < kGoChunk) {
-                s_n0[mine] = rN0; s_n1[mine] = rN1; s_d1[mine] = rD1; s_rgba[mine] = rRGBA;
+                s_q0[mine] = rQ0; s_q1[mine] = rQ1; s_q2[mine] = rQ2; s_rgba[mine] = rRGBA;
                 const float level = acceptance_level<MT>(rRGBA.w);
                 const float band = kLevelBand * level + 1e-6f;
                 s_pos[mine] = make_float4(x0 - rC.x, y0 - rC.y, level - band, rC.z);
@@ -621,7 +661,7 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
             const float4 pos = s_pos[j];
             const float y = pos.y + local_y, s = fmaf(pos.w, y, pos.x + local_x);
             float numerator_rho2, denominator;
-            evaluate_pair(PairForm{s_n0[j], s_n1[j], s_d1[j]}, s, y, numerator_rho2, denominator);
+            evaluate_pair(PairForm{s_q0[j], s_q1[j], s_q2[j]}, s, y, numerator_rho2, denominator);
             const float denominator_rcp = rcp_approx(denominator);
             const float rho2 = numerator_rho2 * denominator_rcp;
             bool ok = valid && rho2 < pos.z;
@@ -669,12 +709,15 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
             v.x += __shfl_xor_sync(0xffffffffu, v.x, 16); v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
             v.z += __shfl_xor_sync(0xffffffffu, v.z, 16); v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
         };
-        both_halves(moments.u0); both_halves(moments.u1); both_halves(moments.v1); both_halves(aC);
+        auto both_halves2 = [](f32x2& v) { v = add2(v, __shfl_xor_sync(0xffffffffu, v, 16)); };
+        both_halves2(moments.uv); both_halves2(moments.u1); both_halves2(moments.u2); both_halves2(moments.v1); both_halves2(moments.v2); both_halves(aC);
+        moments.usy += __shfl_xor_sync(0xffffffffu, moments.usy, 16);
+        moments.vsy += __shfl_xor_sync(0xffffffffu, moments.vsy, 16);
         if constexpr (ABS_GRAD) abs_grad += __shfl_xor_sync(0xffffffffu, abs_grad, 16);
         if ((any >> lane) & 1u) {                        // the two half warps share the four or five reductions of a record
             float4* rec = accum + size_t(g) * 5;
-            if (lane < kGoChunk) { red_add_v4(rec, moments.u0); red_add_v4(rec + 1, moments.u1); }
-            else { red_add_v4(rec + 2, moments.v1); red_add_v4(rec + 3, aC); }
+            if (lane < kGoChunk) { red_add_v4(rec, moments.row(0)); red_add_v4(rec + 1, moments.row(1)); }
+            else { red_add_v4(rec + 2, moments.row(2)); red_add_v4(rec + 3, aC); }
             if constexpr (ABS_GRAD) { if (lane < kGoChunk) red_add_v4(rec + 4, make_float4(abs_grad, 0.0f, 0.0f, 0.0f)); }
         }
         if (__all_sync(0xffffffffu, done)) break;
@@ -736,9 +779,9 @@ __global__ void __launch_bounds__(kChainThreads, 7) preprocess_backward_kernel(
     const float4 dC = accum[size_t(idx) * 5 + 3];
     const float4 T4 = ldg4(reinterpret_cast<const float*>(eval + idx) + 8);
     const float4 centre = ldg4(&pair[idx].cx);       // and shear, 1 / D at the centre
-    const PairMoments moments{centre.w * accum[size_t(idx) * 5], centre.w * accum[size_t(idx) * 5 + 1], centre.w * accum[size_t(idx) * 5 + 2]};
+    const PairForm form{ldg4(&pair[idx].q0.x), ldg4(&pair[idx].q1.x), ldg4(&pair[idx].q2.x)};
     const RowGradients rows = rows_from_moments(affine_planes<double>(ldg4(reinterpret_cast<const float*>(eval + idx)), ldg4(reinterpret_cast<const float*>(eval + idx) + 4), T4,
-                                                              centre.x, centre.y, centre.z), T4, ldg4(&pair[idx].n0.x), ldg4(&pair[idx].n1.x), moments);
+                                                              centre.x, centre.y, centre.z), T4, form, centre.w * accum[size_t(idx) * 5], centre.w * accum[size_t(idx) * 5 + 1], centre.w * accum[size_t(idx) * 5 + 2]);
     // dL/dVPMT4 = -(cx dL/dVPMT1 + cy dL/dVPMT2 + E): the products with the centre are moved to the rows of VPM, where they cancel
     const float4 dT1 = rows.dX, dT2 = rows.dY, dT4 = make_float4(-rows.E.x, -rows.E.y, -rows.E.z, -rows.E.w);
     const float3 c1 = make_float3(dT1.x, dT2.x, dT4.x), c2 = make_float3(dT1.y, dT2.y, dT4.y), c3 = make_float3(dT1.z, dT2.z, dT4.z);
