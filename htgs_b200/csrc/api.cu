@@ -63,6 +63,9 @@ struct Carver {
     }
 };
 
+// GLOBAL_ORDERING splits a key buffer at a 16-byte boundary in its middle (binning.cu: emit_sort_ranges_global).
+inline size_t key_buffer_bytes(const SortPlan& plan, uint64_t capacity) { return size_t(capacity) * size_t(plan.key_bytes) + (plan.key_bytes == 8 ? 16 : 0); }
+
 struct FrameLayout {
     FrameStatus* status;
     PrimBuffers prim;
@@ -94,8 +97,8 @@ FrameLayout carve_frame(void* blob, int n_primitives, int n_tiles, const SortPla
     const uint64_t cap = instance_capacity > 0xfffffff0ull ? 0xfffffff0ull : instance_capacity;
     L.inst.capacity = uint32_t(cap);
     L.inst.sort_blocks_cap = uint32_t((cap + kSortTile - 1) / kSortTile);
-    L.inst.keys[0] = c.take_bytes<void>(size_t(cap) * plan.key_bytes);
-    L.inst.keys[1] = c.take_bytes<void>(size_t(cap) * plan.key_bytes);
+    L.inst.keys[0] = c.take_bytes<void>(key_buffer_bytes(plan, cap));
+    L.inst.keys[1] = c.take_bytes<void>(key_buffer_bytes(plan, cap));
     L.inst.prims[0] = c.take<uint32_t>(size_t(cap));
     L.inst.prims[1] = c.take<uint32_t>(size_t(cap));
     L.inst.sort_scratch = c.take_bytes<void>(sort_scratch_bytes(plan, L.inst.sort_blocks_cap));
@@ -314,14 +317,14 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
     if (prof) cudaEventRecord(ev[0], stream);
     if ((err = launch_preprocess(view.mode, false, scene, view, geo, L.prim, L.status, stream, outline_mode, f.fast)) != cudaSuccess) return fail_cuda(err, "preprocess");
     if (prof) cudaEventRecord(ev[1], stream);
-    if ((err = launch_scan_only(scene, L.prim, L.inst.capacity, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
+    if ((err = launch_scan_only(view.mode, scene, L.prim, L.inst.capacity, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
     if (prof) cudaEventRecord(ev[2], stream);
     *launches += (scene.n_primitives > 0 ? 2 : 0) + 1;
     const uint32_t* prims_sorted = L.inst.prims[plan.final_buffer];
     if (f.fast && !ctx->fast_deterministic) {
         if ((err = launch_bin_unordered(scene, geo, L.prim, L.inst.prims[plan.final_buffer], L.inst.capacity, L.tile_ranges, L.tile_order, L.unordered, L.status, ctx->sm_count,
                                         stream, prof ? ev + 3 : nullptr, launches)) != cudaSuccess) return fail_cuda(err, "unordered binning");
-    } else if ((err = launch_emit_sort_ranges(view.mode, scene, geo, plan, L.prim, L.inst, L.tile_ranges, L.tile_order, L.status, ctx->sm_count, stream,
+    } else if ((err = launch_emit_sort_ranges(scene, view, geo, plan, L.prim, L.inst, L.tile_ranges, L.tile_order, L.status, ctx->sm_count, stream,
                                               prof ? ev + 3 : nullptr, launches)) != cudaSuccess) return fail_cuda(err, "binning");
     if (front_priority) {
         if ((err = cudaEventRecord(ctx->front_end, stream)) != cudaSuccess) return fail_cuda(err, "front event record");
@@ -507,9 +510,22 @@ int htgs_get_intermediates(HtgsContext* ctx, HtgsIntermediates* out) {
     out->eval_records = L.prim.eval;
     out->cull_records = L.prim.cull;
     const int unsorted = (p.n_passes == 0) ? 0 : (p.final_buffer ^ (p.n_passes & 1));   // emission always writes buffer 0
-    out->keys_unsorted = (p.n_passes == 1 || p.n_passes == 0) ? L.inst.keys[unsorted] : nullptr;   // overwritten by later passes otherwise
-    out->prims_unsorted = (p.n_passes == 1 || p.n_passes == 0) ? L.inst.prims[unsorted] : nullptr;
+    const bool by_tile = p.key_bytes != 8;      // GLOBAL_ORDERING emits in depth order: there is no order of emission to show
+    out->keys_unsorted = by_tile && p.n_passes <= 1 ? L.inst.keys[unsorted] : nullptr;   // overwritten by later passes otherwise
+    out->prims_unsorted = by_tile && p.n_passes <= 1 ? L.inst.prims[unsorted] : nullptr;
     out->keys_sorted = L.inst.keys[p.final_buffer];
+    if (!by_tile) {
+        out->keys_sorted = L.inst.keys[0];
+        cudaPointerAttributes attributes{};
+        DeviceGuard guard(ctx->device);
+        cudaError_t err;
+        // a caller's workspace may be gone by now: pointers into it are handed out as before, but nothing is written
+        if (cudaPointerGetAttributes(&attributes, L.inst.keys[0]) != cudaSuccess || attributes.type == cudaMemoryTypeUnregistered) cudaGetLastError();
+        else if (ctx->last_n_instances > 0) {
+            if ((err = launch_global_keys(ctx->last_geo, p, L.prim, L.inst, L.tile_ranges, ctx->front_stream)) != cudaSuccess ||
+                (err = cudaStreamSynchronize(ctx->front_stream)) != cudaSuccess) return fail_cuda(err, "sort keys of the last frame");
+        }
+    }
     out->prims_sorted = L.inst.prims[p.final_buffer];
     out->tile_ranges = reinterpret_cast<const uint32_t*>(L.tile_ranges);
     out->n_tiles = uint32_t(ctx->last_geo.n_tiles);
@@ -651,8 +667,8 @@ InstLayout carve_instance_blob(void* blob, const SortPlan& plan, uint64_t capaci
     // the sorted indices, all that the backward pass reads, come first: it finds them whatever capacity the forward pass had
     L.inst.prims[plan.final_buffer] = c.take<uint32_t>(size_t(cap));
     L.inst.prims[plan.final_buffer ^ 1] = c.take<uint32_t>(size_t(cap));
-    L.inst.keys[0] = c.take_bytes<void>(size_t(cap) * plan.key_bytes);
-    L.inst.keys[1] = c.take_bytes<void>(size_t(cap) * plan.key_bytes);
+    L.inst.keys[0] = c.take_bytes<void>(key_buffer_bytes(plan, cap));
+    L.inst.keys[1] = c.take_bytes<void>(key_buffer_bytes(plan, cap));
     L.inst.sort_scratch = c.take_bytes<void>(sort_scratch_bytes(plan, L.inst.sort_blocks_cap));
     L.bytes = align_up(c.offset);
     return L;
@@ -728,7 +744,7 @@ static int forward_front(HtgsContext* ctx, const HtgsScene* scene, const HtgsVie
     cudaError_t err;
     if ((err = cudaMemsetAsync(L.status, 0, sizeof(FrameStatus), stream)) != cudaSuccess) return fail_cuda(err, "status reset");
     if ((err = launch_preprocess(view->mode, true, *scene, *view, geo, L.prim, L.status, stream, view->mode)) != cudaSuccess) return fail_cuda(err, "preprocess");
-    if ((err = launch_scan_only(*scene, L.prim, capacity, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
+    if ((err = launch_scan_only(view->mode, *scene, L.prim, capacity, L.status, stream)) != cudaSuccess) return fail_cuda(err, "scan");
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
     return HTGS_OK;
 }
@@ -774,7 +790,7 @@ static int forward_finish(HtgsContext* ctx, const HtgsScene* scene, const HtgsVi
     const TileLayout T = carve_tile_blob(blobs->per_tile, geo);
     uint32_t launches = 0;
     cudaError_t err;
-    if ((err = launch_emit_sort_ranges(view->mode, *scene, geo, plan, P.prim, I.inst, T.ranges, T.order, P.status, ctx->sm_count, stream, nullptr, &launches)) != cudaSuccess)
+    if ((err = launch_emit_sort_ranges(*scene, *view, geo, plan, P.prim, I.inst, T.ranges, T.order, P.status, ctx->sm_count, stream, nullptr, &launches)) != cudaSuccess)
         return fail_cuda(err, "binning");
     const BlendOutputs out{image, nullptr, nullptr, true, false, nullptr, 0.0f};
     if ((err = launch_blend(view->mode, BlendTask::training, *view, geo, P.prim, I.inst.prims[plan.final_buffer], T.ranges, T.order, out, X.px, P.status, stream)) != cudaSuccess)

@@ -21,6 +21,7 @@
 #include "kernels.h"
 
 #include <algorithm>
+#include <cstring>
 
 namespace htgs {
 
@@ -36,24 +37,31 @@ FrameGeometry make_geometry(int mode, int width, int height) {
 
 static int bit_length(uint32_t v) { int b = 0; while (v) { ++b; v >>= 1; } return b; }   // rasterization/include/rasterization_utils.h:3-13
 
+// Digits of at most kMaxRadixBits bits, about equally wide; returns how many.
+static int split_digits(int bits, int* width, int* shift) {
+    const int n = (bits + kMaxRadixBits - 1) / kMaxRadixBits;
+    int at = 0;
+    for (int i = 0; i < n; ++i) {
+        width[i] = bits / n + (i < bits % n ? 1 : 0);
+        shift[i] = at;
+        at += width[i];
+    }
+    return n;
+}
+
 SortPlan make_sort_plan(int mode, int n_tiles) {
     SortPlan p{};
     const int tile_bits = bit_length(uint32_t(n_tiles > 0 ? n_tiles - 1 : 0));
     if (mode == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING) { p.key_bytes = 8; p.end_bit = tile_bits + 32; }   // alpha_blend_global_ordering/inference.cu:45
     else { p.end_bit = tile_bits; p.key_bytes = tile_bits <= 16 ? 2 : 4; }                                 // hybrid_blend/inference.cu:121-129
-    p.n_passes = (p.end_bit + kMaxRadixBits - 1) / kMaxRadixBits;
-    int at = 0;
-    for (int i = 0; i < p.n_passes; ++i) {
-        const int base = p.end_bit / p.n_passes, rem = p.end_bit % p.n_passes;
-        p.bits[i] = base + (i < rem ? 1 : 0);
-        p.shift[i] = at;
-        at += p.bits[i];
-    }
+    p.n_passes = split_digits(tile_bits, p.bits, p.shift);
     p.final_buffer = p.n_passes & 1;
     return p;
 }
 
 namespace {
+
+inline size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = kSortTile / kSortThreads;   // 16
@@ -73,12 +81,19 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v) {
 // instead of looping over the array 1024 values at a time with four barriers per round.
 constexpr int kScanThreads = 1024;
 constexpr int kScanRun = 16;            // values per thread and round: 16384 block sums (4.2 M Gaussians) per round
-__global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uint32_t* __restrict__ block_sums, uint32_t* __restrict__ block_offsets,
+// instances: the above.  visible (GLOBAL_ORDERING): adds up the instances, and makes the blocks' visible Gaussians, which lie where the offsets
+// go, into their prefix.  sorted (the same mode, after the sort by depth): the prefix over blocks of 256 visible Gaussians, nothing is published.
+enum class ScanOf { instances, visible, sorted };
+template <ScanOf OF>
+__global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uint32_t* __restrict__ block_sums, uint32_t* block_offsets,
                                                                      uint32_t n_blocks, uint32_t capacity, FrameStatus* status) {
     grid_dependency();
     __shared__ unsigned long long warp_tot[kScanThreads / 32];
     __shared__ unsigned long long carry_s;
-    if (threadIdx.x == 0) carry_s = 0ull;
+    [[maybe_unused]] __shared__ unsigned long long instances_s;
+    if (threadIdx.x == 0) { carry_s = 0ull; instances_s = 0ull; }
+    [[maybe_unused]] unsigned long long instances = 0;
+    if constexpr (OF == ScanOf::sorted) n_blocks = min(n_blocks, (status->n_visible + kPreprocessBlock - 1) / kPreprocessBlock);
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t base = 0; base < n_blocks; base += kScanThreads * kScanRun) {
@@ -86,7 +101,11 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
         uint32_t v[kScanRun];
         unsigned long long mine = 0;
         #pragma unroll
-        for (int i = 0; i < kScanRun; ++i) { v[i] = first + i < n_blocks ? block_sums[first + i] : 0u; mine += v[i]; }
+        for (int i = 0; i < kScanRun; ++i) {
+            v[i] = first + i < n_blocks ? (OF == ScanOf::visible ? block_offsets : block_sums)[first + i] : 0u;
+            mine += v[i];
+            if constexpr (OF == ScanOf::visible) instances += first + i < n_blocks ? block_sums[first + i] : 0u;
+        }
         unsigned long long inc = mine;
         #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= uint32_t(o)) inc += t; }
@@ -110,17 +129,18 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
         if (threadIdx.x == kScanThreads - 1) carry_s = running;
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const unsigned long long total = carry_s;
+    if constexpr (OF == ScanOf::visible) {
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) instances += __shfl_xor_sync(0xffffffffu, instances, o);
+        if (lane == 0) atomicAdd(&instances_s, instances);
+        __syncthreads();
+    }
+    if (OF != ScanOf::sorted && threadIdx.x == 0) {
+        const unsigned long long total = OF == ScanOf::visible ? instances_s : carry_s;
         status->n_instances = total > 0xffffffffull ? 0xffffffffu : uint32_t(total);
         status->overflow = total > (unsigned long long)capacity ? 1u : 0u;
     }
 }
-
-template <typename KeyT> struct KeyOps;
-template <> struct KeyOps<uint16_t> { static __device__ __forceinline__ uint16_t make(uint32_t tile, uint32_t) { return uint16_t(tile); } static __device__ __forceinline__ uint32_t tile(uint16_t k) { return k; } };
-template <> struct KeyOps<uint32_t> { static __device__ __forceinline__ uint32_t make(uint32_t tile, uint32_t) { return tile; } static __device__ __forceinline__ uint32_t tile(uint32_t k) { return k; } };
-template <> struct KeyOps<uint64_t> { static __device__ __forceinline__ uint64_t make(uint32_t tile, uint32_t depth_bits) { return (uint64_t(tile) << 32) | depth_bits; } static __device__ __forceinline__ uint32_t tile(uint64_t k) { return uint32_t(k >> 32); } };
 
 // One block per 256 Gaussians (the blocks of the preprocess kernel), which writes their instances cooperatively: slot j belongs to
 // the Gaussian whose exclusive offset is the last one <= j (eight steps of search); inside a Gaussian the order is row-major over
@@ -129,34 +149,41 @@ template <> struct KeyOps<uint64_t> { static __device__ __forceinline__ uint64_t
 // warp (five steps) where the warps have about equal work gave 51 and 504 us, always 88 and 715: one warp often has most of them.
 // The kernel also clears what the sort and the range kernel count in (`clear`): one launch instead of three.
 struct ClearList { uint4* begin[3]; uint64_t count[3]; uint64_t per_sort_block[3]; };   // 16-byte words: a fixed number, plus so many per sort block of the frame
-template <typename KeyT>
+__device__ __forceinline__ void clear_words(const ClearList& clear, const FrameStatus* status) {
+    const uint64_t sort_blocks = status->overflow ? 0 : (uint64_t(status->n_instances) + kSortTile - 1) / kSortTile;
+    #pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const uint64_t words = clear.count[c] + clear.per_sort_block[c] * sort_blocks;
+        for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < words; i += uint64_t(gridDim.x) * blockDim.x) clear.begin[c][i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+// SORTED (GLOBAL_ORDERING): the blocks are those of the visible Gaussians in depth order, `list`; what has to be cleared has been by then.
+template <typename KeyT, bool SORTED>
 __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
-    const uint32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds, const EvalRecord* __restrict__ eval,
+    const uint32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds, const uint32_t* __restrict__ list,
     const uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ block_offsets, KeyT* __restrict__ keys, uint32_t* __restrict__ prims,
     uint32_t n_primitives, uint32_t grid_w, uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear)
 {
     grid_dependency();
     const bool overflow = status->overflow;
-    const uint64_t sort_blocks = overflow ? 0 : (uint64_t(status->n_instances) + kSortTile - 1) / kSortTile;
-    #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const uint64_t words = clear.count[c] + clear.per_sort_block[c] * sort_blocks;
-        for (uint64_t i = blockIdx.x * kPreprocessBlock + threadIdx.x; i < words; i += uint64_t(gridDim.x) * kPreprocessBlock) clear.begin[c][i] = make_uint4(0u, 0u, 0u, 0u);
-    }
+    if constexpr (!SORTED) clear_words(clear, status);
+    if (SORTED && blockIdx.x * kPreprocessBlock >= status->n_visible) return;
     const uint32_t total = block_sums[blockIdx.x];
     if (total == 0 || overflow) return;   // a frame that does not fit its instance buffers is skipped by every later stage
     __shared__ uint32_t excl[kPreprocessBlock];
-    __shared__ uint4 box[kPreprocessBlock];          // x_min | y_min << 16, width, reciprocal of the width (2^32 / width, rounded up; 0: divide), depth bits
+    __shared__ uint4 box[kPreprocessBlock];          // x_min | y_min << 16, width, reciprocal of the width (2^32 / width, rounded up; 0: divide), Gaussian
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t first = blockIdx.x * kPreprocessBlock;
-    const uint32_t idx = first + threadIdx.x;
-    const uint32_t cnt = idx < n_primitives ? n_touched[idx] : 0u;
+    const uint32_t at = first + threadIdx.x;
+    const bool valid = at < (SORTED ? status->n_visible : n_primitives);
+    const uint32_t idx = SORTED ? (valid ? list[at] : 0u) : at;
+    const uint32_t cnt = valid ? n_touched[idx] : 0u;
     if (cnt) {
         const ushort4 b = bounds[idx];
         const uint32_t w = uint32_t(b.y) - uint32_t(b.x);
         const uint32_t rcp = w > 1 && uint64_t(cnt) * w < (1ull << 32) ? 0xffffffffu / w + 1u : 0u;
-        box[threadIdx.x] = make_uint4(uint32_t(b.x) | (uint32_t(b.z) << 16), w, rcp, sizeof(KeyT) == 8 ? __float_as_uint(eval[idx].mt3.w) : 0u);
+        box[threadIdx.x] = make_uint4(uint32_t(b.x) | (uint32_t(b.z) << 16), w, rcp, idx);
     }
     const uint32_t inc = warp_inclusive_scan(cnt);
     excl[threadIdx.x] = inc - cnt;
@@ -174,8 +201,8 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
         const uint32_t tile = ((b.x >> 16) + ly) * grid_w + (b.x & 0xffffu) + lx;
         const uint64_t dst = base + slot;
         if (dst < capacity) {
-            keys[dst] = KeyOps<KeyT>::make(tile, b.w);
-            prims[dst] = first + owner;
+            keys[dst] = KeyT(tile);
+            prims[dst] = b.w;
         }
     };
     __syncthreads();
@@ -189,8 +216,9 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     }
 }
 
-__device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, uint32_t capacity) {
-    const uint32_t n = status->n_instances;
+// What a sort sorts: the frame's instances, or its visible Gaussians (of which there are no more than instances).
+__device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, uint32_t capacity, bool visible = false) {
+    const uint32_t n = visible ? status->n_visible : status->n_instances;
     return status->overflow ? 0u : (n < capacity ? n : capacity);
 }
 
@@ -215,7 +243,11 @@ constexpr uint32_t kLookbackPolls = 1u << 20;      // about half a second of pol
 constexpr uint32_t kGroup = 32;                    // sort blocks per group
 constexpr int kLookbackBatch = 8;                  // words read per step
 
+constexpr int kDepthRowWords = 1536;     // of the sort by depth: 4 passes of 8 bits, or 3 of 9
+constexpr int kFirstDepthPass = 4;       // its place in tickets and digit_hist; there are at most four passes over the tile
 struct SortScratch {
+    unsigned long long* depth_groups;    // GLOBAL_ORDERING, the sort by depth: [groups][kDepthRowWords], all passes
+    uint32_t* depth_rows;                // [sort_blocks_cap][row_stride]
     uint32_t* tickets;                   // [16]
     uint32_t* digit_hist;                // [8][kMaxRadixBins]
     unsigned long long* groups[8];       // per pass [ceil(sort_blocks_cap / kGroup)][1 << bits]
@@ -233,18 +265,23 @@ __host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32
         sc.groups[i] = reinterpret_cast<unsigned long long*>(p + off);
         off += (n_groups << plan.bits[i]) * sizeof(unsigned long long);
     }
+    const bool by_depth = plan.key_bytes == 8;
+    sc.depth_groups = reinterpret_cast<unsigned long long*>(p + off);
+    if (by_depth) off += n_groups * kDepthRowWords * sizeof(unsigned long long);
     off = (off + 15) & ~size_t(15);
     sc.fixed_bytes = off;
     for (int i = 0; i < plan.n_passes; ++i) {
         sc.rows[i] = reinterpret_cast<uint32_t*>(p + off) + sc.row_stride;
         sc.row_stride += size_t(1) << plan.bits[i];
     }
+    sc.depth_rows = reinterpret_cast<uint32_t*>(p + off) + sc.row_stride;
+    if (by_depth) sc.row_stride += kDepthRowWords;
     sc.row_stride = (sc.row_stride + 3) & ~size_t(3);
     sc.bytes = off + size_t(sort_blocks_cap) * sc.row_stride * sizeof(uint32_t);
     return sc;
 }
 
-struct PassTable { int n_passes; int shift[8]; int bits[8]; };
+struct PassTable { int n_passes; int shift[8]; int bits[8]; bool visible; };
 
 // Digit histograms of all passes in one read of the keys.  A thread takes 16 bytes of consecutive keys per load and
 // counts runs of equal digits before touching shared memory: a Gaussian's instances are neighbouring tiles, so the high
@@ -255,7 +292,7 @@ __global__ void __launch_bounds__(256) radix_histogram_all_kernel(const KeyT* __
     grid_dependency();
     constexpr uint32_t kRun = 16 / sizeof(KeyT);
     __shared__ uint32_t hist[8 * kMaxRadixBins];
-    const uint32_t n = frame_instances(status, capacity);
+    const uint32_t n = frame_instances(status, capacity, passes.visible);
     for (uint32_t i = threadIdx.x; i < uint32_t(passes.n_passes) * kMaxRadixBins; i += 256) hist[i] = 0;
     __syncthreads();
     const uint32_t n_runs = (n + kRun - 1) / kRun;
@@ -324,7 +361,7 @@ template <typename KeyT>
 __global__ void __launch_bounds__(kSortThreads, scatter_blocks_per_sm<KeyT>()) radix_scatter_kernel(
     const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ prims_in, KeyT* __restrict__ keys_out, uint32_t* __restrict__ prims_out,
     const uint32_t* __restrict__ digit_hist, uint32_t* rows, uint32_t row_stride, unsigned long long* groups, uint32_t* ticket,
-    FrameStatus* status, uint32_t capacity, int shift, int bits)
+    FrameStatus* status, uint32_t capacity, int shift, int bits, bool visible)
 {
     grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -339,7 +376,7 @@ __global__ void __launch_bounds__(kSortThreads, scatter_blocks_per_sm<KeyT>()) r
     __shared__ uint32_t warp_tot[kSortWarps];
     __shared__ uint32_t s_blk, s_failed;
 
-    const uint32_t n = frame_instances(status, capacity);
+    const uint32_t n = frame_instances(status, capacity, visible);
     const uint32_t n_blocks = uint32_t((uint64_t(n) + kSortTile - 1) / kSortTile);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -542,12 +579,12 @@ __global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* 
             #pragma unroll
             for (uint32_t i = 0; i < kRangeRun; ++i) k[i] = first + i < n ? keys[first + i] : KeyT(0);
         }
-        uint32_t prev = first ? KeyOps<KeyT>::tile(keys[first - 1]) : 0xffffffffu;
+        uint32_t prev = first ? uint32_t(keys[first - 1]) : 0xffffffffu;
         #pragma unroll
         for (uint32_t i = 0; i < kRangeRun; ++i) {
             const uint32_t at = first + i;
             if (at < n) {
-                const uint32_t tile = KeyOps<KeyT>::tile(k[i]);
+                const uint32_t tile = uint32_t(k[i]);
                 if (at == 0) ranges[tile].x = 0;
                 else if (prev != tile) { ranges[prev].y = at; ranges[tile].x = at; }
                 if (at == n - 1) ranges[tile].y = n;
@@ -566,59 +603,172 @@ __global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* 
     }
 }
 
+// Visible Gaussians of a GLOBAL_ORDERING frame in index order, with the bits of their depth as keys: the input of the sort by depth.
+__global__ void __launch_bounds__(kPreprocessBlock) list_visible_kernel(const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const uint32_t* __restrict__ visible_offsets,
+                                                                        uint32_t* __restrict__ keys, uint32_t* __restrict__ prims, uint32_t n_primitives, uint32_t lowest_key,
+                                                                        const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear) {
+    grid_dependency();
+    clear_words(clear, status);
+    if (status->overflow) return;
+    __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
+    const uint32_t idx = blockIdx.x * kPreprocessBlock + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const bool visible = idx < n_primitives && n_touched[idx] != 0;
+    const uint32_t ballot = __ballot_sync(0xffffffffu, visible);
+    if (lane == 0) warp_tot[warp] = __popc(ballot);
+    __syncthreads();
+    if (!visible) return;
+    uint32_t at = visible_offsets[blockIdx.x] + __popc(ballot & lanemask_lt());
+    #pragma unroll
+    for (int w = 0; w < kPreprocessBlock / 32; ++w) if (w < int(warp)) at += warp_tot[w];
+    keys[at] = __float_as_uint(eval[idx].mt3.w) - lowest_key;
+    prims[at] = idx;
+}
+
+// Instances of every 256 of them, once they are in depth order.
+__global__ void __launch_bounds__(kPreprocessBlock) sum_sorted_kernel(const uint32_t* __restrict__ list, const uint32_t* __restrict__ n_touched, uint32_t* __restrict__ block_sums,
+                                                                      const FrameStatus* __restrict__ status) {
+    grid_dependency();
+    const uint32_t n = status->overflow ? 0u : status->n_visible, i = blockIdx.x * kPreprocessBlock + threadIdx.x;
+    if (blockIdx.x * kPreprocessBlock >= n) return;
+    __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, i < n ? n_touched[list[i]] : 0u);
+    if ((threadIdx.x & 31u) == 0) warp_tot[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    uint32_t total = 0;
+    #pragma unroll
+    for (int w = 0; w < kPreprocessBlock / 32; ++w) total += warp_tot[w];
+    block_sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(256) global_keys_kernel(const uint2* __restrict__ ranges, const uint32_t* __restrict__ prims, const EvalRecord* __restrict__ eval, unsigned long long* __restrict__ keys) {
+    const uint2 range = ranges[blockIdx.x];
+    for (uint32_t i = range.x + threadIdx.x; i < range.y; i += 256) keys[i] = (static_cast<unsigned long long>(blockIdx.x) << 32) | __float_as_uint(eval[prims[i]].mt3.w);
+}
+
+// The passes over `passes`: histogram, then one scatter each, from buffer 0 to buffer n_passes & 1.
+template <typename KeyT>
+cudaError_t launch_radix_sort(const PassTable& passes, KeyT* const (&keys)[2], uint32_t* const (&prims)[2], uint32_t* digit_hist, uint32_t* const* rows, uint32_t row_stride,
+                              unsigned long long* const* groups, uint32_t* tickets, const InstBuffers& inst, uint32_t most_sort_blocks, FrameStatus* status, int sm_count,
+                              cudaStream_t stream, uint32_t* launches) {
+    static PerDeviceOnce configured;
+    const cudaError_t err = configured.run([] { return cudaFuncSetAttribute(radix_scatter_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(scatter_smem_bytes<KeyT>())); });
+    if (err != cudaSuccess || passes.n_passes == 0) return err;
+    const uint32_t hist_grid = std::min<uint32_t>(std::max(most_sort_blocks, 1u), uint32_t(sm_count) * 8u);
+    launch_after(radix_histogram_all_kernel<KeyT>, hist_grid, 256, 0, stream, keys[0], digit_hist, status, inst.capacity, passes);
+    for (int p = 0; p < passes.n_passes; ++p) {
+        const size_t smem = scatter_smem_bytes<KeyT>(passes.bits[p]);
+        const uint32_t resident = uint32_t(std::min<size_t>(scatter_blocks_per_sm<KeyT>(), (227 * 1024) / (smem + 1024)));
+        const uint32_t scatter_grid = std::min<uint32_t>(std::max(most_sort_blocks, 1u), uint32_t(sm_count) * resident);
+        launch_after(radix_scatter_kernel<KeyT>, scatter_grid, kSortThreads, smem, stream, keys[p & 1], prims[p & 1], keys[(p & 1) ^ 1], prims[(p & 1) ^ 1], digit_hist + size_t(p) * kMaxRadixBins,
+                     rows[p], row_stride, groups[p], tickets + p, status, inst.capacity, passes.shift[p], passes.bits[p], passes.visible);
+    }
+    if (launches) *launches += 1u + uint32_t(passes.n_passes);
+    return cudaSuccess;
+}
+
+PassTable tile_passes(const SortPlan& plan) {
+    PassTable t{};
+    t.n_passes = plan.n_passes;
+    for (int p = 0; p < plan.n_passes; ++p) { t.shift[p] = plan.shift[p]; t.bits[p] = plan.bits[p]; }
+    return t;
+}
+
+ClearList clear_list(const SortScratch& sc, const SortPlan& plan, const FrameGeometry& geo, uint2* tile_ranges) {
+    ClearList clear{};      // the buffers are 256-byte aligned and padded to 256 bytes
+    clear.begin[0] = reinterpret_cast<uint4*>(tile_ranges); clear.count[0] = (uint64_t(geo.n_tiles) + 1) / 2;
+    if (sc.row_stride > 0) {
+        clear.begin[1] = reinterpret_cast<uint4*>(sc.tickets); clear.count[1] = sc.fixed_bytes / 16;
+        clear.begin[2] = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(sc.tickets) + sc.fixed_bytes); clear.per_sort_block[2] = sc.row_stride / 4;
+    }
+    (void)plan;
+    return clear;
+}
+
+// A frame without Gaussians or without room for instances.
+template <typename KeyT>
+cudaError_t empty_ranges(const FrameGeometry& geo, const InstBuffers& inst, uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
+    const cudaError_t err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream);
+    if (err != cudaSuccess) return err;
+    if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); }
+    launch_after(tile_ranges_kernel<KeyT>, 1, kOrderThreads, 0, stream, static_cast<const KeyT*>(inst.keys[0]), tile_ranges, tile_order, status, 0u, uint32_t(geo.n_tiles));
+    if (ev) cudaEventRecord(ev[2], stream);
+    if (launches) *launches += 1;
+    return cudaGetLastError();
+}
+
 template <typename KeyT>
 cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst,
                                uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
-    cudaError_t err = cudaSuccess;
-    if (prim_blocks == 0 || inst.capacity == 0) {
-        if ((err = cudaMemsetAsync(tile_ranges, 0, sizeof(uint2) * size_t(geo.n_tiles), stream)) != cudaSuccess) return err;
-        if (ev) { cudaEventRecord(ev[0], stream); cudaEventRecord(ev[1], stream); }
-        launch_after(tile_ranges_kernel<KeyT>, 1, kOrderThreads, 0, stream, static_cast<const KeyT*>(inst.keys[0]), tile_ranges, tile_order, status, 0u, uint32_t(geo.n_tiles));
-        if (ev) cudaEventRecord(ev[2], stream);
-        if (launches) *launches += 1;
-        return cudaGetLastError();
-    }
+    if (prim_blocks == 0 || inst.capacity == 0) return empty_ranges<KeyT>(geo, inst, tile_ranges, tile_order, status, stream, ev, launches);
     const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap);
-    ClearList clear{};      // the buffers are 256-byte aligned and padded to 256 bytes
-    clear.begin[0] = reinterpret_cast<uint4*>(tile_ranges); clear.count[0] = (uint64_t(geo.n_tiles) + 1) / 2;
-    if (plan.n_passes > 0) {
-        clear.begin[1] = reinterpret_cast<uint4*>(sc.tickets); clear.count[1] = sc.fixed_bytes / 16;
-        clear.begin[2] = reinterpret_cast<uint4*>(sc.rows[0]); clear.per_sort_block[2] = sc.row_stride / 4;
-    }
-    launch_after(emit_instances_kernel<KeyT>, prim_blocks, kPreprocessBlock, 0, stream,
-        prim.n_touched, prim.bounds, prim.eval, prim.block_sums, prim.block_offsets, static_cast<KeyT*>(inst.keys[0]), inst.prims[0], n,
-        uint32_t(geo.grid_w), inst.capacity, status, clear);
+    KeyT* const keys[2] = {static_cast<KeyT*>(inst.keys[0]), static_cast<KeyT*>(inst.keys[1])};
+    launch_after(emit_instances_kernel<KeyT, false>, prim_blocks, kPreprocessBlock, 0, stream,
+        prim.n_touched, prim.bounds, nullptr, prim.block_sums, prim.block_offsets, keys[0], inst.prims[0], n,
+        uint32_t(geo.grid_w), inst.capacity, status, clear_list(sc, plan, geo, tile_ranges));
     if (ev) cudaEventRecord(ev[0], stream);
     if (launches) *launches += 1;
-    static PerDeviceOnce configured;
-    err = configured.run([] { return cudaFuncSetAttribute(radix_scatter_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(scatter_smem_bytes<KeyT>())); });
+    const cudaError_t err = launch_radix_sort<KeyT>(tile_passes(plan), keys, inst.prims, sc.digit_hist, sc.rows, uint32_t(sc.row_stride), sc.groups, sc.tickets, inst, inst.sort_blocks_cap,
+                                                    status, sm_count, stream, launches);
     if (err != cudaSuccess) return err;
-    int cur = 0;
-    if (plan.n_passes > 0) {
-        PassTable passes{};
-        passes.n_passes = plan.n_passes;
-        for (int p = 0; p < plan.n_passes; ++p) { passes.shift[p] = plan.shift[p]; passes.bits[p] = plan.bits[p]; }
-        const uint32_t hist_grid = std::min<uint32_t>(inst.sort_blocks_cap ? inst.sort_blocks_cap : 1u, uint32_t(sm_count) * 8u);
-        launch_after(radix_histogram_all_kernel<KeyT>, hist_grid, 256, 0, stream, static_cast<const KeyT*>(inst.keys[0]), sc.digit_hist, status, inst.capacity, passes);
-        if (launches) *launches += 1;
-        for (int p = 0; p < plan.n_passes; ++p) {
-            KeyT* kin = static_cast<KeyT*>(inst.keys[cur]);
-            KeyT* kout = static_cast<KeyT*>(inst.keys[cur ^ 1]);
-            const size_t smem = scatter_smem_bytes<KeyT>(plan.bits[p]);
-            const uint32_t resident = uint32_t(std::min<size_t>(scatter_blocks_per_sm<KeyT>(), (227 * 1024) / (smem + 1024)));
-            const uint32_t scatter_grid = std::min<uint32_t>(inst.sort_blocks_cap ? inst.sort_blocks_cap : 1u, uint32_t(sm_count) * resident);
-            launch_after(radix_scatter_kernel<KeyT>, scatter_grid, kSortThreads, smem, stream,
-                kin, inst.prims[cur], kout, inst.prims[cur ^ 1], sc.digit_hist + size_t(p) * kMaxRadixBins, sc.rows[p],
-                uint32_t(sc.row_stride), sc.groups[p], sc.tickets + p, status, inst.capacity, plan.shift[p], plan.bits[p]);
-            cur ^= 1;
-            if (launches) *launches += 1;
-        }
-    }
     if (ev) cudaEventRecord(ev[1], stream);
-    launch_after(tile_ranges_kernel<KeyT>, uint32_t(sm_count), kOrderThreads, 0, stream, static_cast<const KeyT*>(inst.keys[cur]), tile_ranges, tile_order, status, inst.capacity,
-                                                                                uint32_t(geo.n_tiles));
+    launch_after(tile_ranges_kernel<KeyT>, uint32_t(sm_count), kOrderThreads, 0, stream, keys[plan.final_buffer], tile_ranges, tile_order, status, inst.capacity, uint32_t(geo.n_tiles));
+    if (ev) cudaEventRecord(ev[2], stream);
+    if (launches) *launches += 1;
+    return cudaGetLastError();
+}
+
+// GLOBAL_ORDERING: the lists are in order of depth, Gaussians of equal depth in order of their index.  The reference sorts the instances by 64-bit keys
+// of tile and depth (alpha_blend_global_ordering/inference.cu:40-110); a Gaussian's instances share its depth, so here the visible Gaussians are
+// sorted by depth, then their instances are emitted in that order and sorted by tile alone.  Both sorts are stable, so the lists are the same:
+// three or four passes over a sixth of the Gaussians and two over 16-bit keys take the place of five or six over 64-bit keys.
+// 1.5 M Gaussians, 980 x 545, 2.8 M instances, scan to ranges: 259 -> TODO us.
+//
+// The key buffers (8 bytes an instance, of which the sorts by tile need 2 or 4) hold everything in turn: keys[0] and keys[1] the depth keys and, in
+// their second halves, the Gaussians; the sorted list stays in one of them, the tile keys take both halves of the other.
+template <typename KeyT>
+cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst,
+                                    uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
+    const uint32_t n = uint32_t(scene.n_primitives);
+    const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
+    if (prim_blocks == 0 || inst.capacity == 0) return empty_ranges<KeyT>(geo, inst, tile_ranges, tile_order, status, stream, ev, launches);
+    const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap);
+    // The centres of visible Gaussians lie between the planes (preprocess.cu), so with a positive near plane the distance of their bits from those of
+    // the near plane is all that has to be sorted: 27 bits for 0.2 to 1000.  Otherwise all 32 bits, as the unsigned numbers that the reference's keys hold.
+    int32_t near_bits, far_bits;
+    std::memcpy(&near_bits, &view.near_plane, 4);
+    std::memcpy(&far_bits, &view.far_plane, 4);
+    const bool window = near_bits > 0 && far_bits >= near_bits && far_bits <= 0x7f800000;
+    PassTable depth{};
+    depth.n_passes = split_digits(window ? std::max(bit_length(uint32_t(far_bits - near_bits)), 1) : 32, depth.bits, depth.shift);
+    depth.visible = true;
+    uint32_t* depth_rows[4];
+    unsigned long long* depth_groups[4];
+    const size_t n_groups = (size_t(inst.sort_blocks_cap) + kGroup - 1) / kGroup;
+    for (int p = 0, at = 0; p < depth.n_passes; at += 1 << depth.bits[p], ++p) { depth_rows[p] = sc.depth_rows + at; depth_groups[p] = sc.depth_groups + n_groups * size_t(at); }
+    uint32_t* const depth_keys[2] = {static_cast<uint32_t*>(inst.keys[0]), static_cast<uint32_t*>(inst.keys[1])};
+    uint32_t* const depth_prims[2] = {depth_keys[0] + inst.capacity, depth_keys[1] + inst.capacity};
+    launch_after(list_visible_kernel, prim_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.eval, prim.block_offsets, depth_keys[0], depth_prims[0], n,
+                 window ? uint32_t(near_bits) : 0u, status, clear_list(sc, plan, geo, tile_ranges));
+    const uint32_t most_visible = std::min(n, inst.capacity), visible_blocks = (most_visible + kPreprocessBlock - 1) / kPreprocessBlock;
+    cudaError_t err = launch_radix_sort<uint32_t>(depth, depth_keys, depth_prims, sc.digit_hist + size_t(kFirstDepthPass) * kMaxRadixBins, depth_rows, uint32_t(sc.row_stride), depth_groups,
+                                                  sc.tickets + kFirstDepthPass, inst, (most_visible + kSortTile - 1) / kSortTile, status, sm_count, stream, launches);
+    if (err != cudaSuccess) return err;
+    const uint32_t* list = depth_prims[depth.n_passes & 1];
+    unsigned char* free_buffer = static_cast<unsigned char*>(inst.keys[(depth.n_passes & 1) ^ 1]);
+    KeyT* const keys[2] = {reinterpret_cast<KeyT*>(free_buffer), reinterpret_cast<KeyT*>(free_buffer + align16(size_t(inst.capacity) * 4))};
+    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, prim.block_sums, status);
+    launch_after(scan_block_sums_kernel<ScanOf::sorted>, 1, kScanThreads, 0, stream, prim.block_sums, prim.block_offsets, visible_blocks, inst.capacity, status);
+    launch_after(emit_instances_kernel<KeyT, true>, visible_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.bounds, list, prim.block_sums, prim.block_offsets, keys[0], inst.prims[0], n,
+                 uint32_t(geo.grid_w), inst.capacity, status, ClearList{});
+    if (launches) *launches += 4;
+    if (ev) cudaEventRecord(ev[0], stream);
+    if ((err = launch_radix_sort<KeyT>(tile_passes(plan), keys, inst.prims, sc.digit_hist, sc.rows, uint32_t(sc.row_stride), sc.groups, sc.tickets, inst, inst.sort_blocks_cap,
+                                       status, sm_count, stream, launches)) != cudaSuccess) return err;
+    if (ev) cudaEventRecord(ev[1], stream);
+    launch_after(tile_ranges_kernel<KeyT>, uint32_t(sm_count), kOrderThreads, 0, stream, keys[plan.final_buffer], tile_ranges, tile_order, status, inst.capacity, uint32_t(geo.n_tiles));
     if (ev) cudaEventRecord(ev[2], stream);
     if (launches) *launches += 1;
     return cudaGetLastError();
@@ -628,23 +778,30 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
 
 size_t sort_scratch_bytes(const SortPlan& plan, uint32_t sort_blocks_cap) { return carve_sort_scratch(nullptr, plan, sort_blocks_cap).bytes; }
 
-cudaError_t launch_scan_only(const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream) {
+cudaError_t launch_scan_only(int mode, const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream) {
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
-    launch_after(scan_block_sums_kernel, 1, kScanThreads, 0, stream, prim.block_sums, prim.block_offsets, prim_blocks, capacity, status);
+    const auto kernel = mode == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING ? scan_block_sums_kernel<ScanOf::visible> : scan_block_sums_kernel<ScanOf::instances>;
+    launch_after(kernel, 1, kScanThreads, 0, stream, prim.block_sums, prim.block_offsets, prim_blocks, capacity, status);
     return cudaGetLastError();
 }
 
-cudaError_t launch_emit_sort_ranges(int mode, const HtgsScene& scene, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim,
+cudaError_t launch_emit_sort_ranges(const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim,
                                     const InstBuffers& inst, uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream,
                                     cudaEvent_t* stage_events, uint32_t* launches) {
-    (void)mode;
     switch (plan.key_bytes) {
         case 2: return emit_sort_ranges_t<uint16_t>(scene, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
         case 4: return emit_sort_ranges_t<uint32_t>(scene, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
-        case 8: return emit_sort_ranges_t<uint64_t>(scene, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
+        case 8:
+            return plan.end_bit <= 32 + 16 ? emit_sort_ranges_global<uint16_t>(scene, view, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches)
+                                           : emit_sort_ranges_global<uint32_t>(scene, view, geo, plan, prim, inst, tile_ranges, tile_order, status, sm_count, stream, stage_events, launches);
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_global_keys(const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst, const uint2* tile_ranges, cudaStream_t stream) {
+    global_keys_kernel<<<uint32_t(geo.n_tiles), 256, 0, stream>>>(tile_ranges, inst.prims[plan.final_buffer], prim.eval, static_cast<unsigned long long*>(inst.keys[0]));
+    return cudaGetLastError();
 }
 
 }  // namespace htgs

@@ -50,12 +50,12 @@ struct PrimBuffers {
     PairRecord* pair;         // [N] (training only, else null)
     uint8_t* clamp;           // [N] bit c set: colour channel c was clamped at 0 (training only, else null)
     uint32_t* block_sums;     // [ceil(N/256)] instances emitted by each block of 256 Gaussians
-    uint32_t* block_offsets;  // [ceil(N/256)] exclusive prefix of block_sums
+    uint32_t* block_offsets;  // [ceil(N/256)] exclusive prefix of block_sums (GLOBAL_ORDERING: of the visible Gaussians per block)
     uint32_t* visible_list;   // [N] indices of the Gaussians that survived culling (first n_visible entries, unordered)
 };
 
 struct InstBuffers {
-    void* keys[2];            // ping-pong key buffers, `key_bytes` wide
+    void* keys[2];            // ping-pong key buffers, `key_bytes` wide (GLOBAL_ORDERING: see emit_sort_ranges_global)
     uint32_t* prims[2];       // ping-pong Gaussian indices
     void* sort_scratch;       // ticket counters, digit histograms and look-back words of the radix passes (sort_scratch_bytes)
     uint32_t capacity;        // instances the buffers can hold
@@ -68,9 +68,9 @@ constexpr int kMaxRadixBits = 9;
 constexpr int kMaxRadixBins = 1 << kMaxRadixBits;
 
 struct SortPlan {
-    int key_bytes;     // 2, 4, 8
-    int end_bit;       // bits to sort
-    int n_passes;
+    int key_bytes;     // of the reference's keys: 2, 4, 8 (tile in the upper, depth in the lower half: GLOBAL_ORDERING)
+    int end_bit;       // bits of them that are sorted
+    int n_passes;      // over the tile, of the instances
     int bits[8];       // digit width per pass
     int shift[8];      // digit position per pass
     int final_buffer;  // which ping-pong buffer holds the sorted result
@@ -92,12 +92,15 @@ cudaError_t launch_preprocess(int mode, bool train, const HtgsScene& scene, cons
 
 // binning.cu: scan of block sums, instance emission, stable radix sort, tile ranges.
 // Everything after the scan reads the instance count from `status` on the device.
-cudaError_t launch_scan_only(const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream);
+cudaError_t launch_scan_only(int mode, const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream);
 // `tile_order`: receives the tiles, long lists first (the blend kernels start them in this order).
 // `stage_events` (optional): events recorded after emission, after the sort and after the range kernel.
-cudaError_t launch_emit_sort_ranges(int mode, const HtgsScene& scene, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim,
+cudaError_t launch_emit_sort_ranges(const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim,
                                     const InstBuffers& inst, uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream,
                                     cudaEvent_t* stage_events = nullptr, uint32_t* launches = nullptr);
+
+// The reference's 64-bit keys of a finished GLOBAL_ORDERING frame, which the sort itself does not need, in inst.keys[0].
+cudaError_t launch_global_keys(const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst, const uint2* tile_ranges, cudaStream_t stream);
 
 // binning_unordered.cu: per-tile lists without sort keys (counting sort with atomics; the order inside a list is not
 // defined).  Writes `tile_ranges` and `prims_sorted`; expects `status->n_instances / overflow` from launch_scan_only.

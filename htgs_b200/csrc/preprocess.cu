@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kPreprocessBlock) preprocess_cull_kernel(
         #pragma unroll
         for (int i = 0; i < kPreprocessBlock / 32; ++i) { total += warp_sum[i]; total_vis += warp_vis[i]; }
         out.block_sums[blockIdx.x] = total;
+        if constexpr (MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING) out.block_offsets[blockIdx.x] = total_vis;      // the scan's input for this mode
         list_base = total_vis ? atomicAdd(&status->n_visible, total_vis) : 0u;
     }
     __syncthreads();

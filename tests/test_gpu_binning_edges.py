@@ -28,3 +28,31 @@ def test_sorted_instances_and_ranges(oracle_lib, mode, n, width, height, large):
     want = oracle_lib.bin_instances(got["n_touched"], got["bounds"].astype(np.uint32), got["grid_w"], got["n_tiles"], depth)
     assert info.n_instances == int(got["n_touched"].sum())
     assert np.array_equal(want["sorted_prims"], got["prims_sorted"]) and np.array_equal(want["ranges"], got["ranges"])
+
+
+@pytest.mark.parametrize("near,far", [(0.2, 100.0), (0.2, 3e38), (3.0, 3.0625), (0.0, 100.0), (-1.0, 100.0)])
+@pytest.mark.parametrize("n,width,height", [(1, 16, 16), (257, 16, 16), (5000, 250, 131), (9000, 4128, 4112)])
+def test_global_ordering_lists(oracle_lib, near, far, n, width, height):
+    # sorted by depth first and by tile then: windows of depth bits of one to four passes and none, ties in depth (every Gaussian twice,
+    # the copies far apart), one tile (no pass over it), and more than 65536 tiles
+    import torch
+    from htgs_b200.torch_bindings import _C
+    tb = harness.ours()
+    scene = scenes.tiny_scene(n=n, size=max(width, height), seed=n, mode=2, K=1, sh_degree=1)
+    half = n // 2
+    for a in (scene.positions, scene.scales, scene.rotations):
+        a[half:2 * half] = a[:half]
+    if far < 4.0:
+        scene.positions[:, 2] = near + (far - near) * np.random.default_rng(n).uniform(0.3, 0.7, n)
+        scene.scales[:] *= 1e-2
+    focal = float(max(width, height))
+    view = scenes.make_view(np.eye(4), width, height, focal, focal, width / 2.0, height / 2.0, near, far)
+    tb.rasterize(*harness.scene_tensors(scene), harness.settings_for(tb, scene, view, 2, 1), True, False)
+    torch.cuda.synchronize()
+    info = _C.last_frame_info
+    inter = harness.our_intermediates(0, n, info.n_instances)
+    ob = oracle_lib.bin_instances(inter["n_touched"], inter["bounds"].astype(np.uint32), inter["grid_w"], inter["n_tiles"], inter["eval"][:, 3, 3])
+    assert np.array_equal(ob["sorted_prims"], inter["prims_sorted"])
+    assert np.array_equal(ob["ranges"], inter["ranges"])
+    assert np.array_equal(ob["sorted_keys"], inter["keys_sorted"])
+    assert info.n_instances > 0 or near <= 0.0 or n == 1
