@@ -727,7 +727,8 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
 // 1.5 M Gaussians, 980 x 545, 2.8 M instances, scan to ranges: 259 -> 189 us (four passes of 7 bits; three of 9: 195).
 //
 // The key buffers (8 bytes an instance, of which the sorts by tile need 2 or 4) hold everything in turn: keys[0] and keys[1] the depth keys and, in
-// their second halves, the Gaussians; the sorted list stays in one of them, the tile keys take both halves of the other.
+// their second halves, the Gaussians; the sorted list stays in one of them, with the sums over its blocks in the first half, and the tile keys take both
+// halves of the other.  What the scan left in the per-Gaussian buffers is only read: htgs_forward_finish may be called again on them.
 template <typename KeyT>
 cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view, const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst,
                                     uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream, cudaEvent_t* ev, uint32_t* launches) {
@@ -750,7 +751,7 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
     const size_t n_groups = (size_t(inst.sort_blocks_cap) + kGroup - 1) / kGroup;
     for (int p = 0, at = 0; p < depth.n_passes; at += 1 << depth.bits[p], ++p) { depth_rows[p] = sc.depth_rows + at; depth_groups[p] = sc.depth_groups + n_groups * size_t(at); }
     uint32_t* const depth_keys[2] = {static_cast<uint32_t*>(inst.keys[0]), static_cast<uint32_t*>(inst.keys[1])};
-    uint32_t* const depth_prims[2] = {depth_keys[0] + inst.capacity, depth_keys[1] + inst.capacity};
+    uint32_t* const depth_prims[2] = {depth_keys[0] + inst.capacity + 4, depth_keys[1] + inst.capacity + 4};
     launch_after(list_visible_kernel, prim_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.eval, prim.block_offsets, depth_keys[0], depth_prims[0], n,
                  window ? uint32_t(near_bits) : 0u, status, clear_list(sc, plan, geo, tile_ranges));
     const uint32_t most_visible = std::min(n, inst.capacity), visible_blocks = (most_visible + kPreprocessBlock - 1) / kPreprocessBlock;
@@ -758,11 +759,13 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
                                                   sc.tickets + kFirstDepthPass, inst, (most_visible + kSortTile - 1) / kSortTile, status, sm_count, stream, launches);
     if (err != cudaSuccess) return err;
     const uint32_t* list = depth_prims[depth.n_passes & 1];
+    uint32_t* const sorted_sums = depth_keys[depth.n_passes & 1];       // the sorted depths have done their work: capacity + 4 words for two per 256 visible Gaussians
+    uint32_t* const sorted_offsets = sorted_sums + visible_blocks;
     unsigned char* free_buffer = static_cast<unsigned char*>(inst.keys[(depth.n_passes & 1) ^ 1]);
     KeyT* const keys[2] = {reinterpret_cast<KeyT*>(free_buffer), reinterpret_cast<KeyT*>(free_buffer + align16(size_t(inst.capacity) * 4))};
-    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, prim.block_sums, status);
-    launch_after(scan_block_sums_kernel<ScanOf::sorted>, 1, kScanThreads, 0, stream, prim.block_sums, prim.block_offsets, visible_blocks, inst.capacity, status);
-    launch_after(emit_instances_kernel<KeyT, true>, visible_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.bounds, list, prim.block_sums, prim.block_offsets, keys[0], inst.prims[0], n,
+    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, sorted_sums, status);
+    launch_after(scan_block_sums_kernel<ScanOf::sorted>, 1, kScanThreads, 0, stream, sorted_sums, sorted_offsets, visible_blocks, inst.capacity, status);
+    launch_after(emit_instances_kernel<KeyT, true>, visible_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.bounds, list, sorted_sums, sorted_offsets, keys[0], inst.prims[0], n,
                  uint32_t(geo.grid_w), inst.capacity, status, ClearList{});
     if (launches) *launches += 4;
     if (ev) cudaEventRecord(ev[0], stream);

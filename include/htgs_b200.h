@@ -98,7 +98,7 @@ typedef struct HtgsIntermediates {
     const void* cull_records;      /* [N] 32-byte records */
     const void* keys_unsorted;     /* [n_instances] keys in emission order (key_bytes wide) */
     const uint32_t* prims_unsorted;/* [n_instances] */
-    const void* keys_sorted;       /* [n_instances] (ALPHA_BLEND_GLOBAL_ORDERING: written by htgs_get_intermediates) */
+    const void* keys_sorted;       /* [n_instances] (ALPHA_BLEND_GLOBAL_ORDERING: written by htgs_get_intermediates, into the frame's workspace) */
     const uint32_t* prims_sorted;  /* [n_instances] Gaussian index per sorted instance */
     const uint32_t* tile_ranges;   /* [n_tiles,2] begin,end into the sorted arrays; (0,0) for empty tiles */
     uint32_t n_tiles;
