@@ -194,7 +194,8 @@ template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr size_t tc_bytes = has_tail ? 64 * 16 : 0;
     static constexpr size_t ta_off = tc_off + tc_bytes;
     static constexpr size_t ta_bytes = has_tail ? 64 * 4 : 0;
-    static constexpr size_t stage_off = (ta_off + ta_bytes + 15) & ~size_t(15);
+    static constexpr size_t zero_off = ta_off + ta_bytes;      // 16 bytes of zeros: the terms of a pair that is not accepted
+    static constexpr size_t stage_off = zero_off + 16;
     static constexpr size_t stage_bytes = kBwdThreads * ((ABS_GRAD ? 8 : 5) * 16 + 4 + (MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K ? 8 : 0)) + kBwdSegments * (4 + 1);
     static constexpr size_t core_off = (stage_off + stage_bytes + 15) & ~size_t(15);     // [NT][kBwdCoreRow] core entry of each (staged instance, pixel) pair
     static constexpr size_t core_bytes = has_core ? size_t(kBwdThreads) * kBwdCoreRow : 0;
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
             }
         }
     }
+    if (tid == 0) s_terms[SM::zero_off / 16] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     [[maybe_unused]] CameraCols cam;
     if constexpr (ABS_GRAD) cam = load_camera_cols(VPM);
     request_record(range.x + tid);
@@ -465,26 +467,25 @@ __global__ void __launch_bounds__(kBwdThreads, (BwdSmem<MODE, K, ABS_GRAD>::min_
                 r.rho2 = r.numerator * r.denominator_rcp;
                 if constexpr (kFirstK) {
                     r.ok = valid && r.terms != kNotCore;           // only stored fragments carry gradient (first_k backward.cuh:84-87)
-                    r.terms = r.ok ? r.terms : 0u;
                 } else {
                     r.ok = valid && r.rho2 < pos.z;
                     if (valid && !r.ok && !(r.rho2 > upper_level(pos.z))) r.ok = accepted_by_forward<MT>(eval + s_g[j], x0 + r.column, y0 + r.row);
                 }
                 return r;
             };
-            auto add = [&](Pair r) {                     // of a pair that is not accepted only zeros
-                const float G = r.ok ? exp_approx(-0.5f * r.rho2) : 0.0f;
+            // Of a pair that is not accepted only zeros, read as such: its pixel's gradient may be an infinity or a NaN, which times zero is a NaN.
+            auto add = [&](Pair r) {
                 if (!r.ok) r.rho2 = r.numerator = r.denominator_rcp = 0.0f;
+                const float G = exp_approx(-0.5f * r.rho2);
                 const float alpha = fminf(rgba.w * G, kMaxFragmentAlpha);
-                const float4 term = s_terms[r.terms * 64 + r.p];
+                const float4 term = s_terms[r.ok ? r.terms * 64 + r.p : uint32_t(SM::zero_off / 16)];
                 float dL_dalpha = term.w, scale = 1.0f;
                 if constexpr (SM::has_tail) {            // both, since in almost every step some lanes have the one and some the other
                     const float tail_dL_dalpha = term.w + dot(f3(rgba), f3(term)) + s_ta[r.p] * rcp_approx(fmaxf(1.0f - alpha, kOneMinusAlphaEps));
-                    const bool core = r.terms < uint32_t(SM::core_rows);
+                    const bool core = !r.ok || r.terms < uint32_t(SM::core_rows);
                     scale = core ? 1.0f : alpha;
                     dL_dalpha = core ? dL_dalpha : tail_dL_dalpha;
                 }
-                scale = r.ok ? scale : 0.0f;
                 aC_rg = fma2(low2(term), pack2(scale, scale), aC_rg);
                 aC_b = fmaf(term.z, scale, aC_b);
                 aC_opacity = fmaf(dL_dalpha, G, aC_opacity);
@@ -556,9 +557,9 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
 {
     using MT = ModeTraits<HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING>;
     constexpr uint32_t kTileX = MT::tile_w / 8, kTileY = MT::tile_h / 4;
-    __shared__ float4 s_pair[kGoChunk][33];              // [survivor][pixel]: weight, dL/dalpha * G, rho^2, 1 / D
+    __shared__ float4 s_pair[kGoChunk][33];              // [survivor][pixel]: weight, dL/dalpha * G, rho^2, 1 / D; zeros in the column behind the pixels
     __shared__ float4 s_q0[kGoChunk], s_q1[kGoChunk], s_q2[kGoChunk], s_rgba[kGoChunk], s_pos[kGoChunk];
-    __shared__ float4 s_grad[32];                        // dL/dpixel
+    __shared__ float4 s_grad[33];                        // dL/dpixel, and zeros
     __shared__ uint32_t s_g[kGoChunk], s_queue_prim[kGoQueue], s_queue_mask[kGoQueue];
     const uint32_t lane = threadIdx.x;
     const uint32_t tile = __ldg(tile_order + blockIdx.x / (kTileX * kTileY)), part = blockIdx.x % (kTileX * kTileY);
@@ -576,6 +577,8 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
         rgb_pixel = make_float3(__ldg(image + pixel_idx), __ldg(image + n_pixels + pixel_idx), __ldg(image + 2 * n_pixels + pixel_idx));
     }
     s_grad[lane] = make_float4(grad_pixel.x, grad_pixel.y, grad_pixel.z, 0.0f);
+    if (lane < kGoChunk) s_pair[lane][32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (lane == 0) s_grad[32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     [[maybe_unused]] CameraCols cam;
     if constexpr (ABS_GRAD) cam = load_camera_cols(VPM);
     float3 rgb_pixel_new = make_float3(0, 0, 0);
@@ -707,25 +710,23 @@ __global__ void __launch_bounds__(32) backward_global_kernel(
         float4 aC = make_float4(0, 0, 0, 0);
         [[maybe_unused]] float abs_grad = 0.0f;
         const uint32_t first_pixel = lane & 16u;
-        auto add = [&](uint32_t p, bool valid) {
+        auto add = [&](uint32_t p) {
             const float4 pair = s_pair[mine][p];
             const float4 grad = s_grad[p];
             const float y = offset_y + small_int_to_float(p >> 3), s = fmaf(shear, y, offset_x + small_int_to_float(p & 7u));
-            const float weight = valid ? pair.x : 0.0f, dL_dopacity = valid ? pair.y : 0.0f, rho2 = valid ? pair.z : 0.0f, denominator_rcp = valid ? pair.w : 0.0f;
-            aC.x = fmaf(weight, grad.x, aC.x); aC.y = fmaf(weight, grad.y, aC.y); aC.z = fmaf(weight, grad.z, aC.z);
-            aC.w += dL_dopacity;
-            const float dL_drho2 = -0.5f * opacity * dL_dopacity, u = dL_drho2 * denominator_rcp;
-            add_moments(moments, u, u * rho2, dL_drho2 * rho2, s, y);
+            aC.x = fmaf(pair.x, grad.x, aC.x); aC.y = fmaf(pair.x, grad.y, aC.y); aC.z = fmaf(pair.x, grad.z, aC.z);
+            aC.w += pair.y;
+            const float dL_drho2 = -0.5f * opacity * pair.y, u = dL_drho2 * pair.w;
+            add_moments(moments, u, u * pair.z, dL_drho2 * pair.z, s, y);
             if constexpr (ABS_GRAD) abs_grad += abs_position_gradient(af, u, s, y, x0 + small_int_to_float(p & 7u), y0 + small_int_to_float(p >> 3), cam);
         };
         while (pixels != 0) {
             const uint32_t p0 = first_pixel + uint32_t(__ffs(int(pixels)) - 1);
             pixels &= pixels - 1;
-            const bool second = pixels != 0;
-            const uint32_t p1 = second ? first_pixel + uint32_t(__ffs(int(pixels)) - 1) : p0;
+            const uint32_t p1 = pixels != 0 ? first_pixel + uint32_t(__ffs(int(pixels)) - 1) : 32u;
             pixels &= pixels - 1;
-            add(p0, true);
-            add(p1, second);
+            add(p0);
+            add(p1);
         }
         __syncwarp();
         auto both_halves = [](float4& v) {

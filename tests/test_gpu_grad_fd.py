@@ -78,3 +78,32 @@ def test_gradients_against_finite_differences(oracle_lib, mode, K):
             assert abs(fd - g[ix]) <= 0.02 * abs(fd) + 2e-7, f"{name}{ix}: finite difference {fd:.6e} vs gradient {g[ix]:.6e}"
             agreed += 1
     assert checked >= 20 and agreed >= (2 * checked) // 3, (checked, agreed, skipped)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows", [0, 3])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_bad_pixel_gradient_stays_with_the_gaussians_of_the_pixel(mode, rows, value):
+    # a NaN or an infinity in one pixel's gradient reaches the Gaussians that the pixel accepted and no other; those are the ones that
+    # have a gradient when only this pixel has one
+    import torch
+    tb = harness.ours()
+    scene = scenes.tiny_scene(n=2000, size=64, seed=5, mode=mode, K=8, sh_degree=1)
+
+    def gradients(grad_image):
+        leaves = [t.requires_grad_() for t in harness.scene_tensors(scene)]
+        densification = torch.zeros(rows, scene.n, 1, device="cuda") if rows else torch.empty(0, device="cuda")
+        tb.diff_rasterize(*leaves, densification, harness.settings_for(tb, scene, scene.views[0], mode, 8), False).backward(grad_image)
+        return torch.cat([t.grad.reshape(scene.n, -1) for t in leaves] + ([densification[1:].reshape(rows - 1, scene.n).T] if rows else []), dim=1)
+
+    generator = torch.Generator(device="cuda").manual_seed(1)
+    everywhere = torch.rand(3, 64, 64, device="cuda", generator=generator) + 0.5
+    for y, x in ((20, 37), (32, 32), (47, 24)):
+        only_here, without, bad = torch.zeros_like(everywhere), everywhere.clone(), everywhere.clone()
+        only_here[:, y, x], without[:, y, x], bad[:, y, x] = 1.0, 0.0, value
+        touched = (gradients(only_here) != 0).any(dim=1)
+        assert touched.any() and not touched.all()
+        got, want = gradients(bad), gradients(without)
+        assert torch.isfinite(got[~touched]).all() and not torch.isfinite(got[touched]).all()
+        # sums of one Gaussian over its pixels in another order: a few float32 roundings of the largest gradient
+        assert torch.allclose(got[~touched], want[~touched], rtol=1e-4, atol=1e-5 * float(want.abs().max()))
