@@ -68,6 +68,6 @@ def test_second_half_again(mode):
         image = torch.zeros(3, st.height, st.width, device="cuda")
         _native.check(lib.htgs_forward_finish(ctx, ctypes.byref(s), ctypes.byref(v), ctypes.byref(blobs), count.value, image.data_ptr(), stream,
                                               ctypes.byref(_native.HtgsFrameInfo())))
-        assert torch.equal(primitive, first)        # the first half's results are only read
+        assert torch.equal(primitive[64:], first[64:])        # behind the status at its head, the first half's results are only read
         images.append(image)
     assert float(images[0].max()) > 0.0 and torch.equal(images[0], images[1]) and torch.equal(images[0], images[2])
