@@ -164,6 +164,9 @@ struct HtgsContext {
     FrameGeometry last_geo{};
     uint32_t last_n_instances = 0;
     bool has_last = false;
+    // The 64-bit keys of a GLOBAL_ORDERING frame, which its sort does not need.  In a caller's workspace the frame itself writes them, since that memory
+    // may belong to somebody else once the call has returned; in the context's own they are made when somebody asks.
+    enum class GlobalKeys { none, to_be_made, written } last_keys = GlobalKeys::none;
     HtgsFrameInfo last_info{};
     // the frame whose status has not been read yet (htgs_render_async)
     PendingFrame pending{};
@@ -340,6 +343,10 @@ static int enqueue_frame(HtgsContext* ctx, PendingFrame& f) {
     const bool one_form = f.fast || (f.max_weights && (outline_mode == HTGS_MODE_HYBRID_BLEND || outline_mode == HTGS_MODE_OIT_BLEND));
     *launches += one_form ? 1 : 2;     // blend kernels are launched in two forms (blend.cu)
     if (prof) cudaEventRecord(ev[6], stream);
+    if (f.workspace && plan.key_bytes == 8) {
+        if ((err = launch_global_keys(geo, plan, L.prim, L.inst, L.tile_ranges, L.status, stream)) != cudaSuccess) return fail_cuda(err, "sort keys");
+        *launches += 1;
+    }
     if ((err = cudaMemcpyAsync(ctx->host_status, L.status, sizeof(FrameStatus), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return fail_cuda(err, "status copy");
     if ((err = cudaEventRecord(ctx->frame_done, stream)) != cudaSuccess) return fail_cuda(err, "frame event record");
     return HTGS_OK;
@@ -378,6 +385,7 @@ static int begin_frame(HtgsContext* ctx, const HtgsScene* scene, const HtgsView*
     if ((rc = settle_pending(ctx)) != HTGS_OK) return rc;
     PendingFrame& f = ctx->pending;
     f = PendingFrame{};
+    if (workspace == nullptr && ctx->last_keys == HtgsContext::GlobalKeys::to_be_made) ctx->last_keys = HtgsContext::GlobalKeys::none;     // the last frame's buffers are used again
     f.scene = *scene; f.view = *view;
     f.stream = static_cast<cudaStream_t>(stream_ptr);
     f.geo = make_geometry(view->mode, view->width, view->height);
@@ -423,6 +431,7 @@ static int finish_frame(HtgsContext* ctx, HtgsFrameInfo* info) {
         }
         const FrameStatus st = *ctx->host_status;
         ctx->last_layout = f.layout; ctx->last_plan = f.plan; ctx->last_geo = f.geo; ctx->last_n_instances = st.overflow ? 0 : st.n_instances; ctx->has_last = true;
+        ctx->last_keys = HtgsContext::GlobalKeys::none;
         const uint64_t needed_capacity = uint64_t(st.n_instances) + uint64_t(st.n_instances) / 4 + 4096;
         HtgsFrameInfo& li = ctx->last_info;
         li.n_instances = st.n_instances; li.n_visible = st.n_visible; li.key_bytes = uint32_t(f.plan.key_bytes);
@@ -433,7 +442,11 @@ static int finish_frame(HtgsContext* ctx, HtgsFrameInfo* info) {
         li.workspace_bytes = carve_frame(nullptr, f.scene.n_primitives, f.geo.n_tiles, f.plan, st.overflow ? needed_capacity : f.capacity, false).bytes;
         if (info) *info = li;
         if (st.error) { f.active = false; return fail(HTGS_ERR_DEVICE_FLAG, "a kernel reported an internal error (bounded wait gave up)"); }
-        if (!st.overflow) { f.active = false; return HTGS_OK; }
+        if (!st.overflow) {
+            f.active = false;
+            if (f.plan.key_bytes == 8) ctx->last_keys = internal ? HtgsContext::GlobalKeys::to_be_made : HtgsContext::GlobalKeys::written;
+            return HTGS_OK;
+        }
         f.active = false;
         if (st.n_instances == 0xffffffffu) return fail(HTGS_ERR_INVALID_ARGUMENT, "instance count does not fit 32 bits");
         if (!internal) return fail(HTGS_ERR_WORKSPACE_TOO_SMALL, "workspace too small for the instance buffers of this frame");
@@ -515,16 +528,15 @@ int htgs_get_intermediates(HtgsContext* ctx, HtgsIntermediates* out) {
     out->prims_unsorted = by_tile && p.n_passes <= 1 ? L.inst.prims[unsorted] : nullptr;
     out->keys_sorted = L.inst.keys[p.final_buffer];
     if (!by_tile) {
-        out->keys_sorted = L.inst.keys[0];
-        cudaPointerAttributes attributes{};
-        DeviceGuard guard(ctx->device);
-        cudaError_t err;
-        // a caller's workspace may be gone by now: pointers into it are handed out as before, but nothing is written
-        if (cudaPointerGetAttributes(&attributes, L.inst.keys[0]) != cudaSuccess || attributes.type == cudaMemoryTypeUnregistered) cudaGetLastError();
-        else if (ctx->last_n_instances > 0) {
-            if ((err = launch_global_keys(ctx->last_geo, p, L.prim, L.inst, L.tile_ranges, ctx->front_stream)) != cudaSuccess ||
+        if (ctx->last_keys == HtgsContext::GlobalKeys::to_be_made) {
+            DeviceGuard guard(ctx->device);
+            if (guard.status != cudaSuccess) return fail_cuda(guard.status, "cudaSetDevice");
+            cudaError_t err;
+            if ((err = launch_global_keys(ctx->last_geo, p, L.prim, L.inst, L.tile_ranges, L.status, ctx->front_stream)) != cudaSuccess ||
                 (err = cudaStreamSynchronize(ctx->front_stream)) != cudaSuccess) return fail_cuda(err, "sort keys of the last frame");
+            ctx->last_keys = HtgsContext::GlobalKeys::written;
         }
+        out->keys_sorted = ctx->last_keys == HtgsContext::GlobalKeys::written ? L.inst.keys[0] : nullptr;
     }
     out->prims_sorted = L.inst.prims[p.final_buffer];
     out->tile_ranges = reinterpret_cast<const uint32_t*>(L.tile_ranges);

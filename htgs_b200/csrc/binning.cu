@@ -641,7 +641,9 @@ __global__ void __launch_bounds__(kPreprocessBlock) sum_sorted_kernel(const uint
     block_sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(256) global_keys_kernel(const uint2* __restrict__ ranges, const uint32_t* __restrict__ prims, const EvalRecord* __restrict__ eval, unsigned long long* __restrict__ keys) {
+__global__ void __launch_bounds__(256) global_keys_kernel(const uint2* __restrict__ ranges, const uint32_t* __restrict__ prims, const EvalRecord* __restrict__ eval,
+                                                          unsigned long long* __restrict__ keys, const FrameStatus* __restrict__ status) {
+    if (status->overflow || status->error) return;
     const uint2 range = ranges[blockIdx.x];
     for (uint32_t i = range.x + threadIdx.x; i < range.y; i += 256) keys[i] = (static_cast<unsigned long long>(blockIdx.x) << 32) | __float_as_uint(eval[prims[i]].mt3.w);
 }
@@ -803,8 +805,9 @@ cudaError_t launch_emit_sort_ranges(const HtgsScene& scene, const HtgsView& view
     }
 }
 
-cudaError_t launch_global_keys(const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst, const uint2* tile_ranges, cudaStream_t stream) {
-    global_keys_kernel<<<uint32_t(geo.n_tiles), 256, 0, stream>>>(tile_ranges, inst.prims[plan.final_buffer], prim.eval, static_cast<unsigned long long*>(inst.keys[0]));
+cudaError_t launch_global_keys(const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst, const uint2* tile_ranges, const FrameStatus* status,
+                               cudaStream_t stream) {
+    global_keys_kernel<<<uint32_t(geo.n_tiles), 256, 0, stream>>>(tile_ranges, inst.prims[plan.final_buffer], prim.eval, static_cast<unsigned long long*>(inst.keys[0]), status);
     return cudaGetLastError();
 }
 

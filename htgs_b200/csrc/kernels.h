@@ -99,8 +99,9 @@ cudaError_t launch_emit_sort_ranges(const HtgsScene& scene, const HtgsView& view
                                     const InstBuffers& inst, uint2* tile_ranges, uint32_t* tile_order, FrameStatus* status, int sm_count, cudaStream_t stream,
                                     cudaEvent_t* stage_events = nullptr, uint32_t* launches = nullptr);
 
-// The reference's 64-bit keys of a finished GLOBAL_ORDERING frame, which the sort itself does not need, in inst.keys[0].
-cudaError_t launch_global_keys(const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst, const uint2* tile_ranges, cudaStream_t stream);
+// The reference's 64-bit keys of a GLOBAL_ORDERING frame, which the sort itself does not need, in inst.keys[0]; nothing if the frame ended with an error.
+cudaError_t launch_global_keys(const FrameGeometry& geo, const SortPlan& plan, const PrimBuffers& prim, const InstBuffers& inst, const uint2* tile_ranges, const FrameStatus* status,
+                               cudaStream_t stream);
 
 // binning_unordered.cu: per-tile lists without sort keys (counting sort with atomics; the order inside a list is not
 // defined).  Writes `tile_ranges` and `prims_sorted`; expects `status->n_instances / overflow` from launch_scan_only.

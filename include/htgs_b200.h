@@ -96,9 +96,10 @@ typedef struct HtgsIntermediates {
     const uint16_t* bounds;        /* [N,4] x_min,x_max,y_min,y_max in tiles (undefined where n_touched == 0) */
     const void* eval_records;      /* [N] 80-byte records: vpmt1, vpmt2, vpmt4, mt3, rgba (float4 each) */
     const void* cull_records;      /* [N] 32-byte records */
-    const void* keys_unsorted;     /* [n_instances] keys in emission order (key_bytes wide) */
-    const uint32_t* prims_unsorted;/* [n_instances] */
-    const void* keys_sorted;       /* [n_instances] (ALPHA_BLEND_GLOBAL_ORDERING: written by htgs_get_intermediates, into the frame's workspace) */
+    const void* keys_unsorted;     /* [n_instances] keys in emission order (key_bytes wide); NULL where the sort has overwritten them, as ALPHA_BLEND_GLOBAL_ORDERING always has */
+    const uint32_t* prims_unsorted;/* [n_instances]; NULL with keys_unsorted */
+    const void* keys_sorted;       /* [n_instances]; ALPHA_BLEND_GLOBAL_ORDERING, whose sort does without them: written by the frame into a caller's workspace, by
+                                      htgs_get_intermediates into the context's own; NULL if the frame did not end well */
     const uint32_t* prims_sorted;  /* [n_instances] Gaussian index per sorted instance */
     const uint32_t* tile_ranges;   /* [n_tiles,2] begin,end into the sorted arrays; (0,0) for empty tiles */
     uint32_t n_tiles;

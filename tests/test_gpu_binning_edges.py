@@ -56,3 +56,38 @@ def test_global_ordering_lists(oracle_lib, near, far, n, width, height):
     assert np.array_equal(ob["ranges"], inter["ranges"])
     assert np.array_equal(ob["sorted_keys"], inter["keys_sorted"])
     assert info.n_instances > 0 or near <= 0.0 or n == 1
+
+
+@pytest.mark.parametrize("own", [True, False])
+def test_global_ordering_keys_are_written_while_the_memory_is_the_frames(oracle_lib, own):
+    # the 64-bit keys of a frame, asked for twice; of a caller's workspace also after it went back to the allocator and another tensor has its
+    # memory: the call must not touch that
+    import ctypes
+    import torch
+    from htgs_b200 import _native
+    from htgs_b200.torch_bindings import _C
+    tb = harness.ours()
+    scene = scenes.tiny_scene(n=4000, size=200, seed=3, mode=2, K=1, sh_degree=1)
+    st = harness.settings_for(tb, scene, scene.views[0], 2, 1)
+    tensors = harness.scene_tensors(scene)
+    lib, ctx = _native.lib(), _native.context(0)
+    s, v = _C._scene_view(tensors, st.M, st.VPM, st.cam_position, 2, 1, st.active_sh_bases, st.width, st.height, st.near_plane, st.far_plane, 1.0)
+    image, depth = torch.empty(3, st.height, st.width, device="cuda"), torch.empty(st.height, st.width, device="cuda")
+    info = _native.HtgsFrameInfo()
+    workspace = None if own else torch.empty(lib.htgs_render_workspace_bytes(ctypes.byref(s), ctypes.byref(v), 1 << 18), dtype=torch.uint8, device="cuda")
+    _native.check(lib.htgs_render(ctx, ctypes.byref(s), ctypes.byref(v), image.data_ptr(), depth.data_ptr(), None, 1, 0, None if own else workspace.data_ptr(),
+                                  0 if own else workspace.numel(), torch.cuda.current_stream().cuda_stream, ctypes.byref(info)))
+    for _ in range(2):
+        got = harness.our_intermediates(0, scene.n, info.n_instances)
+        want = oracle_lib.bin_instances(got["n_touched"], got["bounds"].astype(np.uint32), got["grid_w"], got["n_tiles"], got["eval"][:, 3, 3])
+        assert info.n_instances > 1000 and np.array_equal(want["sorted_keys"], got["keys_sorted"]) and np.array_equal(want["sorted_prims"], got["prims_sorted"])
+    if not own:
+        size, address = workspace.numel(), workspace.data_ptr()
+        del workspace
+        other = torch.full((size,), 0x7f, dtype=torch.uint8, device="cuda")
+        assert other.data_ptr() == address
+        torch.cuda.synchronize()
+        inter = _native.HtgsIntermediates()
+        _native.check(lib.htgs_get_intermediates(ctx, ctypes.byref(inter)))
+        torch.cuda.synchronize()
+        assert address <= inter.keys_sorted < address + size and bool((other == 0x7f).all())
