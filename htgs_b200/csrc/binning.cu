@@ -600,6 +600,7 @@ __global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* 
     if (is_last) {
         __threadfence();
         order_tiles(ranges, order, n_tiles);
+        if (threadIdx.x == 0) status->range_blocks_done = 0;      // htgs_forward_finish may be called again on this status
     }
 }
 
