@@ -142,6 +142,13 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
     }
 }
 
+// What a sort sorts: the frame's instances, or its visible Gaussians (of which there are no more than instances).  No more than the buffers hold:
+// htgs_forward_finish may be given a smaller count than htgs_forward_begin counted, and its lists are cut then.
+__device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, uint32_t capacity, bool visible = false) {
+    const uint32_t n = visible ? status->n_visible : status->n_instances;
+    return status->overflow ? 0u : (n < capacity ? n : capacity);
+}
+
 // One block per 256 Gaussians (the blocks of the preprocess kernel), which writes their instances cooperatively: slot j belongs to
 // the Gaussian whose exclusive offset is the last one <= j (eight steps of search); inside a Gaussian the order is row-major over
 // its tile box (rasterization/src/shared_kernels.cu:21-28), so the emitted stream is identical to the reference's.  Bound by
@@ -149,8 +156,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
 // warp (five steps) where the warps have about equal work gave 51 and 504 us, always 88 and 715: one warp often has most of them.
 // The kernel also clears what the sort and the range kernel count in (`clear`): one launch instead of three.
 struct ClearList { uint4* begin[3]; uint64_t count[3]; uint64_t per_sort_block[3]; };   // 16-byte words: a fixed number, plus so many per sort block of the frame
-__device__ __forceinline__ void clear_words(const ClearList& clear, const FrameStatus* status) {
-    const uint64_t sort_blocks = status->overflow ? 0 : (uint64_t(status->n_instances) + kSortTile - 1) / kSortTile;
+__device__ __forceinline__ void clear_words(const ClearList& clear, const FrameStatus* status, uint32_t capacity) {
+    const uint64_t sort_blocks = (uint64_t(frame_instances(status, capacity)) + kSortTile - 1) / kSortTile;
     #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const uint64_t words = clear.count[c] + clear.per_sort_block[c] * sort_blocks;
@@ -166,8 +173,9 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
 {
     grid_dependency();
     const bool overflow = status->overflow;
-    if constexpr (!SORTED) clear_words(clear, status);
-    if (SORTED && blockIdx.x * kPreprocessBlock >= status->n_visible) return;
+    if constexpr (!SORTED) clear_words(clear, status, capacity);
+    const uint32_t n = SORTED ? frame_instances(status, capacity, true) : n_primitives;
+    if (SORTED && blockIdx.x * kPreprocessBlock >= n) return;
     const uint32_t total = block_sums[blockIdx.x];
     if (total == 0 || overflow) return;   // a frame that does not fit its instance buffers is skipped by every later stage
     __shared__ uint32_t excl[kPreprocessBlock];
@@ -176,7 +184,7 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t first = blockIdx.x * kPreprocessBlock;
     const uint32_t at = first + threadIdx.x;
-    const bool valid = at < (SORTED ? status->n_visible : n_primitives);
+    const bool valid = at < n;
     const uint32_t idx = SORTED ? (valid ? list[at] : 0u) : at;
     const uint32_t cnt = valid ? n_touched[idx] : 0u;
     if (cnt) {
@@ -214,12 +222,6 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
         for (uint32_t step = kPreprocessBlock / 2; step > 0; step >>= 1) if (excl[lo + step] <= j) lo += step;
         emit(j, j - excl[lo], lo);
     }
-}
-
-// What a sort sorts: the frame's instances, or its visible Gaussians (of which there are no more than instances).
-__device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, uint32_t capacity, bool visible = false) {
-    const uint32_t n = visible ? status->n_visible : status->n_instances;
-    return status->overflow ? 0u : (n < capacity ? n : capacity);
 }
 
 template <typename KeyT>
@@ -607,9 +609,9 @@ __global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* 
 // Visible Gaussians of a GLOBAL_ORDERING frame in index order, with the bits of their depth as keys: the input of the sort by depth.
 __global__ void __launch_bounds__(kPreprocessBlock) list_visible_kernel(const uint32_t* __restrict__ n_touched, const EvalRecord* __restrict__ eval, const uint32_t* __restrict__ visible_offsets,
                                                                         uint32_t* __restrict__ keys, uint32_t* __restrict__ prims, uint32_t n_primitives, uint32_t lowest_key,
-                                                                        const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear) {
+                                                                        uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear) {
     grid_dependency();
-    clear_words(clear, status);
+    clear_words(clear, status, capacity);
     if (status->overflow) return;
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
     const uint32_t idx = blockIdx.x * kPreprocessBlock + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -621,15 +623,16 @@ __global__ void __launch_bounds__(kPreprocessBlock) list_visible_kernel(const ui
     uint32_t at = visible_offsets[blockIdx.x] + __popc(ballot & lanemask_lt());
     #pragma unroll
     for (int w = 0; w < kPreprocessBlock / 32; ++w) if (w < int(warp)) at += warp_tot[w];
+    if (at >= capacity) return;
     keys[at] = __float_as_uint(eval[idx].mt3.w) - lowest_key;
     prims[at] = idx;
 }
 
 // Instances of every 256 of them, once they are in depth order.
 __global__ void __launch_bounds__(kPreprocessBlock) sum_sorted_kernel(const uint32_t* __restrict__ list, const uint32_t* __restrict__ n_touched, uint32_t* __restrict__ block_sums,
-                                                                      const FrameStatus* __restrict__ status) {
+                                                                      uint32_t capacity, const FrameStatus* __restrict__ status) {
     grid_dependency();
-    const uint32_t n = status->overflow ? 0u : status->n_visible, i = blockIdx.x * kPreprocessBlock + threadIdx.x;
+    const uint32_t n = frame_instances(status, capacity, true), i = blockIdx.x * kPreprocessBlock + threadIdx.x;
     if (blockIdx.x * kPreprocessBlock >= n) return;
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
     const uint32_t sum = __reduce_add_sync(0xffffffffu, i < n ? n_touched[list[i]] : 0u);
@@ -756,7 +759,7 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
     uint32_t* const depth_keys[2] = {static_cast<uint32_t*>(inst.keys[0]), static_cast<uint32_t*>(inst.keys[1])};
     uint32_t* const depth_prims[2] = {depth_keys[0] + inst.capacity + 4, depth_keys[1] + inst.capacity + 4};
     launch_after(list_visible_kernel, prim_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.eval, prim.block_offsets, depth_keys[0], depth_prims[0], n,
-                 window ? uint32_t(near_bits) : 0u, status, clear_list(sc, plan, geo, tile_ranges));
+                 window ? uint32_t(near_bits) : 0u, inst.capacity, status, clear_list(sc, plan, geo, tile_ranges));
     const uint32_t most_visible = std::min(n, inst.capacity), visible_blocks = (most_visible + kPreprocessBlock - 1) / kPreprocessBlock;
     cudaError_t err = launch_radix_sort<uint32_t>(depth, depth_keys, depth_prims, sc.digit_hist + size_t(kFirstDepthPass) * kMaxRadixBins, depth_rows, uint32_t(sc.row_stride), depth_groups,
                                                   sc.tickets + kFirstDepthPass, inst, (most_visible + kSortTile - 1) / kSortTile, status, sm_count, stream, launches);
@@ -766,7 +769,7 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
     uint32_t* const sorted_offsets = sorted_sums + visible_blocks;
     unsigned char* free_buffer = static_cast<unsigned char*>(inst.keys[(depth.n_passes & 1) ^ 1]);
     KeyT* const keys[2] = {reinterpret_cast<KeyT*>(free_buffer), reinterpret_cast<KeyT*>(free_buffer + align16(size_t(inst.capacity) * 4))};
-    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, sorted_sums, status);
+    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, sorted_sums, inst.capacity, status);
     launch_after(scan_block_sums_kernel<ScanOf::sorted>, 1, kScanThreads, 0, stream, sorted_sums, sorted_offsets, visible_blocks, inst.capacity, status);
     launch_after(emit_instances_kernel<KeyT, true>, visible_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.bounds, list, sorted_sums, sorted_offsets, keys[0], inst.prims[0], n,
                  uint32_t(geo.grid_w), inst.capacity, status, ClearList{});

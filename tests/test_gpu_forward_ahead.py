@@ -94,3 +94,20 @@ def test_second_half_again(mode):
         assert status == 0 and torch.equal(order.sort().values, torch.arange(len(order), dtype=torch.int32, device="cuda"))
         assert torch.equal(ranges, results[0][2]) and torch.equal(image, results[0][1])
     assert float(results[0][1].max()) > 0.0
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("share", [0.0, 0.3, 1.0])
+def test_second_half_with_a_smaller_count(mode, share):
+    # a count below that of the first half cuts the lists; nothing is written beyond the blob that belongs to that count, which may have room
+    # for fewer instances than there are visible Gaussians
+    import ctypes
+    import torch
+    *first, primitive, count, _alive = first_half(mode)
+    lib, _, _, v = first[:4]
+    fewer = max(int(count * share), 3)
+    size = lib.htgs_forward_instance_bytes(ctypes.byref(v), fewer)
+    room = torch.full((lib.htgs_forward_instance_bytes(ctypes.byref(v), 2 * count) + (1 << 20),), 0x5a, dtype=torch.uint8, device="cuda")
+    status, image, ranges, _order = second_half(*first, primitive, fewer, room[:size])
+    assert status == 0 and bool((room[size:] == 0x5a).all()) and bool(torch.isfinite(image).all())
+    assert int((ranges[:, 1] - ranges[:, 0]).sum()) == fewer and int(ranges.max()) == fewer
