@@ -143,10 +143,11 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
 }
 
 // What a sort sorts: the frame's instances, or its visible Gaussians (of which there are no more than instances).  No more than the buffers hold:
-// htgs_forward_finish may be given a smaller count than htgs_forward_begin counted, and its lists are cut then.
+// htgs_forward_finish may be given a smaller count than htgs_forward_begin counted, and its lists are cut then.  Nothing once a wait has given up:
+// the output of a pass that did not finish is not a list of valid indices.
 __device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, uint32_t capacity, bool visible = false) {
     const uint32_t n = visible ? status->n_visible : status->n_instances;
-    return status->overflow ? 0u : (n < capacity ? n : capacity);
+    return status->overflow || status->error ? 0u : (n < capacity ? n : capacity);
 }
 
 // One block per 256 Gaussians (the blocks of the preprocess kernel), which writes their instances cooperatively: slot j belongs to
@@ -612,7 +613,7 @@ __global__ void __launch_bounds__(kPreprocessBlock) list_visible_kernel(const ui
                                                                         uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear) {
     grid_dependency();
     clear_words(clear, status, capacity);
-    if (status->overflow) return;
+    if (status->overflow || status->error) return;
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
     const uint32_t idx = blockIdx.x * kPreprocessBlock + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const bool visible = idx < n_primitives && n_touched[idx] != 0;

@@ -111,3 +111,18 @@ def test_second_half_with_a_smaller_count(mode, share):
     status, image, ranges, _order = second_half(*first, primitive, fewer, room[:size])
     assert status == 0 and bool((room[size:] == 0x5a).all()) and bool(torch.isfinite(image).all())
     assert int((ranges[:, 1] - ranges[:, 0]).sum()) == fewer and int(ranges.max()) == fewer
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_second_half_after_an_error(mode):
+    # with the error flag set, as a wait that gave up leaves it, no list is read: every tile is empty, and the call says so
+    import torch
+    from htgs_b200 import _native
+    *first, primitive, count, _alive = first_half(mode)
+    primitive[12:16].view(torch.int32).fill_(2)
+    status, image, ranges, order = second_half(*first, primitive, count)
+    assert status == _native.HTGS_ERR_DEVICE_FLAG and not bool(ranges.any()) and not bool(image.any())
+    assert torch.equal(order.sort().values, torch.arange(len(order), dtype=torch.int32, device="cuda"))
+    primitive[12:16].view(torch.int32).fill_(0)
+    status, image, ranges, _order = second_half(*first, primitive, count)
+    assert status == 0 and bool(image.any()) and int(ranges.max()) == count
