@@ -109,7 +109,7 @@ static_assert(sizeof(FastRecord) == sizeof(EvalRecord), "FastRecord shares the s
 // quadratic in (s, y): y = pixel_y - cy, s = pixel_x - cx + shear * y.  Computed in float64: a rounding of a coefficient is the
 // same at every pixel and does not average out in a gradient that sums thousands of them.
 struct __align__(16) PairRecord {
-    float4 q0, q1, q2;        // coefficients of N and D side by side: q0 = those of 1 and s, q1 = y and ss, q2 = sy and yy
+    float4 n0, n1, d1;        // n0 = N: 1, s, y, ss   n1 = N: sy, yy, D: 1, s   d1 = D: y, ss, sy, yy   (N first: the chain rule reads only that)
     float cx, cy, shear, scale;     // scale: what N and D were multiplied by (1 / D at the centre)
 };
 static_assert(sizeof(PairRecord) == 64, "PairRecord must be 64 bytes");

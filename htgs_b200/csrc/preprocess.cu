@@ -223,9 +223,9 @@ __device__ __forceinline__ PairRecord make_pair_record(const float4& t1, const f
     // N and D grow with the fourth power of sizes in pixels: both are divided by D0
     const double scale = 1.0 / fmax(dot3(d0, d0), 1e-300);
     PairRecord r;
-    r.q0 = make_float4(float(scale * dot3(m0, m0)), float(scale * dot3(d0, d0)), float(2.0 * scale * dot3(m0, ms)), float(2.0 * scale * dot3(d0, ds)));
-    r.q1 = make_float4(float(2.0 * scale * dot3(m0, my)), float(2.0 * scale * dot3(d0, dy)), float(scale * dot3(ms, ms)), float(scale * dot3(ds, ds)));
-    r.q2 = make_float4(float(2.0 * scale * dot3(ms, my)), float(2.0 * scale * dot3(ds, dy)), float(scale * dot3(my, my)), float(scale * dot3(dy, dy)));
+    r.n0 = make_float4(float(scale * dot3(m0, m0)), float(2.0 * scale * dot3(m0, ms)), float(2.0 * scale * dot3(m0, my)), float(scale * dot3(ms, ms)));
+    r.n1 = make_float4(float(2.0 * scale * dot3(ms, my)), float(scale * dot3(my, my)), float(scale * dot3(d0, d0)), float(2.0 * scale * dot3(d0, ds)));
+    r.d1 = make_float4(float(2.0 * scale * dot3(d0, dy)), float(scale * dot3(ds, ds)), float(2.0 * scale * dot3(ds, dy)), float(scale * dot3(dy, dy)));
     r.cx = centre.x; r.cy = centre.y; r.shear = shear; r.scale = float(scale);
     return r;
 }
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kFinishBlock, finish_blocks_per_sm(TRAIN, FAST
                 out.clamp[gi] = clamp_bits;
                 const PairRecord pair = make_pair_record(t1, t2, t4, make_moment_centre<MODE>(t1, t2, t4, box));
                 float4* pdst = reinterpret_cast<float4*>(out.pair + gi);
-                pdst[0] = pair.q0; pdst[1] = pair.q1; pdst[2] = pair.q2; pdst[3] = make_float4(pair.cx, pair.cy, pair.shear, pair.scale);
+                pdst[0] = pair.n0; pdst[1] = pair.n1; pdst[2] = pair.d1; pdst[3] = make_float4(pair.cx, pair.cy, pair.shear, pair.scale);
             }
             if constexpr (FAST) {
                 // The fragment evaluation measures from the projected centre, the outline test from the centre of
