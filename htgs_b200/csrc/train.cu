@@ -205,7 +205,11 @@ template <int MODE, int K, bool ABS_GRAD> struct BwdSmem {
     static constexpr size_t core_off = (stage_off + stage_bytes + 15) & ~size_t(15);     // [NT][kBwdCoreRow] core entry of each (staged instance, pixel) pair
     static constexpr size_t core_bytes = has_core ? size_t(kBwdThreads) * kBwdCoreRow : 0;
     static constexpr size_t total = core_off + core_bytes;
-    static constexpr int max_blocks = 4;      // five spill the pair loop
+    // Five spill the pair loop, which pays only for OIT_BLEND, whose loop reads no buffer (1297 x 840, 1 and 3 M Gaussians: four blocks 291 and 428 us, five 280
+    // and 424; five with one pair per trip 283 and 430, four with one 300 and 444).  The bound of four spills up to 32 bytes in HYBRID_BLEND
+    // with absolute gradients and 20 with K = 32; one pair per trip, which spilled 4 and none, was slower in all of them (1 M Gaussians, absolute gradients, K = 2, 4,
+    // 8, 16, 32: 431, 422, 432, 444, 581 -> 396, 401, 399, 409, 501; K = 32 without: 478 -> 441).
+    static constexpr int max_blocks = MODE == HTGS_MODE_OIT_BLEND && !ABS_GRAD ? 5 : 4;
     static constexpr int min_blocks = int((227 * 1024) / (total + 1024)) < max_blocks ? int((227 * 1024) / (total + 1024)) : max_blocks;   // what the register budget is held to
 };
 
