@@ -356,6 +356,8 @@ __device__ __forceinline__ bool denominator_in_range(const float4& t1, const flo
 // inputs with two bulk copies, the record (in which the cull pass left position and opacity too) and the 16-byte aligned window around
 // its row of coefficients, and reads them from shared memory; strides of 80 and, at degree 3, 208 bytes spread the lanes over the
 // banks.  What bounds it now is DRAM (53 % of its throughput at 600 bytes in 64-byte pieces per Gaussian) and the latency of the float64 chains.
+// Where no coefficients are wanted (degree 0, importance weights) a lane loads its record itself: the copies' round trip through the mbarrier costs more than
+// five loads (16 k Gaussians: 5.5 us, by copies 6.4; 1 M 8.2 and 8.7, importance weights 7.6 and 8.2; 3 M 20.1 and 20.3).
 // Loads by lane -> copies, 3 M Gaussians, 1297 x 840: 88 -> 73 us, training 107 -> 88, relaxed precision 94 -> 79, 1.5 M in GLOBAL_ORDERING 82 -> 65.
 constexpr int kFinishBlock = 128;
 constexpr int kFinishWarps = kFinishBlock / 32;
@@ -384,6 +386,7 @@ __global__ void __launch_bounds__(kFinishBlock, finish_blocks_per_sm(TRAIN, FAST
     __syncwarp();
     unsigned char* my_window = smem + warp * (32u * (layout.window_stride + sizeof(EvalRecord))) + lane * layout.window_stride;
     float4* my_record = reinterpret_cast<float4*>(smem + warp * (32u * (layout.window_stride + sizeof(EvalRecord))) + 32u * layout.window_stride) + lane * 5u;
+    const bool staged = layout.window_bytes != 0;
     const uint32_t n_visible = status->n_visible;
     const float3 cam_position = make_float3(__ldg(cam_position_ptr), __ldg(cam_position_ptr + 1), __ldg(cam_position_ptr + 2));
     const size_t row_bytes = size_t(total_sh_bases) * 12u;
@@ -397,14 +400,19 @@ __global__ void __launch_bounds__(kFinishBlock, finish_blocks_per_sm(TRAIN, FAST
         float4* dst = reinterpret_cast<float4*>(out.eval + gi);
         // the window may reach beyond the ends of the tensor: at the first and last row, if these do not lie on 16-byte boundaries
         const uintptr_t row = sh_begin + size_t(gi) * row_bytes, window = row & ~uintptr_t(15);
-        const bool whole = valid && layout.window_bytes != 0 && window >= sh_begin && window + layout.window_bytes <= sh_end;
-        const uint32_t n_valid = __popc(__ballot_sync(0xffffffffu, valid)), n_whole = __popc(__ballot_sync(0xffffffffu, whole));
-        if (lane == 0) mbar_arrive_expect_tx(bar, n_valid * uint32_t(sizeof(EvalRecord)) + n_whole * layout.window_bytes);
-        __syncwarp();
-        if (valid) bulk_copy_g2s(my_record, dst, uint32_t(sizeof(EvalRecord)), bar);
-        if (whole) bulk_copy_g2s(my_window, reinterpret_cast<const void*>(window), layout.window_bytes, bar);
+        const bool whole = valid && staged && window >= sh_begin && window + layout.window_bytes <= sh_end;
+        float4 t1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), t2 = t1, t4 = t1, m3 = t1, centre_opacity = t1;
+        if (staged) {
+            const uint32_t n_valid = __popc(__ballot_sync(0xffffffffu, valid)), n_whole = __popc(__ballot_sync(0xffffffffu, whole));
+            if (lane == 0) mbar_arrive_expect_tx(bar, n_valid * uint32_t(sizeof(EvalRecord)) + n_whole * layout.window_bytes);
+            __syncwarp();
+            if (valid) bulk_copy_g2s(my_record, dst, uint32_t(sizeof(EvalRecord)), bar);
+            if (whole) bulk_copy_g2s(my_window, reinterpret_cast<const void*>(window), layout.window_bytes, bar);
+        } else if (valid) {
+            t1 = dst[0]; t2 = dst[1]; t4 = dst[2]; m3 = dst[3]; centre_opacity = dst[4];
+        }
         float* coefficients = reinterpret_cast<float*>(my_window + (row & 15u));
-        if (valid && !whole && layout.window_bytes != 0) {
+        if (valid && !whole && staged) {
             const float* from = sh_rest + size_t(gi) * size_t(total_sh_bases) * 3;
             for (int c = 0; c < 3 * (active_sh_bases - 1); ++c) coefficients[c] = __ldg(from + c);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // in front of the copy that the next round puts here
@@ -416,12 +424,14 @@ __global__ void __launch_bounds__(kFinishBlock, finish_blocks_per_sm(TRAIN, FAST
             if constexpr (!FAST) box = out.bounds[gi];
         }
         gi_next = i + step < n_visible ? out.visible_list[i + step] : 0u;
-        if (!mbar_wait_bounded(bar, parity)) {
-            atomicOr(&status->error, 1u);
-            return;
+        if (staged) {
+            if (!mbar_wait_bounded(bar, parity)) {
+                atomicOr(&status->error, 1u);
+                return;
+            }
+            if (valid) { t1 = my_record[0]; t2 = my_record[1]; t4 = my_record[2]; m3 = my_record[3]; centre_opacity = my_record[4]; }
         }
         if (valid) {
-            const float4 t1 = my_record[0], t2 = my_record[1], t4 = my_record[2], m3 = my_record[3], centre_opacity = my_record[4];
             const float3 position = f3(centre_opacity);
             const float opacity = centre_opacity.w;
             uint8_t clamp_bits = 0;
@@ -467,7 +477,7 @@ cudaError_t launch_t(const HtgsScene& scene, const HtgsView& view, const FrameGe
     if (err != cudaSuccess) return err;
     const FinishLayout layout = finish_layout(view.active_sh_bases, scene.sh_0 != nullptr);
     const uint32_t finish_blocks = min((n + kFinishBlock - 1) / kFinishBlock, uint32_t(sm_count_of_current_device()) * uint32_t(finish_blocks_per_sm(TRAIN, FAST)));
-    launch_after(preprocess_finish_kernel<MODE, TRAIN, FAST>, finish_blocks, kFinishBlock, size_t(kFinishBlock) * (layout.window_stride + sizeof(EvalRecord)), stream,
+    launch_after(preprocess_finish_kernel<MODE, TRAIN, FAST>, finish_blocks, kFinishBlock, layout.window_bytes != 0 ? size_t(kFinishBlock) * (layout.window_stride + sizeof(EvalRecord)) : 0, stream,
         scene.sh_0, scene.sh_rest, view.cam_position, prim, status, n, view.active_sh_bases, scene.total_sh_bases, outline_thresholds(outline_mode), layout);
     return cudaGetLastError();
 }
