@@ -382,6 +382,7 @@ __global__ void __launch_bounds__(kSortThreads, scatter_blocks_per_sm<KeyT>()) r
     const uint32_t n = frame_instances(status, capacity, visible);
     const uint32_t n_blocks = uint32_t((uint64_t(n) + kSortTile - 1) / kSortTile);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (n == 0) return;       // without a ticket: the others of a pass in which a wait gave up do not miss this block
 
     // exclusive prefix of the digit totals (same for every sort block)
     for (uint32_t d = threadIdx.x; d < n_bins; d += kSortThreads) digit_base[d] = digit_hist[d];
