@@ -278,7 +278,7 @@ __device__ __forceinline__ bool blend_block(
                     counts[i] = counts[i] && !stopped;
                 }
                 if (stopped) window = before & ((2u << stop_bit) - 1u);
-                if constexpr (STATS) { stat_trips += kPerTrip; stat_trips_inserting += __any_sync(0xffffffffu, enters) ? 1 : 0; stat_insertions += enters ? 1 : 0; }
+                if constexpr (STATS) { stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, enters) ? 1 : 0; stat_insertions += enters ? 1 : 0; }
                 float4 evicted = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (enters) {
                     const uint2 payload = make_uint2(__float_as_uint(in_alpha), s_word[in_j]);   // training: what the backward pass looks up

@@ -122,8 +122,8 @@ struct FrameStatus {
     unsigned int error;           // bounded waits that gave up, bad arguments seen on the device, ...
     unsigned long long candidate_pairs;     // statistics mode of the blend kernels
     unsigned long long accepted_fragments;  // statistics mode of the blend kernels
-    unsigned long long warp_trips;          // statistics mode, HYBRID_BLEND: warp-level evaluations of one candidate per lane
-    unsigned long long warp_trips_inserting;// ... of which at least one lane inserted into its K-buffer
+    unsigned long long warp_trips;          // statistics mode, HYBRID_BLEND: times a warp came to the insertion, behind two or three candidates per lane (K < 4 or a wide depth range: one)
+    unsigned long long warp_trips_inserting;// ... and at least one lane inserted into its K-buffer
     unsigned long long lane_insertions;     // ... and the lanes that inserted
     unsigned int range_blocks_done;         // blocks of the tile-range kernel that have finished; the last one orders the tiles
     unsigned int divide;                    // 1 if a visible Gaussian's |d|^2 may lie outside the range of reciprocal_rn

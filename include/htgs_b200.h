@@ -76,7 +76,7 @@ typedef struct HtgsFrameInfo {
     uint32_t n_instances;        /* (tile, Gaussian) instances */
     uint32_t n_visible;          /* Gaussians that passed culling */
     uint32_t key_bytes;          /* 2, 4 or 8: width of the sort key used */
-    uint32_t end_bit;            /* number of key bits that were sorted */
+    uint32_t end_bit;            /* number of key bits that the order goes by (ALPHA_BLEND_GLOBAL_ORDERING sorts depth and tile one after the other) */
     uint32_t reruns;             /* times the frame was re-run after growing the internal workspace */
     uint32_t device_error;       /* device-side error flags (0 = none) */
     uint32_t kernel_launches;    /* kernels of this library launched for the frame (re-runs included) */
@@ -84,8 +84,9 @@ typedef struct HtgsFrameInfo {
     uint64_t workspace_bytes;    /* bytes a caller-provided workspace must have for this frame */
     uint64_t candidate_pairs;    /* statistics mode only: (pixel, Gaussian) pairs that passed the outline test */
     uint64_t accepted_fragments; /* statistics mode only: fragments accepted by the exact test */
-    uint64_t warp_trips;           /* statistics mode, HYBRID_BLEND: warp-level evaluations of one candidate per lane */
-    uint64_t warp_trips_inserting; /* ... in which at least one lane inserted into its K-buffer */
+    uint64_t warp_trips;           /* statistics mode, HYBRID_BLEND: times a warp came to the insertion into its K-buffers, behind two or three candidates
+                                      per lane, of which one may enter (one candidate with K < 4 and where the planes are too far apart for 32-bit keys) */
+    uint64_t warp_trips_inserting; /* ... and at least one lane inserted */
     uint64_t lane_insertions;      /* ... and the number of lanes that inserted */
 } HtgsFrameInfo;
 

@@ -123,3 +123,29 @@ def test_buffer_filled_to_the_last_entry(mode, K, order):
                 want = render(scene, scene.views[0], mode, K, 0.2, 3e38, median)
                 assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
                 assert got[0].max() > 0.0
+
+
+@pytest.mark.parametrize("far", [100.0, 3e38])
+@pytest.mark.parametrize("K", [4, 8, 16, 32])
+def test_statistics_of_a_buffer_that_every_candidate_enters(K, far):
+    # K Gaussians that every pixel accepts: every time a warp comes to the insertion all of its lanes insert, whatever form the buffer has
+    import torch
+    from htgs_b200 import _native
+    from htgs_b200.torch_bindings import _C
+    scene = scenes.tiny_scene(n=K, size=64, seed=K, mode=0, K=K, sh_degree=1)
+    depth = np.linspace(4.0, 2.0, K)
+    scene.positions[:] = 0.0
+    scene.positions[:, 2] = depth
+    scene.scales[:] = depth[:, None]
+    scene.scales[:, 2] = 1e-3
+    scene.rotations[:] = np.array([1.0, 0.0, 0.0, 0.0], dtype=np.float32)
+    scene.opacities[:] = 0.5
+    lib, ctx = _native.lib(), _native.context(0)
+    lib.htgs_set_collect_stats(ctx, 1)
+    try:
+        image, _ = render(scene, scene.views[0], 0, K, 0.2, far, False)
+        info = _C.last_frame_info
+    finally:
+        lib.htgs_set_collect_stats(ctx, 0)
+    assert image.min() > 0.0 and info.accepted_fragments == info.lane_insertions == K * 64 * 64
+    assert info.warp_trips == info.warp_trips_inserting == K * 64 * 64 // 32
