@@ -82,8 +82,8 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v) {
 constexpr int kScanThreads = 1024;
 constexpr int kScanRun = 16;            // values per thread and round: 16384 block sums (4.2 M Gaussians) per round
 // instances: the above.  visible (GLOBAL_ORDERING): adds up the instances, and makes the blocks' visible Gaussians, which lie where the offsets
-// go, into their prefix.  sorted (the same mode, after the sort by depth): the prefix over blocks of 256 visible Gaussians, nothing is published.
-enum class ScanOf { instances, visible, sorted };
+// go, into their prefix.
+enum class ScanOf { instances, visible };
 template <ScanOf OF>
 __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uint32_t* __restrict__ block_sums, uint32_t* block_offsets,
                                                                      uint32_t n_blocks, uint32_t capacity, FrameStatus* status) {
@@ -93,7 +93,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
     [[maybe_unused]] __shared__ unsigned long long instances_s;
     if (threadIdx.x == 0) { carry_s = 0ull; instances_s = 0ull; }
     [[maybe_unused]] unsigned long long instances = 0;
-    if constexpr (OF == ScanOf::sorted) n_blocks = min(n_blocks, (status->n_visible + kPreprocessBlock - 1) / kPreprocessBlock);
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t base = 0; base < n_blocks; base += kScanThreads * kScanRun) {
@@ -135,7 +134,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
         if (lane == 0) atomicAdd(&instances_s, instances);
         __syncthreads();
     }
-    if (OF != ScanOf::sorted && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
         const unsigned long long total = OF == ScanOf::visible ? instances_s : carry_s;
         status->n_instances = total > 0xffffffffull ? 0xffffffffu : uint32_t(total);
         status->overflow = total > (unsigned long long)capacity ? 1u : 0u;
@@ -165,11 +164,13 @@ __device__ __forceinline__ void clear_words(const ClearList& clear, const FrameS
         for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < words; i += uint64_t(gridDim.x) * blockDim.x) clear.begin[c][i] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
-// SORTED (GLOBAL_ORDERING): the blocks are those of the visible Gaussians in depth order, `list`; what has to be cleared has been by then.
+// SORTED (GLOBAL_ORDERING): the blocks are those of the visible Gaussians in depth order, `list`; what has to be cleared has been by then.  A block adds up
+// the blocks in front of it, of `block_sums` those of its group of 256 and of `group_sums` whole groups, which takes the place of a scan kernel.
+constexpr uint32_t kSumGroup = kPreprocessBlock;
 template <typename KeyT, bool SORTED>
 __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     const uint32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds, const uint32_t* __restrict__ list,
-    const uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ block_offsets, KeyT* __restrict__ keys, uint32_t* __restrict__ prims,
+    const uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ block_offsets, const uint32_t* __restrict__ group_sums, KeyT* __restrict__ keys, uint32_t* __restrict__ prims,
     uint32_t n_primitives, uint32_t grid_w, uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear)
 {
     grid_dependency();
@@ -182,7 +183,15 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     __shared__ uint32_t excl[kPreprocessBlock];
     __shared__ uint4 box[kPreprocessBlock];          // x_min | y_min << 16, width, reciprocal of the width (2^32 / width, rounded up; 0: divide), Gaussian
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
+    [[maybe_unused]] __shared__ uint32_t warp_before[kPreprocessBlock / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if constexpr (SORTED) {
+        const uint32_t group = blockIdx.x / kSumGroup, in_group = blockIdx.x % kSumGroup;
+        uint32_t before = threadIdx.x < in_group ? block_sums[blockIdx.x - in_group + threadIdx.x] : 0u;
+        for (uint32_t i = threadIdx.x; i < group; i += kPreprocessBlock) before += group_sums[i];
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) warp_before[warp] = before;
+    }
     const uint32_t first = blockIdx.x * kPreprocessBlock;
     const uint32_t at = first + threadIdx.x;
     const bool valid = at < n;
@@ -199,10 +208,12 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     if (lane == 31) warp_tot[warp] = inc;
     __syncthreads();
     uint32_t warp_base = 0;
+    uint64_t base = SORTED ? 0u : block_offsets[blockIdx.x];
     #pragma unroll
-    for (int w = 0; w < kPreprocessBlock / 32; ++w)
+    for (int w = 0; w < kPreprocessBlock / 32; ++w) {
         if (w < int(warp)) warp_base += warp_tot[w];
-    const uint64_t base = block_offsets[blockIdx.x];
+        if constexpr (SORTED) base += warp_before[w];
+    }
     auto emit = [&](uint32_t slot, uint32_t local, uint32_t owner) {
         const uint4 b = box[owner];
         const uint32_t ly = b.y == 1u ? local : b.z ? __umulhi(local, b.z) : local / b.y;
@@ -246,18 +257,20 @@ constexpr uint32_t kLookbackPolls = 1u << 20;      // about half a second of pol
 constexpr uint32_t kGroup = 32;                    // sort blocks per group
 constexpr int kLookbackBatch = 8;                  // words read per step
 
-constexpr int kDepthRowWords = 1024;     // of the sort by depth: at most 4 passes of 8 bits
+constexpr int kMostDepthWords = 3 << kMaxRadixBits;     // of the sort by depth: three passes of 9 bits, or four of at most 8
 constexpr int kFirstDepthPass = 4;       // its place in tickets and digit_hist; there are at most four passes over the tile
 struct SortScratch {
-    unsigned long long* depth_groups;    // GLOBAL_ORDERING, the sort by depth: [groups][kDepthRowWords], all passes
+    unsigned long long* depth_groups;    // GLOBAL_ORDERING, the sort by depth: [groups][depth_words], all passes
     uint32_t* depth_rows;                // [sort_blocks_cap][row_stride]
+    uint32_t* group_sums;                // instances of every kSumGroup blocks of the emission
     uint32_t* tickets;                   // [16]
     uint32_t* digit_hist;                // [8][kMaxRadixBins]
     unsigned long long* groups[8];       // per pass [ceil(sort_blocks_cap / kGroup)][1 << bits]
     uint32_t* rows[8];                   // [sort_blocks_cap][row_stride]: the passes' counts of a sort block lie behind one another
     size_t fixed_bytes, row_stride, bytes;
 };
-__host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32_t sort_blocks_cap) {
+// depth_words: words per sort block that the passes over the depth take (0 in the other modes)
+__host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32_t sort_blocks_cap, size_t depth_words) {
     SortScratch sc{};
     unsigned char* p = static_cast<unsigned char*>(base);
     size_t off = 0;
@@ -268,9 +281,10 @@ __host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32
         sc.groups[i] = reinterpret_cast<unsigned long long*>(p + off);
         off += (n_groups << plan.bits[i]) * sizeof(unsigned long long);
     }
-    const bool by_depth = plan.key_bytes == 8;
     sc.depth_groups = reinterpret_cast<unsigned long long*>(p + off);
-    if (by_depth) off += n_groups * kDepthRowWords * sizeof(unsigned long long);
+    off += n_groups * depth_words * sizeof(unsigned long long);
+    sc.group_sums = reinterpret_cast<uint32_t*>(p + off);
+    if (depth_words > 0) off += (size_t(sort_blocks_cap) * (kSortTile / kPreprocessBlock) / kSumGroup + 1) * sizeof(uint32_t);
     off = (off + 15) & ~size_t(15);
     sc.fixed_bytes = off;
     for (int i = 0; i < plan.n_passes; ++i) {
@@ -278,7 +292,7 @@ __host__ SortScratch carve_sort_scratch(void* base, const SortPlan& plan, uint32
         sc.row_stride += size_t(1) << plan.bits[i];
     }
     sc.depth_rows = reinterpret_cast<uint32_t*>(p + off) + sc.row_stride;
-    if (by_depth) sc.row_stride += kDepthRowWords;
+    sc.row_stride += depth_words;
     sc.row_stride = (sc.row_stride + 3) & ~size_t(3);
     sc.bytes = off + size_t(sort_blocks_cap) * sc.row_stride * sizeof(uint32_t);
     return sc;
@@ -630,9 +644,9 @@ __global__ void __launch_bounds__(kPreprocessBlock) list_visible_kernel(const ui
     prims[at] = idx;
 }
 
-// Instances of every 256 of them, once they are in depth order.
+// Instances of every 256 of them, once they are in depth order, and of every 256 such blocks.
 __global__ void __launch_bounds__(kPreprocessBlock) sum_sorted_kernel(const uint32_t* __restrict__ list, const uint32_t* __restrict__ n_touched, uint32_t* __restrict__ block_sums,
-                                                                      uint32_t capacity, const FrameStatus* __restrict__ status) {
+                                                                      uint32_t* __restrict__ group_sums, uint32_t capacity, const FrameStatus* __restrict__ status) {
     grid_dependency();
     const uint32_t n = frame_instances(status, capacity, true), i = blockIdx.x * kPreprocessBlock + threadIdx.x;
     if (blockIdx.x * kPreprocessBlock >= n) return;
@@ -645,6 +659,7 @@ __global__ void __launch_bounds__(kPreprocessBlock) sum_sorted_kernel(const uint
     #pragma unroll
     for (int w = 0; w < kPreprocessBlock / 32; ++w) total += warp_tot[w];
     block_sums[blockIdx.x] = total;
+    atomicAdd(group_sums + blockIdx.x / kSumGroup, total);
 }
 
 __global__ void __launch_bounds__(256) global_keys_kernel(const uint2* __restrict__ ranges, const uint32_t* __restrict__ prims, const EvalRecord* __restrict__ eval,
@@ -682,14 +697,13 @@ PassTable tile_passes(const SortPlan& plan) {
     return t;
 }
 
-ClearList clear_list(const SortScratch& sc, const SortPlan& plan, const FrameGeometry& geo, uint2* tile_ranges) {
+ClearList clear_list(const SortScratch& sc, const FrameGeometry& geo, uint2* tile_ranges) {
     ClearList clear{};      // the buffers are 256-byte aligned and padded to 256 bytes
     clear.begin[0] = reinterpret_cast<uint4*>(tile_ranges); clear.count[0] = (uint64_t(geo.n_tiles) + 1) / 2;
     if (sc.row_stride > 0) {
         clear.begin[1] = reinterpret_cast<uint4*>(sc.tickets); clear.count[1] = sc.fixed_bytes / 16;
         clear.begin[2] = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(sc.tickets) + sc.fixed_bytes); clear.per_sort_block[2] = sc.row_stride / 4;
     }
-    (void)plan;
     return clear;
 }
 
@@ -711,11 +725,11 @@ cudaError_t emit_sort_ranges_t(const HtgsScene& scene, const FrameGeometry& geo,
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
     if (prim_blocks == 0 || inst.capacity == 0) return empty_ranges<KeyT>(geo, inst, tile_ranges, tile_order, status, stream, ev, launches);
-    const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap);
+    const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap, 0);
     KeyT* const keys[2] = {static_cast<KeyT*>(inst.keys[0]), static_cast<KeyT*>(inst.keys[1])};
     launch_after(emit_instances_kernel<KeyT, false>, prim_blocks, kPreprocessBlock, 0, stream,
-        prim.n_touched, prim.bounds, nullptr, prim.block_sums, prim.block_offsets, keys[0], inst.prims[0], n,
-        uint32_t(geo.grid_w), inst.capacity, status, clear_list(sc, plan, geo, tile_ranges));
+        prim.n_touched, prim.bounds, nullptr, prim.block_sums, prim.block_offsets, nullptr, keys[0], inst.prims[0], n,
+        uint32_t(geo.grid_w), inst.capacity, status, clear_list(sc, geo, tile_ranges));
     if (ev) cudaEventRecord(ev[0], stream);
     if (launches) *launches += 1;
     const cudaError_t err = launch_radix_sort<KeyT>(tile_passes(plan), keys, inst.prims, sc.digit_hist, sc.rows, uint32_t(sc.row_stride), sc.groups, sc.tickets, inst, inst.sort_blocks_cap,
@@ -743,7 +757,6 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
     const uint32_t n = uint32_t(scene.n_primitives);
     const uint32_t prim_blocks = (n + kPreprocessBlock - 1) / kPreprocessBlock;
     if (prim_blocks == 0 || inst.capacity == 0) return empty_ranges<KeyT>(geo, inst, tile_ranges, tile_order, status, stream, ev, launches);
-    const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap);
     // The centres of visible Gaussians lie between the planes (preprocess.cu), so with a positive near plane the distance of their bits from those of
     // the near plane is all that has to be sorted: 27 bits for 0.2 to 1000.  Otherwise all 32 bits, as the unsigned numbers that the reference's keys hold.
     int32_t near_bits, far_bits;
@@ -752,8 +765,15 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
     const bool window = near_bits > 0 && far_bits >= near_bits && far_bits <= 0x7f800000;
     PassTable depth{};
     const int depth_bits = window ? std::max(bit_length(uint32_t(far_bits - near_bits)), 1) : 32;
-    depth.n_passes = split_digits(depth_bits, depth.bits, depth.shift, depth_bits <= 28 ? 7 : 8);      // four passes of 7 bits: 103 us, three of 9: 114
+    // Digits: the fewest passes while a pass is mostly latency, shorter digits, whose look-back and ranking are cheaper per sort block, once the sort
+    // blocks fill the GPU.  27 bits, three passes of 9 against four of 7 (kernels alone): 16 k Gaussians 31 us against 37, 400 k 42 / 47, 1 M (166 k visible) 51 / 54,
+    // 3 M 74 / 74, 1.5 M (628 k visible) 114 / 103, 8 M 95 / 83.  How many are visible the host does not know.
+    const uint32_t most_visible = std::min(n, inst.capacity), visible_blocks = (most_visible + kPreprocessBlock - 1) / kPreprocessBlock;
+    depth.n_passes = split_digits(depth_bits, depth.bits, depth.shift, most_visible <= (1u << 19) ? kMaxRadixBits : depth_bits <= 28 ? 7 : 8);
     depth.visible = true;
+    size_t depth_words = 0;
+    for (int p = 0; p < depth.n_passes; ++p) depth_words += size_t(1) << depth.bits[p];
+    const SortScratch sc = carve_sort_scratch(inst.sort_scratch, plan, inst.sort_blocks_cap, depth_words);
     uint32_t* depth_rows[4];
     unsigned long long* depth_groups[4];
     const size_t n_groups = (size_t(inst.sort_blocks_cap) + kGroup - 1) / kGroup;
@@ -761,21 +781,18 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
     uint32_t* const depth_keys[2] = {static_cast<uint32_t*>(inst.keys[0]), static_cast<uint32_t*>(inst.keys[1])};
     uint32_t* const depth_prims[2] = {depth_keys[0] + inst.capacity + 4, depth_keys[1] + inst.capacity + 4};
     launch_after(list_visible_kernel, prim_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.eval, prim.block_offsets, depth_keys[0], depth_prims[0], n,
-                 window ? uint32_t(near_bits) : 0u, inst.capacity, status, clear_list(sc, plan, geo, tile_ranges));
-    const uint32_t most_visible = std::min(n, inst.capacity), visible_blocks = (most_visible + kPreprocessBlock - 1) / kPreprocessBlock;
+                 window ? uint32_t(near_bits) : 0u, inst.capacity, status, clear_list(sc, geo, tile_ranges));
     cudaError_t err = launch_radix_sort<uint32_t>(depth, depth_keys, depth_prims, sc.digit_hist + size_t(kFirstDepthPass) * kMaxRadixBins, depth_rows, uint32_t(sc.row_stride), depth_groups,
                                                   sc.tickets + kFirstDepthPass, inst, (most_visible + kSortTile - 1) / kSortTile, status, sm_count, stream, launches);
     if (err != cudaSuccess) return err;
     const uint32_t* list = depth_prims[depth.n_passes & 1];
-    uint32_t* const sorted_sums = depth_keys[depth.n_passes & 1];       // the sorted depths have done their work: capacity + 4 words for two per 256 visible Gaussians
-    uint32_t* const sorted_offsets = sorted_sums + visible_blocks;
+    uint32_t* const sorted_sums = depth_keys[depth.n_passes & 1];       // the sorted depths have done their work: capacity + 4 words for one per 256 visible Gaussians
     unsigned char* free_buffer = static_cast<unsigned char*>(inst.keys[(depth.n_passes & 1) ^ 1]);
     KeyT* const keys[2] = {reinterpret_cast<KeyT*>(free_buffer), reinterpret_cast<KeyT*>(free_buffer + align16(size_t(inst.capacity) * 4))};
-    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, sorted_sums, inst.capacity, status);
-    launch_after(scan_block_sums_kernel<ScanOf::sorted>, 1, kScanThreads, 0, stream, sorted_sums, sorted_offsets, visible_blocks, inst.capacity, status);
-    launch_after(emit_instances_kernel<KeyT, true>, visible_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.bounds, list, sorted_sums, sorted_offsets, keys[0], inst.prims[0], n,
+    launch_after(sum_sorted_kernel, visible_blocks, kPreprocessBlock, 0, stream, list, prim.n_touched, sorted_sums, sc.group_sums, inst.capacity, status);
+    launch_after(emit_instances_kernel<KeyT, true>, visible_blocks, kPreprocessBlock, 0, stream, prim.n_touched, prim.bounds, list, sorted_sums, nullptr, sc.group_sums, keys[0], inst.prims[0], n,
                  uint32_t(geo.grid_w), inst.capacity, status, ClearList{});
-    if (launches) *launches += 4;
+    if (launches) *launches += 3;
     if (ev) cudaEventRecord(ev[0], stream);
     if ((err = launch_radix_sort<KeyT>(tile_passes(plan), keys, inst.prims, sc.digit_hist, sc.rows, uint32_t(sc.row_stride), sc.groups, sc.tickets, inst, inst.sort_blocks_cap,
                                        status, sm_count, stream, launches)) != cudaSuccess) return err;
@@ -788,7 +805,7 @@ cudaError_t emit_sort_ranges_global(const HtgsScene& scene, const HtgsView& view
 
 }  // namespace
 
-size_t sort_scratch_bytes(const SortPlan& plan, uint32_t sort_blocks_cap) { return carve_sort_scratch(nullptr, plan, sort_blocks_cap).bytes; }
+size_t sort_scratch_bytes(const SortPlan& plan, uint32_t sort_blocks_cap) { return carve_sort_scratch(nullptr, plan, sort_blocks_cap, plan.key_bytes == 8 ? kMostDepthWords : 0).bytes; }
 
 cudaError_t launch_scan_only(int mode, const HtgsScene& scene, const PrimBuffers& prim, uint32_t capacity, FrameStatus* status, cudaStream_t stream) {
     const uint32_t n = uint32_t(scene.n_primitives);
