@@ -144,9 +144,11 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const uin
 // What a sort sorts: the frame's instances, or its visible Gaussians (of which there are no more than instances).  No more than the buffers hold:
 // htgs_forward_finish may be given a smaller count than htgs_forward_begin counted, and its lists are cut then.  Nothing once a wait has given up:
 // the output of a pass that did not finish is not a list of valid indices.
+// One load: kernels of a few microseconds wait for this first (a load per member, the second only if the first was zero: list_visible_kernel 47 -> 56 us at
+// 8 M Gaussians).
 __device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, uint32_t capacity, bool visible = false) {
-    const uint32_t n = visible ? status->n_visible : status->n_instances;
-    return status->overflow || status->error ? 0u : (n < capacity ? n : capacity);
+    const uint4 head = *reinterpret_cast<const uint4*>(status);        // n_instances, overflow, n_visible, error
+    return (head.y | head.w) != 0 ? 0u : min(visible ? head.z : head.x, capacity);
 }
 
 // One block per 256 Gaussians (the blocks of the preprocess kernel), which writes their instances cooperatively: slot j belongs to
@@ -156,8 +158,8 @@ __device__ __forceinline__ uint32_t frame_instances(const FrameStatus* status, u
 // warp (five steps) where the warps have about equal work gave 51 and 504 us, always 88 and 715: one warp often has most of them.
 // The kernel also clears what the sort and the range kernel count in (`clear`): one launch instead of three.
 struct ClearList { uint4* begin[3]; uint64_t count[3]; uint64_t per_sort_block[3]; };   // 16-byte words: a fixed number, plus so many per sort block of the frame
-__device__ __forceinline__ void clear_words(const ClearList& clear, const FrameStatus* status, uint32_t capacity) {
-    const uint64_t sort_blocks = (uint64_t(frame_instances(status, capacity)) + kSortTile - 1) / kSortTile;
+__device__ __forceinline__ void clear_words(const ClearList& clear, uint32_t instances) {
+    const uint64_t sort_blocks = (uint64_t(instances) + kSortTile - 1) / kSortTile;
     #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const uint64_t words = clear.count[c] + clear.per_sort_block[c] * sort_blocks;
@@ -174,12 +176,11 @@ __global__ void __launch_bounds__(kPreprocessBlock) emit_instances_kernel(
     uint32_t n_primitives, uint32_t grid_w, uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear)
 {
     grid_dependency();
-    const bool overflow = status->overflow;
-    if constexpr (!SORTED) clear_words(clear, status, capacity);
-    const uint32_t n = SORTED ? frame_instances(status, capacity, true) : n_primitives;
+    const uint32_t frame = frame_instances(status, capacity, SORTED), n = SORTED ? frame : n_primitives;
+    if constexpr (!SORTED) clear_words(clear, frame);
     if (SORTED && blockIdx.x * kPreprocessBlock >= n) return;
     const uint32_t total = block_sums[blockIdx.x];
-    if (total == 0 || overflow) return;   // a frame that does not fit its instance buffers is skipped by every later stage
+    if (total == 0 || frame == 0) return;   // a frame that does not fit its instance buffers is skipped by every later stage
     __shared__ uint32_t excl[kPreprocessBlock];
     __shared__ uint4 box[kPreprocessBlock];          // x_min | y_min << 16, width, reciprocal of the width (2^32 / width, rounded up; 0: divide), Gaussian
     __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
@@ -372,7 +373,7 @@ __device__ __forceinline__ void block_exclusive_scan_512(uint32_t* vals, uint32_
 // tile, which is staged in shared memory (over the masks) and written out as runs.  The Gaussian indices are requested after
 // the ranking, so that they do not hold registers before.
 // Bound by the latency of a block's phases and their barriers.  7.3 M keys of 16 bits, both passes: 189 -> 123 us; 154 M keys of
-// 32 bits: 3.86 -> 2.78 ms; 2.8 M keys of 64 bits, five passes: 294 -> 236 us.  Six blocks per SM instead of four change nothing.
+// 32 bits: 3.86 -> 2.78 ms.  Six blocks per SM instead of four change nothing.
 template <typename KeyT> constexpr int scatter_blocks_per_sm() { return sizeof(KeyT) == 4 ? 5 : 4; }
 template <typename KeyT>
 __global__ void __launch_bounds__(kSortThreads, scatter_blocks_per_sm<KeyT>()) radix_scatter_kernel(
@@ -584,7 +585,7 @@ template <typename KeyT>
 __global__ void __launch_bounds__(kOrderThreads) tile_ranges_kernel(const KeyT* __restrict__ keys, uint2* __restrict__ ranges, uint32_t* __restrict__ order,
                                                                     FrameStatus* status, uint32_t capacity, uint32_t n_tiles) {
     grid_dependency();
-    constexpr uint32_t kRangeRun = 16 / sizeof(KeyT);            // 8 / 4 / 2 keys per 16-byte load
+    constexpr uint32_t kRangeRun = 16 / sizeof(KeyT);            // 8 or 4 keys per 16-byte load
     const uint32_t n = frame_instances(status, capacity);
     const uint32_t n_runs = (n + kRangeRun - 1) / kRangeRun;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_runs; r += gridDim.x * blockDim.x) {
@@ -627,11 +628,12 @@ __global__ void __launch_bounds__(kPreprocessBlock) list_visible_kernel(const ui
                                                                         uint32_t* __restrict__ keys, uint32_t* __restrict__ prims, uint32_t n_primitives, uint32_t lowest_key,
                                                                         uint32_t capacity, const FrameStatus* __restrict__ status, const __grid_constant__ ClearList clear) {
     grid_dependency();
-    clear_words(clear, status, capacity);
-    if (status->overflow || status->error) return;
-    __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
     const uint32_t idx = blockIdx.x * kPreprocessBlock + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const bool visible = idx < n_primitives && n_touched[idx] != 0;
+    const uint32_t instances = frame_instances(status, capacity);
+    clear_words(clear, instances);
+    if (instances == 0) return;
+    __shared__ uint32_t warp_tot[kPreprocessBlock / 32];
     const uint32_t ballot = __ballot_sync(0xffffffffu, visible);
     if (lane == 0) warp_tot[warp] = __popc(ballot);
     __syncthreads();

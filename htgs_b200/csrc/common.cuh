@@ -115,7 +115,7 @@ struct __align__(16) PairRecord {
 static_assert(sizeof(PairRecord) == 64, "PairRecord must be 64 bytes");
 
 // Device-resident frame status, copied to the host at the end of a call.
-struct FrameStatus {
+struct __align__(16) FrameStatus {      // its first four words are read with one load
     unsigned int n_instances;     // total (tile, Gaussian) instances of the frame
     unsigned int overflow;        // 1 if n_instances exceeded the instance capacity of the workspace
     unsigned int n_visible;       // Gaussians that survived culling
