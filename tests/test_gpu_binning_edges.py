@@ -30,28 +30,23 @@ def test_sorted_instances_and_ranges(oracle_lib, mode, n, width, height, large):
     assert np.array_equal(want["sorted_prims"], got["prims_sorted"]) and np.array_equal(want["ranges"], got["ranges"])
 
 
-ULP = 2.0 ** -22        # of float32 between 2 and 4
-
-
-@pytest.mark.parametrize("near,far", [(0.2, 100.0), (0.2, 3e38), (3.0, 3.0625), (3.0, 3.0 + 16000 * ULP), (3.0, 3.0 + 200 * ULP), (3.0, 3.0 + 100 * ULP), (3.0, 3.0 + ULP), (3.0, 3.0),
-                                      (0.0, 100.0), (-1.0, 100.0)])
+@pytest.mark.parametrize("near,far", [(0.2, 100.0), (0.2, 3e38), (3.0, 3.0625), (0.0, 100.0), (-1.0, 100.0)])
 @pytest.mark.parametrize("n,width,height", [(1, 16, 16), (257, 16, 16), (5000, 250, 131), (9000, 4128, 4112)])
 def test_global_ordering_lists(oracle_lib, near, far, n, width, height):
-    # sorted by depth first and by tile then: windows of 27, 31, 19, 14, 8, 7 and one bits of depth (of none: the same depth for all) and all 32 bits, ties in depth
-    # (every Gaussian twice, the copies far apart), one tile (no pass over it), and more than 65536 tiles
+    # sorted by depth first and by tile then: windows of depth bits of one to four passes and none, ties in depth (every Gaussian twice,
+    # the copies far apart), one tile (no pass over it), and more than 65536 tiles
     import torch
     from htgs_b200.torch_bindings import _C
     tb = harness.ours()
     scene = scenes.tiny_scene(n=n, size=max(width, height), seed=n, mode=2, K=1, sh_degree=1)
-    narrow = 0.0 < near and far < 4.0
-    if narrow:
-        scene.positions[:, 2] = near + ULP * np.random.default_rng(n).integers(0, round((far - near) / ULP) + 1, n)
     half = n // 2
     for a in (scene.positions, scene.scales, scene.rotations):
         a[half:2 * half] = a[:half]
+    if far < 4.0:
+        scene.positions[:, 2] = near + (far - near) * np.random.default_rng(n).uniform(0.3, 0.7, n)
+        scene.scales[:] *= 1e-2
     focal = float(max(width, height))
-    view = scenes.make_view(np.eye(4), width, height, focal, focal, width / 2.0, height / 2.0, *((0.2, 100.0) if narrow else (near, far)))
-    view.near_plane, view.far_plane = near, far           # of the centres; the matrix's planes, for the extents, are wide apart
+    view = scenes.make_view(np.eye(4), width, height, focal, focal, width / 2.0, height / 2.0, near, far)
     tb.rasterize(*harness.scene_tensors(scene), harness.settings_for(tb, scene, view, 2, 1), True, False)
     torch.cuda.synchronize()
     info = _C.last_frame_info
@@ -61,7 +56,37 @@ def test_global_ordering_lists(oracle_lib, near, far, n, width, height):
     assert np.array_equal(ob["ranges"], inter["ranges"])
     assert np.array_equal(ob["sorted_keys"], inter["keys_sorted"])
     assert info.n_instances > 0 or near <= 0.0 or n == 1
-    if narrow and n > 1:
+
+
+ULP = 2.0 ** -22        # of float32 between 2 and 4
+
+
+@pytest.mark.parametrize("far", [3.0625, 3.0 + 16000 * ULP, 3.0 + 200 * ULP, 3.0 + 100 * ULP, 3.0 + ULP, 3.0])
+@pytest.mark.parametrize("n,width,height", [(1, 16, 16), (257, 16, 16), (5000, 250, 131), (9000, 4128, 4112)])
+def test_global_ordering_narrow_windows(oracle_lib, far, n, width, height):
+    # windows of 19, 14, 8, 7 and one bits of depth (of none: the same depth for all), so that the sort takes three passes to one, with the ties in depth of
+    # every Gaussian twice, the copies far apart
+    import torch
+    from htgs_b200.torch_bindings import _C
+    tb = harness.ours()
+    scene = scenes.tiny_scene(n=n, size=max(width, height), seed=n, mode=2, K=1, sh_degree=1)
+    near = 3.0
+    scene.positions[:, 2] = near + ULP * np.random.default_rng(n).integers(0, round((far - near) / ULP) + 1, n)
+    half = n // 2
+    for a in (scene.positions, scene.scales, scene.rotations):
+        a[half:2 * half] = a[:half]
+    focal = float(max(width, height))
+    view = scenes.make_view(np.eye(4), width, height, focal, focal, width / 2.0, height / 2.0, 0.2, 100.0)
+    view.near_plane, view.far_plane = near, far           # of the centres; the matrix's planes, for the extents, are wide apart
+    tb.rasterize(*harness.scene_tensors(scene), harness.settings_for(tb, scene, view, 2, 1), True, False)
+    torch.cuda.synchronize()
+    info = _C.last_frame_info
+    inter = harness.our_intermediates(0, n, info.n_instances)
+    ob = oracle_lib.bin_instances(inter["n_touched"], inter["bounds"].astype(np.uint32), inter["grid_w"], inter["n_tiles"], inter["eval"][:, 3, 3])
+    assert np.array_equal(ob["sorted_prims"], inter["prims_sorted"])
+    assert np.array_equal(ob["ranges"], inter["ranges"])
+    assert np.array_equal(ob["sorted_keys"], inter["keys_sorted"])
+    if n > 1:
         depths = inter["eval"][inter["n_touched"] != 0, 3, 3]
         assert len(np.unique(depths)) < len(depths) and depths.min() >= near and depths.max() <= far
 

@@ -43,6 +43,36 @@ def test_views_above_and_below_the_guess(mode):
     assert float(want[1][0].max()) > 0.0 and not float(want[3][0].abs().max()) > 0.0
 
 
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_second_half_again(mode):
+    # htgs_forward_finish reads the per-Gaussian blob that htgs_forward_begin filled: it may be called on it any number of times
+    import ctypes
+    import torch
+    from htgs_b200 import _native
+    from htgs_b200.torch_bindings import _C
+    scene = scenes.tiny_scene(n=3000, size=256, seed=11, mode=mode, K=8, sh_degree=1)
+    tensors = harness.scene_tensors(scene)
+    st = harness.settings_for(harness.ours(), scene, scene.views[0], mode, 8)
+    lib, ctx, stream = _native.lib(), _native.context(0), torch.cuda.current_stream().cuda_stream
+    s, v = _C._scene_view(tensors, st.M, st.VPM, st.cam_position, mode, 8, st.active_sh_bases, st.width, st.height, st.near_plane, st.far_plane, 1.0)
+    sizes = [ctypes.c_size_t() for _ in range(3)]
+    _native.check(lib.htgs_forward_blob_sizes(ctypes.byref(s), ctypes.byref(v), *(ctypes.byref(x) for x in sizes)))
+    primitive, tile, pixel = (torch.empty(x.value, dtype=torch.uint8, device="cuda") for x in sizes)
+    count = ctypes.c_uint32()
+    _native.check(lib.htgs_forward_begin(ctx, ctypes.byref(s), ctypes.byref(v), primitive.data_ptr(), primitive.numel(), stream, ctypes.byref(count)))
+    instance = torch.empty(lib.htgs_forward_instance_bytes(ctypes.byref(v), count.value), dtype=torch.uint8, device="cuda")
+    blobs = _native.HtgsTrainBlobs(*(x for t in (primitive, tile, instance, pixel) for x in (t.data_ptr(), t.numel())))
+    first = primitive.clone()
+    images = []
+    for _ in range(3):
+        image = torch.zeros(3, st.height, st.width, device="cuda")
+        _native.check(lib.htgs_forward_finish(ctx, ctypes.byref(s), ctypes.byref(v), ctypes.byref(blobs), count.value, image.data_ptr(), stream,
+                                              ctypes.byref(_native.HtgsFrameInfo())))
+        assert torch.equal(primitive[64:], first[64:])        # behind the status at its head, the first half's results are only read
+        images.append(image)
+    assert float(images[0].max()) > 0.0 and torch.equal(images[0], images[1]) and torch.equal(images[0], images[2])
+
+
 def first_half(mode):
     """A scene's training forward up to the instance count: (library, context, scene, view, blob sizes, per-Gaussian blob, count, what has to stay alive)."""
     import ctypes
@@ -82,7 +112,7 @@ def second_half(lib, ctx, s, v, sizes, primitive, count, instance=None):
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2, 3])
-def test_second_half_again(mode):
+def test_second_half_with_other_blobs(mode):
     # htgs_forward_finish leaves the per-Gaussian blob that htgs_forward_begin filled as it was: it may be called on it any number of times, with
     # other blobs for what it writes (an order of the tiles that is missing leaves only tile 0)
     import torch
