@@ -712,7 +712,7 @@ def main():
         "insertion_chain": None if (fast or scene.mode != 0 or not infos[:, 6].mean()) else {
             "warp_trips": float(infos[:, 6].mean()), "share_of_trips_with_an_insertion": float(infos[:, 7].mean() / infos[:, 6].mean()),
             "inserting_lanes_per_such_trip": float(infos[:, 8].mean() / max(infos[:, 7].mean(), 1.0)),
-            "note": "a trip evaluates two candidates per lane (K = 32: three), of which one may enter the K-buffer; the insertion sits behind a per-lane branch, so a warp runs it only when one of its lanes inserts"},
+            "note": "a trip evaluates two candidates per lane (K = 32: three; K < 8: one), of which one may enter the K-buffer; the insertion sits behind a per-lane branch, so a warp runs it only when one of its lanes inserts"},
         "algorithmic": {"pairs": pairs, "accepted_fragments": acc, "candidate_pairs": cand, "flops": blend_flops,
                         "formula": "pairs*54 + accepted*(60+7K), the reference algorithm's work (every pixel of a tile tests every instance of the tile)"},
     }

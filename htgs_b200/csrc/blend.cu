@@ -58,9 +58,16 @@ template <int K, Buffer BUFFER> struct CoreOf { using type = SortedCore<K, 32>; 
 template <int K> struct CoreOf<K, Buffer::keys> { using type = UnsortedCore<K, 32, false>; };
 template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = UnsortedCore<K, 32, true>; };
 // HYBRID_BLEND with the unsorted buffer: candidates that a lane evaluates per trip, of which one may enter the buffer.  With K = 32 the 14 warps
-// that shared memory leaves have registers for a third one, which hides more latency than its repeated evaluations cost; with K = 16 the
-// registers do not suffice (1297 x 840, 3 M Gaussians: two 803 us, three 857; 4K, K = 32: two 29.9 ms, three 28.7, four 31.5).
+// that shared memory leaves have registers for a third one, which hides more latency than its repeated evaluations cost where lists are long and opaque: 4 M
+// Gaussians in dense clusters, 1920 x 1080, two 9.79 ms, three 9.27 (elsewhere two are up to 4 % faster: 3 M, 1297 x 840, 622 and 647 us).
+// With smaller buffers three cost 5 % at K = 4 and 8 and 7 at 16.
 constexpr int candidates_per_trip(int K) { return K >= 32 ? 3 : 2; }
+// Whether one insertion serves a trip.  With four entries in dense clusters few candidates enter, and what a trip decides costs more than the insertions (blend at 4 M as
+// above: 6.09 ms with an insertion per candidate, 6.35 with one per trip; 3 M, 1297 x 840: 346 and 342 us).  With eight, 6.93 and 6.73 ms, 401 and 383 us.
+template <typename SL> constexpr bool merges_insertions(int K) { return SL::Core::unsorted && (K >= 8 || SL::Core::keeps_colour); }
+// Whether entries are appended while there are empty places: its branch costs smaller buffers more than the shorter insertion saves (K = 8, as above: 6.82 ms and
+// 387 us with it, 6.73 and 383 without; K = 16: 7.25 and 414 with it, 7.28 and 424 without), but not where a grid is resident at once (256 x 256: 166 and 170 us).
+template <typename SL> constexpr bool appends_to_empty_places(int K) { return K >= 16 || SL::Core::keeps_colour; }
 struct NoCore { static constexpr bool keeps_colour = false, unsorted = false; static constexpr size_t smem_bytes = 0; };
 
 template <int MODE, int K, Buffer BUFFER, BlendTask TASK> struct SmemLayout {
@@ -111,7 +118,8 @@ __device__ __forceinline__ bool blend_block(
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
-    constexpr bool kMerged = kHybrid && SL::Core::unsorted;
+    constexpr bool kMerged = kHybrid && merges_insertions<SL>(K);
+    constexpr bool kAppends = appends_to_empty_places<SL>(K);
     constexpr int kPerTrip = candidates_per_trip(K);
     constexpr uint32_t kTileX = MT::tile_w / kBlockW, kTileY = MT::tile_h / kBlockH;     // blocks per binning tile
     EvalRecord* s_record = reinterpret_cast<EvalRecord*>(smem + SL::record_off);
@@ -285,12 +293,12 @@ __device__ __forceinline__ bool blend_block(
                     // what falls out is a fragment, or nothing (alpha 0; its colour does not matter)
                     if constexpr (SL::Core::keeps_colour) {
                         float3 rgb = f3(reinterpret_cast<const float4*>(s_record + in_j)[4]);
-                        core.insert(in_depth, payload, last, rgb);
+                        core.template insert<kAppends>(in_depth, payload, last, rgb);
                         evicted = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(last.x));
                     } else {
-                        if (!core.insert(in_depth, payload, last, last_rgb)) last_rgb = colour_of(last.y);
+                        if (!core.template insert<kAppends>(in_depth, payload, last, last_rgb)) last_rgb = colour_of(last.y);
                         evicted = make_float4(last_rgb.x, last_rgb.y, last_rgb.z, __uint_as_float(last.x));
-                        if (core.last(last)) last_rgb = colour_of(last.y);
+                        if (!(kAppends && core.filling()) && core.last(last)) last_rgb = colour_of(last.y);
                     }
                 }
                 #pragma unroll
@@ -301,9 +309,12 @@ __device__ __forceinline__ bool blend_block(
                     }
                 }
             } else if constexpr (kHybrid) {
-                // Two candidates per trip, as above; the buffer and tail updates happen strictly in list order.
-                auto commit = [&](float depth, float alpha, uint32_t j) {
-                    const float4 rgba = reinterpret_cast<const float4*>(s_record + j)[4];
+                // Two candidates per trip, as above; the buffer and tail updates happen strictly in list order.  The colour is loaded ahead where registers
+                // allow (K = 4, frames: 6.17 -> 6.09 ms in dense clusters; K = 2, whose chain is in registers, 303 -> 313 us, training at K = 4 1 % slower).
+                constexpr bool kColourAhead = SL::Core::unsorted && !TRAIN;
+                auto colour_at = [&](uint32_t j) { return reinterpret_cast<const float4*>(s_record + j)[4]; };
+                auto commit = [&](float depth, float alpha, uint32_t j, float4 rgba) {
+                    if constexpr (!kColourAhead) rgba = colour_at(j);
                     float4 frag = make_float4(rgba.x, rgba.y, rgba.z, alpha);
                     if (depth < core.limit() && alpha >= MT::min_alpha_core) {
                         const float limit = core.limit();
@@ -320,16 +331,18 @@ __device__ __forceinline__ bool blend_block(
                 float depth0, depth1, alpha0, alpha1;
                 const bool ok0 = evaluate(v0, j0, depth0, alpha0);
                 const bool ok1 = evaluate(v1, j1, depth1, alpha1);
+                float4 rgba0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), rgba1 = rgba0;
+                if constexpr (kColourAhead) { rgba0 = colour_at(j0); rgba1 = colour_at(j1); }
                 if constexpr (STATS) {   // how often a lane of the warp inserts
                     const bool in0 = ok0 && depth0 < core.limit() && alpha0 >= MT::min_alpha_core;
                     stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in0) ? 1 : 0; stat_insertions += in0 ? 1 : 0;
                 }
-                if (ok0) commit(depth0, alpha0, j0);
+                if (ok0) commit(depth0, alpha0, j0, rgba0);
                 if constexpr (STATS) {
                     const bool in1 = ok1 && depth1 < core.limit() && alpha1 >= MT::min_alpha_core;
                     stat_trips += 1; stat_trips_inserting += __any_sync(0xffffffffu, in1) ? 1 : 0; stat_insertions += in1 ? 1 : 0;
                 }
-                if (ok1) commit(depth1, alpha1, j1);
+                if (ok1) commit(depth1, alpha1, j1, rgba1);
             } else {
                 // The other three modes use the same two-candidates-per-trip shape: both evaluations (divide, expf, depth) are
                 // independent instruction streams; the state updates happen in list order.  A fragment counts iff it passes

@@ -122,7 +122,7 @@ struct __align__(16) FrameStatus {      // its first four words are read with on
     unsigned int error;           // bounded waits that gave up, bad arguments seen on the device, ...
     unsigned long long candidate_pairs;     // statistics mode of the blend kernels
     unsigned long long accepted_fragments;  // statistics mode of the blend kernels
-    unsigned long long warp_trips;          // statistics mode, HYBRID_BLEND: times a warp came to the insertion, behind two or three candidates per lane (K < 4 or a wide depth range: one)
+    unsigned long long warp_trips;          // statistics mode, HYBRID_BLEND: times a warp came to the insertion, behind two or three candidates per lane (K < 8 or a wide depth range: one)
     unsigned long long warp_trips_inserting;// ... and at least one lane inserted into its K-buffer
     unsigned long long lane_insertions;     // ... and the lanes that inserted
     unsigned int range_blocks_done;         // blocks of the tile-range kernel that have finished; the last one orders the tiles

@@ -89,7 +89,6 @@ struct UnsortedCore {
 
     // The entry that falls out next; false if it is an empty one.
     __device__ __forceinline__ bool last(uint2& payload) const {
-        if (filling()) return false;
         payload = pay[(kmax & uint32_t(K - 1)) * THREADS];
         return payload.y != kNoEntry;
     }
@@ -116,9 +115,10 @@ struct UnsortedCore {
         }
     }
 
-    // One or the other.  `evicted` and `colour` of an empty entry are zero, as the caller set them in the beginning.
+    // One or the other; always the latter unless APPENDS.  `evicted` and `colour` of an empty entry are zero, as the caller set them in the beginning.
+    template <bool APPENDS>
     __device__ __forceinline__ bool insert(float depth, uint2 payload, uint2& evicted, float3& colour) {
-        if (!filling()) return replace(depth, payload, evicted, colour);
+        if (!APPENDS || !filling()) return replace(depth, payload, evicted, colour);
         append(depth, payload, colour);
         if constexpr (COLOUR) { colour = make_float3(0.0f, 0.0f, 0.0f); evicted = make_uint2(0u, kNoEntry); }
         return true;

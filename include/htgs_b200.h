@@ -85,7 +85,7 @@ typedef struct HtgsFrameInfo {
     uint64_t candidate_pairs;    /* statistics mode only: (pixel, Gaussian) pairs that passed the outline test */
     uint64_t accepted_fragments; /* statistics mode only: fragments accepted by the exact test */
     uint64_t warp_trips;           /* statistics mode, HYBRID_BLEND: times a warp came to the insertion into its K-buffers, behind two or three candidates
-                                      per lane, of which one may enter (one candidate with K < 4 and where the planes are too far apart for 32-bit keys) */
+                                      per lane, of which one may enter (one candidate with K < 8 and where the planes are too far apart for 32-bit keys) */
     uint64_t warp_trips_inserting; /* ... and at least one lane inserted */
     uint64_t lane_insertions;      /* ... and the number of lanes that inserted */
 } HtgsFrameInfo;
