@@ -59,9 +59,9 @@ template <int K> struct CoreOf<K, Buffer::keys> { using type = UnsortedCore<K, 3
 template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = UnsortedCore<K, 32, true>; };
 // HYBRID_BLEND with the unsorted buffer: candidates that a lane evaluates per trip, of which one may enter the buffer.  With K = 32 the 14 warps
 // that shared memory leaves have registers for a third one, which hides more latency than its repeated evaluations cost where lists are long and opaque: 4 M
-// Gaussians in dense clusters, 1920 x 1080, two 9.79 ms, three 9.27 (elsewhere two are up to 4 % faster: 3 M, 1297 x 840, 622 and 647 us).
-// With smaller buffers three cost 5 % at K = 4 and 8 and 7 at 16.
-constexpr int candidates_per_trip(int K) { return K >= 32 ? 3 : 2; }
+// Gaussians in dense clusters, 1920 x 1080, two 9.79 ms, three 9.27 (elsewhere two are up to 4 % faster: 3 M, 1297 x 840, 622 and 647 us).  A training forward,
+// which writes what lies in the buffer, is faster with two (step at 1 M 1181 and 1261 us), and so are smaller buffers: three cost 5 % at K = 4 and 8 and 7 at 16.
+constexpr int candidates_per_trip(int K, bool train) { return K >= 32 && !train ? 3 : 2; }
 // Whether one insertion serves a trip.  With four entries in dense clusters few candidates enter, and what a trip decides costs more than the insertions (blend at 4 M as
 // above: 6.09 ms with an insertion per candidate, 6.35 with one per trip; 3 M, 1297 x 840: 346 and 342 us).  With eight, 6.93 and 6.73 ms, 401 and 383 us.
 template <typename SL> constexpr bool merges_insertions(int K) { return SL::Core::unsorted && (K >= 8 || SL::Core::keeps_colour); }
@@ -120,7 +120,7 @@ __device__ __forceinline__ bool blend_block(
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
     constexpr bool kMerged = kHybrid && merges_insertions<SL>(K);
     constexpr bool kAppends = appends_to_empty_places<SL>(K);
-    constexpr int kPerTrip = candidates_per_trip(K);
+    constexpr int kPerTrip = candidates_per_trip(K, TRAIN);
     constexpr uint32_t kTileX = MT::tile_w / kBlockW, kTileY = MT::tile_h / kBlockH;     // blocks per binning tile
     EvalRecord* s_record = reinterpret_cast<EvalRecord*>(smem + SL::record_off);
     uint32_t* s_queue_prim = reinterpret_cast<uint32_t*>(smem + SL::queue_prim_off);

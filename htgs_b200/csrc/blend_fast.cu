@@ -37,7 +37,9 @@ constexpr int kFastQueue = 64;       // survivors of the filter that wait for a 
 // 1880: 1745, 1748, 1740, 1726, 1733): lanes that walk their own records read each one's rows again, all together they also evaluate where it does not reach.
 constexpr int kFastDense = 20;
 
-constexpr int kFastPerTrip = 3;      // HYBRID: candidates that a lane evaluates per trip
+// HYBRID: candidates that a lane evaluates per trip.  3 M Gaussians, 1297 x 840, and 4 M in dense clusters, 1920 x 1080, two and three: K = 4 221 and 221 us, 3.79 and 3.80 ms;
+// K = 8 250 and 252, 4.13 and 4.15; K = 16 317 and 301, 5.03 and 4.70 (four: 307, 4.71); K = 32 455 and 481, 6.61 and 6.89.
+constexpr int fast_candidates_per_trip(int K) { return K >= 32 ? 2 : 3; }
 
 template <int MODE, int K> struct FastSmem {
     static constexpr bool has_kbuffer = MODE != HTGS_MODE_OIT_BLEND;
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
             // goes back into the window (3 M Gaussians, 1297 x 840, K = 16: an insertion per candidate 623 us; candidates per trip two 617, three
             // 580, four 595; K = 32 at 1 M: 576, -, 537, 540).  A shorter insertion into empty places, as there, does not pay here (582).
             if constexpr (kHybrid) {
+                constexpr int kFastPerTrip = fast_candidates_per_trip(K);
                 while (__any_sync(0xffffffffu, window >= 0x10000u)) {
                     const uint32_t before = window;
                     uint32_t bit[kFastPerTrip];
