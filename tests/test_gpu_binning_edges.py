@@ -124,3 +124,26 @@ def test_global_ordering_keys_are_written_while_the_memory_is_the_frames(oracle_
         _native.check(lib.htgs_get_intermediates(ctx, ctypes.byref(inter)))
         torch.cuda.synchronize()
         assert address <= inter.keys_sorted < address + size and bool((other == 0x7f).all())
+
+
+@pytest.mark.parametrize("far", [100.0, 3e38])
+@pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1])
+def test_global_ordering_digits(oracle_lib, n, far):
+    # on either side of the number of Gaussians from which the sort by depth takes more and shorter digits, with windows of 27 and 31 bits
+    import torch
+    from htgs_b200.torch_bindings import _C
+    tb = harness.ours()
+    scene = scenes.tiny_scene(n=n, size=512, seed=n, mode=2, K=1, sh_degree=0)
+    scene.scales[:] *= 0.1
+    half = n // 2
+    for a in (scene.positions, scene.scales, scene.rotations):
+        a[half:2 * half] = a[:half]
+    view = scenes.make_view(np.eye(4), 512, 512, 512.0, 512.0, 256.0, 256.0, 0.2, far)
+    tb.rasterize(*harness.scene_tensors(scene), harness.settings_for(tb, scene, view, 2, 1), True, False)
+    torch.cuda.synchronize()
+    info = _C.last_frame_info
+    inter = harness.our_intermediates(0, n, info.n_instances)
+    ob = oracle_lib.bin_instances(inter["n_touched"], inter["bounds"].astype(np.uint32), inter["grid_w"], inter["n_tiles"], inter["eval"][:, 3, 3])
+    assert info.n_instances > n          # so that the buffers do not bound the number of visible Gaussians
+    assert np.array_equal(ob["sorted_prims"], inter["prims_sorted"]) and np.array_equal(ob["ranges"], inter["ranges"])
+    assert np.array_equal(ob["sorted_keys"], inter["keys_sorted"])
