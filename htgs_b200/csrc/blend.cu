@@ -31,7 +31,7 @@
 //
 // Blocks start in the order of `tile_order`, long lists first: the last blocks of a launch are short ones.
 //
-// What bounds it: instruction issue (74 % of the issue slots at 1.5 M Gaussians, 1297 x 840, K = 16; a fifth of the instructions are
+// What bounds it: instruction issue (77 % of the issue slots at 1 M Gaussians, 1297 x 840, K = 16; a fifth of the instructions are
 // insertions, a quarter filter, window and compositing), at the 22 warps per SM that the K-buffers leave (K = 32: 14).  3 M
 // Gaussians, 1297 x 840, K = 16: 788 us; 8 M, 4K, K = 32: 27.8 ms.
 #include <algorithm>

@@ -355,7 +355,7 @@ __device__ __forceinline__ bool denominator_in_range(const float4& t1, const flo
 // costs the L1 a look-up per lane, for 45 coefficients, 16 floats of the rows, position and opacity.  So each lane fetches its
 // inputs with two bulk copies, the record (in which the cull pass left position and opacity too) and the 16-byte aligned window around
 // its row of coefficients, and reads them from shared memory; strides of 80 and, at degree 3, 208 bytes spread the lanes over the
-// banks.  What bounds it now is DRAM (53 % of its throughput at 600 bytes in 64-byte pieces per Gaussian) and the latency of the float64 chains.
+// banks.  What bounds it now is DRAM (40 to 47 % of its throughput at 600 bytes in 64-byte pieces per Gaussian) and the latency of the float64 chains.
 // Where no coefficients are wanted (degree 0, importance weights) a lane loads its record itself: the copies' round trip through the mbarrier costs more than
 // five loads (16 k Gaussians: 5.5 us, by copies 6.4; 1 M 8.2 and 8.7, importance weights 7.6 and 8.2; 3 M 20.1 and 20.3).
 // Loads by lane -> copies, 3 M Gaussians, 1297 x 840: 88 -> 73 us, training 107 -> 88, relaxed precision 94 -> 79, 1.5 M in GLOBAL_ORDERING 82 -> 65.
@@ -370,6 +370,8 @@ inline FinishLayout finish_layout(int active_sh_bases, bool colour) {
     const uint32_t bytes = (12u * uint32_t(active_sh_bases - 1) + 12u + 15u) & ~15u;      // a row starts up to 12 bytes behind a 16-byte boundary
     return {bytes, (bytes / 16u) % 2u ? bytes : bytes + 16u};                             // an odd number of 16-byte words
 }
+// Relaxed precision: five blocks spill 28 bytes, four none; both passes of the preprocess at four, five and six blocks: 1 M Gaussians 36.6, 37.6 and 39.5 us, 3 M 93, 92 and
+// 95, 8 M 224, 227 and 233, 4 M in dense clusters, 1920 x 1080, 274, 279 and 288 (loads by lane, without a bound: 39, 100, 247, 314).
 constexpr int finish_blocks_per_sm(bool train, bool fast) { return train || fast ? 5 : 6; }
 template <int MODE, bool TRAIN, bool FAST>
 __global__ void __launch_bounds__(kFinishBlock, finish_blocks_per_sm(TRAIN, FAST)) preprocess_finish_kernel(
