@@ -38,8 +38,10 @@ constexpr int kFastQueue = 64;       // survivors of the filter that wait for a 
 constexpr int kFastDense = 20;
 
 // HYBRID: candidates that a lane evaluates per trip.  3 M Gaussians, 1297 x 840, and 4 M in dense clusters, 1920 x 1080, two and three: K = 4 221 and 221 us, 3.79 and 3.80 ms;
-// K = 8 250 and 252, 4.13 and 4.15; K = 16 317 and 301, 5.03 and 4.70 (four: 307, 4.71); K = 32 455 and 481, 6.61 and 6.89.
-constexpr int fast_candidates_per_trip(int K) { return K >= 32 ? 2 : 3; }
+// K = 8 250 and 252, 4.13 and 4.15; K = 16 317 and 301, 5.03 and 4.70 (four: 307, 4.71); K = 32 455 and 481, 6.61 and 6.89.  K = 32 stays with three all the same: how far a lane
+// is ahead decides between entries whose keys agree but for the depth bits that the position takes, so with two some pixels differ by up to 1e-3, also under
+// htgs_set_fast_deterministic.
+constexpr int kFastPerTrip = 3;
 
 template <int MODE, int K> struct FastSmem {
     static constexpr bool has_kbuffer = MODE != HTGS_MODE_OIT_BLEND;
@@ -327,7 +329,6 @@ __global__ void __launch_bounds__(kFastThreads) blend_fast_kernel(
             // goes back into the window (3 M Gaussians, 1297 x 840, K = 16: an insertion per candidate 623 us; candidates per trip two 617, three
             // 580, four 595; K = 32 at 1 M: 576, -, 537, 540).  A shorter insertion into empty places, as there, does not pay here (582).
             if constexpr (kHybrid) {
-                constexpr int kFastPerTrip = fast_candidates_per_trip(K);
                 while (__any_sync(0xffffffffu, window >= 0x10000u)) {
                     const uint32_t before = window;
                     uint32_t bit[kFastPerTrip];
