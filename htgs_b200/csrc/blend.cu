@@ -62,9 +62,10 @@ template <int K> struct CoreOf<K, Buffer::keys_and_colours> { using type = Unsor
 // Gaussians in dense clusters, 1920 x 1080, two 9.79 ms, three 9.27 (elsewhere two are up to 4 % faster: 3 M, 1297 x 840, 622 and 647 us).  A training forward,
 // which writes what lies in the buffer, is faster with two (step at 1 M 1181 and 1261 us), and so are smaller buffers: three cost 5 % at K = 4 and 8 and 7 at 16.
 constexpr int candidates_per_trip(int K, bool train) { return K >= 32 && !train ? 3 : 2; }
-// Whether one insertion serves a trip.  With four entries in dense clusters few candidates enter, and what a trip decides costs more than the insertions (blend at 4 M as
-// above: 6.09 ms with an insertion per candidate, 6.35 with one per trip; 3 M, 1297 x 840: 346 and 342 us).  With eight, 6.93 and 6.73 ms, 401 and 383 us.
-template <typename SL> constexpr bool merges_insertions(int K) { return SL::Core::unsorted && (K >= 8 || SL::Core::keeps_colour); }
+// Whether one insertion serves a trip.  With four entries in long lists, of which few candidates enter, what a trip decides costs more than the insertions (blend at 4 M as
+// above: 6.09 ms with an insertion per candidate, 6.35 with one per trip; 3 M, 1297 x 840: 346 and 342 us).  A training step is faster with one per trip there too (400 k, 980 x
+// 545: 626 and 615 us).  With eight entries, 6.93 and 6.73 ms, 401 and 383 us.
+template <typename SL> constexpr bool merges_insertions(int K, bool train) { return SL::Core::unsorted && (K >= 8 || train || SL::Core::keeps_colour); }
 // Whether entries are appended while there are empty places: its branch costs smaller buffers more than the shorter insertion saves (K = 8, as above: 6.82 ms and
 // 387 us with it, 6.73 and 383 without; K = 16: 7.25 and 414 with it, 7.28 and 424 without), but not where a grid is resident at once (256 x 256: 166 and 170 us).
 template <typename SL> constexpr bool appends_to_empty_places(int K) { return K >= 16 || SL::Core::keeps_colour; }
@@ -118,7 +119,7 @@ __device__ __forceinline__ bool blend_block(
     constexpr bool kHybrid = MODE == HTGS_MODE_HYBRID_BLEND;
     constexpr bool kFirstK = MODE == HTGS_MODE_ALPHA_BLEND_FIRST_K;
     constexpr bool kGlobal = MODE == HTGS_MODE_ALPHA_BLEND_GLOBAL_ORDERING;
-    constexpr bool kMerged = kHybrid && merges_insertions<SL>(K);
+    constexpr bool kMerged = kHybrid && merges_insertions<SL>(K, TRAIN);
     constexpr bool kAppends = appends_to_empty_places<SL>(K);
     constexpr int kPerTrip = candidates_per_trip(K, TRAIN);
     constexpr uint32_t kTileX = MT::tile_w / kBlockW, kTileY = MT::tile_h / kBlockH;     // blocks per binning tile
@@ -310,8 +311,8 @@ __device__ __forceinline__ bool blend_block(
                 }
             } else if constexpr (kHybrid) {
                 // Two candidates per trip, as above; the buffer and tail updates happen strictly in list order.  The colour is loaded ahead where registers
-                // allow (K = 4, frames: 6.17 -> 6.09 ms in dense clusters; K = 2, whose chain is in registers, 303 -> 313 us, training at K = 4 1 % slower).
-                constexpr bool kColourAhead = SL::Core::unsorted && !TRAIN;
+                // allow (K = 4: 6.17 -> 6.09 ms in dense clusters; K = 2, whose chain is in registers, 303 -> 313 us).
+                constexpr bool kColourAhead = SL::Core::unsorted;
                 auto colour_at = [&](uint32_t j) { return reinterpret_cast<const float4*>(s_record + j)[4]; };
                 auto commit = [&](float depth, float alpha, uint32_t j, float4 rgba) {
                     if constexpr (!kColourAhead) rgba = colour_at(j);
@@ -743,7 +744,10 @@ cudaError_t launch_k(const BlendLaunch& l, BlendTask task, const HtgsView& view)
         if constexpr (MODE == HTGS_MODE_HYBRID_BLEND) {
             constexpr size_t smem = SmemLayout<MODE, K, Buffer::keys_and_colours, BlendTask::image>::total;
             constexpr int per_sm = int((227 * 1024) / (smem + 1024)) < 32 ? int((227 * 1024) / (smem + 1024)) : 32;
-            if (task == BlendTask::image && l.geo.n_tiles * 2 <= per_sm * sm_count_of_current_device())
+            // With four entries the colours cost little shared memory, and one insertion per trip pays until lists are long: up to four times the resident grid
+            // (blend with the colours and without: 500 x 400, 60 k 53 and 64 us; 800 x 600, 200 k 104 and 113; 980 x 545, 400 k 167 and 180; 1297 x 840, 400 k 147 and 141).
+            constexpr int grids = K == 4 ? 4 : 1;
+            if (task == BlendTask::image && l.geo.n_tiles * 2 <= grids * per_sm * sm_count_of_current_device())
                 return launch_task<MODE, K, Buffer::keys_and_colours, BlendTask::image>(l, window.base);
         }
         return launch_buffer<MODE, K, Buffer::keys>(l, task, window.base);

@@ -149,3 +149,19 @@ def test_statistics_of_a_buffer_that_every_candidate_enters(K, far):
         lib.htgs_set_collect_stats(ctx, 0)
     assert image.min() > 0.0 and info.accepted_fragments == info.lane_insertions == K * 64 * 64
     assert info.warp_trips == info.warp_trips_inserting == K * 64 * 64 // 32
+
+
+@pytest.mark.parametrize("width,height", [(752, 776), (752, 784), (1000, 1000)])
+@pytest.mark.parametrize("n", [3, 4, 5, 9, 6000])
+def test_four_entries_with_and_without_colours(n, width, height):
+    # on either side of the number of tiles from which a buffer of four entries does without colours and inserts per candidate (148 multiprocessors of 31 blocks)
+    scene, view = scene_with_ties(n, width, height, 4, 0)
+    if n < 10:      # Gaussians that every pixel near the centre sees, one short of a full buffer to more than fit
+        scene.positions[:, :2] = 0.0
+        scene.scales[:] = 0.5
+        scene.opacities[:] = 0.4
+    for median in (False, True):
+        got = render(scene, view, 0, 4, 0.2, 100.0, median)
+        want = render(scene, view, 0, 4, 0.2, 3e38, median)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        assert got[0].max() > 0.0
